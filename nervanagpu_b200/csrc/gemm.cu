@@ -3,9 +3,10 @@
 // Mirrors NervanaGPU.dot / batched_dot (nervanagpu/nervanagpu.py:820-1105) and the C interface
 // nervana_hgemm (nervanagpu/kernels/C_interface/nervana_c_api.h:31-128).
 //
-// Shapes whose operands TMA can address (16-byte aligned base, leading dimensions that are
-// multiples of 8 elements) run on the tcgen05 engine; anything else runs on a plain SIMT
-// kernel so that every legal call of the reference API still executes on the GPU.
+// Everything runs on the tcgen05 engine. Operands that TMA cannot address (base not 16-byte
+// aligned, leading dimension or batch stride no multiple of 8 elements) are first copied into
+// rows that it can (pack_rows_kernel). The plain CUDA-core kernel serves ng_hgemm_simt, the
+// second opinion of the tests.
 #include <algorithm>
 
 #include "../../include/nervana_b200.h"
@@ -109,13 +110,66 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(SimtGemmArgs g) {
   }
 }
 
-bool tma_ok(const void* p, long long ld) {
-  return (reinterpret_cast<uintptr_t>(p) & 15u) == 0 && (ld & 7) == 0;
+// ------------------------------------------------------------------------------------------
+// Copy of an operand with rows at odd addresses into rows of a multiple of 8 elements.
+// ------------------------------------------------------------------------------------------
+struct PackArgs {
+  const __half* src;
+  uint4* dst;
+  long long ld, zstride;    // of src, in elements
+  uint32_t rows, cols8, cols, total;   // rows per batch entry; 16-byte groups per row; elements per row; groups in all
+};
+
+// Each thread moves 8 elements. Their 16 bytes start at any even address: two aligned 16-byte
+// loads (the second is the neighbour's first, an L1 hit, and is left out where nothing of it is
+// needed, so that no load leaves the 16-byte granules that hold the operand) and a byte shift.
+__device__ __forceinline__ void pack_group(const PackArgs& a, uint32_t i) {
+  const uint32_t r = i / a.cols8, g = i - r * a.cols8;
+  const uint32_t z = r / a.rows;
+  const __half* s = a.src + z * a.zstride + static_cast<long long>(r - z * a.rows) * a.ld + g * 8;
+  const uint32_t sh = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(s)) & 15u;
+  const uint4* q = reinterpret_cast<const uint4*>(reinterpret_cast<uintptr_t>(s) & ~uintptr_t(15));
+  const uint32_t need = min(8u, a.cols - g * 8) * 2u;     // bytes that exist
+  const uint4 lo = __ldg(q);
+  uint4 hi = make_uint4(0u, 0u, 0u, 0u);
+  if (sh + need > 16u) hi = __ldg(q + 1);
+  uint32_t w0 = lo.x, w1 = lo.y, w2 = lo.z, w3 = lo.w, w4 = hi.x, w5 = hi.y, w6 = hi.z, w7 = hi.w;
+  if (sh & 8u) { w0 = w2; w1 = w3; w2 = w4; w3 = w5; w4 = w6; w5 = w7; }
+  if (sh & 4u) { w0 = w1; w1 = w2; w2 = w3; w3 = w4; w4 = w5; }
+  const uint32_t bits = (sh & 2u) * 8u;
+  a.dst[i] = make_uint4(__funnelshift_r(w0, w1, bits), __funnelshift_r(w1, w2, bits), __funnelshift_r(w2, w3, bits),
+                        __funnelshift_r(w3, w4, bits));
+}
+
+// Both operands in one launch, the groups of the second behind those of the first. Bound by the
+// memory traffic (the copies stay in L2 for the product that follows).
+__global__ void __launch_bounds__(256) pack_rows_kernel(PackArgs a, PackArgs b) {
+  grid_dependency_wait();
+  grid_launch_dependents();   // the product sets itself up meanwhile and waits for the copies
+  const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+  if (i < a.total) pack_group(a, i);
+  else if (i - a.total < b.total) pack_group(b, i - a.total);
+}
+
+// Fills `a` for an operand of `nz` entries of rows x cols elements; false when it is too large.
+bool plan_pack(PackArgs& a, const void* src, long long ld, long long zstride, long long nz, long long rows, long long cols) {
+  a.src = static_cast<const __half*>(src);
+  a.ld = ld; a.zstride = zstride;
+  const long long c8 = (cols + 7) / 8, total = nz * rows * c8;
+  if (total > 0x3fffffffll) return false;
+  a.rows = static_cast<uint32_t>(rows); a.cols = static_cast<uint32_t>(cols);
+  a.cols8 = static_cast<uint32_t>(c8); a.total = static_cast<uint32_t>(total);
+  return true;
+}
+
+bool tma_ok(const void* p, long long ld, long long zstride) {
+  return (reinterpret_cast<uintptr_t>(p) & 15u) == 0 && (ld & 7) == 0 && (zstride & 7) == 0;
 }
 
 }  // namespace
 
-int run_gemm(const GemmCall& g, cudaStream_t stream) {
+int run_gemm(const GemmCall& call, cudaStream_t stream) {
+  GemmCall g = call;
   if (!g.A || !g.B || !g.C) return fail(NG_ERR_INVALID_ARG, "null operand");
   if (g.m <= 0 || g.n <= 0 || g.k <= 0) return fail(NG_ERR_INVALID_ARG, "m, n, k must be positive");
   if (g.a_t && g.b_t) return fail(NG_ERR_UNSUPPORTED, "op 'tt' is not supported");
@@ -130,8 +184,16 @@ int run_gemm(const GemmCall& g, cudaStream_t stream) {
   ea.seed_lo = static_cast<uint32_t>(g.seed); ea.seed_hi = static_cast<uint32_t>(g.seed >> 32);
   ea.rng_offset = g.rng_offset;
 
-  const bool batched_ok = g.loops == 1 && (g.az % 8 == 0) && (g.bz % 8 == 0);
-  const bool use_tc = !g.force_simt && tma_ok(g.A, g.lda) && tma_ok(g.B, g.ldb) && batched_ok;
+  // one batch dimension per operand: independent products, or products summed into one output
+  const bool sum = g.loops > 1;
+  const long long zsa = sum ? g.alz : g.az, zsb = sum ? g.blz : g.bz;
+  const int nza = zsa == 0 ? 1 : (sum ? g.loops : g.batch), nzb = zsb == 0 ? 1 : (sum ? g.loops : g.batch);
+  PackArgs packA = {}, packB = {};
+  bool use_tc = !g.force_simt && !(sum && g.batch > 1);
+  if (use_tc && !tma_ok(g.A, g.lda, zsa))
+    use_tc = plan_pack(packA, g.A, g.lda, zsa, nza, g.a_t ? g.k : g.m, g.a_t ? g.m : g.k);
+  if (use_tc && !tma_ok(g.B, g.ldb, zsb))
+    use_tc = plan_pack(packB, g.B, g.ldb, zsb, nzb, g.b_t ? g.n : g.k, g.b_t ? g.k : g.n);
   if (!use_tc) {
     SimtGemmArgs s;
     s.A = static_cast<const __half*>(g.A); s.B = static_cast<const __half*>(g.B); s.C = g.C;
@@ -152,7 +214,9 @@ int run_gemm(const GemmCall& g, cudaStream_t stream) {
   p.M = g.m; p.N = g.n;
   p.tiles_n = (g.n + p.block_n - 1) / p.block_n;
   p.nz = g.batch;
-  p.num_kb = (g.k + kChunk - 1) / kChunk;
+  p.red_chunks = (g.k + kChunk - 1) / kChunk;
+  if (static_cast<long long>(p.red_chunks) * g.loops > 0x7fffffffll) return fail(NG_ERR_TOO_LARGE, "reduction too long");
+  p.num_kb = p.red_chunks * g.loops;
   tc_pick_tile_rows(c, p, static_cast<long long>(p.tiles_n) * p.nz, p.num_kb);
   // Two or more row tiles and 128 or 256 columns: CTA pairs (a 256-row tile over two SMs, each of
   // which loads half of the B columns).
@@ -172,7 +236,8 @@ int run_gemm(const GemmCall& g, cudaStream_t stream) {
   lay.a_merge = !merge_off && g.a_t && g.m % kChunk == 0;
   lay.b_merge_static = !merge_off && !g.b_t && g.n % kChunk == 0 && bn_cta >= 2 * kChunk;
   tc_fill_mma(p, lay);
-  p.a_zmul = g.az != 0; p.b_zmul = g.bz != 0;
+  p.a_zmul = !sum && nza > 1; p.b_zmul = !sum && nzb > 1;
+  p.a_lmul = sum && nza > 1; p.b_lmul = sum && nzb > 1;
   p.C = g.C; p.Cold = g.beta != 0.0f ? g.C : nullptr;
   p.ldc = g.ldc; p.c_zstride = g.cz;
   p.alpha = g.alpha; p.beta = g.beta; p.relu = g.relu; p.sr_bits = g.sr_bits; p.out_f32 = g.out_f32;
@@ -182,6 +247,40 @@ int run_gemm(const GemmCall& g, cudaStream_t stream) {
   p.seed_lo = ea.seed_lo; p.seed_hi = ea.seed_hi; p.rng_offset = g.rng_offset;
   p.splits = choose_splits(c, static_cast<long long>(p.tiles_m) * p.tiles_n * p.nz, p.num_kb,
                            static_cast<long long>(g.m) * g.n * g.batch);
+  if (p.splits > 1 && (g.n & 7)) {
+    // partials with whole 16-byte groups per row: they leave through the staged output stage, and
+    // the second stage stores the columns that exist
+    p.n_store = g.n;
+    p.N = (g.n + 7) & ~7;
+  }
+  if (packA.total || packB.total) {
+    size_t off = p.splits > 1 ? static_cast<size_t>(p.splits) * p.nz * p.M * p.N * sizeof(float) : 0;
+    off = (off + 255) & ~size_t(255);
+    const size_t bytesA = (static_cast<size_t>(packA.total) * 16 + 255) & ~size_t(255);
+    int rc = ensure_workspace(c, stream, off + bytesA + static_cast<size_t>(packB.total) * 16);
+    if (rc != NG_OK) return rc;
+    uint8_t* room = reinterpret_cast<uint8_t*>(c->ws) + off;
+    if (packA.total) {
+      packA.dst = reinterpret_cast<uint4*>(room);
+      g.A = room; g.lda = packA.cols8 * 8ll; g.az = g.alz = nza > 1 ? g.lda * packA.rows : 0;
+    }
+    if (packB.total) {
+      packB.dst = reinterpret_cast<uint4*>(room + bytesA);
+      g.B = room + bytesA; g.ldb = packB.cols8 * 8ll; g.bz = g.blz = nzb > 1 ? g.ldb * packB.rows : 0;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((packA.total + packB.total + 255u) / 256u);
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = tuning().dependent_launch != 0 ? 1 : 0;
+    NG_CUDA(cudaLaunchKernelEx(&cfg, pack_rows_kernel, packA, packB));
+    NG_CHECK_LAUNCH();
+  }
+  const uint64_t zbytesA = static_cast<uint64_t>(sum ? g.alz : g.az) * 2, zbytesB = static_cast<uint64_t>(sum ? g.blz : g.bz) * 2;
 
   // Tensor maps. Dimension 0 is the contiguous one; dimension 2 walks the batch.
   CUtensorMap mapA, mapB;
@@ -191,15 +290,15 @@ int run_gemm(const GemmCall& g, cudaStream_t stream) {
     uint32_t box[5] = {kChunk, 1, 1, 1, 1};
     if (g.a_t) { dims[0] = g.m; dims[1] = g.k; box[1] = kChunk; }
     else       { dims[0] = g.k; dims[1] = g.m; box[1] = kTileM * p.m_halves; }
-    dims[2] = g.az != 0 ? g.batch : 1;
+    dims[2] = nza;
     str[0] = static_cast<uint64_t>(g.lda) * 2;
-    str[1] = g.az != 0 ? static_cast<uint64_t>(g.az) * 2 : str[0] * dims[1];
+    str[1] = nza > 1 ? zbytesA : str[0] * dims[1];
     str[2] = str[1] * dims[2];
     str[3] = str[2];
     if (lay.a_merge) {   // (m_lo, k, m_hi, batch)
-      dims[0] = kChunk; dims[1] = g.k; dims[2] = g.m / kChunk; dims[3] = g.az != 0 ? g.batch : 1;
+      dims[0] = kChunk; dims[1] = g.k; dims[2] = g.m / kChunk; dims[3] = nza;
       str[0] = static_cast<uint64_t>(g.lda) * 2; str[1] = 128;
-      str[2] = g.az != 0 ? static_cast<uint64_t>(g.az) * 2 : str[0] * dims[1];
+      str[2] = nza > 1 ? zbytesA : str[0] * dims[1];
       str[3] = str[2] * dims[3];
       box[1] = kChunk; box[2] = 2;
     }
@@ -212,15 +311,15 @@ int run_gemm(const GemmCall& g, cudaStream_t stream) {
     uint32_t box[5] = {kChunk, 1, 1, 1, 1};
     if (g.b_t) { dims[0] = g.k; dims[1] = g.n; box[1] = bn_cta; }
     else       { dims[0] = g.n; dims[1] = g.k; box[1] = kChunk; }
-    dims[2] = g.bz != 0 ? g.batch : 1;
+    dims[2] = nzb;
     str[0] = static_cast<uint64_t>(g.ldb) * 2;
-    str[1] = g.bz != 0 ? static_cast<uint64_t>(g.bz) * 2 : str[0] * dims[1];
+    str[1] = nzb > 1 ? zbytesB : str[0] * dims[1];
     str[2] = str[1] * dims[2];
     str[3] = str[2];
     if (lay.b_merge_static) {   // (n_lo, k, n_hi, batch)
-      dims[0] = kChunk; dims[1] = g.k; dims[2] = g.n / kChunk; dims[3] = g.bz != 0 ? g.batch : 1;
+      dims[0] = kChunk; dims[1] = g.k; dims[2] = g.n / kChunk; dims[3] = nzb;
       str[0] = static_cast<uint64_t>(g.ldb) * 2; str[1] = 128;
-      str[2] = g.bz != 0 ? static_cast<uint64_t>(g.bz) * 2 : str[0] * dims[1];
+      str[2] = nzb > 1 ? zbytesB : str[0] * dims[1];
       str[3] = str[2] * dims[3];
       box[1] = kChunk; box[2] = bn_cta / kChunk;
     }

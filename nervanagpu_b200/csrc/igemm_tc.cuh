@@ -46,7 +46,8 @@ struct TcParams {
                        // [z * taps_per_z, (z + 1) * taps_per_z), at most acc_groups * acc_taps of them
   int nz_out;          // number of output slices (= nz unless taps are grouped or stacked, then
                        // nz = ceil(nz_out / (acc_groups * acc_taps)))
-  int M, N;            // logical output extent (rows, cols)
+  int M, N;            // logical output extent (rows, cols); split products: N is the pitch of the partials
+  int n_store;         // columns that exist in the output (0 = N; differs for ragged split products only)
 
   // ---- MMA descriptors (host-built)
   uint32_t idesc;
@@ -76,9 +77,10 @@ struct TcParams {
                                    //   3 GEMM, map (n_lo, k, n_hi, batch), every tile
                                    //   4 tap blocks, N = 128: a box per pixel, map (n_lo, x, y, chan, n_hi)
   int kb_rows;                     // reduction rows per k-block (64, or 16..64 for small C in fprop)
-  int a_zmul, b_zmul;              // batched GEMM: coordinate in dim 2 = z * zmul
+  int a_zmul, b_zmul;              // batched GEMM: batch coordinate = z * zmul + loop * lmul, where the
+  int a_lmul, b_lmul;              // k-blocks walk `red_chunks` blocks of every summed product in turn
+  int red_chunks;                  // fprop: ceil(C/kb_rows); bprop: ceil(K/64); GEMM: ceil(k/64)
   // conv geometry (unused by TC_GEMM)
-  int red_chunks;                  // fprop: ceil(C/kb_rows); bprop: ceil(K/64)
   int RS, S, R;                    // filter taps (tap blocks when tap_w/tap_h > 1)
   int tap_w, tap_h;                // input pixels per tap step: 1, or the tap-block size of the
                                    // few-channel modes where one box carries a block of taps

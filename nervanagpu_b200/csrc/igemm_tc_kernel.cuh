@@ -71,7 +71,7 @@ __device__ __forceinline__ Tap decode_tap(const TcParams& p, int trs) {
 struct Walk {
   ChunkPos cp;
   Tap tap;
-  int trs, rc, kb;
+  int trs, rc;
 };
 
 // Exact division for the strided gather of the backward pass: returns false when `num` is not
@@ -242,9 +242,11 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
       wk.cp = {0, 0, 0, 0, true};   // fprop/bprop: pixel chunk of this B box; update: walks
       wk.tap = {0, 0, 0};           // fprop/bprop: walks the filter taps; update: fixed (z)
       wk.trs = 0; wk.rc = 0;        // tap number and reduction-chunk number inside the tap
-      wk.kb = it.kb0;
       bool tap_live = true;         // update: this A box's tap exists (last group may be short)
-      if (kMode == TC_FPROP || kMode == TC_BPROP) {
+      if (kMode == TC_GEMM) {   // trs counts the products that are summed into one output
+        wk.trs = fast_div(it.kb0, p.fd_red);
+        wk.rc = it.kb0 - wk.trs * p.red_chunks;
+      } else if (kMode == TC_FPROP || kMode == TC_BPROP) {
         // (b_merge 4: a box carries the two chunks of one pixel)
         if (!is_a) wk.cp = decode_chunk(p, n0 / kChunk + (p.b_merge == 4 ? 2 * bi : bi));
         if (p.b_merge == 1 || p.b_merge == 2) {
@@ -276,19 +278,20 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
       auto coords = [&](const Walk& s, int& c0, int& c1, int& c2, int& c3, int& c4) {
         const ChunkPos& cp = s.cp;
         const Tap& tap = s.tap;
-        const int trs = s.trs, rc = s.rc, kb = s.kb;
+        const int trs = s.trs, rc = s.rc;
         c0 = c1 = c2 = c3 = c4 = 0;
         {
           if (kMode == TC_GEMM) {
-            const int k0 = kb * kChunk;
+            const int k0 = rc * kChunk;
+            const int za = it.z * p.a_zmul + trs * p.a_lmul, zb = it.z * p.b_zmul + trs * p.b_lmul;
             if (is_a) {
-              if (p.a_merge) { c1 = k0; c2 = (m0 + kTileM * bi) / kChunk; c3 = it.z * p.a_zmul; }
-              else if (p.a_mn_major) { c0 = m0 + kChunk * bi; c1 = k0; c2 = it.z * p.a_zmul; }
-              else { c0 = k0; c1 = m0; c2 = it.z * p.a_zmul; }
+              if (p.a_merge) { c1 = k0; c2 = (m0 + kTileM * bi) / kChunk; c3 = za; }
+              else if (p.a_mn_major) { c0 = m0 + kChunk * bi; c1 = k0; c2 = za; }
+              else { c0 = k0; c1 = m0; c2 = za; }
             } else {
-              if (p.b_merge == 3) { c1 = k0; c2 = n0 / kChunk; c3 = it.z * p.b_zmul; }
-              else if (p.b_mn_major) { c0 = n0 + kChunk * bi; c1 = k0; c2 = it.z * p.b_zmul; }
-              else { c0 = k0; c1 = n0; c2 = it.z * p.b_zmul; }
+              if (p.b_merge == 3) { c1 = k0; c2 = n0 / kChunk; c3 = zb; }
+              else if (p.b_mn_major) { c0 = n0 + kChunk * bi; c1 = k0; c2 = zb; }
+              else { c0 = k0; c1 = n0; c2 = zb; }
             }
           } else if (kMode == TC_FPROP) {
             if (is_a) {  // filter rows c of tap trs, 64 output channels wide
@@ -342,8 +345,9 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
       };
       // step a walker to the next k-block
       auto advance = [&](Walk& s) {
-        ++s.kb;
-        if (kMode == TC_FPROP || kMode == TC_BPROP) {
+        if (kMode == TC_GEMM) {
+          if (++s.rc == p.red_chunks) { s.rc = 0; ++s.trs; }
+        } else if (kMode == TC_FPROP || kMode == TC_BPROP) {
           if (++s.rc == p.red_chunks) {
             s.rc = 0;
             ++s.trs;
@@ -862,12 +866,13 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
 // lanes matter when there are many partitions of a small output: one thread walking 70 slices
 // one after the other is a chain of 70 dependent memory latencies.
 // ------------------------------------------------------------------------------------------
-__global__ void splitk_reduce_kernel(const float* __restrict__ ws, int splits, int lanes, int nz, int M, int N,
+// The partials have rows of N columns, of which the first n_out exist in the output.
+__global__ void splitk_reduce_kernel(const float* __restrict__ ws, int splits, int lanes, int nz, int M, int N, int n_out,
                                      void* C, const void* Cold, long long ldc, long long c_zstride, int out_f32,
                                      int vec_ok, EpiArgs ea, int c_row_chunks, int c_row_len) {
   grid_dependency_wait();     // (launched while the product that writes the partials drains)
   grid_launch_dependents();
-  const int groups_per_row = (N + 7) / 8;
+  const int groups_per_row = (n_out + 7) / 8;
   const long long total = static_cast<long long>(nz) * M * groups_per_row;
   const long long slice = static_cast<long long>(nz) * M * N;
   const long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
@@ -880,13 +885,13 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, int splits, i
   const int row = static_cast<int>(zr % M);
   const int z = static_cast<int>(zr / M);
   const int col = g * 8;
-  const int nvalid = min(8, N - col);
+  const int nvalid = min(8, n_out - col);
   float v[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) v[j] = 0.0f;
   const float* src = ws + zr * N + col + sub * slice;
   const long long step = slice * lanes;
-  const bool v4 = (N & 3) == 0 && nvalid == 8;
+  const bool v4 = (N & 3) == 0 && col + 8 <= N;
   if (live) {
     if (v4) {
       int s = sub;
@@ -934,7 +939,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, int splits, i
   const int esz = out_f32 ? 4 : 2;
   uint8_t* crow = static_cast<uint8_t*>(C) + off * esz;
   const uint8_t* oldrow = Cold ? static_cast<const uint8_t*>(Cold) + off * esz : nullptr;
-  const unsigned long long lin = (static_cast<unsigned long long>(z) * M + row) * static_cast<unsigned long long>(N) + col;
+  const unsigned long long lin = (static_cast<unsigned long long>(z) * M + row) * static_cast<unsigned long long>(n_out) + col;
   if (out_f32)
     epi_store8<true>(ea, v, crow, oldrow, gcol, lin, nvalid, vec_ok != 0);
   else

@@ -411,7 +411,8 @@ int tc_launch(DeviceCtx* c, const CUtensorMap& mapA, const CUtensorMap& mapB, Tc
     EpiArgs ea;
     ea.alpha = p.alpha; ea.beta = p.beta; ea.relu = p.relu; ea.sr_bits = p.sr_bits;
     ea.seed_lo = p.seed_lo; ea.seed_hi = p.seed_hi; ea.rng_offset = p.rng_offset;
-    const long long groups = static_cast<long long>(p.nz_out) * p.M * ((p.N + 7) / 8);
+    const int n_out = p.n_store > 0 ? p.n_store : p.N;
+    const long long groups = static_cast<long long>(p.nz_out) * p.M * ((n_out + 7) / 8);
     const int lanes = splitk_reduce_lanes(groups, p.splits, c->sm_count);
     const long long blocks = (groups * lanes + 255) / 256;
     if (blocks > 0x7fffffffll) return fail(NG_ERR_TOO_LARGE, "output too large for the split-K reduction");
@@ -425,7 +426,7 @@ int tc_launch(DeviceCtx* c, const CUtensorMap& mapA, const CUtensorMap& mapB, Tc
     cfg.attrs = attr;
     cfg.numAttrs = tuning().dependent_launch != 0 ? 1 : 0;
     NG_CUDA(cudaLaunchKernelEx(&cfg, splitk_reduce_kernel, static_cast<const float*>(p.ws), p.splits, lanes, p.nz_out,
-                               p.M, p.N, p.C, p.Cold, p.ldc, p.c_zstride, p.out_f32, p.vec_ok, ea, p.c_row_chunks,
+                               p.M, p.N, n_out, p.C, p.Cold, p.ldc, p.c_zstride, p.out_f32, p.vec_ok, ea, p.c_row_chunks,
                                p.c_row_len));
     NG_CHECK_LAUNCH();
   }
@@ -580,7 +581,7 @@ extern "C" int ng_hgemm_static_scratch(const void* A, const void* B, void* C, in
   p.nz = 1;
   p.nz_out = 1;
   p.acc_groups = 1;
-  p.num_kb = (k + kChunk - 1) / kChunk;
+  p.num_kb = p.red_chunks = (k + kChunk - 1) / kChunk;
   TcOperandLayout lay;
   lay.a_mn_major = a_t ? 1 : 0;
   lay.b_mn_major = b_t ? 0 : 1;
@@ -640,7 +641,7 @@ extern "C" int ng_hgemm_static_scratch(const void* A, const void* B, void* C, in
     const long long groups = static_cast<long long>(m) * ((n + 7) / 8);
     const int lanes = ngb::splitk_reduce_lanes(groups, p.splits, slots->sm_count);
     const int blocks = static_cast<int>((groups * lanes + 255) / 256);
-    splitk_reduce_kernel<<<blocks, 256, 0, stream>>>(p.ws, p.splits, lanes, 1, m, n, C, p.Cold, ldc, 0, 0, p.vec_ok,
+    splitk_reduce_kernel<<<blocks, 256, 0, stream>>>(p.ws, p.splits, lanes, 1, m, n, n, C, p.Cold, ldc, 0, 0, p.vec_ok,
                                                      ea, 0, 0);
     NG_CHECK_LAUNCH();
   }

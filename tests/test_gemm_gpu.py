@@ -123,6 +123,49 @@ def test_batched_dot(ng):
     assert_close(dS.get(), refs, 2.0 ** -10 * np.abs(refs) + 2e-2, "batched loops")
 
 
+@pytest.mark.parametrize("op", ["nn", "nt", "tn"])
+@pytest.mark.parametrize("mnk", [(1, 1, 1), (7, 9, 8), (127, 129, 63), (130, 250, 65), (257, 31, 1030)])
+def test_operands_at_odd_addresses(ng, op, mnk):
+    """Views whose rows start at every even address: bases one to seven elements behind a 16-byte
+    boundary and odd leading dimensions. The copies that TMA reads and the products equal the oracle."""
+    m, n, k = mnk
+    rng = np.random.default_rng(13 + m)
+    for shift in (1, 2, 5, 7):
+        A, B = _operands(rng, m, n, k, op)
+        bigA = np.full((A.shape[0], A.shape[1] + 9), np.nan, np.float16)
+        bigB = np.full((B.shape[0], B.shape[1] + 9 - shift), np.nan, np.float16)
+        bigA[:, shift:shift + A.shape[1]] = A
+        bigB[:, :B.shape[1]] = B
+        dA = ng.array(bigA)[:, shift:shift + A.shape[1]]
+        dB = ng.array(bigB)[:, :B.shape[1]]
+        C0 = rng.standard_normal((m, n)).astype(np.float16)
+        C = ng.array(C0)
+        ng.dot(dA.T if op[0] == "t" else dA, dB.T if op[1] == "t" else dB, C, alpha=0.5, beta=0.25)
+        ref = rm.gemm(A, B, op[0] == "t", op[1] == "t", alpha=0.5, beta=0.25, C=C0)
+        tol = rn16_tol(ref, rm.gemm_abs(A, B, op[0] == "t", op[1] == "t"), k) + 2.0 ** -11 * np.abs(C0.astype(np.float32))
+        assert_close(C.get(), ref, tol, "%s %s +%d" % (op, mnk, shift))
+
+
+@pytest.mark.parametrize("dims", [(2, 8, 8, 8), (3, 129, 72, 65), (5, 33, 17, 130), (17, 128, 128, 64), (1, 40, 24, 72)])
+@pytest.mark.parametrize("shared", [None, "A", "B"])
+def test_batched_dot_forms(ng, dims, shared):
+    """Independent products and products summed over the batch, either operand shared by all of
+    them, reductions that end inside a 64-wide block of every product, odd sizes."""
+    b, m, n, k = dims
+    rng = np.random.default_rng(17 + b)
+    A = rng.standard_normal((m, k) if shared == "A" else (b, m, k)).astype(np.float16)
+    B = rng.standard_normal((k, n) if shared == "B" else (b, k, n)).astype(np.float16)
+    a3, b3 = (np.broadcast_to(x.astype(np.float32), (b,) + x.shape[-2:]) for x in (A, B))
+    each = np.matmul(a3, b3)
+    mag = np.matmul(np.abs(a3), np.abs(b3))
+    C, S = ng.empty((b, m, n)), ng.empty((m, n))
+    ng.batched_dot(ng.array(A), ng.array(B), C)
+    assert_close(C.get(), each, rn16_tol(each, mag, k), "independent %s" % (dims,))
+    ng.batched_dot(ng.array(A), ng.array(B), S, relu=True)
+    total = np.maximum(each.sum(axis=0), 0)
+    assert_close(S.get(), total, rn16_tol(total, mag.sum(axis=0), k * b), "summed %s" % (dims,))
+
+
 def test_reference_c_interface(ng, lib):
     """nervana_hgemm / nervana_hgemm_colmajor keep the reference's signatures and conventions."""
     rng = np.random.default_rng(9)
