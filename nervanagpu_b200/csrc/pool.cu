@@ -11,7 +11,7 @@
 // windows that contain it in increasing (k,m,p,q) order and sum, in fp32, the errors of those
 // whose argmax it is. Overlapping windows so need neither atomics nor a zero-fill pass and the
 // result is deterministic. Windows that do not overlap take one pass. The common 2-D shapes
-// (3x3/2, 2x2/2, 3x3/3 without padding) have compile-time specialisations. The innermost
+// (2x2/2, 3x3/3, 3x3/2 and 3x3/1) have compile-time specialisations. The innermost
 // dimension N is contiguous: each thread owns 8 images (one 16-byte lane) when N % 8 == 0, else 1.
 #include <algorithm>
 #include <cfloat>
@@ -187,357 +187,587 @@ __global__ void pool_gather_kernel(PoolGeo g, const int* __restrict__ arg, const
 }
 
 // ------------------------------------------------------------------------------------------
-// Specialised 2-D windows (J = T = 1, no padding, fp16, N % 8 == 0): compile-time R,S and strides,
-// grid (x: pixel of the plane and image lane, y: channel): two index divisions per thread.
+// Common 2-D windows (J = T = 1, rows of whole 16-byte vectors): window, strides and padding are
+// compile-time constants. A thread owns one 16-byte vector of images and walks a strip of L rows
+// of outputs (inputs, on the way back) of one pixel column, so that an input row that several of
+// its windows share is read and reduced along x once: with one output per thread a 3x3 stride-1
+// window fetches every input nine times through L1, with strips of four rows 4.5 times, and takes
+// nine compares per output instead of six. Measured (fp16, forward / backward, before -> now):
+// 3x3/1 pad 1 on 192 x 28 x 28 x 128: 63.7 -> 18.7 us (4.1 TB/s) / 236 -> 85 us; 3x3/2 on
+// 64 x 55 x 55 x 128: 16.9 -> 10.2 us (6.0 TB/s); 2x2/2 on 64 x 224 x 224 x 64 backward without a
+// record: 164 -> 136 us (6.8 TB/s, HBM bound); 2x2/2 fp32 on 50 x 107 x 107 x 112: 78 -> 47 us /
+// 363 -> 87 us (6.7 TB/s). The 3x3/1 backward pass is bound by its compares: every input is tested
+// against the records of nine windows (strips of 1, 2, 3, 4 rows: 90, 85, 92, 88 us).
 // ------------------------------------------------------------------------------------------
-struct Lanes8 {
-  float v[8];
+template <typename T>
+struct Vec16;
+
+// Eight fp16 images. Maxima stay in fp16, in packed pairs: a mask per pair says which of the two
+// running maxima a candidate beats, and maxima and tap numbers (16 bits each) are merged under it.
+template <>
+struct Vec16<__half> {
+  static constexpr int kLanes = 8;
+  uint32_t w[4];
+  __device__ void load(const __half* p) {
+    const uint4 r = __ldg(reinterpret_cast<const uint4*>(p));
+    w[0] = r.x; w[1] = r.y; w[2] = r.z; w[3] = r.w;
+  }
+  __device__ void store(__half* p) const { *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]); }
+  __device__ void to_float(float (&f)[8]) const {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+      f[2 * i] = v.x; f[2 * i + 1] = v.y;
+    }
+  }
+  __device__ void from_float(const float (&f)[8]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __half2 h = __floats2half2_rn(f[2 * i], f[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+  }
 };
-__device__ __forceinline__ Lanes8 load8(const __half* p) {
-  const uint4 r = *reinterpret_cast<const uint4*>(p);
-  const __half2* h = reinterpret_cast<const __half2*>(&r);
-  Lanes8 o;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 f = __half22float2(h[i]);
-    o.v[2 * i] = f.x;
-    o.v[2 * i + 1] = f.y;
+template <>
+struct Vec16<float> {
+  static constexpr int kLanes = 4;
+  float w[4];
+  __device__ void load(const float* p) {
+    const float4 r = __ldg(reinterpret_cast<const float4*>(p));
+    w[0] = r.x; w[1] = r.y; w[2] = r.z; w[3] = r.w;
   }
-  return o;
-}
-__device__ __forceinline__ void store8(__half* p, const float (&v)[8]) {
-  uint4 r;
-  __half2* h = reinterpret_cast<__half2*>(&r);
+  __device__ void store(float* p) const { *reinterpret_cast<float4*>(p) = make_float4(w[0], w[1], w[2], w[3]); }
+  __device__ void to_float(float (&f)[4]) const {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) h[i] = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
-  *reinterpret_cast<uint4*>(p) = r;
-}
+    for (int i = 0; i < 4; ++i) f[i] = w[i];
+  }
+  __device__ void from_float(const float (&f)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = f[i];
+  }
+};
 
-// max and first-argmax (tap id r*S+s) of window (p,q) of channel plane `plane` for 8 images
-template <int R, int S, int SH, int SW>
-__device__ __forceinline__ void window2d(const __half* __restrict__ plane, int H, int W, int N, int p, int q, int n0,
-                                         float (&best)[8], int (&arg)[8]) {
-#pragma unroll
-  for (int i = 0; i < 8; ++i) { best[i] = -FLT_MAX; arg[i] = 0; }
-  // all taps are requested before the first compare, so that R*S loads are in flight per thread
-  uint4 raw[R * S];
-  bool ok[R * S];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-      const int y = p * SH + r, x = q * SW + s;
-      ok[r * S + s] = y < H && x < W;
-      raw[r * S + s] = make_uint4(0, 0, 0, 0);
-      if (ok[r * S + s]) raw[r * S + s] = __ldg(reinterpret_cast<const uint4*>(plane + (static_cast<long long>(y) * W + x) * N + n0));
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < R * S; ++k) {
-    if (!ok[k]) continue;
-    const __half2* h = reinterpret_cast<const __half2*>(&raw[k]);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 f = __half22float2(h[i]);
-      if (f.x > best[2 * i]) { best[2 * i] = f.x; arg[2 * i] = k; }
-      if (f.y > best[2 * i + 1]) { best[2 * i + 1] = f.y; arg[2 * i + 1] = k; }
-    }
-  }
-}
-
-template <int R, int S, int SH, int SW>
-__global__ void __launch_bounds__(256) pool2d_fprop_kernel(const __half* __restrict__ I, __half* __restrict__ O,
-                                                          uint8_t* __restrict__ arg_out, int H, int W, int N,
-                                                          int P, int Q, int mask_pos) {
-  // one thread per output pixel and vector of 8 images; x walks (p, q, lane) of one channel plane
-  // so that no thread of a block is idle whatever Q is
-  const int nvec = N >> 3;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= P * Q * nvec) return;
-  const int pq = t / nvec;
-  const int n0 = (t - pq * nvec) << 3;
-  const int p = pq / Q, q = pq - p * Q;
-  const int c = blockIdx.y;
-  const __half* plane = I + static_cast<long long>(c) * H * W * N;
-  // All taps are requested before the first compare. The compares stay in fp16 (the inputs are
-  // fp16, so the order is the same as in fp32) on packed pairs: a mask per pair says which of
-  // the two running maxima a tap beats, and maxima and tap numbers are merged under that mask;
-  // three instructions per pair and tap instead of converting every value to fp32.
-  uint4 raw[R * S];
-  bool ok[R * S];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-      const int y = p * SH + r, x = q * SW + s;
-      ok[r * S + s] = y < H && x < W;
-      raw[r * S + s] = make_uint4(0, 0, 0, 0);
-      if (ok[r * S + s])
-        raw[r * S + s] = __ldg(reinterpret_cast<const uint4*>(plane + (static_cast<long long>(y) * W + x) * N + n0));
-    }
-  }
-  uint32_t best[4], arg[4];   // two fp16 maxima / two 16-bit tap numbers per word
-#pragma unroll
-  for (int i = 0; i < 4; ++i) { best[i] = 0xfc00fc00u; arg[i] = 0u; }   // -inf, tap 0
-#pragma unroll
-  for (int k = 0; k < R * S; ++k) {
-    if (!ok[k]) continue;
-    const uint32_t w[4] = {raw[k].x, raw[k].y, raw[k].z, raw[k].w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t m = __hgt2_mask(*reinterpret_cast<const __half2*>(&w[i]), *reinterpret_cast<const __half2*>(&best[i]));
-      best[i] = (w[i] & m) | (best[i] & ~m);
-      arg[i] = ((static_cast<uint32_t>(k) * 0x00010001u) & m) | (arg[i] & ~m);
-    }
-  }
-  const long long o = ((static_cast<long long>(c) * P + p) * Q + q) * N + n0;
-  if (O) *reinterpret_cast<uint4*>(O + o) = make_uint4(best[0], best[1], best[2], best[3]);
-  if (arg_out) {
-    // one byte per output: the tap (r*S + s) of the first maximum. mask_pos 1: a window whose
-    // maximum is not positive names no tap (its error is dropped); mask_pos 2: such windows are
-    // flagged in bit 7 and the backward pass decides whether the flag counts.
-    if (mask_pos) {
-      const uint32_t zero2 = 0u;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t pos = __hgt2_mask(*reinterpret_cast<const __half2*>(&best[i]), *reinterpret_cast<const __half2*>(&zero2));
-        arg[i] = mask_pos == 1 ? ((arg[i] & pos) | (0x00ff00ffu & ~pos)) : (arg[i] | (0x00800080u & ~pos));
-      }
-    }
-    uint2 packed;
-    packed.x = __byte_perm(arg[0], arg[1], 0x6420);   // low byte of each 16-bit tap number
-    packed.y = __byte_perm(arg[2], arg[3], 0x6420);
-    *reinterpret_cast<uint2*>(arg_out + o) = packed;
-  }
-}
-
-// Backward, second stage: the thread that owns the SH x SW input block (a, b) reads the recorded
-// argmax and the error of each overlapping window once and credits the block input it names.
-template <int R, int S, int SH, int SW>
-__global__ void __launch_bounds__(256) pool2d_gather_kernel(const uint8_t* __restrict__ arg,
-                                                           const __half* __restrict__ E,
-                                                           __half* __restrict__ dI, int H, int W, int N, int P, int Q,
-                                                           int BW, uint32_t byte_and) {
-  // byte_and 0x7f7f7f7f drops the "maximum not positive" flag of recorded argmax bytes (no ReLU
-  // mask wanted); with 0xffffffff a flagged byte is >= 128 and matches no tap.
-  constexpr int WP = (R + SH - 1) / SH, WQ = (S + SW - 1) / SW;
-  const int nvec = N >> 3;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int BH = (H + SH - 1) / SH;
-  if (t >= BH * BW * nvec) return;
-  const int ab = t / nvec;
-  const int n0 = (t - ab * nvec) << 3;
-  const int a = ab / BW, b = ab - a * BW;
-  const int c = blockIdx.y;
-  float acc[SH][SW][8];
-#pragma unroll
-  for (int dy = 0; dy < SH; ++dy)
-#pragma unroll
-    for (int dx = 0; dx < SW; ++dx)
-#pragma unroll
-      for (int i = 0; i < 8; ++i) acc[dy][dx][i] = 0.0f;
-  // the records and errors of all overlapping windows are requested before any is used
-  uint2 rec[WP * WQ];
-  uint4 err[WP * WQ];
-  bool live[WP * WQ];
-#pragma unroll
-  for (int wp = 0; wp < WP; ++wp) {
-#pragma unroll
-    for (int wq = 0; wq < WQ; ++wq) {
-      const int p = a - (WP - 1) + wp, q = b - (WQ - 1) + wq;
-      const int w = wp * WQ + wq;
-      live[w] = p >= 0 && p < P && q >= 0 && q < Q;
-      rec[w] = make_uint2(0xffffffffu, 0xffffffffu);
-      err[w] = make_uint4(0, 0, 0, 0);
-      if (live[w]) {
-        const long long o = ((static_cast<long long>(c) * P + p) * Q + q) * N + n0;
-        rec[w] = __ldg(reinterpret_cast<const uint2*>(arg + o));
-        err[w] = __ldg(reinterpret_cast<const uint4*>(E + o));
-      }
-    }
-  }
-#pragma unroll
-  for (int wp = 0; wp < WP; ++wp) {
-#pragma unroll
-    for (int wq = 0; wq < WQ; ++wq) {
-      if (!live[wp * WQ + wq]) continue;
-      uint2 pk = rec[wp * WQ + wq];
-      pk.x &= byte_and;
-      pk.y &= byte_and;
-      const int idx[8] = {static_cast<int>(pk.x & 255u), static_cast<int>((pk.x >> 8) & 255u),
-                          static_cast<int>((pk.x >> 16) & 255u), static_cast<int>(pk.x >> 24),
-                          static_cast<int>(pk.y & 255u), static_cast<int>((pk.y >> 8) & 255u),
-                          static_cast<int>((pk.y >> 16) & 255u), static_cast<int>(pk.y >> 24)};
-      Lanes8 e;
-      {
-        const __half2* h = reinterpret_cast<const __half2*>(&err[wp * WQ + wq]);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 f = __half22float2(h[i]);
-          e.v[2 * i] = f.x;
-          e.v[2 * i + 1] = f.y;
-        }
-      }
-#pragma unroll
-      for (int dy = 0; dy < SH; ++dy) {
-        const int r = (WP - 1 - wp) * SH + dy;     // tap row of block input dy inside window p
-        if (r >= R) continue;
-#pragma unroll
-        for (int dx = 0; dx < SW; ++dx) {
-          const int s = (WQ - 1 - wq) * SW + dx;
-          if (s >= S) continue;
-          const int tap = r * S + s;
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            if (idx[i] == tap) acc[dy][dx][i] += e.v[i];
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int dy = 0; dy < SH; ++dy) {
-    const int y = a * SH + dy;
-    if (y >= H) break;
-#pragma unroll
-    for (int dx = 0; dx < SW; ++dx) {
-      const int x = b * SW + dx;
-      if (x >= W) break;
-      store8(dI + ((static_cast<long long>(c) * H + y) * W + x) * N + n0, acc[dy][dx]);
-    }
-  }
-}
-
-// Each thread owns the SH x SW block of inputs at block coordinates (a, b). The windows that
-// overlap the block are visited in increasing (p, q) order; a window's error goes to the block
-// input that is its first maximum. Same sums in the same order as the per-element gather.
-template <int R, int S, int SH, int SW>
-__global__ void __launch_bounds__(256) pool2d_bprop_kernel(const __half* __restrict__ I, const __half* __restrict__ E,
-                                                          __half* __restrict__ dI, int H, int W, int N, int P, int Q,
-                                                          int BW, int mask_pos) {
-  constexpr int WP = (R + SH - 1) / SH, WQ = (S + SW - 1) / SW;
-  const int nvec = N >> 3;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int BH = (H + SH - 1) / SH;
-  if (t >= BH * BW * nvec) return;
-  const int ab = t / nvec;
-  const int n0 = (t - ab * nvec) << 3;
-  const int a = ab / BW, b = ab - a * BW;
-  const int c = blockIdx.y;
-  const __half* plane = I + static_cast<long long>(c) * H * W * N;
-  float acc[SH][SW][8];
-#pragma unroll
-  for (int dy = 0; dy < SH; ++dy)
-#pragma unroll
-    for (int dx = 0; dx < SW; ++dx)
-#pragma unroll
-      for (int i = 0; i < 8; ++i) acc[dy][dx][i] = 0.0f;
-#pragma unroll
-  for (int wp = 0; wp < WP; ++wp) {
-    const int p = a - (WP - 1) + wp;
-    if (p < 0 || p >= P) continue;
-#pragma unroll
-    for (int wq = 0; wq < WQ; ++wq) {
-      const int q = b - (WQ - 1) + wq;
-      if (q < 0 || q >= Q) continue;
-      float best[8];
-      int arg[8];
-      window2d<R, S, SH, SW>(plane, H, W, N, p, q, n0, best, arg);
-      if (mask_pos) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if (!(best[i] > 0.0f)) arg[i] = 255;
-      }
-      const Lanes8 e = load8(E + ((static_cast<long long>(c) * P + p) * Q + q) * N + n0);
-#pragma unroll
-      for (int dy = 0; dy < SH; ++dy) {
-        constexpr int dummy = 0;
-        (void)dummy;
-        const int r = (WP - 1 - wp) * SH + dy;   // tap row of block input dy inside window p
-        if (r >= R) continue;
-#pragma unroll
-        for (int dx = 0; dx < SW; ++dx) {
-          const int s = (WQ - 1 - wq) * SW + dx;
-          if (s >= S) continue;
-          const int tap = r * S + s;
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            if (arg[i] == tap) acc[dy][dx][i] += e.v[i];
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int dy = 0; dy < SH; ++dy) {
-    const int y = a * SH + dy;
-    if (y >= H) break;
-#pragma unroll
-    for (int dx = 0; dx < SW; ++dx) {
-      const int x = b * SW + dx;
-      if (x >= W) break;
-      store8(dI + ((static_cast<long long>(c) * H + y) * W + x) * N + n0, acc[dy][dx]);
-    }
-  }
-}
-
-template <int R, int S, int SH, int SW>
-int launch_pool2d(const PoolGeo& g, const void* I, const void* EO, void* out, int mode, int* arg_ws,
-                  cudaStream_t stream) {
-  const int nvec = g.N / 8;
-  dim3 fgrid((g.P * g.Q * nvec + 255) / 256, g.C);
-  if (mode == 0) {
-    pool2d_fprop_kernel<R, S, SH, SW><<<fgrid, 256, 0, stream>>>(
-        static_cast<const __half*>(I), static_cast<__half*>(const_cast<void*>(EO)), nullptr, g.H, g.W, g.N, g.P, g.Q, 0);
-    NG_CHECK_LAUNCH();
-  } else if (mode == 3) {
-    // forward pass that also records each window's argmax (bit 7: maximum not positive) in the
-    // caller's buffer, for a later backward pass that then need not look at the input again
-    pool2d_fprop_kernel<R, S, SH, SW><<<fgrid, 256, 0, stream>>>(
-        static_cast<const __half*>(I), static_cast<__half*>(const_cast<void*>(EO)), reinterpret_cast<uint8_t*>(arg_ws),
-        g.H, g.W, g.N, g.P, g.Q, 2);
-    NG_CHECK_LAUNCH();
-  } else if (mode == 4 || mode == 5) {
-    // backward pass from a recorded argmax; mode 5 also applies the ReLU mask of the layer below
-    const int BH = (g.H + SH - 1) / SH, BW = (g.W + SW - 1) / SW;
-    dim3 grid((BH * BW * nvec + 255) / 256, g.C);
-    pool2d_gather_kernel<R, S, SH, SW><<<grid, 256, 0, stream>>>(
-        reinterpret_cast<const uint8_t*>(arg_ws), static_cast<const __half*>(EO), static_cast<__half*>(out), g.H, g.W,
-        g.N, g.P, g.Q, BW, mode == 5 ? 0xffffffffu : 0x7f7f7f7fu);
-    NG_CHECK_LAUNCH();
-  } else if (R <= SH && S <= SW) {
-    // windows do not overlap: one pass, each block of inputs sees at most one window
-    const int BH = (g.H + SH - 1) / SH, BW = (g.W + SW - 1) / SW;
-    dim3 grid((BH * BW * nvec + 255) / 256, g.C);
-    pool2d_bprop_kernel<R, S, SH, SW><<<grid, 256, 0, stream>>>(
-        static_cast<const __half*>(I), static_cast<const __half*>(EO), static_cast<__half*>(out), g.H, g.W, g.N, g.P,
-        g.Q, BW, mode == 2);
-    NG_CHECK_LAUNCH();
+// One byte per image: the tap that holds a window's first maximum.
+template <typename T>
+struct ArgBytes;
+template <>
+struct ArgBytes<__half> { uint32_t w[2]; };
+template <>
+struct ArgBytes<float> { uint32_t w[1]; };
+template <typename T>
+__device__ __forceinline__ ArgBytes<T> load_args(const uint8_t* p) {
+  ArgBytes<T> a;
+  if (sizeof(T) == 2) {
+    const uint2 r = __ldg(reinterpret_cast<const uint2*>(p));
+    a.w[0] = r.x; a.w[sizeof(T) == 2 ? 1 : 0] = r.y;
   } else {
-    uint8_t* arg8 = reinterpret_cast<uint8_t*>(arg_ws);
-    pool2d_fprop_kernel<R, S, SH, SW><<<fgrid, 256, 0, stream>>>(static_cast<const __half*>(I), nullptr, arg8, g.H,
-                                                                g.W, g.N, g.P, g.Q, mode == 2);
-    NG_CHECK_LAUNCH();
-    const int BH = (g.H + SH - 1) / SH, BW = (g.W + SW - 1) / SW;
-    dim3 grid((BH * BW * nvec + 255) / 256, g.C);
-    pool2d_gather_kernel<R, S, SH, SW><<<grid, 256, 0, stream>>>(arg8, static_cast<const __half*>(EO),
-                                                                 static_cast<__half*>(out), g.H, g.W, g.N, g.P, g.Q, BW,
-                                                                 0xffffffffu);
-    NG_CHECK_LAUNCH();
+    a.w[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
   }
+  return a;
+}
+
+// Running maximum and tap of its first occurrence, per image.
+template <typename T>
+struct Best;
+template <>
+struct Best<__half> {
+  uint32_t best[4], arg[4];
+  __device__ void init() {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { best[i] = 0xfc00fc00u; arg[i] = 0u; }   // -inf, tap 0
+  }
+  __device__ void merge(int i, uint32_t v, uint32_t a) {
+    const uint32_t m = __hgt2_mask(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&best[i]));
+    best[i] = (v & m) | (best[i] & ~m);
+    arg[i] = (a & m) | (arg[i] & ~m);
+  }
+  __device__ void take(const Vec16<__half>& v, int tap) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) merge(i, v.w[i], static_cast<uint32_t>(tap) * 0x00010001u);
+  }
+  __device__ void raise(const Vec16<__half>& v) {   // the maximum without its tap
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __half2 h = __hmax2(*reinterpret_cast<const __half2*>(&best[i]), *reinterpret_cast<const __half2*>(&v.w[i]));
+      best[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+  }
+  __device__ void take(const Best<__half>& row, int tap) {   // the row's taps start at `tap`
+#pragma unroll
+    for (int i = 0; i < 4; ++i) merge(i, row.best[i], row.arg[i] + static_cast<uint32_t>(tap) * 0x00010001u);
+  }
+  __device__ Vec16<__half> value() const {
+    Vec16<__half> v;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v.w[i] = best[i];
+    return v;
+  }
+  // mask_pos 1: a window whose maximum is not positive names no tap (its error is dropped);
+  // mask_pos 2: such windows are flagged in bit 7 and the backward pass decides
+  __device__ ArgBytes<__half> bytes(int mask_pos) const {
+    uint32_t a[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      a[i] = arg[i];
+      if (mask_pos) {
+        const uint32_t zero2 = 0u;
+        const uint32_t pos = __hgt2_mask(*reinterpret_cast<const __half2*>(&best[i]), *reinterpret_cast<const __half2*>(&zero2));
+        a[i] = mask_pos == 1 ? ((a[i] & pos) | (0x00ff00ffu & ~pos)) : (a[i] | (0x00800080u & ~pos));
+      }
+    }
+    ArgBytes<__half> o;
+    o.w[0] = __byte_perm(a[0], a[1], 0x6420);   // low byte of each 16-bit tap number
+    o.w[1] = __byte_perm(a[2], a[3], 0x6420);
+    return o;
+  }
+  // `e` where the maximum is tap `tap`, zero elsewhere
+  __device__ Vec16<__half> credit(const Vec16<__half>& e, int tap) const {
+    Vec16<__half> v;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v.w[i] = e.w[i] & __vcmpeq2(arg[i], static_cast<uint32_t>(tap) * 0x00010001u);
+    return v;
+  }
+  __device__ void drop_not_positive() {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t zero2 = 0u;
+      arg[i] |= ~__hgt2_mask(*reinterpret_cast<const __half2*>(&best[i]), *reinterpret_cast<const __half2*>(&zero2));
+    }
+  }
+};
+template <>
+struct Best<float> {
+  float best[4];
+  uint32_t arg[4];
+  __device__ void init() {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { best[i] = -FLT_MAX; arg[i] = 0u; }
+  }
+  __device__ void take(const Vec16<float>& v, int tap) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (v.w[i] > best[i]) { best[i] = v.w[i]; arg[i] = static_cast<uint32_t>(tap); }
+  }
+  __device__ void raise(const Vec16<float>& v) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) best[i] = v.w[i] > best[i] ? v.w[i] : best[i];
+  }
+  __device__ void take(const Best<float>& row, int tap) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (row.best[i] > best[i]) { best[i] = row.best[i]; arg[i] = row.arg[i] + static_cast<uint32_t>(tap); }
+  }
+  __device__ Vec16<float> value() const {
+    Vec16<float> v;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v.w[i] = best[i];
+    return v;
+  }
+  __device__ ArgBytes<float> bytes(int mask_pos) const {
+    ArgBytes<float> o;
+    o.w[0] = 0u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      uint32_t a = arg[i];
+      if (mask_pos && !(best[i] > 0.0f)) a = mask_pos == 1 ? 255u : (a | 128u);
+      o.w[0] |= a << (8 * i);
+    }
+    return o;
+  }
+  __device__ Vec16<float> credit(const Vec16<float>& e, int tap) const {
+    Vec16<float> v;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v.w[i] = arg[i] == static_cast<uint32_t>(tap) ? e.w[i] : 0.0f;
+    return v;
+  }
+  __device__ void drop_not_positive() {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (!(best[i] > 0.0f)) arg[i] = 0xffffffffu;
+  }
+};
+
+struct Plane2d {
+  int H, W, N, P, Q, strips;
+};
+// thread -> (strip, pixel column, first image of its vector); false past the end
+__device__ __forceinline__ bool strip_pos(const Plane2d& g, int columns, int lanes, int& strip, int& x, int& n0) {
+  const uint32_t nvec = static_cast<uint32_t>(g.N / lanes), t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t px = t / nvec;
+  n0 = static_cast<int>(t - px * nvec) * lanes;
+  strip = static_cast<int>(px / static_cast<uint32_t>(columns));
+  x = static_cast<int>(px) - strip * columns;
+  return strip < g.strips;
+}
+
+// Forward pass. Rows are reduced along x first (first maximum of the
+// row), then along y: the order in which ties are broken stays (r, s).
+// kKind: the maximum alone, the maximum (O, may be null) and its tap (arg_out), or the mean.
+enum Pool2dKind : int { P2_MAX = 0, P2_MAX_ARG = 1, P2_AVG = 2 };
+template <typename T, int R, int S, int SH, int SW, int PH, int PW, int L, int kKind>
+__global__ void __launch_bounds__(256) pool2d_fprop_kernel(Plane2d g, const T* __restrict__ I, T* __restrict__ O,
+                                                          uint8_t* __restrict__ arg_out, int mask_pos) {
+  constexpr bool kAvg = kKind == P2_AVG;
+  constexpr int V = Vec16<T>::kLanes, NR = (L - 1) * SH + R;
+  int strip, q, n0;
+  if (!strip_pos(g, g.Q, V, strip, q, n0)) return;
+  const int p0 = strip * L, y0 = p0 * SH - PH, x0 = q * SW - PW;
+  const T* plane = I + static_cast<long long>(blockIdx.y) * g.H * g.W * g.N + n0;
+  const long long out0 = ((static_cast<long long>(blockIdx.y) * g.P + p0) * g.Q + q) * g.N + n0;
+  // (a window without padding lies inside the tensor; a strip may run past the last window)
+  auto inside = [&](int j, int s) {
+    const int y = y0 + j, x = x0 + s;
+    return (PH == 0 || y >= 0) && ((PH == 0 && L == 1) || y < g.H) && (PW == 0 || (x >= 0 && x < g.W));
+  };
+  Vec16<T> raw[2][S];
+  auto fetch = [&](int j, Vec16<T> (&row)[S]) {
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+      if (inside(j, s)) row[s].load(plane + (static_cast<long long>(y0 + j) * g.W + x0 + s) * g.N);
+  };
+  fetch(0, raw[0]);
+  Best<T> win[L];
+  float acc[kAvg ? L : 1][V];
+#pragma unroll
+  for (int j = 0; j < NR; ++j) {
+    if (j + 1 < NR) fetch(j + 1, raw[(j + 1) & 1]);   // one row ahead of the reduction
+    Best<T> row;
+    float sum[V];
+    if (kAvg) {
+#pragma unroll
+      for (int i = 0; i < V; ++i) sum[i] = 0.0f;
+    } else {
+      row.init();
+    }
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      if (!inside(j, s)) continue;
+      if (kAvg) {
+        float f[V];
+        raw[j & 1][s].to_float(f);
+#pragma unroll
+        for (int i = 0; i < V; ++i) sum[i] += f[i];
+      } else {
+        if (kKind == P2_MAX) row.raise(raw[j & 1][s]);
+        else row.take(raw[j & 1][s], s);
+      }
+    }
+#pragma unroll
+    for (int l = 0; l < L; ++l) {
+      const int r = j - l * SH;
+      if (r < 0 || r >= R) continue;
+      if (kAvg) {
+#pragma unroll
+        for (int i = 0; i < V; ++i) acc[kAvg ? l : 0][i] = r == 0 ? sum[i] : acc[kAvg ? l : 0][i] + sum[i];
+      } else {
+        if (r == 0) win[l].init();
+        if (kKind == P2_MAX) win[l].raise(row.value());
+        else win[l].take(row, r * S);
+      }
+      if (r == R - 1 && p0 + l < g.P) {
+        const long long o = out0 + static_cast<long long>(l) * g.Q * g.N;
+        if (kAvg) {
+          Vec16<T> v;
+#pragma unroll
+          for (int i = 0; i < V; ++i) acc[kAvg ? l : 0][i] *= 1.0f / static_cast<float>(R * S);
+          v.from_float(acc[kAvg ? l : 0]);
+          v.store(O + o);
+        } else {
+          if (kKind == P2_MAX || O) win[l].value().store(O + o);
+          if (kKind == P2_MAX_ARG) {
+            const ArgBytes<T> a = win[l].bytes(mask_pos);
+            if (sizeof(T) == 2) *reinterpret_cast<uint2*>(arg_out + o) = make_uint2(a.w[0], a.w[sizeof(T) == 2 ? 1 : 0]);
+            else *reinterpret_cast<uint32_t*>(arg_out + o) = a.w[0];
+          }
+        }
+      }
+    }
+  }
+}
+
+// Backward pass from the recorded argmax bytes (maximum) or of the mean. A thread owns a column of
+// L blocks of SH x SW inputs; it reads the error of every window that overlaps them once, in
+// increasing (p, q) order, and adds it, in fp32, to the input that the record names.
+// byte_and 0x7f7f7f7f drops the "maximum not positive" flag of the records (no ReLU mask wanted);
+// with 0xffffffff a flagged byte is >= 128 and matches no tap.
+template <typename T, int R, int S, int SH, int SW, int PH, int PW, int L, bool kAvg>
+__global__ void __launch_bounds__(256) pool2d_gather_kernel(Plane2d g, int BW, const uint8_t* __restrict__ arg,
+                                                           const T* __restrict__ E, T* __restrict__ dI,
+                                                           uint32_t byte_and) {
+  constexpr int V = Vec16<T>::kLanes, WP = (R + SH - 1) / SH, WQ = (S + SW - 1) / SW, NP = L + WP - 1;
+  int strip, b, n0;
+  if (!strip_pos(g, BW, V, strip, b, n0)) return;
+  const int a0 = strip * L;
+  const long long win0 = static_cast<long long>(blockIdx.y) * g.P * g.Q * g.N + n0;
+  float acc[L][SH][SW][V];
+#pragma unroll
+  for (int l = 0; l < L; ++l)
+#pragma unroll
+    for (int dy = 0; dy < SH; ++dy)
+#pragma unroll
+      for (int dx = 0; dx < SW; ++dx)
+#pragma unroll
+        for (int i = 0; i < V; ++i) acc[l][dy][dx][i] = 0.0f;
+  auto live = [&](int j, int wq) {
+    const int p = a0 - (WP - 1) + j, q = b - (WQ - 1) + wq;
+    return p >= 0 && p < g.P && q >= 0 && q < g.Q;
+  };
+  ArgBytes<T> rec[2][WQ];
+  Vec16<T> err[2][WQ];
+  auto fetch = [&](int j, int slot) {
+#pragma unroll
+    for (int wq = 0; wq < WQ; ++wq)
+      if (live(j, wq)) {
+        const long long o = win0 + (static_cast<long long>(a0 - (WP - 1) + j) * g.Q + b - (WQ - 1) + wq) * g.N;
+        if (!kAvg) rec[slot][wq] = load_args<T>(arg + o);
+        err[slot][wq].load(E + o);
+      }
+  };
+  fetch(0, 0);
+#pragma unroll
+  for (int j = 0; j < NP; ++j) {
+    if (j + 1 < NP) fetch(j + 1, (j + 1) & 1);
+#pragma unroll
+    for (int wq = 0; wq < WQ; ++wq) {
+      if (!live(j, wq)) continue;
+      float e[V];
+      err[j & 1][wq].to_float(e);
+      uint32_t idx[V];
+      if (!kAvg) {
+#pragma unroll
+        for (int i = 0; i < V; ++i) idx[i] = ((rec[j & 1][wq].w[i >> 2] & byte_and) >> (8 * (i & 3))) & 255u;
+      }
+#pragma unroll
+      for (int l = 0; l < L; ++l)
+#pragma unroll
+        for (int dy = 0; dy < SH; ++dy) {
+          const int r = (l + WP - 1 - j) * SH + dy;      // tap row of this input inside window row j
+          if (r < 0 || r >= R) continue;
+#pragma unroll
+          for (int dx = 0; dx < SW; ++dx) {
+            const int s = (WQ - 1 - wq) * SW + dx;
+            if (s >= S) continue;
+#pragma unroll
+            for (int i = 0; i < V; ++i)
+              if (kAvg || idx[i] == static_cast<uint32_t>(r * S + s)) acc[l][dy][dx][i] += e[i];
+          }
+        }
+    }
+  }
+#pragma unroll
+  for (int l = 0; l < L; ++l)
+#pragma unroll
+    for (int dy = 0; dy < SH; ++dy) {
+      const int y = (a0 + l) * SH + dy - PH;
+      if (y < 0 || y >= g.H) continue;
+#pragma unroll
+      for (int dx = 0; dx < SW; ++dx) {
+        const int x = b * SW + dx - PW;
+        if (x < 0 || x >= g.W) continue;
+        Vec16<T> v;
+        if (kAvg) {
+#pragma unroll
+          for (int i = 0; i < V; ++i) acc[l][dy][dx][i] *= 1.0f / static_cast<float>(R * S);
+        }
+        v.from_float(acc[l][dy][dx]);
+        v.store(dI + ((static_cast<long long>(blockIdx.y) * g.H + y) * g.W + x) * g.N + n0);
+      }
+    }
+}
+
+// Backward pass when windows do not overlap, without a record: the thread of block (a, b) reads its
+// window, finds the first maximum and writes the whole block.
+template <typename T, int R, int S, int SH, int SW>
+__global__ void __launch_bounds__(256) pool2d_bprop_kernel(Plane2d g, int BW, const T* __restrict__ I,
+                                                          const T* __restrict__ E, T* __restrict__ dI, int mask_pos) {
+  constexpr int V = Vec16<T>::kLanes;
+  int a, b, n0;
+  if (!strip_pos(g, BW, V, a, b, n0)) return;
+  const long long base = (static_cast<long long>(blockIdx.y) * g.H + a * SH) * g.W + b * SW;
+  Best<T> best;
+  Vec16<T> e;
+  best.init();
+  const bool live = a < g.P && b < g.Q;     // (a ragged border belongs to no window)
+  if (live) {
+    Vec16<T> raw[R * S];
+#pragma unroll
+    for (int k = 0; k < R * S; ++k)
+      raw[k].load(I + (base + static_cast<long long>(k / S) * g.W + k % S) * g.N + n0);
+    e.load(E + ((static_cast<long long>(blockIdx.y) * g.P + a) * g.Q + b) * g.N + n0);
+#pragma unroll
+    for (int k = 0; k < R * S; ++k) best.take(raw[k], k);
+    if (mask_pos) best.drop_not_positive();
+  }
+#pragma unroll
+  for (int dy = 0; dy < SH; ++dy) {
+    if (a * SH + dy >= g.H) break;
+#pragma unroll
+    for (int dx = 0; dx < SW; ++dx) {
+      if (b * SW + dx >= g.W) break;
+      Vec16<T> v;
+      if (live && dy < R && dx < S) {
+        v = best.credit(e, dy * S + dx);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v.w[i] = 0;
+      }
+      v.store(dI + (base + static_cast<long long>(dy) * g.W + dx) * g.N + n0);
+    }
+  }
+}
+
+// mode: 0 forward, 1 backward, 2 backward + ReLU mask, 3 forward that records the argmax in `arg`
+// (bit 7: maximum not positive), 4 / 5 backward from such a record without / with the ReLU mask.
+template <typename T, int R, int S, int SH, int SW, int PH, int PW, int LF, int LB, bool kAvg>
+int launch_pool2d_strips(const PoolGeo& g, const T* I, T* EO, T* out, int mode, uint8_t* arg, cudaStream_t stream) {
+  const int nvec = g.N / Vec16<T>::kLanes, planes = g.C * g.D;
+  Plane2d f = {g.H, g.W, g.N, g.P, g.Q, (g.P + LF - 1) / LF};
+  const int BH = (g.H + PH + SH - 1) / SH, BW = (g.W + PW + SW - 1) / SW;
+  Plane2d b = {g.H, g.W, g.N, g.P, g.Q, (BH + LB - 1) / LB};
+  auto grid = [&](int strips, int columns) {
+    return dim3(static_cast<unsigned>((1ll * strips * columns * nvec + 255) / 256), planes);
+  };
+  if (mode == 0) {
+    pool2d_fprop_kernel<T, R, S, SH, SW, PH, PW, LF, kAvg ? P2_AVG : P2_MAX><<<grid(f.strips, g.Q), 256, 0, stream>>>(
+        f, I, EO, nullptr, 0);
+    NG_CHECK_LAUNCH();
+    return NG_OK;
+  }
+  if (!kAvg && mode == 3) {
+    pool2d_fprop_kernel<T, R, S, SH, SW, PH, PW, LF, P2_MAX_ARG><<<grid(f.strips, g.Q), 256, 0, stream>>>(f, I, EO, arg, 2);
+    NG_CHECK_LAUNCH();
+    return NG_OK;
+  }
+  if (!kAvg && mode < 3) {
+    if constexpr (R <= SH && S <= SW) {
+      b.strips = BH;
+      pool2d_bprop_kernel<T, R, S, SH, SW><<<grid(BH, BW), 256, 0, stream>>>(b, BW, I, EO, out, mode == 2);
+      NG_CHECK_LAUNCH();
+      return NG_OK;
+    } else {
+      pool2d_fprop_kernel<T, R, S, SH, SW, PH, PW, LF, P2_MAX_ARG><<<grid(f.strips, g.Q), 256, 0, stream>>>(
+          f, I, nullptr, arg, mode == 2);
+      NG_CHECK_LAUNCH();
+    }
+  }
+  pool2d_gather_kernel<T, R, S, SH, SW, PH, PW, LB, kAvg><<<grid(b.strips, BW), 256, 0, stream>>>(
+      b, BW, arg, EO, out, mode == 4 ? 0x7f7f7f7fu : 0xffffffffu);
+  NG_CHECK_LAUNCH();
   return NG_OK;
 }
 
-// returns NG_OK when a specialised kernel ran, 1 when the generic path must be used
-int try_pool2d(const PoolGeo& g, const void* I, const void* EO, void* out, int mode, int* arg_ws,
+// Strips where they leave enough threads for the device, single rows elsewhere.
+template <typename T, int R, int S, int SH, int SW, int PH, int PW, int LF, int LB, bool kAvg>
+int launch_pool2d(const DeviceCtx* c, const PoolGeo& g, const void* I, const void* EO, void* out, int mode, void* arg,
+                  cudaStream_t stream) {
+  const T* in = static_cast<const T*>(I);
+  T* eo = static_cast<T*>(const_cast<void*>(EO));
+  const long long threads = 1ll * g.C * g.D * g.P * g.Q * (g.N / Vec16<T>::kLanes);
+  if (threads >= 4ll * 1024 * c->sm_count)
+    return launch_pool2d_strips<T, R, S, SH, SW, PH, PW, LF, LB, kAvg>(g, in, eo, static_cast<T*>(out), mode,
+                                                                      static_cast<uint8_t*>(arg), stream);
+  return launch_pool2d_strips<T, R, S, SH, SW, PH, PW, 1, 1, kAvg>(g, in, eo, static_cast<T*>(out), mode,
+                                                                  static_cast<uint8_t*>(arg), stream);
+}
+
+// The window shapes that have kernels of their own: NG_OK when one ran, 1 when the general path must.
+template <typename T, bool kAvg>
+int try_pool2d(const DeviceCtx* c, const PoolGeo& g, const void* I, const void* EO, void* out, int mode, void* arg,
                cudaStream_t stream) {
-  const bool plain = g.J == 1 && g.T == 1 && g.D == 1 && g.str_j == 1 && g.str_d == 1 && g.pad_j == 0 &&
-                     g.pad_d == 0 && g.pad_h == 0 && g.pad_w == 0 && g.N % 8 == 0 && g.C <= 65535 && g.H <= 65535 &&
-                     (reinterpret_cast<uintptr_t>(I) & 15u) == 0 && (reinterpret_cast<uintptr_t>(EO) & 15u) == 0 &&
-                     (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
-  if (!plain) return 1;
-  if (g.R == 3 && g.S == 3 && g.str_h == 2 && g.str_w == 2) return launch_pool2d<3, 3, 2, 2>(g, I, EO, out, mode, arg_ws, stream);
-  if (g.R == 2 && g.S == 2 && g.str_h == 2 && g.str_w == 2) return launch_pool2d<2, 2, 2, 2>(g, I, EO, out, mode, arg_ws, stream);
-  if (g.R == 3 && g.S == 3 && g.str_h == 3 && g.str_w == 3) return launch_pool2d<3, 3, 3, 3>(g, I, EO, out, mode, arg_ws, stream);
+  auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+  const bool plain = g.J == 1 && g.T == 1 && g.str_j == 1 && g.str_d == 1 && g.pad_j == 0 && g.pad_d == 0 &&
+                     g.N % Vec16<T>::kLanes == 0 && 1ll * g.C * g.D <= 65535 && al(I) && al(EO) && al(out) &&
+                     1ll * (g.H + g.R) * (g.W + g.S) * (g.N / Vec16<T>::kLanes) < 0x7fffffffll;
+  if (!plain || g.R != g.S || g.str_h != g.str_w || g.pad_h != g.pad_w) return 1;
+#define NG_POOL2D(r, st, pd, lf, lb) \
+  if (g.R == r && g.str_h == st && g.pad_h == pd) return launch_pool2d<T, r, r, st, st, pd, pd, lf, lb, kAvg>(c, g, I, EO, out, mode, arg, stream)
+  NG_POOL2D(3, 2, 0, 3, 1);
+  NG_POOL2D(2, 2, 0, 1, 1);
+  NG_POOL2D(3, 3, 0, 1, 1);
+  NG_POOL2D(3, 1, 1, 4, 2);
+  NG_POOL2D(3, 2, 1, 3, 1);
+#undef NG_POOL2D
   return 1;
+}
+
+// ------------------------------------------------------------------------------------------
+// Windows without padding in any number of dimensions: every tap of every window exists, at the
+// same distance from the window's first element. A thread owns one window and vector of images
+// and requests eight taps at a time; HBM bound. 2x2x2x2 on 64 x 16 x 56 x 56 x 32, fp16: forward
+// 54.9 -> 35.1 us (6.2 TB/s), backward 88 -> 65.8 us (6.4 TB/s).
+// ------------------------------------------------------------------------------------------
+constexpr int kTapTable = 64;
+struct TapTable {
+  int n;
+  int off[kTapTable];   // elements, in (j, t, r, s) order
+};
+bool make_tap_table(const PoolGeo& g, TapTable& t) {
+  if (g.pad_j || g.pad_d || g.pad_h || g.pad_w) return false;
+  const long long n = 1ll * g.J * g.T * g.R * g.S;
+  if (n > kTapTable || 1ll * g.J * g.D * g.H * g.W * g.N > 0x7fffffffll || 1ll * g.K * g.M * g.P * g.Q * g.N > 0x7fffffffll)
+    return false;
+  t.n = 0;
+  for (int j = 0; j < g.J; ++j)
+    for (int d = 0; d < g.T; ++d)
+      for (int r = 0; r < g.R; ++r)
+        for (int s = 0; s < g.S; ++s) t.off[t.n++] = (((j * g.D + d) * g.H + r) * g.W + s) * g.N;
+  return true;
+}
+template <typename T>
+__device__ __forceinline__ const T* window_base(const PoolGeo& g, const T* I, uint32_t t) {
+  const uint32_t nvec = static_cast<uint32_t>(g.N / Vec16<T>::kLanes);
+  uint32_t r = t / nvec;
+  const int n0 = static_cast<int>(t - r * nvec) * Vec16<T>::kLanes;
+  uint32_t d = r / g.Q;
+  const int q = static_cast<int>(r - d * g.Q);
+  r = d / g.P;
+  const int p = static_cast<int>(d - r * g.P);
+  d = r / g.M;
+  const int m = static_cast<int>(r - d * g.M);
+  return I + (((1ll * d * g.str_j * g.D + m * g.str_d) * g.H + p * g.str_h) * g.W + q * g.str_w) * g.N + n0;
+}
+template <typename T, bool kArg>
+__device__ __forceinline__ void table_max(const TapTable& taps, const T* base, Best<T>& best) {
+  best.init();
+  for (int k = 0; k < taps.n; k += 8) {
+    Vec16<T> raw[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (k + u < taps.n) raw[u].load(base + taps.off[k + u]);
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (k + u < taps.n) {
+        if (kArg) best.take(raw[u], k + u);
+        else best.raise(raw[u]);
+      }
+  }
+}
+template <typename T>
+__global__ void __launch_bounds__(256) pool_table_fprop_kernel(PoolGeo g, const __grid_constant__ TapTable taps,
+                                                              uint32_t total, const T* __restrict__ I, T* __restrict__ O) {
+  const uint32_t t = blockIdx.x * 256u + threadIdx.x;
+  if (t >= total) return;
+  Best<T> best;
+  table_max<T, false>(taps, window_base(g, I, t), best);
+  best.value().store(O + static_cast<size_t>(t) * Vec16<T>::kLanes);
+}
+// Backward pass when the windows tile the input exactly: the window's inputs are written where it
+// was read, the error at the first maximum and zero elsewhere.
+template <typename T>
+__global__ void __launch_bounds__(256) pool_table_bprop_kernel(PoolGeo g, const __grid_constant__ TapTable taps,
+                                                              uint32_t total, const T* __restrict__ I,
+                                                              const T* __restrict__ E, T* __restrict__ dI, int mask_pos) {
+  const uint32_t t = blockIdx.x * 256u + threadIdx.x;
+  if (t >= total) return;
+  Vec16<T> e;
+  e.load(E + static_cast<size_t>(t) * Vec16<T>::kLanes);
+  const T* base = window_base(g, I, t);
+  Best<T> best;
+  table_max<T, true>(taps, base, best);
+  if (mask_pos) best.drop_not_positive();
+  T* out = dI + (base - I);
+#pragma unroll 4
+  for (int k = 0; k < taps.n; ++k) best.credit(e, k).store(out + taps.off[k]);
 }
 
 int grid_for(long long total, const DeviceCtx* c) {
@@ -698,6 +928,10 @@ __global__ void pool_bprop_op_kernel(PoolGeo g, int op, const T* __restrict__ I,
 template <typename T, int VW>
 int run_pool_op(const PoolGeo& g, int op, const void* I, const void* E, void* out, bool backward, DeviceCtx* c,
                 cudaStream_t stream) {
+  if (op == POOL_AVG) {
+    const int rc = try_pool2d<T, true>(c, g, I, backward ? E : out, out, backward, nullptr, stream);
+    if (rc <= 0) return rc;
+  }
   const bool vec = g.N % VW == 0 && (reinterpret_cast<uintptr_t>(I) & 15u) == 0 &&
                    (reinterpret_cast<uintptr_t>(E) & 15u) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
   const long long out_elems = 1ll * g.K * g.M * g.P * g.Q * g.N;
@@ -735,12 +969,18 @@ int run_pool(const PoolGeo& g, const void* I, const void* EO, void* out, int mod
     if (rc != NG_OK) return rc;
     arg_ws = reinterpret_cast<int*>(c->ws);
   }
-  if (sizeof(T) == 2) {
-    const int rc = try_pool2d(g, I, EO, out, mode, arg_ws, stream);
+  {
+    const int rc = try_pool2d<T, false>(c, g, I, EO, out, mode, arg_ws, stream);
     if (rc <= 0) return rc;
   }
+  TapTable taps;
+  const bool table = vec && make_tap_table(g, taps);
   if (mode != 0 && tiles_exactly(g)) {
-    if (vec)
+    if (table)
+      pool_table_bprop_kernel<T><<<static_cast<unsigned>((out_elems / VW + 255) / 256), 256, 0, stream>>>(
+          g, taps, static_cast<uint32_t>(out_elems / VW), static_cast<const T*>(I), static_cast<const T*>(EO),
+          static_cast<T*>(out), mode == 2);
+    else if (vec)
       pool_bprop_tiled_kernel<T, VW><<<grid_for(out_elems / VW, c), 256, 0, stream>>>(
           g, static_cast<const T*>(I), static_cast<const T*>(EO), static_cast<T*>(out), mode == 2);
     else
@@ -751,7 +991,10 @@ int run_pool(const PoolGeo& g, const void* I, const void* EO, void* out, int mod
   }
   if (mode == 0) {
     T* O = static_cast<T*>(const_cast<void*>(EO));
-    if (vec)
+    if (table)
+      pool_table_fprop_kernel<T><<<static_cast<unsigned>((out_elems / VW + 255) / 256), 256, 0, stream>>>(
+          g, taps, static_cast<uint32_t>(out_elems / VW), static_cast<const T*>(I), O);
+    else if (vec)
       pool_fprop_kernel<T, VW><<<grid_for(out_elems / VW, c), 256, 0, stream>>>(g, static_cast<const T*>(I), O, nullptr, 0);
     else
       pool_fprop_kernel<T, 1><<<grid_for(out_elems, c), 256, 0, stream>>>(g, static_cast<const T*>(I), O, nullptr, 0);
@@ -868,8 +1111,11 @@ int ng_pool_fprop_argmax(const ng_pool_desc* d, int dtype_bytes, const void* I, 
   if (!I || !O || !argmax) return fail(NG_ERR_INVALID_ARG, "null tensor");
   if (dtype_bytes != 2 || (reinterpret_cast<uintptr_t>(argmax) & 7u))
     return fail(NG_ERR_UNSUPPORTED, "recorded argmax needs fp16 tensors and an 8-byte aligned buffer");
-  if (!current_ctx()) return NG_ERR_CUDA;
-  rc = try_pool2d(g, I, O, O, 3, static_cast<int*>(argmax), static_cast<cudaStream_t>(stream));
+  const DeviceCtx* c = current_ctx();
+  if (!c) return NG_ERR_CUDA;
+  size_t bytes = 0;
+  ng_pool_argmax_bytes(d, dtype_bytes, &bytes);
+  rc = bytes == 0 ? 1 : try_pool2d<__half, false>(c, g, I, O, O, 3, argmax, static_cast<cudaStream_t>(stream));
   if (rc > 0) return fail(NG_ERR_UNSUPPORTED, "this pooling shape has no recorded-argmax path (see ng_pool_argmax_bytes)");
   return rc;
 }
@@ -882,9 +1128,12 @@ int ng_pool_bprop_argmax(const ng_pool_desc* d, int dtype_bytes, const void* arg
   if (!argmax || !E || !gradI) return fail(NG_ERR_INVALID_ARG, "null tensor");
   if (dtype_bytes != 2 || (reinterpret_cast<uintptr_t>(argmax) & 7u))
     return fail(NG_ERR_UNSUPPORTED, "recorded argmax needs fp16 tensors and an 8-byte aligned buffer");
-  if (!current_ctx()) return NG_ERR_CUDA;
-  rc = try_pool2d(g, nullptr, E, gradI, relu_mask ? 5 : 4,
-                  static_cast<int*>(const_cast<void*>(argmax)), static_cast<cudaStream_t>(stream));
+  const DeviceCtx* c = current_ctx();
+  if (!c) return NG_ERR_CUDA;
+  size_t bytes = 0;
+  ng_pool_argmax_bytes(d, dtype_bytes, &bytes);
+  rc = bytes == 0 ? 1 : try_pool2d<__half, false>(c, g, nullptr, E, gradI, relu_mask ? 5 : 4, const_cast<void*>(argmax),
+                                                  static_cast<cudaStream_t>(stream));
   if (rc > 0) return fail(NG_ERR_UNSUPPORTED, "this pooling shape has no recorded-argmax path (see ng_pool_argmax_bytes)");
   return rc;
 }

@@ -161,3 +161,40 @@ def test_avg_and_l2_refuse_the_max_only_extensions(ng):
     dI, dE, dB = ng.empty(layer.dimI), ng.empty(layer.dimO), ng.empty(layer.dimI)
     with pytest.raises(ValueError):
         ng.bprop_pool(layer, dI, dE, dB, relu_mask=True)
+
+
+WINDOWS = {"3x3_s2": (3, 2, 0), "2x2_s2": (2, 2, 0), "3x3_s3": (3, 3, 0), "3x3_s1_p1": (3, 1, 1), "3x3_s2_p1": (3, 2, 1)}
+
+
+@pytest.mark.parametrize("dtype", [np.float16, np.float32])
+@pytest.mark.parametrize("size", ["single_rows", "strips"])
+@pytest.mark.parametrize("name", sorted(WINDOWS))
+def test_window_shapes_with_kernels_of_their_own(ng, name, size, dtype):
+    """Maximum (bit for bit) and mean of the window shapes that are compiled in, few outputs (one row
+    per thread) and many (strips of rows), map sizes that leave ragged strips and borders."""
+    R, st, pad = WINDOWS[name]
+    lanes = 8 if dtype is np.float16 else 4
+    n, c, h, w = 16, 3, 7, 10
+    if size == "strips":      # over 4096 threads of one output each per SM
+        n, c, h, w = 72 * lanes, 40, 14 * st + 5, 15 * st + 4
+    cfg = (n, c, 1, h, w, 1, 1, R, R, 0, 0, pad, pad, 1, 1, st, st)
+    pd = rm.PoolDims(*cfg)
+    rng = np.random.default_rng(5 + R + st)
+    I = (rng.integers(0, 12, pd.dimI) / 8.0).astype(dtype)      # plenty of ties
+    E = rng.uniform(-1, 1, pd.dimO).astype(dtype)
+    refO, refB = rm.pool_max_fast(pd, I, E)
+    layer, O, B = _run(ng, cfg, I, E, dtype)
+    assert np.array_equal(O, refO.astype(dtype))
+    assert np.array_equal(B, refB.astype(dtype))
+    if size == "strips":
+        return
+    refO, refB = rm.pool_avg_l2(pd, I, "avg", E)
+    layer = ng.pool_layer(dtype, "avg", *cfg)
+    dI, dE = ng.array(I, dtype=dtype), ng.array(E, dtype=dtype)
+    dO, dB = ng.empty(layer.dimO, dtype=dtype), ng.empty(layer.dimI, dtype=dtype)
+    ng.fprop_pool(layer, dI, dO)
+    ng.bprop_pool(layer, dI, dE, dB)
+    # nine fp32 additions of values up to 1.5 in another order, then one rounding to the stored type
+    unit = 2.0 ** -11 if dtype is np.float16 else 2.0 ** -24
+    assert np.all(np.abs(dO.get() - refO) <= unit * np.abs(refO) + 9 * 2.0 ** -24 * 1.5)
+    assert np.all(np.abs(dB.get() - refB) <= unit * np.abs(refB) + 9 * 2.0 ** -24)
