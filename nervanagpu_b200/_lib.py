@@ -1,9 +1,11 @@
 """ctypes binding of libnervana_b200.so (the C ABI declared in include/nervana_b200.h).
 
-This is the only place that touches the shared library. There is no CPU fallback: if the
+This and the native half of the host path (_native, csrc/pyext.cpp: the calls a program makes
+thousands of times) are the only places that touch the shared library. There is no CPU fallback: if the
 library is missing or the device is not an sm_100 GPU, calls raise.
 """
 import ctypes
+import importlib
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -139,6 +141,23 @@ SIGNATURES = {
                                                ctypes.c_bool, ctypes.c_bool, c_void_p, c_int]),
 }
 
+class _Native(object):
+    """The native module, loaded when it is first used: the build script is part of this package and
+    must be importable before there is anything to load. `prepare` (set by the package) gets the
+    module before its first use."""
+    prepare = None
+
+    def __getattr__(self, name):
+        try:
+            module = importlib.import_module(__package__ + "._native")
+        except ImportError as e:
+            raise ImportError("%s: build it with `python -m nervanagpu_b200.build`" % e)
+        self.prepare(module)
+        self.__dict__.update((k, v) for k, v in module.__dict__.items() if not k.startswith("__"))
+        return self.__dict__[name]
+
+
+native = _Native()
 _lib = None
 _initialised = set()
 

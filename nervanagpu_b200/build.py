@@ -1,14 +1,17 @@
-"""Builds libnervana_b200.so (sm_100a only) in-tree with nvcc.
+"""Builds libnervana_b200.so (sm_100a only) and the CPython module _native.so in-tree.
 
 Usage: python -m nervanagpu_b200.build [--force] [--verbose]
 """
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libnervana_b200.so")
+EXT = os.path.join(HERE, "_native.so")     # CPython module: the native half of the host path
+EXT_SOURCE = os.path.join(CSRC, "pyext.cpp")
 
 SOURCES = ["runtime.cu", "tc_host.cu", "gemm.cu", "conv.cu", "pool.cu", "ew_rt.cu", "legacy_api.cu", "comm.cu"]
 
@@ -62,6 +65,14 @@ def build(force=False, verbose=False):
         r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
         if r.returncode != 0:
             raise RuntimeError("link failed:\n" + r.stdout)
+    if force or _newer(EXT, [EXT_SOURCE, LIB, headers[-1]]):
+        cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+               "-Wall", "-Wno-missing-field-initializers", "-Wno-cast-function-type",
+               "-I" + sysconfig.get_paths()["include"], EXT_SOURCE, "-o", EXT,
+               "-L" + HERE, "-lnervana_b200", "-Wl,-rpath,$ORIGIN"]
+        r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        if r.returncode != 0:
+            raise RuntimeError("build of _native.so failed:\n" + r.stdout)
     return LIB
 
 

@@ -26,6 +26,7 @@ import hashlib
 import numpy as np
 
 from . import _lib
+from ._lib import native as _native
 
 # ---------------------------------------------------------------------------------------------
 # operator tables: name -> (arity, C expression template)
@@ -64,6 +65,9 @@ _float_ops = {
 }
 
 _reduction_ops = ("sum", "max", "min", "argmax", "argmin")
+
+# every operation by number, for the keys of the native half
+operation_numbers = {name: i for i, name in enumerate(sorted(_float_ops) + list(_reduction_ops))}
 
 _CTYPES = {
     "f2": "__half", "f4": "float", "u1": "unsigned char", "i1": "signed char",
@@ -893,13 +897,6 @@ def _rowvec_config(plan, depth):
     return ("row", lpr, ch, ch <= 4, "".join(kinds))
 
 
-class _Launch(object):
-    """A prepared launch: compiled kernel, marshalled arguments, grid. Reused while the same
-    expression is applied to tensors with the same device layout (the common case in a training
-    loop), so that the per-call host cost is a dictionary lookup and one C call."""
-    __slots__ = ("kernel", "holders", "argv", "grid", "block", "offset_holder", "keepalive")
-
-
 _launch_cache = {}
 _LAUNCH_CACHE_LIMIT = 4096
 
@@ -969,19 +966,26 @@ def _prepare(args):
             grid, block = ((n_rows + rows_per_block - 1) // rows_per_block, 1, 1), (32 * rows_per_block, 1, 1)
         else:
             grid, block = (n_rows, 1, 1), (threads, 1, 1)
-    launch = _Launch()
     push(ctypes.c_uint, 0)          # seed lo (filled per call)
     push(ctypes.c_uint, 0)          # seed hi
     push(ctypes.c_uint, 0)          # rng offset
     push(ctypes.c_int, sr)
-    launch.kernel = kernel
-    launch.holders = holders
-    launch.argv = (ctypes.c_void_p * len(holders))(*[ctypes.cast(ctypes.pointer(h), ctypes.c_void_p) for h in holders])
-    launch.grid, launch.block = grid, block
-    # The entry holds raw addresses, not tensors: it is found again only through a key made of the
+    # The launch holds raw addresses, not tensors: it is found again only through a key made of the
     # same addresses and layouts, so it never outlives the meaning of its arguments.
-    launch.keepalive = None
-    return launch
+    argv = (ctypes.c_void_p * len(holders))(*[ctypes.addressof(h) for h in holders])
+    return _native.Launch(kernel.value, grid, block, ctypes.addressof(argv), *[ctypes.addressof(h) for h in holders[-4:-1]],
+                          (holders, argv))
+
+
+def prepare_assignment(out, value):
+    """The prepared launch of out[...] = value (a node, tensor or number); None for an empty tensor.
+    Called by the native half when it meets an expression for the first time."""
+    from .nervanagpu import OpTreeNode
+    args = OpTreeNode({"op": "assign"}, out, value).traverse([])
+    if out.size == 0:
+        _analyse(args)              # still validate the expression
+        return None
+    return _prepare(args)
 
 
 def call_compound_kernel(rand_state, *args):
@@ -1004,18 +1008,10 @@ def call_compound_kernel(rand_state, *args):
         if len(_launch_cache) >= _LAUNCH_CACHE_LIMIT:
             _launch_cache.clear()
         _launch_cache[key] = launch
-    h = launch.holders
-    seed = rand_state.seed if rand_state is not None else 0
-    h[-4].value = seed & 0xFFFFFFFF
-    h[-3].value = (seed >> 32) & 0xFFFFFFFF
-    h[-2].value = rand_state.next_offset() if rand_state is not None else 0
     backend = out.backend
     repeat = backend.bench if (backend is not None and type(backend.bench) is int and backend.bench > 1) else 1
-    lib = _lib.init()
-    g, b = launch.grid, launch.block
     for _ in range(repeat):
-        _lib.check(lib.ng_ew_launch(launch.kernel, g[0], g[1], g[2], b[0], b[1], b[2], 0, launch.argv,
-                                    backend.stream if backend is not None else None))
+        _native.run(launch, backend, rand_state)
     return out
 
 

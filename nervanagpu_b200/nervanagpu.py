@@ -15,11 +15,15 @@ import weakref
 import numpy as np
 
 from . import _lib
-from .float_ew import call_compound_kernel
+from ._lib import native as _native
+from .float_ew import call_compound_kernel, operation_numbers, prepare_assignment
 from .layers import ConvLayer, DeconvLayer, PoolLayer
 
 _none_slice = slice(None, None, None)
 _DTYPES = (np.float16, np.float32, np.uint8, np.int8, np.uint16, np.int16, np.uint32, np.int32)
+_DTYPE_OF = {}      # accepted dtype arguments -> dtype object
+for _t in _DTYPES:
+    _DTYPE_OF[_t] = _DTYPE_OF[np.dtype(_t)] = np.dtype(_t)
 
 
 def _contiguous_strides(shape):
@@ -67,13 +71,15 @@ class GPUTensor(object):
 
     def __init__(self, backend, shape, dtype=np.float16, allocator=mem_alloc, base=None, gpudata=None,
                  strides=None, take_array=None, is_trans=False, name=None, rounding=0):
-        assert dtype in _DTYPES or np.dtype(dtype).type in _DTYPES
-        dtype = np.dtype(dtype)
+        given, dtype = dtype, _DTYPE_OF.get(dtype)
+        if dtype is None:
+            assert np.dtype(given).type in _DTYPES
+            dtype = np.dtype(given)
         try:
+            shape = tuple(map(int, shape))
             size = 1
             for dim in shape:
                 size *= dim
-            shape = tuple(int(d) for d in shape)
         except TypeError:
             assert isinstance(shape, (int, np.integer))
             size = shape
@@ -245,6 +251,8 @@ class GPUTensor(object):
                               rounding=self.rounding)
 
     def _assign(self, value):
+        if type(value) is OpTreeNode:
+            return _assign_to(self, value)
         stream = self.backend.stream
         if isinstance(value, (int, float)):
             if self.is_contiguous:
@@ -260,17 +268,17 @@ class GPUTensor(object):
                 else:
                     _lib.check(lib.ng_memset_d32_async(self.ptr, struct.unpack("I", bits)[0], self.size, stream))
             else:
-                OpTreeNode.build("assign", self, value)
+                _assign_to(self, value)
 
         elif isinstance(value, GPUTensor):
             if self.is_contiguous and value.is_contiguous and self.dtype == value.dtype and not value.is_trans:
                 if self.size:
                     _lib.check(_lib.init().ng_memcpy_d2d_async(self.ptr, value.ptr, self.nbytes, stream))
             else:
-                OpTreeNode.build("assign", self, value)
+                _assign_to(self, value)
 
         elif isinstance(value, OpTreeNode):
-            OpTreeNode.build("assign", self, value)
+            _assign_to(self, value)
 
         elif isinstance(value, np.ndarray):
             self.set(value)
@@ -337,33 +345,33 @@ class GPUTensor(object):
             return OpTreeNode.build("assign", out, self.T)
         return self.T
 
-    def __add__(self, other): return OpTreeNode.build("add", self, other)
-    def __sub__(self, other): return OpTreeNode.build("sub", self, other)
-    def __mul__(self, other): return OpTreeNode.build("mul", self, other)
-    def __div__(self, other): return OpTreeNode.build("div", self, other)
-    def __truediv__(self, other): return OpTreeNode.build("div", self, other)
-    def __pow__(self, other): return OpTreeNode.build("pow", self, other)
-    def __radd__(self, other): return OpTreeNode.build("add", other, self)
-    def __rsub__(self, other): return OpTreeNode.build("sub", other, self)
-    def __rmul__(self, other): return OpTreeNode.build("mul", other, self)
-    def __rdiv__(self, other): return OpTreeNode.build("div", other, self)
-    def __rtruediv__(self, other): return OpTreeNode.build("div", other, self)
-    def __rpow__(self, other): return OpTreeNode.build("pow", other, self)
-    def __eq__(self, other): return OpTreeNode.build("eq", self, other)
-    def __ne__(self, other): return OpTreeNode.build("ne", self, other)
-    def __lt__(self, other): return OpTreeNode.build("lt", self, other)
-    def __le__(self, other): return OpTreeNode.build("le", self, other)
-    def __gt__(self, other): return OpTreeNode.build("gt", self, other)
-    def __ge__(self, other): return OpTreeNode.build("ge", self, other)
-    def __abs__(self): return OpTreeNode.build("abs", self, None)
-    def __neg__(self): return OpTreeNode.build("neg", self, None)
+    def __add__(self, other): return _node(_OPS["add"], self, other)
+    def __sub__(self, other): return _node(_OPS["sub"], self, other)
+    def __mul__(self, other): return _node(_OPS["mul"], self, other)
+    def __div__(self, other): return _node(_OPS["div"], self, other)
+    def __truediv__(self, other): return _node(_OPS["div"], self, other)
+    def __pow__(self, other): return _node(_OPS["pow"], self, other)
+    def __radd__(self, other): return _node(_OPS["add"], other, self)
+    def __rsub__(self, other): return _node(_OPS["sub"], other, self)
+    def __rmul__(self, other): return _node(_OPS["mul"], other, self)
+    def __rdiv__(self, other): return _node(_OPS["div"], other, self)
+    def __rtruediv__(self, other): return _node(_OPS["div"], other, self)
+    def __rpow__(self, other): return _node(_OPS["pow"], other, self)
+    def __eq__(self, other): return _node(_OPS["eq"], self, other)
+    def __ne__(self, other): return _node(_OPS["ne"], self, other)
+    def __lt__(self, other): return _node(_OPS["lt"], self, other)
+    def __le__(self, other): return _node(_OPS["le"], self, other)
+    def __gt__(self, other): return _node(_OPS["gt"], self, other)
+    def __ge__(self, other): return _node(_OPS["ge"], self, other)
+    def __abs__(self): return _node(_OPS["abs"], self, None)
+    def __neg__(self): return _node(_OPS["neg"], self, None)
 
-    def __iadd__(self, other): return OpTreeNode.build("add", self, other, out=self)
-    def __isub__(self, other): return OpTreeNode.build("sub", self, other, out=self)
-    def __imul__(self, other): return OpTreeNode.build("mul", self, other, out=self)
-    def __idiv__(self, other): return OpTreeNode.build("div", self, other, out=self)
-    def __itruediv__(self, other): return OpTreeNode.build("div", self, other, out=self)
-    def __ipow__(self, other): return OpTreeNode.build("pow", self, other, out=self)
+    def __iadd__(self, other): return _build(_OPS["add"], self, other, self)
+    def __isub__(self, other): return _build(_OPS["sub"], self, other, self)
+    def __imul__(self, other): return _build(_OPS["mul"], self, other, self)
+    def __idiv__(self, other): return _build(_OPS["div"], self, other, self)
+    def __itruediv__(self, other): return _build(_OPS["div"], self, other, self)
+    def __ipow__(self, other): return _build(_OPS["pow"], self, other, self)
 
 
 class RandState(object):
@@ -528,18 +536,24 @@ class NervanaGPU(object):
                            grid_P, grid_Q, update_size)
 
     def fprop_conv(self, layer, I, F, O, alpha=1.0, relu=False, repeat=1):
+        if repeat == 1 and not self.bench and _native.conv(0, self, layer, I, F, O, alpha, relu):
+            return 0, 0
         assert layer.sizeI == I.size
         assert layer.sizeF == F.size
         assert layer.sizeO == O.size
         return self._execute_conv(layer, "fprop", I, F, O, alpha, relu, repeat)
 
     def bprop_conv(self, layer, F, E, grad_I, alpha=1.0, repeat=1):
+        if repeat == 1 and not self.bench and _native.conv(1, self, layer, F, E, grad_I, alpha, False):
+            return 0, 0
         assert layer.sizeF == F.size
         assert layer.sizeO == E.size
         assert layer.sizeI == grad_I.size
         return self._execute_conv(layer, "bprop", E, F, grad_I, alpha, False, repeat)
 
     def update_conv(self, layer, I, E, grad_F, alpha=1.0, repeat=1):
+        if repeat == 1 and not self.bench and _native.conv(2, self, layer, I, E, grad_F, alpha, False):
+            return 0, 0
         assert layer.sizeI == I.size
         assert layer.sizeO == E.size
         assert layer.sizeF == grad_F.size
@@ -594,6 +608,8 @@ class NervanaGPU(object):
         """argmax: optional uint8 tensor of pool_argmax_bytes(layer) elements that receives each
         window's argmax, for bprop_pool(..., argmax=) (an extension: the reference's backward
         kernel rescans the windows, nervanagpu/nervanagpu.py:780-787)."""
+        if repeat == 1 and not self.bench and _native.pool(self, layer, I, O, None, 0, argmax):
+            return None
         assert layer.sizeI == I.size
         assert layer.sizeO == O.size
         return self._execute_pool(layer, I, O, None, 0, repeat, argmax)
@@ -603,6 +619,8 @@ class NervanaGPU(object):
         I, in the same pass (an extension: the reference runs it as a separate element-wise
         kernel, nervanagpu/layers.py:87-96). argmax: the record a forward pass over the same I
         left (see fprop_pool); I is then not read."""
+        if repeat == 1 and not self.bench and _native.pool(self, layer, I, E, grad_I, 2 if relu_mask else 1, argmax):
+            return None
         assert layer.sizeI == I.size
         assert layer.sizeO == E.size
         assert layer.sizeI == grad_I.size
@@ -657,6 +675,8 @@ class NervanaGPU(object):
         and is accepted and ignored. stochastic_round: None = use C.rounding (the reference
         behaviour, nervanagpu/nervanagpu.py:1071-1072), else True / mantissa bits / 0.
         """
+        if repeat == 1 and not self.bench and _native.dot(self, A, B, C, alpha, beta, relu, stochastic_round) is not None:
+            return C
         assert A.dtype.type == B.dtype.type == C.dtype.type
         assert min(A.strides) == 1
         assert min(B.strides) == 1
@@ -693,6 +713,9 @@ class NervanaGPU(object):
     def batched_dot(self, A, B, C, alpha=1.0, beta=0.0, relu=False, repeat=1, size=None, stochastic_round=None):
         """Batched GEMM (nervanagpu/nervanagpu.py:820-957): 3-D operands carry the batch in dim 0.
         A 3-D C gives one product per batch entry; a 2-D C sums the products over the batch."""
+        if (repeat == 1 and not self.bench and
+                _native.batched_dot(self, A, B, C, alpha, beta, relu, stochastic_round) is not None):
+            return C
         assert A.dtype.type == B.dtype.type == C.dtype.type
         dima = dimb = dimc = 0
         ldaz = ldbz = ldcz = 0
@@ -752,36 +775,36 @@ class NervanaGPU(object):
         call_compensated_sum(self, sum_tensor, cmp_tensor, add_tensor, cmp_scale, add_scale)
 
     # ---- lazy numpy-style operations -------------------------------------------------------
-    def add(self, a, b, out=None): return OpTreeNode.build("add", a, b, out=out)
-    def subtract(self, a, b, out=None): return OpTreeNode.build("sub", a, b, out=out)
-    def multiply(self, a, b, out=None): return OpTreeNode.build("mul", a, b, out=out)
-    def divide(self, a, b, out=None): return OpTreeNode.build("div", a, b, out=out)
-    def true_divide(self, a, b, out=None): return OpTreeNode.build("div", a, b, out=out)
-    def power(self, a, b, out=None): return OpTreeNode.build("pow", a, b, out=out)
-    def reciprocal(self, a, out=None): return OpTreeNode.build("div", 1, a, out=out)
-    def negative(self, a, out=None): return OpTreeNode.build("neg", a, None, out=out)
-    def sgn(self, a, out=None): return OpTreeNode.build("sgn", a, None, out=out)
-    def absolute(self, a, out=None): return OpTreeNode.build("abs", a, None, out=out)
-    def fabs(self, a, out=None): return OpTreeNode.build("abs", a, None, out=out)
-    def sqrt(self, a, out=None): return OpTreeNode.build("sqrt", a, None, out=out)
-    def square(self, a, out=None): return OpTreeNode.build("sqr", a, None, out=out)
-    def exp(self, a, out=None): return OpTreeNode.build("exp", a, None, out=out)
-    def exp2(self, a, out=None): return OpTreeNode.build("exp2", a, None, out=out)
-    def log(self, a, out=None): return OpTreeNode.build("log", a, None, out=out)
-    def log2(self, a, out=None): return OpTreeNode.build("log2", a, None, out=out)
-    def sig(self, a, out=None): return OpTreeNode.build("sig", a, None, out=out)
-    def sig2(self, a, out=None): return OpTreeNode.build("sig2", a, None, out=out)
-    def tanh(self, a, out=None): return OpTreeNode.build("tanh", a, None, out=out)
-    def tanh2(self, a, out=None): return OpTreeNode.build("tanh2", a, None, out=out)
-    def finite(self, a, out=None): return OpTreeNode.build("finite", a, None, out=out)
-    def equal(self, a, b, out=None): return OpTreeNode.build("eq", a, b, out=out)
-    def not_equal(self, a, b, out=None): return OpTreeNode.build("ne", a, b, out=out)
-    def less(self, a, b, out=None): return OpTreeNode.build("lt", a, b, out=out)
-    def less_equal(self, a, b, out=None): return OpTreeNode.build("le", a, b, out=out)
-    def greater(self, a, b, out=None): return OpTreeNode.build("gt", a, b, out=out)
-    def greater_equal(self, a, b, out=None): return OpTreeNode.build("ge", a, b, out=out)
-    def maximum(self, a, b, out=None): return OpTreeNode.build("maximum", a, b, out=out)
-    def minimum(self, a, b, out=None): return OpTreeNode.build("minimum", a, b, out=out)
+    def add(self, a, b, out=None): return _build(_OPS["add"], a, b, out)
+    def subtract(self, a, b, out=None): return _build(_OPS["sub"], a, b, out)
+    def multiply(self, a, b, out=None): return _build(_OPS["mul"], a, b, out)
+    def divide(self, a, b, out=None): return _build(_OPS["div"], a, b, out)
+    def true_divide(self, a, b, out=None): return _build(_OPS["div"], a, b, out)
+    def power(self, a, b, out=None): return _build(_OPS["pow"], a, b, out)
+    def reciprocal(self, a, out=None): return _build(_OPS["div"], 1, a, out)
+    def negative(self, a, out=None): return _build(_OPS["neg"], a, None, out)
+    def sgn(self, a, out=None): return _build(_OPS["sgn"], a, None, out)
+    def absolute(self, a, out=None): return _build(_OPS["abs"], a, None, out)
+    def fabs(self, a, out=None): return _build(_OPS["abs"], a, None, out)
+    def sqrt(self, a, out=None): return _build(_OPS["sqrt"], a, None, out)
+    def square(self, a, out=None): return _build(_OPS["sqr"], a, None, out)
+    def exp(self, a, out=None): return _build(_OPS["exp"], a, None, out)
+    def exp2(self, a, out=None): return _build(_OPS["exp2"], a, None, out)
+    def log(self, a, out=None): return _build(_OPS["log"], a, None, out)
+    def log2(self, a, out=None): return _build(_OPS["log2"], a, None, out)
+    def sig(self, a, out=None): return _build(_OPS["sig"], a, None, out)
+    def sig2(self, a, out=None): return _build(_OPS["sig2"], a, None, out)
+    def tanh(self, a, out=None): return _build(_OPS["tanh"], a, None, out)
+    def tanh2(self, a, out=None): return _build(_OPS["tanh2"], a, None, out)
+    def finite(self, a, out=None): return _build(_OPS["finite"], a, None, out)
+    def equal(self, a, b, out=None): return _build(_OPS["eq"], a, b, out)
+    def not_equal(self, a, b, out=None): return _build(_OPS["ne"], a, b, out)
+    def less(self, a, b, out=None): return _build(_OPS["lt"], a, b, out)
+    def less_equal(self, a, b, out=None): return _build(_OPS["le"], a, b, out)
+    def greater(self, a, b, out=None): return _build(_OPS["gt"], a, b, out)
+    def greater_equal(self, a, b, out=None): return _build(_OPS["ge"], a, b, out)
+    def maximum(self, a, b, out=None): return _build(_OPS["maximum"], a, b, out)
+    def minimum(self, a, b, out=None): return _build(_OPS["minimum"], a, b, out)
 
     def clip(self, a, a_min, a_max, out=None):
         return self.minimum(self.maximum(a, a_min), a_max, out=out)
@@ -790,25 +813,25 @@ class NervanaGPU(object):
         if axis is None:
             assert partial is not None
             return self.sum(self.sum(a, axis=1, out=partial), axis=0, out=out)
-        return OpTreeNode.build("sum", a, None, axis=axis, out=out)
+        return _reduce("sum", a, axis, out)
 
     def max(self, a, axis=None, partial=None, out=None, keepdims=True):
         if axis is None:
             assert partial is not None
             return self.max(self.max(a, axis=1, out=partial), axis=0, out=out)
-        return OpTreeNode.build("max", a, None, axis=axis, out=out)
+        return _reduce("max", a, axis, out)
 
     def min(self, a, axis=None, partial=None, out=None, keepdims=True):
         if axis is None:
             assert partial is not None
             return self.min(self.min(a, axis=1, out=partial), axis=0, out=out)
-        return OpTreeNode.build("min", a, None, axis=axis, out=out)
+        return _reduce("min", a, axis, out)
 
     def argmax(self, a, axis=1, out=None, keepdims=True):
-        return OpTreeNode.build("argmax", a, None, axis=axis, out=out)
+        return _reduce("argmax", a, axis, out)
 
     def argmin(self, a, axis=1, out=None, keepdims=True):
-        return OpTreeNode.build("argmin", a, None, axis=axis, out=out)
+        return _reduce("argmin", a, axis, out)
 
     def mean(self, a, axis=None, partial=None, out=None, keepdims=True):
         shape = OpTreeNode.shape(a)
@@ -816,7 +839,7 @@ class NervanaGPU(object):
             assert partial is not None
             return self.multiply(self.sum(self.sum(a, axis=1, out=partial), axis=0),
                                  1.0 / (shape[0] * shape[1]), out=out)
-        return self.multiply(self.sum(a, axis=axis), 1.0 / shape[axis], out=out)
+        return _build(_OPS["mul"], _reduce("sum", a, axis, None), 1.0 / shape[axis], out)
 
     def var(self, a, axis=None, partial=None, out=None, keepdims=True):
         if axis is None:
@@ -829,7 +852,7 @@ class NervanaGPU(object):
         return self.sqrt(self.var(a, axis=axis, partial=partial, out=out))
 
     def rand(self, out=None):
-        return OpTreeNode.build("rand", None, None, out=out)
+        return _build(_OPS["rand"], None, None, out)
 
     def dropout(self, keep=0.5, out=None):
         return self.less_equal(self.rand(), keep, out=out)
@@ -841,6 +864,36 @@ class NervanaGPU(object):
         if axis not in (0, 1):
             raise ValueError("bad axis for onehot")
         return OpTreeNode.build("onehot", None, None, idx=indices, axis=axis, out=out)
+
+
+# The operation records of expression nodes. They are never changed, so equal ones are one object.
+_OPS = {name: {"op": name} for name in operation_numbers}
+_AXIS_OPS = {(name, axis): {"op": name, "axis": axis} for name in operation_numbers for axis in (0, 1)}
+
+
+def _node(op_dict, a, b):
+    """An OpTreeNode, or NotImplemented when an operand is no tensor, node or number."""
+    return _native.node(op_dict, a, b)
+
+
+def _build(op_dict, a, b, out):
+    """A node, or, given somewhere to put the result, the assignment."""
+    node = _node(op_dict, a, b)
+    if out is None or node is NotImplemented:
+        return node
+    return _assign_to(out, node)
+
+
+def _reduce(op, a, axis, out):
+    op_dict = _AXIS_OPS.get((op, axis))
+    return _build({"op": op, "axis": axis} if op_dict is None else op_dict, a, None, out)
+
+
+def _assign_to(out, value):
+    """out[...] = value (a node, tensor or number) as one generated kernel."""
+    if _native.assign(out, value) is None:
+        OpTreeNode(_OPS["assign"], out, value).execute()
+    return out
 
 
 class OpTreeNode(tuple):
@@ -855,16 +908,21 @@ class OpTreeNode(tuple):
 
     @staticmethod
     def build(op, a, b, out=None, **kwargs):
-        for arg in (a, b):
-            if not isinstance(arg, (int, float, GPUTensor, OpTreeNode, type(None))):
-                return NotImplemented
-        op_dict = {"op": op}
-        op_dict.update(kwargs)
-        node = OpTreeNode(op_dict, a, b)
+        if not kwargs:
+            op_dict = _OPS.get(op)
+        elif len(kwargs) == 1 and "axis" in kwargs:
+            op_dict = _AXIS_OPS.get((op, kwargs["axis"]))
+        else:
+            op_dict = None
+        if op_dict is None:
+            op_dict = dict(kwargs, op=op)
+        node = _node(op_dict, a, b)
+        if node is NotImplemented:
+            return node
         if op == "assign":
             return node.execute()
         if out is not None:
-            return OpTreeNode({"op": "assign"}, out, node).execute()
+            return _assign_to(out, node)
         return node
 
     def execute(self):
@@ -891,31 +949,31 @@ class OpTreeNode(tuple):
         if type(node) is GPUTensor:
             return node.shape
         if type(node) is OpTreeNode:
-            max_shape = [1, 1]
-            for item in node.traverse(list()):
-                if type(item) is GPUTensor:
-                    for i in range(2):
-                        max_shape[i] = max(max_shape[i], item.shape[i])
-            return tuple(max_shape)
+            a, b = OpTreeNode.shape(node[1]), OpTreeNode.shape(node[2])
+            return (max(a[0], b[0]), max(a[1], b[1]))
         return (1, 1)
 
-    def __add__(self, other): return self.build("add", self, other)
-    def __sub__(self, other): return self.build("sub", self, other)
-    def __mul__(self, other): return self.build("mul", self, other)
-    def __div__(self, other): return self.build("div", self, other)
-    def __truediv__(self, other): return self.build("div", self, other)
-    def __pow__(self, other): return self.build("pow", self, other)
-    def __radd__(self, other): return self.build("add", other, self)
-    def __rsub__(self, other): return self.build("sub", other, self)
-    def __rmul__(self, other): return self.build("mul", other, self)
-    def __rdiv__(self, other): return self.build("div", other, self)
-    def __rtruediv__(self, other): return self.build("div", other, self)
-    def __rpow__(self, other): return self.build("pow", other, self)
-    def __eq__(self, other): return self.build("eq", self, other)
-    def __ne__(self, other): return self.build("ne", self, other)
-    def __lt__(self, other): return self.build("lt", self, other)
-    def __le__(self, other): return self.build("le", self, other)
-    def __gt__(self, other): return self.build("gt", self, other)
-    def __ge__(self, other): return self.build("ge", self, other)
-    def __abs__(self): return self.build("abs", self, None)
-    def __neg__(self): return self.build("neg", self, None)
+    def __add__(self, other): return _node(_OPS["add"], self, other)
+    def __sub__(self, other): return _node(_OPS["sub"], self, other)
+    def __mul__(self, other): return _node(_OPS["mul"], self, other)
+    def __div__(self, other): return _node(_OPS["div"], self, other)
+    def __truediv__(self, other): return _node(_OPS["div"], self, other)
+    def __pow__(self, other): return _node(_OPS["pow"], self, other)
+    def __radd__(self, other): return _node(_OPS["add"], other, self)
+    def __rsub__(self, other): return _node(_OPS["sub"], other, self)
+    def __rmul__(self, other): return _node(_OPS["mul"], other, self)
+    def __rdiv__(self, other): return _node(_OPS["div"], other, self)
+    def __rtruediv__(self, other): return _node(_OPS["div"], other, self)
+    def __rpow__(self, other): return _node(_OPS["pow"], other, self)
+    def __eq__(self, other): return _node(_OPS["eq"], self, other)
+    def __ne__(self, other): return _node(_OPS["ne"], self, other)
+    def __lt__(self, other): return _node(_OPS["lt"], self, other)
+    def __le__(self, other): return _node(_OPS["le"], self, other)
+    def __gt__(self, other): return _node(_OPS["gt"], self, other)
+    def __ge__(self, other): return _node(_OPS["ge"], self, other)
+    def __abs__(self): return _node(_OPS["abs"], self, None)
+    def __neg__(self): return _node(_OPS["neg"], self, None)
+
+
+_native.prepare = lambda module: module.setup(GPUTensor, OpTreeNode, prepare_assignment, _lib.check,
+                                              tuple(np.dtype(t) for t in _DTYPES), operation_numbers)
