@@ -40,31 +40,77 @@ __device__ __forceinline__ void sr_bits8(const EpiArgs& e, unsigned long long e8
 // Stochastic rounding of 8 consecutive outputs to fp16, out of line: ten Philox rounds inlined at
 // every use made the tensor-core kernel's code several times larger than the instruction cache
 // (and the round-to-nearest path paid for it in instruction-cache misses). `lin` is the linear
-// index of the first element; groups that do not start on a multiple of 8 (ragged rows) draw
-// per element.
-static __device__ __noinline__ uint4 sr_round8(EpiArgs e, unsigned long long lin, float v0, float v1, float v2, float v3,
-                                        float v4, float v5, float v6, float v7) {
+// index of the first element.
+static __device__ __noinline__ uint4 sr_round8_any(EpiArgs e, unsigned long long lin, float v0, float v1, float v2,
+                                                   float v3, float v4, float v5, float v6, float v7) {
   const float v[8] = {v0, v1, v2, v3, v4, v5, v6, v7};
   __half h[8];
-  if ((lin & 7ull) == 0ull) {
-    uint32_t rnd[8];
-    sr_bits8(e, lin >> 3, rnd);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) h[i] = f2h_sr(v[i], rnd[i], e.sr_bits);
-  } else {
 #pragma unroll 1
-    for (int i = 0; i < 8; ++i) {
-      uint32_t r8[8];
-      const unsigned long long li = lin + i;
-      sr_bits8(e, li >> 3, r8);
-      h[i] = f2h_sr(v[i], r8[li & 7ull], e.sr_bits);
-    }
+  for (int i = 0; i < 8; ++i) {
+    uint32_t r8[8];
+    const unsigned long long li = lin + i;
+    sr_bits8(e, li >> 3, r8);
+    h[i] = f2h_sr(v[i], r8[li & 7ull], e.sr_bits);
   }
   uint4 o;
   __half2* oh = reinterpret_cast<__half2*>(&o);
 #pragma unroll
   for (int i = 0; i < 4; ++i) oh[i] = __halves2half2(h[2 * i], h[2 * i + 1]);
   return o;
+}
+
+// The same results for formats that keep at least 7 mantissa bits (16 random bits per element).
+// f2h_sr on a normal number adds the random bits below the kept mantissa bits and truncates. Eight
+// of them go through that form together, truncated in pairs by one conversion; one test over all
+// eight finds the values that need the full form (non-zero but below the fp16 normal range, infinite
+// or NaN; a zero comes out as itself either way). A group that does not start on a multiple of 8
+// (ragged rows, kAligned false) takes its bits from two Philox blocks.
+template <bool kAligned>
+static __device__ __forceinline__ uint4 sr_round8_fast(const EpiArgs& e, unsigned long long lin, const float (&v)[8]) {
+  uint4 o;
+  uint32_t* ow = &o.x;
+  uint32_t w[4];           // random bits of two elements per word
+  {
+    const unsigned long long e8 = lin >> 3;
+    const Philox4 a = philox4x32_10(static_cast<uint32_t>(e8), static_cast<uint32_t>(e8 >> 32), e.rng_offset, 0u,
+                                    e.seed_lo, e.seed_hi);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = a.v[i];
+    const uint32_t skip = kAligned ? 0u : static_cast<uint32_t>(lin) & 7u;
+    if (skip) {
+      const unsigned long long f8 = e8 + 1;
+      const Philox4 b = philox4x32_10(static_cast<uint32_t>(f8), static_cast<uint32_t>(f8 >> 32), e.rng_offset, 0u,
+                                      e.seed_lo, e.seed_hi);
+      uint32_t t[8] = {a.v[0], a.v[1], a.v[2], a.v[3], b.v[0], b.v[1], b.v[2], b.v[3]};
+      if (skip & 4u) { t[0] = t[2]; t[1] = t[3]; t[2] = t[4]; t[3] = t[5]; t[4] = t[6]; t[5] = t[7]; }
+      if (skip & 2u) { t[0] = t[1]; t[1] = t[2]; t[2] = t[3]; t[3] = t[4]; t[4] = t[5]; }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = __funnelshift_r(t[i], t[i + 1], (skip & 1u) * 16u);
+    }
+  }
+  const uint32_t mask = (1u << (23 - e.sr_bits)) - 1u;
+  uint32_t low = 0u;       // largest of: twice the bits, less the smallest fp16-normal number's
+  float top = 0.0f;        // largest magnitude, NaN if there is one
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t b0 = __float_as_uint(v[2 * i]), b1 = __float_as_uint(v[2 * i + 1]);
+    low = max(low, max(2u * b0 - (113u << 24), 2u * b1 - (113u << 24)));
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(fabsf(v[2 * i])));
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(fabsf(v[2 * i + 1])));
+    const uint32_t r0 = (b0 + (w[i] & mask)) & ~mask, r1 = (b1 + ((w[i] >> 16) & mask)) & ~mask;
+    asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(ow[i]) : "f"(__uint_as_float(r1)), "f"(__uint_as_float(r0)));
+  }
+  // (a zero gives exactly 143 << 24, a number below the range more, one inside it less)
+  if (low > (143u << 24) || !(top <= 3.402823466e+38f))
+    o = sr_round8_any(e, lin, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
+  return o;
+}
+
+static __device__ __noinline__ uint4 sr_round8(EpiArgs e, unsigned long long lin, float v0, float v1, float v2, float v3,
+                                        float v4, float v5, float v6, float v7) {
+  if (e.sr_bits < 7) return sr_round8_any(e, lin, v0, v1, v2, v3, v4, v5, v6, v7);
+  const float v[8] = {v0, v1, v2, v3, v4, v5, v6, v7};
+  return sr_round8_fast<false>(e, lin, v);
 }
 
 __device__ __forceinline__ float epi_scale(const EpiArgs& e, float acc) {
@@ -154,12 +200,22 @@ __device__ __noinline__ void epi_store8_call(EpiArgs e, float v0, float v1, floa
 
 // Same arithmetic as epi_store8 for 8 consecutive, fully valid, 16-byte aligned outputs, but the
 // result is returned in registers (one 16-byte vector of fp16, or two of fp32) so the caller can
-// stage it in shared memory for a bulk tensor store. `oldp` points at the 8 old values or is null.
+// stage it in shared memory. `oldp` points at the 8 old values or is null; nvalid > 0: only so many
+// of them exist, at any address.
 template <bool F32OUT>
 __device__ __forceinline__ void epi_pack8(const EpiArgs& e, float (&v)[8], const void* oldp, unsigned long long lin,
-                                          uint4& lo, uint4& hi) {
+                                          uint4& lo, uint4& hi, int nvalid = 0) {
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = epi_scale(e, v[i]);
+  if (nvalid > 0) {
+    if (e.beta != 0.0f && oldp) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i < nvalid)
+          v[i] = fmaf(e.beta, F32OUT ? static_cast<const float*>(oldp)[i] : __half2float(static_cast<const __half*>(oldp)[i]), v[i]);
+    }
+    oldp = nullptr;
+  }
   if (F32OUT) {
     if (e.beta != 0.0f && oldp) {
       const float4 a = reinterpret_cast<const float4*>(oldp)[0], b = reinterpret_cast<const float4*>(oldp)[1];

@@ -130,15 +130,19 @@ __device__ __forceinline__ WorkItem decode_work(const TcParams& p, int w) {
 
 // One instance per mode (kMode = p.mode): the producer of each carries only its own coordinate
 // code, which keeps the single-warp roles' loops short in the instruction cache.
-// kLean instances serve the common output stage only (tiles staged through shared memory,
-// alpha 1, no beta term, round to nearest, or raw split-K partials) and carry no other.
+// kLean instances serve one common output stage only and carry no other: 1, tiles staged through
+// shared memory, alpha 1, no beta term, round to nearest, or raw split-K partials; 2 (products), the
+// same rounded stochastically. Called out of line, one group of eight at a time, the Philox rounds
+// were a chain of latencies that two warps per scheduler cannot hide; in line, the four groups of a
+// load interleave. 3072^3, rounded stochastically: 63.6 us before, 50 with the shorter rounding,
+// 45.7 in line (to nearest: 39.4 us).
 // kPair instances run as clusters of two CTAs on the two SMs of a pair (tcgen05 cta_group::2):
 // a work item is a tile of 256 rows, 128 in the tensor memory of each CTA; each CTA loads its own
 // 128 rows of A and its own half of the columns of B (plain TMA loads, no multicast) and the MMA,
 // issued by one thread of the first CTA, reads both halves of B from the two shared memories. Per
 // flop each SM takes in a third fewer operand bytes than with a 128-row tile of its own, and the
 // accumulators stay double-buffered across tiles.
-template <int kMode, bool kLean, bool kPair = false>
+template <int kMode, int kLean, bool kPair = false>
 __global__ void __launch_bounds__(kTcThreads, 1)
 igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                 const __grid_constant__ CUtensorMap mapBm, const __grid_constant__ TcParams p) {
@@ -150,6 +154,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
   // output staging (staged epilogue only), then the control block
   const uint32_t epi_base = smem_base + ring_bytes;
   const bool staged = kLean || p.store_staged != 0;
+  const bool ragged = kMode == TC_GEMM && kLean == 0 && p.store_staged == 2;
   const uint32_t epi_bytes = staged ? kEpiStageBytes : 0u;
 
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_gen + ring_bytes + epi_bytes);
@@ -604,7 +609,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     ea.seed_lo = p.seed_lo; ea.seed_hi = p.seed_hi; ea.rng_offset = p.rng_offset;
     // the common case gets a short path of its own: the epilogue is bound by instruction latency
     // (two warps per scheduler), so every instruction fewer counts
-    const bool plain = kLean || (ea.alpha == 1.0f && ea.beta == 0.0f && ea.sr_bits == 0);
+    const bool plain = kLean == 1 || (kLean == 0 && ea.alpha == 1.0f && ea.beta == 0.0f && ea.sr_bits == 0);
     const bool wide = p.m_halves == 2;
     // two warps share each group of 32 TMEM lanes and split the columns between them
     const int col_group = (warp - 2) >> 2;
@@ -685,6 +690,22 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
               const uint32_t swz = static_cast<uint32_t>(lane & 7);
               // (no "memory" clobber on the staging stores: they are ordered with the loads of the
               // write-out by being volatile and by the __syncwarp between them)
+              if (kLean == 2) {
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                  float v[8];
+#pragma unroll
+                  for (int i = 0; i < 8; ++i) {
+                    v[i] = __uint_as_float(r[g * 8 + i]);
+                    if (ea.relu) v[i] = fmaxf(v[i], 0.0f);
+                  }
+                  const uint4 h = sr_round8_fast<true>(ea, lin_row + colb + sub * 32 + g * 8, v);
+                  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(
+                                   rowb + ((static_cast<uint32_t>(sub * 4 + g) ^ swz) << 4)),
+                               "r"(h.x), "r"(h.y), "r"(h.z), "r"(h.w));
+                }
+                continue;
+              }
               if (plain && f32) {
                 // raw fp32 (split-K partials; fp32 results with alpha 1, beta 0): registers to staging
 #pragma unroll
@@ -730,7 +751,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                 const bool live = row_ok && col < p.N;
                 if (f32) {   // 8 fp32 = two chunks
                   epi_pack8<true>(ea, v, (live && oldrow) ? oldrow + static_cast<long long>(col) * 4 : nullptr,
-                                  lin_row + col, lo, hi);
+                                  lin_row + col, lo, hi, ragged ? min(8, p.N - col) : 0);
                   const int j = g * 2;
                   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rowb + (((j) ^ (lane & 7)) << 4)),
                                "r"(lo.x), "r"(lo.y), "r"(lo.z), "r"(lo.w));
@@ -738,7 +759,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                                "r"(hi.x), "r"(hi.y), "r"(hi.z), "r"(hi.w));
                 } else {                       // 8 fp16 = one chunk
                   epi_pack8<false>(ea, v, (live && oldrow) ? oldrow + static_cast<long long>(col) * 2 : nullptr,
-                                   lin_row + col, lo, hi);
+                                   lin_row + col, lo, hi, ragged ? min(8, p.N - col) : 0);
                   const int j = sub * 4 + g;
                   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rowb + ((j ^ (lane & 7)) << 4)),
                                "r"(lo.x), "r"(lo.y), "r"(lo.z), "r"(lo.w));
@@ -760,6 +781,30 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
               } else {
                 gbase = static_cast<uint8_t*>(p.C) + static_cast<long long>(zt_warp) * p.c_zstride * esz;
                 gstride = p.ldc * esz;
+              }
+              if (ragged) {
+                // rows that start at any address: one row per step, a warp's lanes side by side
+                const uint32_t elem = f32 ? lane & 3 : lane & 7, part = f32 ? lane >> 2 : lane >> 3;
+                uint8_t* gp = gbase + row0 * gstride + static_cast<long long>(colb + lane) * esz;
+                const int rows = min(32, p.M - row0);
+                const bool c0 = colb + lane < p.N, c1 = !f32 && colb + 32 + lane < p.N;
+#pragma unroll 4
+                for (int t = 0; t < rows; ++t, gp += gstride) {
+                  const uint32_t src = buf + static_cast<uint32_t>(t) * 128u + elem * esz;
+                  if (f32) {
+                    uint32_t v;
+                    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(src + ((part ^ (t & 7)) << 4)));
+                    if (c0) *reinterpret_cast<uint32_t*>(gp) = v;
+                  } else {
+                    uint16_t a, b;
+                    asm volatile("ld.shared.b16 %0, [%1];" : "=h"(a) : "r"(src + ((part ^ (t & 7)) << 4)));
+                    asm volatile("ld.shared.b16 %0, [%1];" : "=h"(b) : "r"(src + (((part + 4) ^ (t & 7)) << 4)));
+                    if (c0) *reinterpret_cast<uint16_t*>(gp) = a;
+                    if (c1) *reinterpret_cast<uint16_t*>(gp + 64) = b;
+                  }
+                }
+                __syncwarp();
+                continue;
               }
               const int j = lane & 7;
               int gcol = colb + j * (16 / esz);

@@ -142,9 +142,12 @@ void tc_fill_mma(TcParams& p, const TcOperandLayout& lay) {
 }
 
 // How tiles leave the epilogue: 1 = staged through swizzled shared memory and written out by the
-// warps in whole 128-byte rows, 0 = straight from registers (output not 16-byte addressable).
+// warps in whole 128-byte rows, 2 = staged, written out row by row in single elements (products
+// whose rows are not 16-byte addressable), 0 = straight from registers (stacked taps only).
 static int pick_store_mode(TcParams& p) {
-  if ((p.N & 7) != 0) return 0;
+  const int ragged = p.mode == TC_GEMM && p.splits == 1 ? 2 : 0;
+  p.c_box_cols = p.splits == 1 && !p.out_f32 ? 64 : 32;
+  if ((p.N & 7) != 0) return ragged;
   // stacked taps: a warp's 32 rows must belong to one tap
   if (p.acc_taps > 1 && (p.pack_rows & 31) != 0) return 0;
   const bool partial = p.splits > 1;
@@ -156,14 +159,13 @@ static int pick_store_mode(TcParams& p) {
     row_bytes = static_cast<uint64_t>(p.N) * 4;
     z_bytes = row_bytes * p.M;
   } else {
-    if (!p.vec_ok) return 0;
+    if (!p.vec_ok) return ragged;
     base = p.C;
     row_bytes = static_cast<uint64_t>(p.ldc) * esz;
     z_bytes = p.nz_out > 1 ? static_cast<uint64_t>(p.c_zstride) * esz : row_bytes * p.M;
-    if (z_bytes == 0) return 0;
+    if (z_bytes == 0) return ragged;
   }
-  if ((reinterpret_cast<uintptr_t>(base) & 15u) || (row_bytes & 15u) || (z_bytes & 15u)) return 0;
-  p.c_box_cols = 128 / esz;
+  if ((reinterpret_cast<uintptr_t>(base) & 15u) || (row_bytes & 15u) || (z_bytes & 15u)) return ragged;
   return 1;
 }
 
@@ -303,17 +305,18 @@ int tc_launch(DeviceCtx* c, const CUtensorMap& mapA, const CUtensorMap& mapB, Tc
   }
   if (!c->smem_attr_set) {
 #define NG_TC_SMEM_ATTR(mode)                                                                                        \
-  NG_CUDA(cudaFuncSetAttribute(igemm_tc_kernel<mode, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit)); \
-  NG_CUDA(cudaFuncSetAttribute(igemm_tc_kernel<mode, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit))
+  NG_CUDA(cudaFuncSetAttribute(igemm_tc_kernel<mode, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit)); \
+  NG_CUDA(cudaFuncSetAttribute(igemm_tc_kernel<mode, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit))
     NG_TC_SMEM_ATTR(TC_GEMM);
+    NG_CUDA(cudaFuncSetAttribute(igemm_tc_kernel<TC_GEMM, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
     NG_TC_SMEM_ATTR(TC_FPROP);
     NG_TC_SMEM_ATTR(TC_BPROP);
     NG_TC_SMEM_ATTR(TC_UPDATE);
 #undef NG_TC_SMEM_ATTR
 #define NG_TC_SMEM_ATTR_PAIR(mode)                                                                                 \
-  NG_CUDA(cudaFuncSetAttribute(igemm_tc_kernel<mode, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
+  NG_CUDA(cudaFuncSetAttribute(igemm_tc_kernel<mode, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
                                kSmemLimit));                                                                       \
-  NG_CUDA(cudaFuncSetAttribute(igemm_tc_kernel<mode, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit))
+  NG_CUDA(cudaFuncSetAttribute(igemm_tc_kernel<mode, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit))
     NG_TC_SMEM_ATTR_PAIR(TC_GEMM);
     NG_TC_SMEM_ATTR_PAIR(TC_FPROP);
     NG_TC_SMEM_ATTR_PAIR(TC_BPROP);
@@ -354,8 +357,12 @@ int tc_launch(DeviceCtx* c, const CUtensorMap& mapA, const CUtensorMap& mapB, Tc
   }
   if (!mapBm && (launch.b_merge == 1 || launch.b_merge == 2)) launch.b_merge = 0;
   const CUtensorMap& mapB2 = mapBm ? *mapBm : mapB;
-  // the lean instances: staged tiles, and either raw split-K partials or alpha 1 / no beta / round to nearest
-  const bool lean = tuning().lean_kernels != 0 && launch.store_staged &&
+  // the lean instances: staged tiles, and either raw split-K partials or alpha 1 / no beta, rounded to
+  // nearest, or stochastically to at least 7 bits in rows of whole groups (see kLean)
+  const bool lean_sr = tuning().lean_kernels != 0 && launch.mode == TC_GEMM && launch.store_staged == 1 && !launch.pair &&
+                       launch.splits == 1 && launch.alpha == 1.0f && launch.beta == 0.0f && launch.sr_bits >= 7 &&
+                       !launch.out_f32;
+  const bool lean = tuning().lean_kernels != 0 && launch.store_staged == 1 &&
                     (launch.splits > 1 || (launch.alpha == 1.0f && launch.beta == 0.0f && launch.sr_bits == 0));
   if (launch.pair) {
     // clusters of two CTAs
@@ -372,8 +379,8 @@ int tc_launch(DeviceCtx* c, const CUtensorMap& mapA, const CUtensorMap& mapB, Tc
     cfg.attrs = attr;
     cfg.numAttrs = 1;
 #define NG_TC_LAUNCH_PAIR(mode)                                                                              \
-  if (lean) NG_CUDA(cudaLaunchKernelEx(&cfg, igemm_tc_kernel<mode, true, true>, mapA, mapB, mapB2, launch));  \
-  else NG_CUDA(cudaLaunchKernelEx(&cfg, igemm_tc_kernel<mode, false, true>, mapA, mapB, mapB2, launch))
+  if (lean) NG_CUDA(cudaLaunchKernelEx(&cfg, igemm_tc_kernel<mode, 1, true>, mapA, mapB, mapB2, launch));  \
+  else NG_CUDA(cudaLaunchKernelEx(&cfg, igemm_tc_kernel<mode, 0, true>, mapA, mapB, mapB2, launch))
     switch (launch.mode) {
       case TC_GEMM: NG_TC_LAUNCH_PAIR(TC_GEMM); break;
       case TC_FPROP: NG_TC_LAUNCH_PAIR(TC_FPROP); break;
@@ -395,10 +402,13 @@ int tc_launch(DeviceCtx* c, const CUtensorMap& mapA, const CUtensorMap& mapB, Tc
   cfg.attrs = attr;
   cfg.numAttrs = tuning().dependent_launch != 0 ? 1 : 0;
 #define NG_TC_LAUNCH(mode)                                                                                      \
-  if (lean) NG_CUDA(cudaLaunchKernelEx(&cfg, igemm_tc_kernel<mode, true, false>, mapA, mapB, mapB2, launch));  \
-  else NG_CUDA(cudaLaunchKernelEx(&cfg, igemm_tc_kernel<mode, false, false>, mapA, mapB, mapB2, launch))
+  if (lean) NG_CUDA(cudaLaunchKernelEx(&cfg, igemm_tc_kernel<mode, 1, false>, mapA, mapB, mapB2, launch));  \
+  else NG_CUDA(cudaLaunchKernelEx(&cfg, igemm_tc_kernel<mode, 0, false>, mapA, mapB, mapB2, launch))
   switch (launch.mode) {
-    case TC_GEMM: NG_TC_LAUNCH(TC_GEMM); break;
+    case TC_GEMM:
+      if (lean_sr) NG_CUDA(cudaLaunchKernelEx(&cfg, igemm_tc_kernel<TC_GEMM, 2, false>, mapA, mapB, mapB2, launch));
+      else NG_TC_LAUNCH(TC_GEMM);
+      break;
     case TC_FPROP: NG_TC_LAUNCH(TC_FPROP); break;
     case TC_BPROP: NG_TC_LAUNCH(TC_BPROP); break;
     case TC_UPDATE: NG_TC_LAUNCH(TC_UPDATE); break;
@@ -479,7 +489,7 @@ int static_setup(int dev, StaticSlots** out) {
     s.scratch = static_cast<float*>(p);
     NG_CUDA(cudaGetSymbolAddress(&p, g_static_status));
     s.status = static_cast<int*>(p);
-    NG_CUDA(cudaFuncSetAttribute(igemm_tc_kernel<TC_GEMM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
+    NG_CUDA(cudaFuncSetAttribute(igemm_tc_kernel<TC_GEMM, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
     s.ready = true;
   }
   *out = &s;
@@ -632,7 +642,7 @@ extern "C" int ng_hgemm_static_scratch(const void* A, const void* B, void* C, in
   p.wait_limit_ns = kWaitLimitNs;
   p.full_items = p.total_items = static_cast<int>(total);
   ngb::fill_fast_divs(p);
-  igemm_tc_kernel<TC_GEMM, false><<<grid, kTcThreads, smem, stream>>>(mapA, mapB, mapB, p);
+  igemm_tc_kernel<TC_GEMM, 0><<<grid, kTcThreads, smem, stream>>>(mapA, mapB, mapB, p);
   NG_CHECK_LAUNCH();
   EpiArgs ea;
   ea.alpha = alpha; ea.beta = beta; ea.relu = relu; ea.sr_bits = sr_bits;

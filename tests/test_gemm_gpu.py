@@ -220,3 +220,24 @@ def test_cta_pair_instances_match_the_oracle(ng, lib, op):
     finally:
         assert lib.ng_tune(b"pair_mma", -1) == 0
     assert lib.ng_sync() == 0
+
+
+@pytest.mark.parametrize("bits", [10, 7, 4])
+@pytest.mark.parametrize("scale", [0, -12, -20])
+@pytest.mark.parametrize("mnk", [(256, 256, 64), (130, 264, 40), (130, 131, 40), (64, 72, 1024)])
+def test_stochastic_rounding_forms_agree_bit_for_bit(ng, lib, mnk, scale, bits):
+    """Small integers times a power of two: every sum is exact whatever its order, so the vectorised,
+    the ragged and the split-K output stages must round each element with the same random bits as the
+    element-by-element form of the CUDA-core kernel. Scales put the results in the normal and in the
+    subnormal fp16 range; zeros occur in all of them."""
+    m, n, k = mnk
+    rng = np.random.default_rng(3)
+    A = rng.integers(-3, 4, (m, k)).astype(np.float16)
+    B = (rng.integers(-3, 4, (k, n)) * 2.0 ** scale * (1 + 2.0 ** -4)).astype(np.float16)
+    A[5], B[:, 7] = 0, 0
+    dA, dB, c1, c2 = ng.array(A), ng.array(B), ng.empty((m, n)), ng.empty((m, n))
+    for fn, c in ((lib.ng_hgemm, c1), (lib.ng_hgemm_simt, c2)):
+        assert fn(dA.ptr, dB.ptr, c.ptr, 0, 0, m, n, k, k, n, n, 1.0, 0.0, 0, bits, 99, 7, None) == 0
+    a, b = c1.get(), c2.get()
+    assert np.array_equal(a, b)
+    assert (a[5] == 0).all() and (a[:, 7] == 0).all() and (a != 0).sum() > a.size // 2
