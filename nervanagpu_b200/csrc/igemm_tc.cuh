@@ -23,6 +23,17 @@ struct FastDiv {
   uint32_t mul, shr, d;
 };
 
+// Where a column of the GEMM's view of a pixel space lies in memory. Columns are numbered in 64-wide
+// chunks, `row_chunks` per image row; the first row_len elements of a row exist. row_chunks 0:
+// columns are stored as they are numbered. n 0: the rows follow one another. n > 0: the pixels
+// (n images each) are those of one phase of a strided layer, x / y / z elements apart.
+struct ColumnMap {
+  int row_chunks, row_len;
+  int n, x, y_count;
+  long long y, z;
+  FastDiv fd_chunks, fd_n, fd_y;
+};
+
 struct TcParams {
   // ---- work decomposition: item = ((split * nz + z) * tiles_n + tile_n) * tiles_m + tile_m
   int tiles_m, tiles_n, nz, splits;
@@ -88,6 +99,8 @@ struct TcParams {
   int str_d, str_h, str_w;
   int inner_tap;                   // N in flattened-(W,N) mode else 0
   int x_tap;                       // 0 in flattened mode else 1
+  int phase_w;                     // > 1: the input is a copy whose rows are split into this many x phases
+                                   // (strided layers in flattened mode): tap s reads phase s % phase_w
   int dec_cpi, dec_q, dec_p, dec_m;  // chunk decode of the pixel space the chunks walk
   int oob_y;                       // a y/p coordinate that is out of range (forces zero fill)
 
@@ -104,16 +117,12 @@ struct TcParams {
   int store_staged;                // 1: tiles leave through swizzled shared memory, written out in
                                    // whole 128-byte rows; 0: stored straight from registers
   int c_box_cols;                  // columns per staged box (128 bytes worth: 64 fp16 / 32 fp32)
-  // Convolution outputs over a flattened (x, n) pixel space whose image rows are not a multiple
-  // of 64 elements: the column space is padded to c_row_chunks chunks per image row, of which
-  // the first c_row_len elements exist in memory (row r starts at column r * c_row_len of C).
-  // 0 = columns are stored as they are numbered.
-  int c_row_chunks, c_row_len;
+  ColumnMap cmap;                  // convolution outputs
   uint32_t seed_lo, seed_hi, rng_offset;
   float* ws;                       // split-K partials [split][z][M][N] when splits > 1
   int* status;                     // device status word
   // divisors of the tile / chunk / tap decodes, filled in by the launch code
-  FastDiv fd_tiles_m, fd_tiles_n, fd_nz, fd_cpi, fd_q, fd_p, fd_RS, fd_S, fd_red, fd_crow;
+  FastDiv fd_tiles_m, fd_tiles_n, fd_nz, fd_cpi, fd_q, fd_p, fd_RS, fd_S, fd_red, fd_phase;
   unsigned long long wait_limit_ns;   // bound of every wait inside the kernel
 };
 

@@ -57,6 +57,7 @@ __device__ __forceinline__ ChunkPos decode_chunk(const TcParams& p, int chunk) {
 
 struct Tap {
   int t, r, s;
+  int sq, sp;   // s / phase_w and s % phase_w (phase_w > 1 only)
 };
 __device__ __forceinline__ Tap decode_tap(const TcParams& p, int trs) {
   Tap tp;
@@ -64,6 +65,8 @@ __device__ __forceinline__ Tap decode_tap(const TcParams& p, int trs) {
   const int rs = trs - tp.t * p.RS;
   tp.r = fast_div(rs, p.fd_S);
   tp.s = rs - tp.r * p.S;
+  tp.sq = fast_div(tp.s, p.fd_phase);
+  tp.sp = tp.s - tp.sq * p.phase_w;
   return tp;
 }
 
@@ -74,19 +77,20 @@ struct Walk {
   int trs, rc;
 };
 
-// Exact division for the strided gather of the backward pass: returns false when `num` is not
-// a multiple of `den` (that tap does not touch this pixel).
-__device__ __forceinline__ bool div_exact(int num, int den, int& out) {
-  if (den == 1) {
-    out = num;
-    return true;
+// Memory offset (elements, inside a row of the output) of column `col`, a multiple of 8; false for
+// columns that pad an image row to whole chunks.
+__device__ __forceinline__ bool map_column(const ColumnMap& m, int col, long long& off) {
+  const int ch = col >> 6;
+  const int r = fast_div(ch, m.fd_chunks);
+  const int within = (ch - r * m.row_chunks) * kChunk + (col & (kChunk - 1));
+  if (within >= m.row_len) return false;
+  if (m.n == 0) {
+    off = static_cast<long long>(r) * m.row_len + within;
+  } else {
+    const int x = fast_div(within, m.fd_n), z = fast_div(r, m.fd_y);
+    off = z * m.z + (r - z * m.y_count) * m.y + static_cast<long long>(x) * m.x + (within - x * m.n);
   }
-  if (num < 0) {
-    out = -1;  // out of range either way
-    return true;
-  }
-  out = num / den;
-  return out * den == num;
+  return true;
 }
 
 // Row coordinate of a box that must read zeros (a chunk past the end of the pixel space): this far
@@ -227,7 +231,8 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     uint32_t phase = 0;
     bool ok = true;
     // steps of the box coordinates per tap (s, r, t) and per reduction chunk, see below
-    const bool linear = (kMode == TC_FPROP || (kMode == TC_BPROP && p.str_w == 1 && p.str_h == 1 && p.str_d == 1));
+    constexpr bool linear = kMode == TC_FPROP || kMode == TC_BPROP;
+    const bool phased = kMode == TC_FPROP && p.phase_w > 1 && !is_a;
     int ls[5] = {0, 0, 0, 0, 0}, lr[5] = {0, 0, 0, 0, 0}, lt[5] = {0, 0, 0, 0, 0}, lc[5] = {0, 0, 0, 0, 0};
     int steps_for = -1;   // form of the B box (0 per chunk, 1 merged) the steps were taken for; -1 = not yet
     for (int w = w_first; w < total_work && ok; w += w_step) {
@@ -245,7 +250,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
       // values costs this single warp more than the MMAs of a k-block take.
       Walk wk;
       wk.cp = {0, 0, 0, 0, true};   // fprop/bprop: pixel chunk of this B box; update: walks
-      wk.tap = {0, 0, 0};           // fprop/bprop: walks the filter taps; update: fixed (z)
+      wk.tap = {0, 0, 0, 0, 0};     // fprop/bprop: walks the filter taps; update: fixed (z)
       wk.trs = 0; wk.rc = 0;        // tap number and reduction-chunk number inside the tap
       bool tap_live = true;         // update: this A box's tap exists (last group may be short)
       if (kMode == TC_GEMM) {   // trs counts the products that are summed into one output
@@ -303,32 +308,26 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
               if (p.a_merge) { c1 = rc * p.kb_rows; c2 = (m0 + kTileM * bi) / kChunk; c3 = trs; }
               else { c0 = m0 + kChunk * bi; c1 = trs; c2 = rc * p.kb_rows; }
             } else {     // input pixels of this chunk shifted by the tap
-              c0 = cp.inner0 + (tap.s - p.pad_w) * p.inner_tap;
-              c1 = (cp.q * p.str_w - p.pad_w + tap.s * p.tap_w) * p.x_tap;
+              c0 = cp.inner0 + ((p.phase_w > 1 ? tap.sq : tap.s) - p.pad_w) * p.inner_tap;
+              c1 = p.phase_w > 1 ? tap.sp : (cp.q * p.str_w - p.pad_w + tap.s * p.tap_w) * p.x_tap;
               c2 = cp.valid ? cp.p * p.str_h - p.pad_h + tap.r * p.tap_h : p.oob_y + kFarRows;
               c3 = cp.m * p.str_d - p.pad_d + tap.t;
               c4 = rc * p.kb_rows;
             }
           } else if (kMode == TC_BPROP) {
-            if (is_a) {  // filter rows c0.., 64 output channels k of tap trs
-              c0 = rc * kChunk; c1 = trs; c2 = m0;
-            } else {     // error pixels that reach this input pixel through tap trs
-              bool v = cp.valid;
-              int q = 0, pp = 0, mm = 0;
-              if (p.x_tap) {
-                v &= div_exact(cp.q + p.pad_w - tap.s, p.str_w, q);
-                c0 = cp.inner0;
-              } else {
-                c0 = cp.inner0 + (p.pad_w - tap.s) * p.inner_tap;
-              }
-              v &= div_exact(cp.p + p.pad_h - tap.r, p.str_h, pp);
-              v &= div_exact(cp.m + p.pad_d - tap.t, p.str_d, mm);
-              c1 = q; c2 = v ? pp : p.oob_y + kFarRows; c3 = mm; c4 = rc * kChunk;
+            if (is_a) {  // filter rows c0.., 64 output channels k of the tap
+              c0 = rc * kChunk; c1 = tap.s; c2 = tap.r; c3 = tap.t; c4 = m0;
+            } else {     // error pixels that reach this input pixel through the tap
+              c0 = cp.inner0 + (p.x_tap ? 0 : (p.pad_w - tap.s) * p.inner_tap);
+              c1 = p.x_tap ? cp.q + p.pad_w - tap.s : 0;
+              c2 = cp.valid ? cp.p + p.pad_h - tap.r : p.oob_y + kFarRows;
+              c3 = cp.m + p.pad_d - tap.t;
+              c4 = rc * kChunk;
             }
           } else {  // TC_UPDATE: k-block = one 64-element chunk of the (m,p,q,n) space
             if (is_a != (p.swap_ab != 0)) {  // input pixels under tap z, 128 channels c
-              c0 = cp.inner0 + (tap.s - p.pad_w) * p.inner_tap;
-              c1 = (cp.q * p.str_w - p.pad_w + tap.s * p.tap_w) * p.x_tap;
+              c0 = cp.inner0 + ((p.phase_w > 1 ? tap.sq : tap.s) - p.pad_w) * p.inner_tap;
+              c1 = p.phase_w > 1 ? tap.sp : (cp.q * p.str_w - p.pad_w + tap.s * p.tap_w) * p.x_tap;
               c2 = tap_live ? cp.p * p.str_h - p.pad_h + tap.r * p.tap_h : p.oob_y;
               c3 = cp.m * p.str_d - p.pad_d + tap.t;
               c4 = p.swap_ab ? 0 : m0;
@@ -356,8 +355,9 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
           if (++s.rc == p.red_chunks) {
             s.rc = 0;
             ++s.trs;
+            if (kMode == TC_FPROP && ++s.tap.sp == p.phase_w) { s.tap.sp = 0; ++s.tap.sq; }
             if (++s.tap.s == p.S) {
-              s.tap.s = 0;
+              s.tap.s = s.tap.sq = s.tap.sp = 0;
               if (++s.tap.r == p.R) { s.tap.r = 0; ++s.tap.t; }
             }
           }
@@ -387,7 +387,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
       int lb0 = 0, lb1 = 0, lb2 = 0, lb3 = 0, lb4 = 0;          // coordinates at tap (0, 0, 0), chunk 0
       if (linear && act) {
         Walk o = wk;
-        o.tap = {0, 0, 0}; o.trs = 0; o.rc = 0;
+        o.tap = {0, 0, 0, 0, 0}; o.trs = 0; o.rc = 0;
         coords(o, lb0, lb1, lb2, lb3, lb4);
         if (steps_for != static_cast<int>(merged)) {
           steps_for = static_cast<int>(merged);
@@ -396,7 +396,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
           int b0, b1, b2, b3, b4, d0, d1, d2, d3, d4;
           coords(o, b0, b1, b2, b3, b4);
           Walk q = o;
-          q.tap.s = 1; q.trs = 1;
+          q.tap.s = q.tap.sq = 1; q.trs = 1;   // (phased input: the step from one group of phases to the next)
           coords(q, d0, d1, d2, d3, d4);
           ls[0] = d0 - b0; ls[1] = d1 - b1; ls[2] = d2 - b2; ls[3] = d3 - b3; ls[4] = d4 - b4;
           q = o; q.tap.r = 1; q.trs = p.S;
@@ -415,12 +415,13 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         // (All lanes poll: one polling lane plus a broadcast measured the same or slower.)
         int c0 = 0, c1 = 0, c2 = 0, c3 = 0, c4 = 0;
         if (linear) {
-          const int ts = wk.tap.s, tr = wk.tap.r, tt = wk.tap.t, rc = wk.rc;
+          const int ts = phased ? wk.tap.sq : wk.tap.s, tr = wk.tap.r, tt = wk.tap.t, rc = wk.rc;
           c0 = lb0 + ts * ls[0] + tr * lr[0] + tt * lt[0] + rc * lc[0];
           c1 = lb1 + ts * ls[1] + tr * lr[1] + tt * lt[1] + rc * lc[1];
           c2 = lb2 + ts * ls[2] + tr * lr[2] + tt * lt[2] + rc * lc[2];
           c3 = lb3 + ts * ls[3] + tr * lr[3] + tt * lt[3] + rc * lc[3];
           c4 = lb4 + ts * ls[4] + tr * lr[4] + tt * lt[4] + rc * lc[4];
+          if (phased) c1 += wk.tap.sp;
         } else if (act) {
           coords(wk, c0, c1, c2, c3, c4);
         }
@@ -807,19 +808,11 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                 continue;
               }
               const int j = lane & 7;
-              int gcol = colb + j * (16 / esz);
+              long long gcol = colb + j * (16 / esz);
               bool col_live = gcol < p.N && zt_warp < p.nz_out;
-              if (kConvOut && !partial && p.c_row_chunks) {
-                // Flattened pixel space whose image rows are padded to whole 64-element chunks:
-                // this box is chunk `ch` of the padded space; it holds elements [cq * 64, +64) of
-                // image row r, of which only those below c_row_len exist in memory.
-                const int ch = colb >> 6;
-                const int r = fast_div(ch, p.fd_crow);
-                const int cq = ch - r * p.c_row_chunks;
-                gcol = r * p.c_row_len + cq * kChunk + j * 8;
-                col_live = col_live && cq * kChunk + j * 8 < p.c_row_len;
-              }
-              uint8_t* gp = gbase + (row0 + (lane >> 3)) * gstride + static_cast<long long>(gcol) * esz;
+              // (convolutions: one 64-wide box is one chunk of the pixel space)
+              if (kConvOut && !partial && p.cmap.row_chunks) col_live = col_live && map_column(p.cmap, colb + j * 8, gcol);
+              uint8_t* gp = gbase + (row0 + (lane >> 3)) * gstride + gcol * esz;
               uint4 v[8];
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
@@ -914,7 +907,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
 // The partials have rows of N columns, of which the first n_out exist in the output.
 __global__ void splitk_reduce_kernel(const float* __restrict__ ws, int splits, int lanes, int nz, int M, int N, int n_out,
                                      void* C, const void* Cold, long long ldc, long long c_zstride, int out_f32,
-                                     int vec_ok, EpiArgs ea, int c_row_chunks, int c_row_len) {
+                                     int vec_ok, EpiArgs ea, ColumnMap cmap) {
   grid_dependency_wait();     // (launched while the product that writes the partials drains)
   grid_launch_dependents();
   const int groups_per_row = (n_out + 7) / 8;
@@ -970,25 +963,17 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, int splits, i
     for (int j = 0; j < 8; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], d);
   }
   if (!live || sub != 0) return;
-  int gcol = col;
-  if (c_row_chunks) {
-    // padded image rows (see TcParams::c_row_chunks): the partials are laid out in the padded
-    // column space, the output is not
-    const int ch = col >> 6;
-    const int r = ch / c_row_chunks;
-    const int within = (ch - r * c_row_chunks) * kChunk + (col & 63);
-    if (within >= c_row_len) return;
-    gcol = r * c_row_len + within;
-  }
-  const long long off = z * c_zstride + static_cast<long long>(row) * ldc;
+  long long gcol = col;      // (the partials are laid out in the padded column space, the output is not)
+  if (cmap.row_chunks && !map_column(cmap, col, gcol)) return;
+  const long long off = z * c_zstride + static_cast<long long>(row) * ldc + gcol;
   const int esz = out_f32 ? 4 : 2;
   uint8_t* crow = static_cast<uint8_t*>(C) + off * esz;
   const uint8_t* oldrow = Cold ? static_cast<const uint8_t*>(Cold) + off * esz : nullptr;
   const unsigned long long lin = (static_cast<unsigned long long>(z) * M + row) * static_cast<unsigned long long>(n_out) + col;
   if (out_f32)
-    epi_store8<true>(ea, v, crow, oldrow, gcol, lin, nvalid, vec_ok != 0);
+    epi_store8<true>(ea, v, crow, oldrow, 0, lin, nvalid, vec_ok != 0);
   else
-    epi_store8<false>(ea, v, crow, oldrow, gcol, lin, nvalid, vec_ok != 0);
+    epi_store8<false>(ea, v, crow, oldrow, 0, lin, nvalid, vec_ok != 0);
 }
 
 }  // namespace ngb

@@ -48,7 +48,10 @@ static void fill_fast_divs(TcParams& p) {
   p.fd_RS = make_fast_div(p.RS);
   p.fd_S = make_fast_div(p.S);
   p.fd_red = make_fast_div(p.red_chunks);
-  p.fd_crow = make_fast_div(p.c_row_chunks);
+  p.fd_phase = make_fast_div(p.phase_w);
+  p.cmap.fd_chunks = make_fast_div(p.cmap.row_chunks);
+  p.cmap.fd_n = make_fast_div(p.cmap.n);
+  p.cmap.fd_y = make_fast_div(p.cmap.y_count);
 }
 
 // Bytes a K-major A descriptor may read past its (short) slot; kept inside the allocation.
@@ -343,7 +346,7 @@ int tc_launch(DeviceCtx* c, const CUtensorMap& mapA, const CUtensorMap& mapB, Tc
     grid = 2 * static_cast<int>(std::min<long long>(total, c->sm_count / 2));   // one pair per work item in flight
   }
   p.store_staged = pick_store_mode(p);
-  if (p.c_row_chunks && !p.store_staged)
+  if (p.cmap.row_chunks && !p.store_staged)
     return fail(NG_ERR_UNSUPPORTED, "internal: padded image rows need the staged output stage");
   if (!p.wait_limit_ns) p.wait_limit_ns = c->wait_limit_ns;
   const uint32_t smem = p.stages * p.stage_bytes + 1024u + kCtrlBytes + (p.store_staged ? kEpiStageBytes : 0u) +
@@ -436,8 +439,7 @@ int tc_launch(DeviceCtx* c, const CUtensorMap& mapA, const CUtensorMap& mapB, Tc
     cfg.attrs = attr;
     cfg.numAttrs = tuning().dependent_launch != 0 ? 1 : 0;
     NG_CUDA(cudaLaunchKernelEx(&cfg, splitk_reduce_kernel, static_cast<const float*>(p.ws), p.splits, lanes, p.nz_out,
-                               p.M, p.N, n_out, p.C, p.Cold, p.ldc, p.c_zstride, p.out_f32, p.vec_ok, ea, p.c_row_chunks,
-                               p.c_row_len));
+                               p.M, p.N, n_out, p.C, p.Cold, p.ldc, p.c_zstride, p.out_f32, p.vec_ok, ea, p.cmap));
     NG_CHECK_LAUNCH();
   }
   return NG_OK;
@@ -652,7 +654,7 @@ extern "C" int ng_hgemm_static_scratch(const void* A, const void* B, void* C, in
     const int lanes = ngb::splitk_reduce_lanes(groups, p.splits, slots->sm_count);
     const int blocks = static_cast<int>((groups * lanes + 255) / 256);
     splitk_reduce_kernel<<<blocks, 256, 0, stream>>>(p.ws, p.splits, lanes, 1, m, n, n, C, p.Cold, ldc, 0, 0, p.vec_ok,
-                                                     ea, 0, 0);
+                                                     ea, p.cmap);
     NG_CHECK_LAUNCH();
   }
   return NG_OK;

@@ -339,3 +339,36 @@ def test_layer_argument_checks(ng):
     with pytest.raises(TypeError):
         ng.fprop_conv(layer, ng.empty(layer.dimI, dtype=np.float32), ng.empty(layer.dimF, dtype=np.float32),
                       ng.empty(layer.dimO, dtype=np.float32))
+
+
+STRIDED = {
+    # minibatches that are no multiple of 64 (split copies of the input), and multiples of it (phases of
+    # the backward pass alone); filters shorter than the stride, padding larger than a phase, 3-D
+    "n8_3x3_s2": (8, 24, 16, 1, 5, 5, 1, 3, 3, 0, 1, 1, 1, 2, 2),
+    "n24_5x5_s3": (24, 40, 72, 1, 17, 14, 1, 5, 5, 0, 2, 2, 1, 3, 3),
+    "n88_7x7_s2_c96": (88, 96, 72, 1, 13, 15, 1, 7, 7, 0, 3, 3, 1, 2, 2),
+    "n16_1x1_s2": (16, 64, 136, 1, 9, 8, 1, 1, 1, 0, 0, 0, 1, 2, 2),
+    "n40_2x3_s3_h1": (40, 17, 64, 1, 8, 16, 1, 2, 3, 0, 0, 1, 1, 1, 3),
+    "n32_3d_s222": (32, 32, 32, 5, 6, 7, 3, 3, 3, 1, 1, 1, 2, 2, 2),
+    "n16_c3_5x5_s2": (16, 3, 24, 1, 12, 11, 1, 5, 5, 0, 2, 2, 1, 2, 2),
+    "n64_3x3_s2": (64, 130, 72, 1, 9, 12, 1, 3, 3, 0, 1, 1, 1, 2, 2),
+    "n128_1x1_s2": (128, 64, 64, 1, 7, 7, 1, 1, 1, 0, 0, 0, 1, 2, 2),
+    "n64_4x4_s4_pad3": (64, 16, 32, 1, 10, 9, 1, 4, 4, 0, 3, 3, 1, 4, 4),
+    "n64_2x2_s3": (64, 48, 64, 1, 11, 10, 1, 2, 2, 0, 1, 0, 1, 3, 3),
+}
+
+
+@pytest.mark.parametrize("name", sorted(STRIDED))
+def test_strided_layers_run_on_the_tensor_core_path(ng, lib, name):
+    import ctypes
+    cfg = STRIDED[name]
+    cd = rm.ConvDims(*cfg)
+    I, F, E = _inputs(cd, 1007)
+    ref = {"O": rm.conv_fprop_fast(cd, I, F, relu=True), "gradI": rm.conv_bprop_fast(cd, F, E),
+           "gradF": rm.conv_update_fast(cd, I, E)}
+    before, after = ctypes.c_ulonglong(0), ctypes.c_ulonglong(0)
+    assert lib.ng_fallback_launch_count(ctypes.byref(before)) == 0
+    got = _run_all(ng, _layer(ng, cfg, "auto"), I, F, E, relu=True)
+    assert lib.ng_fallback_launch_count(ctypes.byref(after)) == 0
+    assert after.value == before.value
+    _check(cd, got, I, F, E, ref, name)
