@@ -25,9 +25,10 @@ enum Dtype : int { kF16 = 0, kF32 = 1 };   // positions in the tuple that setup(
 PyObject *g_tensor_type, *g_node_type, *g_prepare, *g_check, *g_dtypes, *g_ops;
 PyObject* g_cache;   // expression key -> Launch
 constexpr Py_ssize_t kCacheLimit = 4096;
+constexpr int kMaxArgs = 1024;   // 4 KB of kernel parameters of 4 bytes and more
 
 PyObject *s_gpudata, *s_shape, *s_strides, *s_dtype, *s_is_trans, *s_rounding, *s_take_array, *s_backend, *s_stream,
-    *s_value, *s_ptr, *s_bench, *s_rand_state, *s_seed, *s_offset, *s_op, *s_axis, *s_desc, *s_path, *s_sizeI, *s_sizeF,
+    *s_value, *s_ptr, *s_bench, *s_rand_state, *s_seed, *s_offset, *s_op, *s_axis, *s_as_parameter, *s_desc, *s_path, *s_sizeI, *s_sizeF,
     *s_sizeO;
 
 // "not the plain case": forget the error, let the Python form of the call take over
@@ -43,6 +44,16 @@ PyObject* failed(int rc) {   // raises NervanaError with the library's message
     PyErr_SetString(PyExc_RuntimeError, "library call failed");
   }
   return nullptr;
+}
+
+// A C call as ctypes makes it: other threads run meanwhile. A launch waits while the stream's queue
+// is full, and what the queued kernels wait for may be another thread's launch.
+template <typename F>
+int without_gil(F call) {
+  PyThreadState* state = PyEval_SaveThread();
+  const int rc = call();
+  PyEval_RestoreThread(state);
+  return rc;
 }
 
 // owned reference that goes away with its scope
@@ -152,31 +163,33 @@ bool read_tensor(PyObject* o, Tensor& t) {
   else {
     long long v;
     if (!to_ll(ro.o, v)) return false;
+    if (v < 0 || v > 255) return false;   // (one byte of an expression's key)
     t.rounding = static_cast<int>(v);
   }
   return t.is_trans >= 0;
 }
 
+// The forms of a stream that ctypes takes for a void pointer: None, an int, a c_void_p, or an object
+// that says in _as_parameter_ which of these it stands for (a torch.cuda.Stream does).
 bool read_stream(PyObject* backend, void*& stream) {
-  if (backend == Py_None) {
-    stream = nullptr;
-    return true;
+  stream = nullptr;
+  if (backend == Py_None) return true;
+  PyObject* s = PyObject_GetAttr(backend, s_stream);
+  for (int depth = 0; s && depth < 8; ++depth) {
+    if (s == Py_None || PyLong_Check(s)) {
+      Ref v(s);
+      if (s != Py_None) stream = reinterpret_cast<void*>(PyLong_AsUnsignedLongLong(s));
+      return !PyErr_Occurred();
+    }
+    PyObject* next = PyObject_GetAttr(s, s_as_parameter);
+    if (!next) {
+      PyErr_Clear();
+      next = PyObject_GetAttr(s, s_value);
+    }
+    Py_SETREF(s, next);
   }
-  Ref s(PyObject_GetAttr(backend, s_stream));
-  if (!s) return false;
-  if (s.o == Py_None) {
-    stream = nullptr;
-    return true;
-  }
-  Ref v(PyLong_Check(s.o) ? Py_NewRef(s.o) : PyObject_GetAttr(s.o, s_value));
-  if (!v) return false;
-  if (v.o == Py_None) {
-    stream = nullptr;
-    return true;
-  }
-  if (!PyLong_Check(v.o)) return false;
-  stream = reinterpret_cast<void*>(PyLong_AsUnsignedLongLong(v.o));
-  return !PyErr_Occurred();
+  Py_XDECREF(s);
+  return false;
 }
 
 // The position of a RandState (or None) in its random stream, moved on by one.
@@ -210,7 +223,7 @@ struct Launch {
   void* kernel;
   unsigned grid[3], block[3];
   void** argv;
-  uint32_t *seed_lo, *seed_hi, *offset;
+  int n_args;      // the last four: seed low, seed high, random offset, rounding
   PyObject* keep;
 };
 
@@ -219,41 +232,49 @@ void launch_dealloc(PyObject* self) {
   Py_TYPE(self)->tp_free(self);
 }
 
-// Launch(kernel, grid, block, address of the argument pointers, of seed low, seed high and offset, owner)
+// Launch(kernel, grid, block, address and number of the argument pointers, owner)
 PyObject* launch_new(PyTypeObject* type, PyObject* args, PyObject*) {
-  unsigned long long kernel, argv, lo, hi, off;
+  unsigned long long kernel, argv;
   unsigned g[3], b[3];
+  int n_args;
   PyObject* keep;
-  if (!PyArg_ParseTuple(args, "K(III)(III)KKKKO", &kernel, &g[0], &g[1], &g[2], &b[0], &b[1], &b[2], &argv, &lo, &hi,
-                        &off, &keep))
+  if (!PyArg_ParseTuple(args, "K(III)(III)KiO", &kernel, &g[0], &g[1], &g[2], &b[0], &b[1], &b[2], &argv, &n_args, &keep))
     return nullptr;
+  if (n_args < 4 || n_args > kMaxArgs) {
+    PyErr_SetString(PyExc_ValueError, "too many kernel arguments");
+    return nullptr;
+  }
   Launch* l = reinterpret_cast<Launch*>(type->tp_alloc(type, 0));
   if (!l) return nullptr;
   l->kernel = reinterpret_cast<void*>(kernel);
   memcpy(l->grid, g, sizeof(g));
   memcpy(l->block, b, sizeof(b));
   l->argv = reinterpret_cast<void**>(argv);
-  l->seed_lo = reinterpret_cast<uint32_t*>(lo);
-  l->seed_hi = reinterpret_cast<uint32_t*>(hi);
-  l->offset = reinterpret_cast<uint32_t*>(off);
+  l->n_args = n_args;
   l->keep = Py_NewRef(keep);
   return reinterpret_cast<PyObject*>(l);
 }
 
 PyTypeObject g_launch_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
-// Runs a prepared launch on the backend's stream with the next random offset of `rs`.
-int launch_run(Launch* l, PyObject* backend, PyObject* rs, bool& plain) {
+// Runs a prepared launch on the backend's stream with the next random offset of `rs`. The caller
+// holds a reference to it: another thread may run it at the same time, or drop it from the cache.
+int launch_run(const Launch* l, PyObject* backend, PyObject* rs, bool& plain) {
   unsigned long long seed;
   unsigned off;
   void* stream;
   plain = read_stream(backend, stream) && next_random(rs, seed, off);
   if (!plain) return NG_ERR_INVALID_ARG;
-  *l->seed_lo = static_cast<uint32_t>(seed);
-  *l->seed_hi = static_cast<uint32_t>(seed >> 32);
-  *l->offset = off;
-  return ng_ew_launch(l->kernel, l->grid[0], l->grid[1], l->grid[2], l->block[0], l->block[1], l->block[2], 0, l->argv,
-                      stream);
+  uint32_t lo = static_cast<uint32_t>(seed), hi = static_cast<uint32_t>(seed >> 32);
+  void* argv[kMaxArgs];
+  memcpy(argv, l->argv, sizeof(void*) * l->n_args);
+  argv[l->n_args - 4] = &lo;
+  argv[l->n_args - 3] = &hi;
+  argv[l->n_args - 2] = &off;
+  return without_gil([&] {
+    return ng_ew_launch(l->kernel, l->grid[0], l->grid[1], l->grid[2], l->block[0], l->block[1], l->block[2], 0, argv,
+                        stream);
+  });
 }
 
 // Key of an expression: everything its prepared launch depends on, in postfix order. A tensor
@@ -295,7 +316,7 @@ struct Key {
     const Py_ssize_t items = PyDict_GET_SIZE(d);
     if (items == 2) {
       PyObject* a = PyDict_GetItemWithError(d, s_axis);
-      if (!to_ll(a, axis)) return false;
+      if (!to_ll(a, axis) || axis < 0 || axis > 1) return false;
     } else if (items != 1) {
       return false;
     }
@@ -448,10 +469,11 @@ PyObject* py_dot(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 8 || !read_tensor(args[1], p.a) || !read_tensor(args[2], p.b) || !read_tensor(args[3], p.c) || p.a.nd != 2 ||
       p.b.nd != 2 || p.c.nd != 2 || !read_product(args, p, 0, 0, 0))
     return decline();
-  const int rc = ng_hgemm(reinterpret_cast<void*>(p.a.ptr), reinterpret_cast<void*>(p.b.ptr),
-                          reinterpret_cast<void*>(p.c.ptr), p.a.is_trans, p.b.is_trans, p.m, p.n, p.k,
-                          static_cast<int>(p.lda), static_cast<int>(p.ldb), static_cast<int>(p.ldc), p.alpha, p.beta,
-                          p.relu, p.sr, p.seed, p.off, p.stream);
+  const int rc = without_gil([&] {
+    return ng_hgemm(reinterpret_cast<void*>(p.a.ptr), reinterpret_cast<void*>(p.b.ptr), reinterpret_cast<void*>(p.c.ptr),
+                    p.a.is_trans, p.b.is_trans, p.m, p.n, p.k, static_cast<int>(p.lda), static_cast<int>(p.ldb),
+                    static_cast<int>(p.ldc), p.alpha, p.beta, p.relu, p.sr, p.seed, p.off, p.stream);
+  });
   if (rc != NG_OK) return failed(rc);
   return Py_NewRef(args[3]);
 }
@@ -465,12 +487,14 @@ PyObject* py_batched_dot(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if ((fa && fb && p.b.shape[0] != batch) || (fc && p.c.shape[0] != batch) || batch < 1 || batch > 0x7fffffff)
     return decline();
   if (!read_product(args, p, fa, fb, fc)) return decline();
-  const int rc = ng_hgemm_batched(reinterpret_cast<void*>(p.a.ptr), reinterpret_cast<void*>(p.b.ptr),
-                                  reinterpret_cast<void*>(p.c.ptr), p.a.is_trans, p.b.is_trans, p.m, p.n, p.k,
-                                  static_cast<int>(p.lda), static_cast<int>(p.ldb), static_cast<int>(p.ldc), p.alpha,
-                                  p.beta, p.relu, p.sr, p.seed, p.off, fc ? static_cast<int>(batch) : 1,
-                                  fc ? 1 : static_cast<int>(batch), fa ? p.a.strides[0] : 0, fb ? p.b.strides[0] : 0,
-                                  fc ? p.c.strides[0] : 0, p.stream);
+  const int rc = without_gil([&] {
+    return ng_hgemm_batched(reinterpret_cast<void*>(p.a.ptr), reinterpret_cast<void*>(p.b.ptr),
+                            reinterpret_cast<void*>(p.c.ptr), p.a.is_trans, p.b.is_trans, p.m, p.n, p.k,
+                            static_cast<int>(p.lda), static_cast<int>(p.ldb), static_cast<int>(p.ldc), p.alpha, p.beta,
+                            p.relu, p.sr, p.seed, p.off, fc ? static_cast<int>(batch) : 1,
+                            fc ? 1 : static_cast<int>(batch), fa ? p.a.strides[0] : 0, fb ? p.b.strides[0] : 0,
+                            fc ? p.c.strides[0] : 0, p.stream);
+  });
   if (rc != NG_OK) return failed(rc);
   return Py_NewRef(args[3]);
 }
@@ -504,10 +528,11 @@ PyObject* py_conv(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return decline();
   if (a.dtype != kF16 || b.dtype != kF16 || !(c.dtype == kF16 || (pass == 2 && c.dtype == kF32))) return decline();
   void *pa = reinterpret_cast<void*>(a.ptr), *pb = reinterpret_cast<void*>(b.ptr), *pc = reinterpret_cast<void*>(c.ptr);
-  int rc;
-  if (pass == 0) rc = ng_conv_fprop(&d, pa, pb, pc, alpha, relu, static_cast<int>(path), stream);
-  else if (pass == 1) rc = ng_conv_bprop(&d, pa, pb, pc, alpha, static_cast<int>(path), stream);
-  else rc = ng_conv_update(&d, pa, pb, pc, c.dtype == kF32, alpha, static_cast<int>(path), stream);
+  const int rc = without_gil([&] {
+    if (pass == 0) return ng_conv_fprop(&d, pa, pb, pc, alpha, relu, static_cast<int>(path), stream);
+    if (pass == 1) return ng_conv_bprop(&d, pa, pb, pc, alpha, static_cast<int>(path), stream);
+    return ng_conv_update(&d, pa, pb, pc, c.dtype == kF32, alpha, static_cast<int>(path), stream);
+  });
   if (rc != NG_OK) return failed(rc);
   Py_RETURN_TRUE;
 }
@@ -534,11 +559,11 @@ PyObject* py_pool(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const int esz = in.dtype == kF16 ? 2 : 4;
   void *pi = reinterpret_cast<void*>(in.ptr), *pe = reinterpret_cast<void*>(eo.ptr), *po = reinterpret_cast<void*>(out.ptr),
        *pr = reinterpret_cast<void*>(arg.ptr);
-  int rc;
-  if (mode == 0) rc = record ? ng_pool_fprop_argmax(&d, esz, pi, pe, pr, stream) : ng_pool_fprop(&d, esz, pi, pe, stream);
-  else if (record) rc = ng_pool_bprop_argmax(&d, esz, pr, pe, po, mode == 2, stream);
-  else if (mode == 1) rc = ng_pool_bprop(&d, esz, pi, pe, po, stream);
-  else rc = ng_pool_bprop_relu(&d, esz, pi, pe, po, stream);
+  const int rc = without_gil([&] {
+    if (mode == 0) return record ? ng_pool_fprop_argmax(&d, esz, pi, pe, pr, stream) : ng_pool_fprop(&d, esz, pi, pe, stream);
+    if (record) return ng_pool_bprop_argmax(&d, esz, pr, pe, po, mode == 2, stream);
+    return mode == 1 ? ng_pool_bprop(&d, esz, pi, pe, po, stream) : ng_pool_bprop_relu(&d, esz, pi, pe, po, stream);
+  });
   if (rc != NG_OK) return failed(rc);
   Py_RETURN_TRUE;
 }
@@ -571,6 +596,7 @@ PyMODINIT_FUNC PyInit__native(void) {
                {&s_is_trans, "is_trans"}, {&s_rounding, "rounding"}, {&s_take_array, "take_array"},
                {&s_backend, "backend"}, {&s_stream, "stream"}, {&s_value, "value"}, {&s_ptr, "ptr"}, {&s_bench, "bench"},
                {&s_rand_state, "rand_state"}, {&s_seed, "seed"}, {&s_offset, "offset"}, {&s_op, "op"}, {&s_axis, "axis"},
+               {&s_as_parameter, "_as_parameter_"},
                {&s_desc, "desc"}, {&s_path, "path"}, {&s_sizeI, "sizeI"}, {&s_sizeF, "sizeF"}, {&s_sizeO, "sizeO"}};
   for (auto& x : names)
     if (!(*x.slot = PyUnicode_InternFromString(x.text))) return nullptr;

@@ -966,15 +966,14 @@ def _prepare(args):
             grid, block = ((n_rows + rows_per_block - 1) // rows_per_block, 1, 1), (32 * rows_per_block, 1, 1)
         else:
             grid, block = (n_rows, 1, 1), (threads, 1, 1)
-    push(ctypes.c_uint, 0)          # seed lo (filled per call)
+    push(ctypes.c_uint, 0)          # seed lo (each call passes its own)
     push(ctypes.c_uint, 0)          # seed hi
     push(ctypes.c_uint, 0)          # rng offset
     push(ctypes.c_int, sr)
     # The launch holds raw addresses, not tensors: it is found again only through a key made of the
     # same addresses and layouts, so it never outlives the meaning of its arguments.
     argv = (ctypes.c_void_p * len(holders))(*[ctypes.addressof(h) for h in holders])
-    return _native.Launch(kernel.value, grid, block, ctypes.addressof(argv), *[ctypes.addressof(h) for h in holders[-4:-1]],
-                          (holders, argv))
+    return _native.Launch(kernel.value, grid, block, ctypes.addressof(argv), len(holders), (holders, argv))
 
 
 def prepare_assignment(out, value):

@@ -294,3 +294,45 @@ def test_compensated_sum_matches_the_kahan_model_and_keeps_small_updates(ng, dty
     ng.compensated_sum(dS, dC, ng.array(a, dtype=dtype))
     s2, c2 = _kahan_model(s, c, a, 0.0, 1.0)
     assert np.array_equal(dS.get(), s2) and np.array_equal(dC.get(), c2) and dC.kahan_count == 1
+
+
+class _StandsFor(object):
+    """An object that names its stream in _as_parameter_, as a torch.cuda.Stream does."""
+
+    def __init__(self, handle):
+        self._as_parameter_ = handle
+
+
+@pytest.mark.parametrize("form", ["none", "c_void_p", "int", "object"])
+def test_every_form_of_a_stream_is_taken_by_expressions_products_and_pooling(ng, form):
+    rng = np.random.default_rng(31)
+    handle = ng.new_stream()
+    ng.stream = {"none": None, "c_void_p": handle, "int": handle.value, "object": _StandsFor(handle)}[form]
+    try:
+        a = rng.uniform(-1, 1, (64, 128)).astype(np.float16)
+        b = rng.uniform(-1, 1, (128, 64)).astype(np.float16)
+        A, B, C, D = ng.array(a), ng.array(b), ng.empty((64, 64)), ng.empty((64, 64))
+        D[:] = ng.max(A[:, :64], axis=1) + A[:, :64] * 2.0
+        ng.dot(A, B, C)
+        layer = ng.pool_layer(np.float16, "max", 64, 1, 1, 8, 8, 1, 1, 2, 2)
+        I, O = ng.empty(layer.dimI), ng.empty(layer.dimO)
+        I[:] = 3.0
+        ng.fprop_pool(layer, I, O)
+        ng.synchronize()
+        h = a[:, :64].astype(np.float32)
+        np.testing.assert_array_equal(D.get(), (h.max(axis=1, keepdims=True) + h * np.float32(2.0)).astype(np.float16))
+        ref = a.astype(np.float64) @ b.astype(np.float64)
+        np.testing.assert_allclose(C.get().astype(np.float64), ref, rtol=2.0 ** -10, atol=1e-4)
+        assert (O.get() == 3.0).all()
+    finally:
+        ng.stream = None
+        ng.synchronize()
+
+
+def test_an_axis_that_does_not_exist_is_refused_after_one_that_does(ng):
+    A, O = ng.ones((8, 16), dtype=np.float32), ng.empty((8, 1), dtype=np.float32)
+    O[:] = ng.sum(A, axis=1)
+    assert (O.get() == 16).all()
+    for axis in (257, 256 + 255, -255):      # equal to 1 or -1 in the low byte
+        with pytest.raises(Exception):
+            O[:] = ng.sum(A, axis=axis)
