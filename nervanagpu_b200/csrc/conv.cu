@@ -497,6 +497,39 @@ void set_update_groups(TcParams& p, int taps, int a_rows) {
   p.nz_out = taps;
 }
 
+// Partitions of a weight update that replaces a form with shorter sums. The error of an fp32 sum grows with
+// its length, so long ones run as up to `max_waves` waves of partitions instead of one. Exchanged operands:
+// 64 -> 64, 3x3x3, 16x56x56, 32 images 4.6e-5 off the sum in 64 bits (plain form 6.5e-5), 24 -> 16, 7x7,
+// 80x80, 96 images 1.5e-5 (1.8e-5; one wave 2.3e-5). Strided: 96 -> 72, 5x5, 51x51, 88 images 3.8e-6
+// (CUDA cores 4.9e-6; 85 k-blocks per partition 6.0e-6).
+int shorter_partitions(const DeviceCtx* c, long long tiles, int num_kb, int splits, long long out_elems, int max_waves) {
+  for (int w = 2; w <= max_waves && num_kb / splits > 64; ++w) {
+    const long long s = std::min<long long>(kMaxSplits, 1ll * w * c->sm_count / tiles);
+    if (s > splits && s * out_elems * 4 <= (256ll << 20)) splits = static_cast<int>(s);
+  }
+  return splits;
+}
+
+// Rows of one tap among the MMA columns of update_swapped: whole groups of 8, and no more than 16 boxes
+// per column tile (a lane of the producer warp loads each).
+int swap_rows(int C) { return std::max(16, (C + 7) / 8 * 8); }
+// Whether the update of a layer with few channels exchanges its operands (update_swapped). Plainly,
+// `stack` taps share the 128 rows of an MMA whose columns are the filters, and 64 columns cost what 256
+// do; exchanged, `per` taps share the 256 columns. It pays where that halves the MMAs, or with no more than
+// 64 filters takes a third of them: 64 -> 64, 3x3x3, 16x56x56, 32 images 1010 -> 724 us; 48 -> 128, 5x5,
+// 28x28, 128 images 79 -> 54; 64 -> 64, 3x3, 56x56, 128 images 103 -> 85. Otherwise the operand feed, larger
+// by the error boxes, eats the gain (64 -> 128, 3x3, 112x112, 64 images: 237 and 249 us), and so it does
+// where 16-row taps stack eight high in the plain form (16 -> 32, 5x5: 34 and 38). Small layers lose the
+// 3 us of the transposition (40 -> 48, 3x3, 14x14, 128 images: 21.5 and 23.6).
+bool wants_update_swap(const Geo& g, long long chunks) {
+  if (tuning().update_swap == 0 || g.C > 64 || g.K > kTileM) return false;
+  if (tuning().update_swap == 2) return true;    // (tests: every shape)
+  const int rows = swap_rows(g.C), taps = g.T * g.R * g.S;
+  const int stack = kTileM / rows, per = 256 / rows;
+  const int accs = (taps + stack - 1) / stack, tiles = (taps + per - 1) / per;
+  return rows > 16 && 2 * accs >= (g.K <= 64 ? 3 : 4) * tiles && (accs - tiles) * chunks > 3000;
+}
+
 // Column tile of the weight update (output channels): the smallest multiple of 64 that covers K
 // in the fewest tiles, so that K = 192 or 384 does not pay for 256-wide MMAs.
 int update_block_n(int K) {
@@ -654,21 +687,36 @@ __global__ void filter_unpack_t_kernel(Geo g, TapBlock tb, int per, int ld, cons
 }
 
 // Few filters (K <= 128) as well as few channels: the roles of the operands are exchanged, so that
-// the 128 MMA rows carry the filters and the 256 MMA columns carry the rows of several tap blocks
-// (an MMA with 64 columns costs nearly as much as one with 256). Column tile j owns tap blocks
+// the 128 MMA rows carry the filters and the 256 MMA columns carry the rows of several taps or tap
+// blocks (an MMA with 64 columns costs nearly as much as one with 256). Column tile j owns tap blocks
 // [j * per, (j + 1) * per); its B operand is their input boxes stacked, its A operand the error box.
-int update_tapblock_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, const void* I, const void* E,
-                            void* gradF, int out_f32, float alpha, cudaStream_t stream) {
+// `tb`: the tap blocks of a first layer, or single taps (bw = bh = 1) of swap_rows(C) rows each.
+int update_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, ChunkMode mode, bool phased, const void* I,
+                   const void* E, void* gradF, int out_f32, float alpha, cudaStream_t stream) {
   const int ntb = g.T * tb.nr * tb.ns;
-  const long long span = 1ll * g.M * g.P * g.Q * g.N;
+  const bool blocks = tb.bw > 1 || tb.bh > 1;
   const int per = 256 / tb.rows;
   const int tiles = (ntb + per - 1) / per;
   const int ld = tiles * 256;
-  const size_t dt_bytes = static_cast<size_t>(g.K) * ld * 4;
-  const size_t dt_off = (kMaxSplits * dt_bytes + 255) & ~size_t(255);
-  int rc = ensure_workspace(c, stream, dt_off + dt_bytes);
+  // second buffer: the gradient in tap order, then copies of the operands (the partials of the split
+  // reduction are in the first)
+  const bool blocked_i = !blocks && !phased && wants_chan_block(g.D, g.H, g.W, g.N, ntb);
+  const bool blocked_e = !blocks && wants_chan_block(g.M, g.P, g.Q, g.N, ntb);
+  const size_t dt_bytes = (static_cast<size_t>(g.K) * ld * 4 + 255) & ~size_t(255);
+  const size_t i_bytes = phased ? phase_split_bytes(g) : (blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0);
+  const size_t e_bytes = blocked_e ? chan_block_bytes(g.K, g.M, g.P, g.Q, g.N) : 0;
+  void* aux = nullptr;
+  int rc = ensure_aux(c, stream, dt_bytes + i_bytes + e_bytes, &aux);
   if (rc != NG_OK) return rc;
-  float* Dt = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(c->ws) + dt_off);
+  float* Dt = static_cast<float*>(aux);
+  void* copy_i = static_cast<uint8_t*>(aux) + dt_bytes;
+  void* copy_e = static_cast<uint8_t*>(copy_i) + i_bytes;
+  if (phased) rc = phase_split(g, I, copy_i, stream);
+  else if (blocked_i) rc = chan_block(c, stream, I, copy_i, g.C, g.D, g.H, g.W, g.N);
+  if (rc == NG_OK && blocked_e) rc = chan_block(c, stream, E, copy_e, g.K, g.M, g.P, g.Q, g.N);
+  if (rc != NG_OK) return rc;
+  if (i_bytes) I = copy_i;
+  if (e_bytes) E = copy_e;
   TcParams p = {};
   p.mode = TC_UPDATE;
   p.swap_ab = 1;
@@ -682,19 +730,22 @@ int update_tapblock_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, cons
   lay.a_box_rows = std::min(g.K, kTileM);
   lay.b_box_rows = tb.rows;
   lay.b_box_count = per;
-  p.num_kb = static_cast<int>(span / kChunk);
+  p.num_kb = g.M * g.P * row_chunks(g.N, g.Q, mode);
   tc_fill_mma(p, lay);
-  fill_taps(p, g, CH_PIXEL);
+  fill_taps(p, g, mode);
   p.R = tb.nr; p.S = tb.ns; p.RS = tb.nr * tb.ns; p.tap_w = tb.bw; p.tap_h = tb.bh;
-  fill_decode(p, g.N, g.Q, g.P, g.M, CH_PIXEL);
+  if (phased) fill_phases(p, g);
+  fill_decode(p, g.N, g.Q, g.P, g.M, mode);
   p.oob_y = g.H;
   p.C = Dt; p.Cold = nullptr; p.ldc = ld; p.c_zstride = 0;
   p.alpha = alpha; p.beta = 0.0f; p.relu = 0; p.sr_bits = 0; p.out_f32 = 1; p.vec_ok = 1;
   p.splits = choose_splits(c, p.tiles_n, p.num_kb, 1ll * g.K * ld);
+  if (!blocks) p.splits = shorter_partitions(c, tiles, p.num_kb, p.splits, 1ll * g.K * ld, 2);
   CUtensorMap mapA, mapB;
-  rc = act_map(&mapA, E, g.K, g.M, g.P, g.Q, g.N, CH_PIXEL, lay.a_box_rows);
+  rc = act_map(&mapA, E, g.K, g.M, g.P, g.Q, g.N, mode, lay.a_box_rows, blocked_e);
   if (rc != NG_OK) return rc;
-  rc = act_map_tapblock(&mapB, I, g, tb);
+  rc = blocks ? act_map_tapblock(&mapB, I, g, tb)
+              : (phased ? phase_map(&mapB, I, g, tb.rows) : act_map(&mapB, I, g.C, g.D, g.H, g.W, g.N, mode, tb.rows, blocked_i));
   if (rc != NG_OK) return rc;
   rc = tc_launch(c, mapA, mapB, p, stream);
   if (rc != NG_OK) return rc;
@@ -708,7 +759,7 @@ int update_tapblock(DeviceCtx* c, const Geo& g, const TapBlock& tb, const void* 
   const bool swap_ok = tuning().update_swap != 0;
   // (worth it when the tap blocks fill at least half of a 256-column tile)
   if (swap_ok && g.K <= kTileM && g.T * tb.nr * tb.ns * tb.rows >= 128)
-    return update_tapblock_swapped(c, g, tb, I, E, gradF, out_f32, alpha, stream);
+    return update_swapped(c, g, tb, CH_PIXEL, false, I, E, gradF, out_f32, alpha, stream);
   const int ntb = g.T * tb.nr * tb.ns;
   const long long span = 1ll * g.M * g.P * g.Q * g.N;
   // workspace: [split-K partials of the engine, at most 32 splits][Dp]
@@ -1136,6 +1187,11 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
       return NG_OK;
     }
   }
+  if (direct && wants_update_swap(g, 1ll * g.M * g.P * row_chunks(g.N, g.Q, mode))) {
+    TapBlock taps;
+    taps.bw = taps.bh = 1; taps.rows = swap_rows(g.C); taps.nr = g.R; taps.ns = g.S; taps.ok = true;
+    return update_swapped(c, g, taps, mode, phased, I, E, gradF, out_f32, alpha, stream);
+  }
   if (direct) {
     TcParams p = {};
     p.mode = TC_UPDATE;
@@ -1165,6 +1221,8 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
     p.C = gradF; p.Cold = nullptr; p.ldc = 1ll * RST * g.K; p.c_zstride = g.K;
     p.alpha = alpha; p.beta = 0.0f; p.relu = 0; p.sr_bits = 0; p.out_f32 = out_f32; p.vec_ok = 1;
     p.splits = choose_splits(c, 1ll * p.tiles_m * p.tiles_n * p.nz, p.num_kb, 1ll * g.C * g.K * RST);
+    if (phased)
+      p.splits = shorter_partitions(c, 1ll * p.tiles_m * p.tiles_n * p.nz, p.num_kb, p.splits, 1ll * g.C * g.K * RST, 4);
     CUtensorMap mapA, mapB;
     // large channel planes: the product reads copies in (z, y, chan, x, n) order
     const bool blocked_i = !phased && wants_chan_block(g.D, g.H, g.W, g.N, RST);

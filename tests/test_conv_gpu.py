@@ -372,3 +372,43 @@ def test_strided_layers_run_on_the_tensor_core_path(ng, lib, name):
     assert lib.ng_fallback_launch_count(ctypes.byref(after)) == 0
     assert after.value == before.value
     _check(cd, got, I, F, E, ref, name)
+
+
+EXCHANGED = {
+    # few channels and filters, many taps: whole and last, partly filled column tiles of taps; rows per tap
+    # that are and are not a divisor of 256; ragged image rows; a phase-split input; 3-D
+    "c64_k64_3d": (32, 64, 64, 4, 14, 14, 3, 3, 3, 1, 1, 1, 1, 1, 1),
+    "c33_k72_5x5": (64, 33, 72, 1, 12, 11, 1, 5, 5, 0, 2, 2, 1, 1, 1),
+    "c17_k128_7x7_n8": (8, 17, 128, 1, 13, 13, 1, 7, 7, 0, 3, 3, 1, 1, 1),
+    "c64_k8_3x3": (128, 64, 8, 1, 9, 9, 1, 3, 3, 0, 1, 1, 1, 1, 1),
+    "c48_k128_5x5_s2_n24": (24, 48, 128, 1, 17, 15, 1, 5, 5, 0, 2, 2, 1, 2, 2),
+    "c16_k16_1x1": (64, 16, 16, 1, 8, 8, 1, 1, 1, 0, 0, 0, 1, 1, 1),
+}
+
+
+@pytest.mark.parametrize("name", sorted(EXCHANGED))
+@pytest.mark.parametrize("half", [False, True])
+def test_update_with_exchanged_operands(ng, lib, name, half):
+    cfg = EXCHANGED[name]
+    cd = rm.ConvDims(*cfg)
+    I, F, E = _inputs(cd, 1011)
+    layer = _layer(ng, cfg, "auto")
+    dI, dE = ng.array(I), ng.array(E)
+    ref = rm.conv_update_fast(cd, I, E)
+    got = []
+    try:
+        for form in (2, 0):
+            assert lib.ng_tune(b"update_swap", form) == 0
+            dU = ng.empty(layer.dimF, dtype=np.float16 if half else np.float32)
+            ng.update_conv(layer, dI, dE, dU)
+            got.append(dU.get().astype(np.float64))
+    finally:
+        assert lib.ng_tune(b"update_swap", -1) == 0
+    # 16 2^-24 |a|_2 |b|_2 (as for the full-size layers), the norms of n values bounded by the largest;
+    # fp16 results are rounded once more
+    n = int(np.prod(cd.MPQ)) * cd.N
+    tol = 16 * 2.0 ** -24 * n * float(np.abs(I).max()) * float(np.abs(E).max())
+    if half:
+        tol = tol + 2.0 ** -11 * np.abs(ref) + 2.0 ** -25
+    for g in got:
+        assert (np.abs(g - ref) <= tol).all(), name
