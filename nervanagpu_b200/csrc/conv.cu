@@ -268,6 +268,16 @@ int filter_map(CUtensorMap* m, const void* base, const Geo& g, uint32_t box_c) {
   return make_tensor_map(m, base, dims, str, box);
 }
 
+// filter (C, T, R, S, K) with T x R x S taps seen as (k, s, r, t, c)
+int filter_map_rows(CUtensorMap* m, const void* base, int K, int S, int R, int T, int C, uint32_t box_c) {
+  const uint64_t k = 2ull * K;
+  const uint64_t dims[5] = {static_cast<uint64_t>(K), static_cast<uint64_t>(S), static_cast<uint64_t>(R),
+                            static_cast<uint64_t>(T), static_cast<uint64_t>(C)};
+  const uint64_t str[4] = {k, k * S, k * S * R, k * S * R * T};
+  const uint32_t box[5] = {kChunk, 1, 1, 1, box_c};
+  return make_tensor_map(m, base, dims, str, box);
+}
+
 // One phase of the backward pass: the taps t0 + str_d * jt, r0 + str_h * jr, s0 + str_w * js of the
 // filter, seen as (k, js, jr, jt, c)
 int filter_map_phase(CUtensorMap* m, const void* base, const Geo& g, const int first[3], const int count[3], uint32_t box_c) {
@@ -294,6 +304,53 @@ void fill_decode(TcParams& p, int N, int X, int Y, int Z, ChunkMode mode) {
   p.dec_q = mode == CH_FLAT ? 1 : X;
   p.dec_p = Y;
   p.dec_m = Z;
+}
+
+// Two image rows per tile (see kLean 3 of the kernel), or one? Both by the model of tc_pick_tile: tiles run in
+// waves of one per SM, a k-block costs the larger of its operand feed and its MMAs. (A layer of less than a
+// wave of tiles is split over the SMs in the plain form, and is not with two rows: its waves count in
+// parts there, in whole here.) `M` output channels, `a_rows` rows of A that the plain form loads, `taps`
+// filter taps in R rows, images of `rows` rows of `row_cols` columns in `planes` planes. 0 = one row, else
+// block_n, a multiple of bn_step. Measured, one row -> two: 64 -> 64, 3x3x3, 16x56x56, 32 images forward
+// 620 -> 470 us, backward 636 -> 470; 64 -> 128, 3x3, 112x112, 64 images backward 300 -> 212; 64 -> 192, 5x5,
+// 27x27, 128 images backward 95 -> 85; 3 -> 64, 11x11 stride 4, 224x224, 128 images forward 56 -> 48; 24 ->
+// 16, 7x7, 80x80, 96 images 350 -> 240 and 352 -> 263. Forced on a layer of less than a wave (48 -> 40, 3x3,
+// 30x30, 24 images, backward) 15.3 -> 17.3.
+int pick_row_stack(const DeviceCtx* c, int M, int a_rows, int taps, int R, int red_chunks, int kb_rows, int rows,
+                   long long planes, long long row_cols, float alpha, int bn_step = 64) {
+  const int mode = tuning().row_stack;
+  if (mode == 0 || tuning().lean_kernels == 0 || M > kChunk || R < 2 || rows < 2 || alpha != 1.0f) return 0;
+  const double mma = (kb_rows / 16) * 66.0 + 30.0;
+  auto best = [&](int a, long long cols, int num_kb, bool whole, int& block_n) {
+    double t_best = -1.0;
+    for (int bn = 256; bn >= 128; bn -= bn_step) {
+      const long long tiles = (cols + bn - 1) / bn, sm = c->sm_count;
+      const double waves = tiles < sm && !whole ? static_cast<double>(tiles) / sm : static_cast<double>((tiles + sm - 1) / sm);
+      const double t = waves * (num_kb * std::max((a + bn) * kb_rows * 2.0 / 100, mma) + 600.0);
+      if (t_best < 0.0 || t < t_best) { t_best = t; block_n = bn; }
+    }
+    return t_best;
+  };
+  int bn1 = 256, bn2 = 256;
+  const double one = best(a_rows, planes * rows * row_cols, taps * red_chunks, false, bn1);
+  const double two = best(2 * a_rows, planes * ((rows + 1) / 2) * row_cols, taps / R * (R + 1) * red_chunks, true, bn2);
+  return mode == 2 || two < 0.95 * one ? bn2 : 0;
+}
+// The columns of a product over pairs of image rows: `x` elements from pixel to pixel of the output, `y`
+// from row to row, `z` from plane to plane.
+void fill_row_pairs(TcParams& p, int block_n, int N, int X, int rows, long long planes, ChunkMode mode, int x,
+                    long long y, long long z) {
+  p.row_stack = 1;
+  p.block_n = block_n;
+  p.m_halves = p.tiles_m = 1;
+  p.cmap.row_chunks = row_chunks(N, X, mode);
+  p.cmap.row_len = X * N;
+  p.cmap.n = N; p.cmap.x = x; p.cmap.y = 2 * y; p.cmap.z = z;
+  p.cmap.y_count = (rows + 1) / 2;
+  p.cmap.pair_rows = rows;
+  p.N = static_cast<int>(planes * p.cmap.y_count * p.cmap.row_chunks * kChunk);
+  p.tiles_n = (p.N + block_n - 1) / block_n;
+  p.nz_out = 2;
 }
 
 int pick_kb_rows(int C) {
@@ -631,15 +688,28 @@ int fprop_tapblock(DeviceCtx* c, const Geo& g, const TapBlock& tb, const void* I
   lay.a_merge = !merge_off && g.K % kChunk == 0 && g.K > kChunk;
   lay.a_chunks = (g.K + kChunk - 1) / kChunk;
   lay.b_pair = !merge_off && g.N == 2 * kChunk && g.D == 1;
+  // (tap blocks as high as the stride: the next image row meets the same input rows one block later)
+  const int row_cols = row_chunks(g.N, g.Q, CH_PIXEL) * kChunk;
+  const int stack = g.str_h == tb.bh ? pick_row_stack(c, g.K, kChunk, ntb, tb.nr, 1, tb.rows, g.P, g.M, row_cols, alpha, lay.b_pair ? 128 : 64) : 0;
+  if (stack) {
+    fill_row_pairs(p, stack, g.N, g.Q, g.P, g.M, CH_PIXEL, g.N, 1ll * g.Q * g.N, 1ll * g.P * g.Q * g.N);
+    p.num_kb = ntb / tb.nr * (tb.nr + 1);
+    lay.a_merge = 0;
+    lay.a_chunks = 2;
+  }
   tc_fill_mma(p, lay);
   fill_taps(p, g, CH_PIXEL);
-  p.R = tb.nr; p.S = tb.ns; p.RS = tb.nr * tb.ns; p.tap_w = tb.bw; p.tap_h = tb.bh;
-  fill_decode(p, g.N, g.Q, g.P, g.M, CH_PIXEL);
+  p.R = tb.nr + (stack ? 1 : 0); p.S = tb.ns; p.RS = p.R * tb.ns; p.tap_w = tb.bw; p.tap_h = tb.bh;
+  if (stack) p.str_h = 2 * g.str_h;
+  fill_decode(p, g.N, g.Q, stack ? p.cmap.y_count : g.P, g.M, CH_PIXEL);
   p.oob_y = g.H;
-  p.C = O; p.Cold = nullptr; p.ldc = cols; p.c_zstride = 0;
+  p.C = O; p.Cold = nullptr; p.ldc = cols; p.c_zstride = stack ? 1ll * g.Q * g.N : 0;
   p.alpha = alpha; p.beta = 0.0f; p.relu = relu; p.sr_bits = 0; p.out_f32 = 0; p.vec_ok = 1;
   CUtensorMap mapA, mapB;
-  {  // packed filter seen as (k, tap block, row), or as (k_lo, row, k_hi, tap block)
+  if (stack) {
+    rc = filter_map_rows(&mapA, Fp, g.K, tb.ns, tb.nr, g.T, tb.rows, tb.rows);
+    if (rc != NG_OK) return rc;
+  } else {  // packed filter seen as (k, tap block, row), or as (k_lo, row, k_hi, tap block)
     uint64_t dims[5] = {static_cast<uint64_t>(g.K), static_cast<uint64_t>(ntb), static_cast<uint64_t>(tb.rows), 1, 1};
     uint64_t str[4];
     str[0] = 1ull * g.K * 2; str[1] = str[0] * ntb; str[2] = str[1] * tb.rows; str[3] = str[2];
@@ -933,17 +1003,26 @@ int bprop_phase(DeviceCtx* c, const Geo& g, const int first[3], ChunkMode mode, 
   p.num_kb = taps[0] * taps[1] * taps[2] * p.red_chunks;
   tc_pick_tile(c, p, cols, p.num_kb, kChunk);
   // fewer input channels than tile rows (one row tile): the filter box carries the real rows only
-  const int a_rows = p.tiles_m == 1 ? std::min(kTileM * p.m_halves, (g.C + 7) / 8 * 8) : kTileM * p.m_halves;
+  int a_rows = p.tiles_m == 1 ? std::min(kTileM * p.m_halves, (g.C + 7) / 8 * 8) : kTileM * p.m_halves;
+  const int n_taps = taps[0] * taps[1] * taps[2];
+  const int stack = pick_row_stack(c, g.C, a_rows, n_taps, taps[1], p.red_chunks, kChunk, n[1], n[0],
+                                   1ll * row_chunks(g.N, n[2], mode) * kChunk, alpha);
+  const long long out_row = 1ll * g.str_h * g.W * g.N;
+  if (stack) {
+    fill_row_pairs(p, stack, g.N, n[2], n[1], n[0], mode, g.str_w * g.N, out_row, 1ll * g.str_d * g.H * g.W * g.N);
+    p.num_kb = n_taps / taps[1] * (taps[1] + 1) * p.red_chunks;
+    lay.a_box_count = 2;
+  }
   lay.a_box_rows = a_rows;
   tc_fill_mma(p, lay);
-  p.RS = taps[1] * taps[2]; p.S = taps[2]; p.R = taps[1];
-  p.pad_d = lo[0]; p.pad_h = lo[1]; p.pad_w = lo[2];
+  p.S = taps[2]; p.R = taps[1] + (stack ? 1 : 0); p.RS = p.R * taps[2];
+  p.pad_d = lo[0]; p.pad_h = lo[1] + (stack ? 1 : 0); p.pad_w = lo[2];
   p.inner_tap = mode == CH_FLAT ? g.N : 0;
   p.x_tap = mode == CH_FLAT ? 0 : 1;
-  fill_decode(p, g.N, n[2], n[1], n[0], mode);
+  fill_decode(p, g.N, n[2], stack ? p.cmap.y_count : n[1], n[0], mode);
   p.oob_y = g.P;
   p.C = static_cast<__half*>(gradI) + ((1ll * off[0] * g.H + off[1]) * g.W + off[2]) * g.N;
-  p.Cold = nullptr; p.ldc = 1ll * g.D * g.H * g.W * g.N; p.c_zstride = 0;
+  p.Cold = nullptr; p.ldc = 1ll * g.D * g.H * g.W * g.N; p.c_zstride = stack ? out_row : 0;
   p.alpha = alpha; p.beta = 0.0f; p.relu = 0; p.sr_bits = 0; p.out_f32 = 0; p.vec_ok = 1;
   CUtensorMap mapA, mapB, mapBm;
   int rc = filter_map_phase(&mapA, F, g, first, taps, a_rows);
@@ -956,7 +1035,7 @@ int bprop_phase(DeviceCtx* c, const Geo& g, const int first[3], ChunkMode mode, 
     copied = aux;
   }
   if (blocked) E = copied;
-  p.splits = choose_splits(c, 1ll * p.tiles_m * p.tiles_n, p.num_kb, 1ll * g.C * cols, true);
+  if (!stack) p.splits = choose_splits(c, 1ll * p.tiles_m * p.tiles_n, p.num_kb, 1ll * g.C * cols, true);
   rc = act_map(&mapB, E, g.K, g.M, g.P, g.Q, g.N, mode, kChunk, blocked);
   if (rc != NG_OK) return rc;
   // the error pixels of a column tile inside one image row as one box
@@ -1068,19 +1147,28 @@ int ng_conv_fprop(const ng_conv_desc* d, const void* I, const void* F, void* O, 
   lay.a_merge = !merge_off && g.K % kChunk == 0 && g.K > kChunk &&
                 filter_map_merged(&mapA, F, g, lay.kb_rows) == NG_OK;
   lay.a_chunks = (g.K + kChunk - 1) / kChunk;
+  const int stack = g.str_h == 1 ? pick_row_stack(c, g.K, kChunk, RST, g.R, p.red_chunks, lay.kb_rows, g.P, g.M,
+                                                  1ll * row_chunks(g.N, g.Q, mode) * kChunk, alpha)
+                                 : 0;
+  if (stack) {
+    fill_row_pairs(p, stack, g.N, g.Q, g.P, g.M, mode, g.N, 1ll * g.Q * g.N, 1ll * g.P * g.Q * g.N);
+    p.num_kb = g.T * (g.R + 1) * g.S * p.red_chunks;
+    lay.a_chunks = 2;
+  }
   tc_fill_mma(p, lay);
   fill_taps(p, g, mode);
   if (phased) fill_phases(p, g);
-  fill_decode(p, g.N, g.Q, g.P, g.M, mode);
+  if (stack) { ++p.R; p.RS += g.S; p.str_h = 2; }
+  fill_decode(p, g.N, g.Q, stack ? p.cmap.y_count : g.P, g.M, mode);
   p.oob_y = g.H;
-  p.C = O; p.Cold = nullptr; p.ldc = ldo; p.c_zstride = 0;
+  p.C = O; p.Cold = nullptr; p.ldc = ldo; p.c_zstride = stack ? 1ll * g.Q * g.N : 0;
   p.alpha = alpha; p.beta = 0.0f; p.relu = relu; p.sr_bits = 0; p.out_f32 = 0; p.vec_ok = 1;
   if (!lay.a_merge) {
-    rc = filter_map(&mapA, F, g, lay.kb_rows);
+    rc = stack ? filter_map_rows(&mapA, F, g.K, g.S, g.R, g.T, g.C, lay.kb_rows) : filter_map(&mapA, F, g, lay.kb_rows);
     if (rc != NG_OK) return rc;
   }
   // few tiles (a small minibatch, e.g. the shard of one GPU): the reduction is split over the SMs too
-  p.splits = choose_splits(c, 1ll * p.tiles_m * p.tiles_n, p.num_kb, 1ll * g.K * cols, true);
+  if (!stack) p.splits = choose_splits(c, 1ll * p.tiles_m * p.tiles_n, p.num_kb, 1ll * g.K * cols, true);
   if (phased) {
     const size_t bytes = phase_split_bytes(g);
     void* copy = nullptr;

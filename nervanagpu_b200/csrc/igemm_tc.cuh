@@ -26,9 +26,12 @@ struct FastDiv {
 // Where a column of the GEMM's view of a pixel space lies in memory. Columns are numbered in 64-wide
 // chunks, `row_chunks` per image row; the first row_len elements of a row exist. row_chunks 0:
 // columns are stored as they are numbered. n 0: the rows follow one another. n > 0: the pixels
-// (n images each) are those of one phase of a strided layer, x / y / z elements apart.
+// (n images each) are those of one phase of a strided layer, x / y / z elements apart. pair_rows > 0:
+// the rows come in pairs (y elements from pair to pair), of which the second half of the last one does
+// not exist when pair_rows, the number of rows, is odd.
 struct ColumnMap {
   int row_chunks, row_len;
+  int pair_rows;
   int n, x, y_count;
   long long y, z;
   FastDiv fd_chunks, fd_n, fd_y;
@@ -52,6 +55,8 @@ struct TcParams {
   int acc_taps;        // weight update only: taps stacked along the rows of one accumulator (each
                        // `pack_rows` rows: t * pack_rows <= 128), so that a tap with few rows does
                        // not cost a whole 128-row MMA; 1 otherwise
+  int row_stack;       // forward / backward pass with at most 64 output channels: 1 = a tile's 128 rows are the
+                       // channels of two image rows (see kLean 3 of the kernel); R is then one more than the filter's
   int pack_rows;       // rows per stacked tap (= rows of one A box)
   int taps_per_z;      // weight update with groups / stacking: work item z owns output slices
                        // [z * taps_per_z, (z + 1) * taps_per_z), at most acc_groups * acc_taps of them
@@ -75,6 +80,7 @@ struct TcParams {
   uint32_t a_bytes;                // B region starts at this offset inside a stage
   int a_boxes, b_boxes;            // TMA boxes per stage per operand
   uint32_t a_box_bytes, b_box_bytes;
+  uint32_t a_box_step;             // from one A box to the next in the slot
 
   // ---- producer
   int mode;

@@ -79,7 +79,8 @@ struct Walk {
 
 // Memory offset (elements, inside a row of the output) of column `col`, a multiple of 8; false for
 // columns that pad an image row to whole chunks.
-__device__ __forceinline__ bool map_column(const ColumnMap& m, int col, long long& off) {
+// `slice`: which row of a pair.
+__device__ __forceinline__ bool map_column(const ColumnMap& m, int col, int slice, long long& off) {
   const int ch = col >> 6;
   const int r = fast_div(ch, m.fd_chunks);
   const int within = (ch - r * m.row_chunks) * kChunk + (col & (kChunk - 1));
@@ -87,8 +88,9 @@ __device__ __forceinline__ bool map_column(const ColumnMap& m, int col, long lon
   if (m.n == 0) {
     off = static_cast<long long>(r) * m.row_len + within;
   } else {
-    const int x = fast_div(within, m.fd_n), z = fast_div(r, m.fd_y);
-    off = z * m.z + (r - z * m.y_count) * m.y + static_cast<long long>(x) * m.x + (within - x * m.n);
+    const int x = fast_div(within, m.fd_n), z = fast_div(r, m.fd_y), y = r - z * m.y_count;
+    if (m.pair_rows && 2 * y + slice >= m.pair_rows) return false;
+    off = z * m.z + y * m.y + static_cast<long long>(x) * m.x + (within - x * m.n);
   }
   return true;
 }
@@ -139,7 +141,17 @@ __device__ __forceinline__ WorkItem decode_work(const TcParams& p, int w) {
 // same rounded stochastically. Called out of line, one group of eight at a time, the Philox rounds
 // were a chain of latencies that two warps per scheduler cannot hide; in line, the four groups of a
 // load interleave. 3072^3, rounded stochastically: 63.6 us before, 50 with the shorter rounding,
-// 45.7 in line (to nearest: 39.4 us).
+// 45.7 in line (to nearest: 39.4 us). 3, output stage 1 and two image rows per tile:
+//
+// Two image rows per tile (row_stack; forward and backward pass, at most 64 output channels, filters of
+// R >= 2 rows, rows of the input one apart from row to row of the output). Half of a 128-row MMA was
+// padding there, and every input row was fetched R times. Rows 0-63 of the accumulator hold the channels
+// of image row 2y, rows 64-127 those of row 2y + 1. The R + 1 input rows that the two need are walked
+// once: row i meets filter row i for the first and i - 1 for the second, the two stacked as the A operand
+// (backward pass: i - 1 and i, the error rows run the other way), so that two image rows cost R + 1 steps
+// instead of 2 R. The first and the last of them belong to one half only: the MMA leaves the lanes of the
+// other alone (a product with zeros would spread infinities beyond the filter's reach). They come last,
+// so that the first k-block may overwrite both halves.
 // kPair instances run as clusters of two CTAs on the two SMs of a pair (tcgen05 cta_group::2):
 // a work item is a tile of 256 rows, 128 in the tensor memory of each CTA; each CTA loads its own
 // 128 rows of A and its own half of the columns of B (plain TMA loads, no multicast) and the MMA,
@@ -157,6 +169,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
   const uint32_t ring_bytes = static_cast<uint32_t>(p.stages) * p.stage_bytes;
   // output staging (staged epilogue only), then the control block
   const uint32_t epi_base = smem_base + ring_bytes;
+  constexpr bool kStack = kLean == 3;
   const bool staged = kLean || p.store_staged != 0;
   const bool ragged = kMode == TC_GEMM && kLean == 0 && p.store_staged == 2;
   const uint32_t epi_bytes = staged ? kEpiStageBytes : 0u;
@@ -226,7 +239,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     const int bi = is_a ? lane : lane - p.a_boxes;
     const CUtensorMap* map = is_a ? &mapA : &mapB;
     bool merged = false;   // this item's B operand comes as one box (convolutions, see b_merge)
-    const uint32_t box_off = is_a ? bi * p.a_box_bytes : p.a_bytes + bi * p.b_box_bytes;
+    const uint32_t box_off = is_a ? bi * p.a_box_step : p.a_bytes + bi * p.b_box_bytes;
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
@@ -305,7 +318,8 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
             }
           } else if (kMode == TC_FPROP) {
             if (is_a) {  // filter rows c of tap trs, 64 output channels wide
-              if (p.a_merge) { c1 = rc * p.kb_rows; c2 = (m0 + kTileM * bi) / kChunk; c3 = trs; }
+              if (kStack) { c1 = tap.s; c2 = tap.r - bi; c3 = tap.t; c4 = rc * p.kb_rows; }   // (rows outside: zeros)
+              else if (p.a_merge) { c1 = rc * p.kb_rows; c2 = (m0 + kTileM * bi) / kChunk; c3 = trs; }
               else { c0 = m0 + kChunk * bi; c1 = trs; c2 = rc * p.kb_rows; }
             } else {     // input pixels of this chunk shifted by the tap
               c0 = cp.inner0 + ((p.phase_w > 1 ? tap.sq : tap.s) - p.pad_w) * p.inner_tap;
@@ -316,11 +330,11 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
             }
           } else if (kMode == TC_BPROP) {
             if (is_a) {  // filter rows c0.., 64 output channels k of the tap
-              c0 = rc * kChunk; c1 = tap.s; c2 = tap.r; c3 = tap.t; c4 = m0;
+              c0 = rc * kChunk; c1 = tap.s; c2 = kStack ? tap.r - 1 + bi : tap.r; c3 = tap.t; c4 = m0;
             } else {     // error pixels that reach this input pixel through the tap
               c0 = cp.inner0 + (p.x_tap ? 0 : (p.pad_w - tap.s) * p.inner_tap);
               c1 = p.x_tap ? cp.q + p.pad_w - tap.s : 0;
-              c2 = cp.valid ? cp.p + p.pad_h - tap.r : p.oob_y + kFarRows;
+              c2 = cp.valid ? cp.p * (kStack ? 2 : 1) + p.pad_h - tap.r : p.oob_y + kFarRows;
               c3 = cp.m + p.pad_d - tap.t;
               c4 = rc * kChunk;
             }
@@ -415,7 +429,9 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         // (All lanes poll: one polling lane plus a broadcast measured the same or slower.)
         int c0 = 0, c1 = 0, c2 = 0, c3 = 0, c4 = 0;
         if (linear) {
-          const int ts = phased ? wk.tap.sq : wk.tap.s, tr = wk.tap.r, tt = wk.tap.t, rc = wk.rc;
+          // (two image rows: input rows 1 to R first, then row 0)
+          const int tr = !kStack ? wk.tap.r : (wk.tap.r + 1 == p.R ? 0 : wk.tap.r + 1);
+          const int ts = phased ? wk.tap.sq : wk.tap.s, tt = wk.tap.t, rc = wk.rc;
           c0 = lb0 + ts * ls[0] + tr * lr[0] + tt * lt[0] + rc * lc[0];
           c1 = lb1 + ts * ls[1] + tr * lr[1] + tt * lt[1] + rc * lc[1];
           c2 = lb2 + ts * ls[2] + tr * lr[2] + tt * lt[2] + rc * lc[2];
@@ -550,7 +566,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         // loop, the count switch and the first-k-block test inside, the same work took the issuing
         // warp ~900 cycles per k-block of four MMAs instead of ~570 (the tensor pipe needs 512).
 #define NG_STEADY_LOOP(count, two)                                                                                  \
-  for (; ok && kb < it.kb1; ++kb) {                                                                                 \
+  for (; ok && kb < stop; ++kb) {                                                                                   \
     if (!wait_operands()) { ok = false; break; }                                                                    \
     if (issuer) {                                                                                                   \
       tc_mma_f16_run<kPair, count>(d_base, a_lo0 | sa, a_hi, b_lo0 | (sa + b_off), b_hi, idesc, 1u, a_kstep, b_kstep); \
@@ -560,7 +576,42 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     }                                                                                                               \
     release_and_step();                                                                                             \
   }
-        if (halves == 1) {
+        if (kStack) {
+          // two image rows: per filter plane the input rows that both halves need, then the last and the first
+          const int row_kb = p.S * p.red_chunks;
+          for (int stop = it.kb0; ok && stop < it.kb1;) {
+            stop += (p.R - 2) * row_kb;
+            switch (mma_per_kb) {
+              case 4: NG_STEADY_LOOP(4, false) break;
+              case 3: NG_STEADY_LOOP(3, false) break;
+              case 2: NG_STEADY_LOOP(2, false) break;
+              default: NG_STEADY_LOOP(1, false) break;
+            }
+            for (int edge = 0; edge < 2; ++edge) {
+              stop += row_kb;
+              // (forward: filter row R does not exist for the first image row, row -1 not for the second)
+              const uint32_t off_lo = (edge == 0) == (kMode == TC_FPROP) ? 0xffffffffu : 0u, off_hi = ~off_lo;
+#define NG_STACK_MMA(count) \
+  tc_mma_f16_run_half<count>(d_base, a_lo0 | sa, a_hi, b_lo0 | (sa + b_off), b_hi, idesc, off_lo, off_hi, a_kstep, b_kstep)
+              for (; ok && kb < stop; ++kb) {
+                if (!wait_operands()) { ok = false; break; }
+                if (issuer) {
+                  switch (mma_per_kb) {
+                    case 4: NG_STACK_MMA(4); break;
+                    case 3: NG_STACK_MMA(3); break;
+                    case 2: NG_STACK_MMA(2); break;
+                    default: NG_STACK_MMA(1); break;
+                  }
+                }
+                release_and_step();
+              }
+#undef NG_STACK_MMA
+            }
+          }
+        }
+        const int stop = it.kb1;
+        if (kStack) {
+        } else if (halves == 1) {
           switch (mma_per_kb) {
             case 4: NG_STEADY_LOOP(4, false) break;
             case 3: NG_STEADY_LOOP(3, false) break;
@@ -610,7 +661,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     ea.seed_lo = p.seed_lo; ea.seed_hi = p.seed_hi; ea.rng_offset = p.rng_offset;
     // the common case gets a short path of its own: the epilogue is bound by instruction latency
     // (two warps per scheduler), so every instruction fewer counts
-    const bool plain = kLean == 1 || (kLean == 0 && ea.alpha == 1.0f && ea.beta == 0.0f && ea.sr_bits == 0);
+    const bool plain = kLean == 1 || kStack || (kLean == 0 && ea.alpha == 1.0f && ea.beta == 0.0f && ea.sr_bits == 0);
     const bool wide = p.m_halves == 2;
     // two warps share each group of 32 TMEM lanes and split the columns between them
     const int col_group = (warp - 2) >> 2;
@@ -651,6 +702,12 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
             row0 = lane_group * 32 - sub_w * p.pack_rows;
             zt_warp = (sub_w < p.acc_taps && acc_first + sub_w < z_end) ? acc_first + sub_w : p.nz_out;
           }
+        }
+        if (kStack) {     // lanes 64-127 are the same channels of the next image row
+          zt = zt_warp = lane_group >> 1;
+          row0 = (lane_group & 1) * 32;
+          row = row0 + lane;
+          row_ok = row < p.M;
         }
         // whole accumulator beyond M (or beyond the last tap): nothing accumulated, nothing to store
         const bool half_live = rt * kTileM < p.M && acc_first < z_end && (!wide || h < it.live);
@@ -811,7 +868,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
               long long gcol = colb + j * (16 / esz);
               bool col_live = gcol < p.N && zt_warp < p.nz_out;
               // (convolutions: one 64-wide box is one chunk of the pixel space)
-              if (kConvOut && !partial && p.cmap.row_chunks) col_live = col_live && map_column(p.cmap, colb + j * 8, gcol);
+              if (kConvOut && !partial && p.cmap.row_chunks) col_live = col_live && map_column(p.cmap, colb + j * 8, zt_warp, gcol);
               uint8_t* gp = gbase + (row0 + (lane >> 3)) * gstride + gcol * esz;
               uint4 v[8];
 #pragma unroll
@@ -964,7 +1021,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, int splits, i
   }
   if (!live || sub != 0) return;
   long long gcol = col;      // (the partials are laid out in the padded column space, the output is not)
-  if (cmap.row_chunks && !map_column(cmap, col, gcol)) return;
+  if (cmap.row_chunks && !map_column(cmap, col, 0, gcol)) return;
   const long long off = z * c_zstride + static_cast<long long>(row) * ldc + gcol;
   const int esz = out_f32 ? 4 : 2;
   uint8_t* crow = static_cast<uint8_t*>(C) + off * esz;

@@ -91,7 +91,7 @@ void tc_fill_mma(TcParams& p, const TcOperandLayout& lay) {
     int chunks = tile_rows / kChunk;
     if (!lay.a_merge && p.m_halves == 1 && lay.a_chunks > 0) chunks = std::min(chunks, lay.a_chunks);
     p.a_boxes = lay.a_merge ? p.m_halves : chunks;
-    p.a_box_bytes = lay.a_merge ? 2u * mn_box : mn_box;
+    p.a_box_bytes = p.a_box_step = lay.a_merge ? 2u * mn_box : mn_box;
     p.a_merge = lay.a_merge;
     p.a_desc_lo = desc_lo(mn_box);
     p.a_kstep = 2048u >> 4;
@@ -99,10 +99,11 @@ void tc_fill_mma(TcParams& p, const TcOperandLayout& lay) {
   } else {
     if (p.acc_groups < 1) p.acc_groups = 1;
     if (p.acc_taps < 1) p.acc_taps = 1;
-    p.a_boxes = p.acc_groups * p.acc_taps;   // grouped update: one A box per tap of every accumulator
+    p.a_boxes = lay.a_box_count > 0 ? lay.a_box_count : p.acc_groups * p.acc_taps;   // grouped update: one A box per tap of every accumulator
     // a box may deliver fewer rows than the tile has (few-channel update): the rest of the
     // slot keeps stale data whose products land in rows that are never stored
-    p.a_box_bytes = (lay.a_box_rows ? lay.a_box_rows : tile_rows) * 128u;
+    p.a_box_bytes = p.a_box_step = (lay.a_box_rows ? lay.a_box_rows : tile_rows) * 128u;
+    if (lay.a_box_count > 0) p.a_box_step = tile_rows / lay.a_box_count * 128u;
     p.a_desc_lo = desc_lo(16);
     p.a_kstep = 32u >> 4;
     p.a_half_step = ((p.acc_groups > 1 || p.acc_taps > 1) ? p.acc_taps * p.a_box_bytes : kTileM * 128u) >> 4;
@@ -113,7 +114,7 @@ void tc_fill_mma(TcParams& p, const TcOperandLayout& lay) {
   // A slot: the rows the box delivers. When that is fewer than the MMA's 128 rows the instruction
   // also reads what follows (the B slot, the next stage, the staging area: all inside this CTA's
   // allocation); those products fall in accumulator rows that are never stored.
-  p.a_bytes = p.a_boxes * p.a_box_bytes;
+  p.a_bytes = p.a_boxes * p.a_box_step;
   if (lay.b_mn_major) {
     // one box per 64-column chunk, or (b_merge_static) one box for the whole column tile
     // (b_pair: one box per pixel, its two image groups)
@@ -314,6 +315,8 @@ int tc_launch(DeviceCtx* c, const CUtensorMap& mapA, const CUtensorMap& mapB, Tc
     NG_CUDA(cudaFuncSetAttribute(igemm_tc_kernel<TC_GEMM, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
     NG_TC_SMEM_ATTR(TC_FPROP);
     NG_TC_SMEM_ATTR(TC_BPROP);
+    NG_CUDA(cudaFuncSetAttribute(igemm_tc_kernel<TC_FPROP, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
+    NG_CUDA(cudaFuncSetAttribute(igemm_tc_kernel<TC_BPROP, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
     NG_TC_SMEM_ATTR(TC_UPDATE);
 #undef NG_TC_SMEM_ATTR
 #define NG_TC_SMEM_ATTR_PAIR(mode)                                                                                 \
@@ -348,6 +351,8 @@ int tc_launch(DeviceCtx* c, const CUtensorMap& mapA, const CUtensorMap& mapB, Tc
   p.store_staged = pick_store_mode(p);
   if (p.cmap.row_chunks && !p.store_staged)
     return fail(NG_ERR_UNSUPPORTED, "internal: padded image rows need the staged output stage");
+  if (p.row_stack && (p.store_staged != 1 || p.splits != 1 || p.alpha != 1.0f || p.tiles_m != 1 || p.m_halves != 1 || p.M > kChunk))
+    return fail(NG_ERR_INVALID_ARG, "internal: this product cannot hold two image rows per tile");
   if (!p.wait_limit_ns) p.wait_limit_ns = c->wait_limit_ns;
   const uint32_t smem = p.stages * p.stage_bytes + 1024u + kCtrlBytes + (p.store_staged ? kEpiStageBytes : 0u) +
                         a_overread(p);
@@ -412,8 +417,14 @@ int tc_launch(DeviceCtx* c, const CUtensorMap& mapA, const CUtensorMap& mapB, Tc
       if (lean_sr) NG_CUDA(cudaLaunchKernelEx(&cfg, igemm_tc_kernel<TC_GEMM, 2, false>, mapA, mapB, mapB2, launch));
       else NG_TC_LAUNCH(TC_GEMM);
       break;
-    case TC_FPROP: NG_TC_LAUNCH(TC_FPROP); break;
-    case TC_BPROP: NG_TC_LAUNCH(TC_BPROP); break;
+    case TC_FPROP:
+      if (launch.row_stack) NG_CUDA(cudaLaunchKernelEx(&cfg, igemm_tc_kernel<TC_FPROP, 3, false>, mapA, mapB, mapB2, launch));
+      else NG_TC_LAUNCH(TC_FPROP);
+      break;
+    case TC_BPROP:
+      if (launch.row_stack) NG_CUDA(cudaLaunchKernelEx(&cfg, igemm_tc_kernel<TC_BPROP, 3, false>, mapA, mapB, mapB2, launch));
+      else NG_TC_LAUNCH(TC_BPROP);
+      break;
     case TC_UPDATE: NG_TC_LAUNCH(TC_UPDATE); break;
     default: return fail(NG_ERR_INVALID_ARG, "internal: unknown tensor-core mode");
   }

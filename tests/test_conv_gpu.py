@@ -412,3 +412,59 @@ def test_update_with_exchanged_operands(ng, lib, name, half):
         tol = tol + 2.0 ** -11 * np.abs(ref) + 2.0 ** -25
     for g in got:
         assert (np.abs(g - ref) <= tol).all(), name
+
+
+ROW_PAIRS = {
+    # at most 64 output channels in one pass or both: odd and even numbers of rows, filters of two rows and
+    # more, ragged image rows, planes, phases of a strided backward pass, tap blocks, a phase-split input
+    "c64_k64_h7": (64, 64, 64, 1, 7, 9, 1, 3, 3, 0, 1, 1, 1, 1, 1),
+    "c33_k24_2x3_n8": (8, 33, 24, 1, 6, 5, 1, 2, 3, 0, 0, 1, 1, 1, 1),
+    "c16_k72_5x5_n128": (128, 16, 72, 1, 9, 8, 1, 5, 5, 0, 2, 2, 1, 1, 1),
+    "c32_k48_3d": (32, 32, 48, 3, 5, 6, 3, 3, 3, 1, 1, 1, 1, 1, 1),
+    "c130_k64_valid": (64, 130, 64, 1, 9, 9, 1, 3, 3, 0, 0, 0, 1, 1, 1),
+    "c40_k72_5x5_s2": (64, 40, 72, 1, 12, 11, 1, 5, 5, 0, 2, 2, 1, 2, 2),
+    "c40_k64_3x5_s3_n24": (24, 40, 64, 1, 11, 10, 1, 3, 5, 0, 1, 2, 1, 1, 3),
+    "c3_k64_11x11_s4_n128": (128, 3, 64, 1, 23, 23, 1, 11, 11, 0, 3, 3, 1, 4, 4),
+    "c3_k40_11x11_s4_n64": (64, 3, 40, 1, 27, 23, 1, 11, 11, 0, 3, 3, 1, 4, 4),
+}
+
+
+@pytest.mark.parametrize("name", sorted(ROW_PAIRS))
+def test_two_image_rows_per_tile(ng, lib, name):
+    cfg = ROW_PAIRS[name]
+    cd = rm.ConvDims(*cfg)
+    I, F, E = _inputs(cd, 1013)
+    ref = {"O": rm.conv_fprop_fast(cd, I, F, relu=True), "gradI": rm.conv_bprop_fast(cd, F, E),
+           "gradF": rm.conv_update_fast(cd, I, E)}
+    layer = _layer(ng, cfg, "auto")
+    # an infinity reaches the outputs under the filter and no others
+    I2, E2 = I.copy(), E.copy()
+    I2[1, 0, I.shape[2] // 2, 3, 5] = np.inf
+    E2[2, 0, E.shape[2] // 2, 1, 4] = -np.inf
+    got, finite = {}, []
+    try:
+        for form in (0, 2):
+            assert lib.ng_tune(b"row_stack", form) == 0
+            pad = 4096              # guard cells around the outputs
+            bufs = [ng.empty((n + 2 * pad,)) for n in (layer.sizeO, layer.sizeI)]
+            views = []
+            for buf, n, dim in zip(bufs, (layer.sizeO, layer.sizeI), (layer.dimO, layer.dimI)):
+                buf.fill(7.0)
+                views.append(buf[pad:pad + n].reshape(dim))
+            dU = ng.empty(layer.dimF, dtype=np.float32)
+            ng.fprop_conv(layer, ng.array(I), ng.array(F), views[0], relu=True)
+            ng.bprop_conv(layer, ng.array(F), ng.array(E), views[1])
+            ng.update_conv(layer, ng.array(I), ng.array(E), dU)
+            got = {"O": views[0].get(), "gradI": views[1].get(), "gradF": dU.get()}
+            _check(cd, got, I, F, E, ref, name)
+            for buf in bufs:
+                h = buf.get()
+                assert (h[:pad] == 7.0).all() and (h[-pad:] == 7.0).all(), name + ": wrote outside the tensor"
+            ng.fprop_conv(layer, ng.array(I2), ng.array(F), views[0])
+            ng.bprop_conv(layer, ng.array(F), ng.array(E2), views[1])
+            finite.append([np.isfinite(v.get()) for v in views])
+    finally:
+        assert lib.ng_tune(b"row_stack", -1) == 0
+    for one, two in zip(*finite):
+        assert np.array_equal(one, two), name
+        assert not one.all()
