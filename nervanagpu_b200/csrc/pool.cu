@@ -266,15 +266,21 @@ __device__ __forceinline__ ArgBytes<T> load_args(const uint8_t* p) {
   return a;
 }
 
+// The tap that a window keeps when none of its values is above the initial maximum (NaN, minus infinity, in
+// fp32 the lowest number). The general kernels keep input pixel 0, whether it lies in the window or not:
+// `none` says so, and no_tap is the tap that no gradient goes to. The unpadded fp16 windows of 2-D data keep
+// their own first tap.
+constexpr uint32_t no_tap = 255u;
+
 // Running maximum and tap of its first occurrence, per image.
 template <typename T>
 struct Best;
 template <>
 struct Best<__half> {
   uint32_t best[4], arg[4];
-  __device__ void init() {
+  __device__ void init(uint32_t tap = 0u) {   // `tap` stays where no value is above the first
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { best[i] = 0xfc00fc00u; arg[i] = 0u; }   // -inf, tap 0
+    for (int i = 0; i < 4; ++i) { best[i] = 0xfc00fc00u; arg[i] = tap * 0x00010001u; }   // -inf
   }
   __device__ void merge(int i, uint32_t v, uint32_t a) {
     const uint32_t m = __hgt2_mask(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&best[i]));
@@ -339,9 +345,9 @@ template <>
 struct Best<float> {
   float best[4];
   uint32_t arg[4];
-  __device__ void init() {
+  __device__ void init(uint32_t tap = 0u) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { best[i] = -FLT_MAX; arg[i] = 0u; }
+    for (int i = 0; i < 4; ++i) { best[i] = -FLT_MAX; arg[i] = tap; }
   }
   __device__ void take(const Vec16<float>& v, int tap) {
 #pragma unroll
@@ -389,6 +395,7 @@ struct Best<float> {
 
 struct Plane2d {
   int H, W, N, P, Q, strips;
+  int none;    // see no_tap
 };
 // thread -> (strip, pixel column, first image of its vector); false past the end
 __device__ __forceinline__ bool strip_pos(const Plane2d& g, int columns, int lanes, int& strip, int& x, int& n0) {
@@ -460,7 +467,11 @@ __global__ void __launch_bounds__(256) pool2d_fprop_kernel(Plane2d g, const T* _
 #pragma unroll
         for (int i = 0; i < V; ++i) acc[kAvg ? l : 0][i] = r == 0 ? sum[i] : acc[kAvg ? l : 0][i] + sum[i];
       } else {
-        if (r == 0) win[l].init();
+        if (r == 0) {
+          const int top = y0 + l * SH;
+          const bool has0 = blockIdx.y == 0 && top <= 0 && top + R > 0 && x0 <= 0 && x0 + S > 0;
+          win[l].init(!g.none ? 0u : (has0 ? static_cast<uint32_t>(-top * S - x0) : no_tap));
+        }
         if (kKind == P2_MAX) win[l].raise(row.value());
         else win[l].take(row, r * S);
       }
@@ -586,7 +597,7 @@ __global__ void __launch_bounds__(256) pool2d_bprop_kernel(Plane2d g, int BW, co
   const long long base = (static_cast<long long>(blockIdx.y) * g.H + a * SH) * g.W + b * SW;
   Best<T> best;
   Vec16<T> e;
-  best.init();
+  best.init(g.none && !(blockIdx.y == 0 && a == 0 && b == 0) ? no_tap : 0u);
   const bool live = a < g.P && b < g.Q;     // (a ragged border belongs to no window)
   if (live) {
     Vec16<T> raw[R * S];
@@ -621,9 +632,10 @@ __global__ void __launch_bounds__(256) pool2d_bprop_kernel(Plane2d g, int BW, co
 template <typename T, int R, int S, int SH, int SW, int PH, int PW, int LF, int LB, bool kAvg>
 int launch_pool2d_strips(const PoolGeo& g, const T* I, T* EO, T* out, int mode, uint8_t* arg, cudaStream_t stream) {
   const int nvec = g.N / Vec16<T>::kLanes, planes = g.C * g.D;
-  Plane2d f = {g.H, g.W, g.N, g.P, g.Q, (g.P + LF - 1) / LF};
+  const int none = !(sizeof(T) == 2 && g.D == 1 && PH == 0 && PW == 0);
+  Plane2d f = {g.H, g.W, g.N, g.P, g.Q, (g.P + LF - 1) / LF, none};
   const int BH = (g.H + PH + SH - 1) / SH, BW = (g.W + PW + SW - 1) / SW;
-  Plane2d b = {g.H, g.W, g.N, g.P, g.Q, (BH + LB - 1) / LB};
+  Plane2d b = {g.H, g.W, g.N, g.P, g.Q, (BH + LB - 1) / LB, none};
   auto grid = [&](int strips, int columns) {
     return dim3(static_cast<unsigned>((1ll * strips * columns * nvec + 255) / 256), planes);
   };
@@ -727,8 +739,8 @@ __device__ __forceinline__ const T* window_base(const PoolGeo& g, const T* I, ui
   return I + (((1ll * d * g.str_j * g.D + m * g.str_d) * g.H + p * g.str_h) * g.W + q * g.str_w) * g.N + n0;
 }
 template <typename T, bool kArg>
-__device__ __forceinline__ void table_max(const TapTable& taps, const T* base, Best<T>& best) {
-  best.init();
+__device__ __forceinline__ void table_max(const TapTable& taps, const T* base, uint32_t first, Best<T>& best) {
+  best.init(first);
   for (int k = 0; k < taps.n; k += 8) {
     Vec16<T> raw[8];
 #pragma unroll
@@ -748,7 +760,7 @@ __global__ void __launch_bounds__(256) pool_table_fprop_kernel(PoolGeo g, const 
   const uint32_t t = blockIdx.x * 256u + threadIdx.x;
   if (t >= total) return;
   Best<T> best;
-  table_max<T, false>(taps, window_base(g, I, t), best);
+  table_max<T, false>(taps, window_base(g, I, t), 0u, best);
   best.value().store(O + static_cast<size_t>(t) * Vec16<T>::kLanes);
 }
 // Backward pass when the windows tile the input exactly: the window's inputs are written where it
@@ -763,7 +775,7 @@ __global__ void __launch_bounds__(256) pool_table_bprop_kernel(PoolGeo g, const 
   e.load(E + static_cast<size_t>(t) * Vec16<T>::kLanes);
   const T* base = window_base(g, I, t);
   Best<T> best;
-  table_max<T, true>(taps, base, best);
+  table_max<T, true>(taps, base, base - I < g.N ? 0u : no_tap, best);
   if (mask_pos) best.drop_not_positive();
   T* out = dI + (base - I);
 #pragma unroll 4
