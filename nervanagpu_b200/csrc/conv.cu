@@ -164,42 +164,46 @@ int chan_block(DeviceCtx* c, cudaStream_t stream, const void* src, void* dst, in
 // product itself needs no other change than this walk over the taps. One read and one write of the
 // input; the CUDA-core kernels it replaces ran at 2.3 TFLOP/s: 96 -> 72 channels, 5x5 stride 2,
 // 102x102, 88 images, 100.8 -> 0.8 ms.
-int phase_row(const Geo& g) { return g.Q + (g.S - 1) / g.str_w; }       // pixels per phase of a row
-size_t phase_split_bytes(const Geo& g) {
-  return (static_cast<size_t>(2) * g.C * g.D * g.H * g.str_w * phase_row(g) * g.N + 255) & ~size_t(255);
+// The update multiplies a row's last chunk, zeros in the error tensor past the row's end, with whatever the
+// copy holds there: with ragged rows its copy has a row of Q pixels for every tap instead (`phases` = S), so
+// that a NaN or infinity meets no zero of a tap that does not reach it.
+int update_phases(const Geo& g) { return (1ll * g.Q * g.N) % kChunk == 0 ? g.str_w : std::max(g.str_w, g.S); }
+int phase_row(const Geo& g, int phases) { return g.Q + (g.S - 1) / phases; }       // pixels per phase of a row
+size_t phase_split_bytes(const Geo& g, int phases) {
+  return (static_cast<size_t>(2) * g.C * g.D * g.H * phases * phase_row(g, phases) * g.N + 255) & ~size_t(255);
 }
 // one block per (z, y, c) row
-__global__ void __launch_bounds__(128) phase_split_kernel(Geo g, int wp, const uint4* __restrict__ I, uint4* __restrict__ dst) {
+__global__ void __launch_bounds__(128) phase_split_kernel(Geo g, int phases, int wp, const uint4* __restrict__ I, uint4* __restrict__ dst) {
   const int nvec = g.N >> 3, c = blockIdx.x % g.C;
   const long long zy = blockIdx.x / g.C;
   const uint4* src = I + (1ll * c * g.D * g.H + zy) * g.W * nvec;
-  uint4* out = dst + 1ll * blockIdx.x * g.str_w * wp * nvec;
-  for (int i = threadIdx.x; i < g.str_w * wp * nvec; i += 128) {
+  uint4* out = dst + 1ll * blockIdx.x * phases * wp * nvec;
+  for (int i = threadIdx.x; i < phases * wp * nvec; i += 128) {
     const int pix = i / nvec, ph = pix / wp;
     const int x = (pix - ph * wp) * g.str_w + ph - g.pad_w;
     out[i] = x >= 0 && x < g.W ? __ldg(src + x * nvec + (i - pix * nvec)) : make_uint4(0, 0, 0, 0);
   }
 }
-int phase_split(const Geo& g, const void* I, void* dst, cudaStream_t stream) {
+int phase_split(const Geo& g, int phases, const void* I, void* dst, cudaStream_t stream) {
   const long long rows = 1ll * g.C * g.D * g.H;
   if (rows > 0x7fffffffll) return fail(NG_ERR_TOO_LARGE, "tensor too large for the phase-split copy");
-  phase_split_kernel<<<static_cast<unsigned>(rows), 128, 0, stream>>>(g, phase_row(g), static_cast<const uint4*>(I),
+  phase_split_kernel<<<static_cast<unsigned>(rows), 128, 0, stream>>>(g, phases, phase_row(g, phases), static_cast<const uint4*>(I),
                                                                       static_cast<uint4*>(dst));
   NG_CHECK_LAUNCH();
   return NG_OK;
 }
 // the copy seen as (x' n, phase, y, z, chan)
-int phase_map(CUtensorMap* m, const void* base, const Geo& g, uint32_t box_chan) {
-  const uint64_t row = 2ull * phase_row(g) * g.N;
-  const uint64_t dims[5] = {1ull * phase_row(g) * g.N, static_cast<uint64_t>(g.str_w), static_cast<uint64_t>(g.H),
+int phase_map(CUtensorMap* m, const void* base, const Geo& g, int phases, uint32_t box_chan) {
+  const uint64_t row = 2ull * phase_row(g, phases) * g.N;
+  const uint64_t dims[5] = {1ull * phase_row(g, phases) * g.N, static_cast<uint64_t>(phases), static_cast<uint64_t>(g.H),
                             static_cast<uint64_t>(g.D), static_cast<uint64_t>(g.C)};
-  const uint64_t chan = row * g.str_w;
+  const uint64_t chan = row * phases;
   const uint64_t str[4] = {row, chan * g.C, chan * g.C * g.H, chan};
   const uint32_t box[5] = {kChunk, 1, 1, 1, box_chan};
   return make_tensor_map(m, base, dims, str, box);
 }
-void fill_phases(TcParams& p, const Geo& g) {
-  p.phase_w = g.str_w;
+void fill_phases(TcParams& p, int phases) {
+  p.phase_w = phases;
   p.pad_w = 0;         // (part of the copy)
 }
 
@@ -773,7 +777,7 @@ int update_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, ChunkMode mod
   const bool blocked_i = !blocks && !phased && wants_chan_block(g.D, g.H, g.W, g.N, ntb);
   const bool blocked_e = !blocks && wants_chan_block(g.M, g.P, g.Q, g.N, ntb);
   const size_t dt_bytes = (static_cast<size_t>(g.K) * ld * 4 + 255) & ~size_t(255);
-  const size_t i_bytes = phased ? phase_split_bytes(g) : (blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0);
+  const size_t i_bytes = phased ? phase_split_bytes(g, update_phases(g)) : (blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0);
   const size_t e_bytes = blocked_e ? chan_block_bytes(g.K, g.M, g.P, g.Q, g.N) : 0;
   void* aux = nullptr;
   int rc = ensure_aux(c, stream, dt_bytes + i_bytes + e_bytes, &aux);
@@ -781,7 +785,7 @@ int update_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, ChunkMode mod
   float* Dt = static_cast<float*>(aux);
   void* copy_i = static_cast<uint8_t*>(aux) + dt_bytes;
   void* copy_e = static_cast<uint8_t*>(copy_i) + i_bytes;
-  if (phased) rc = phase_split(g, I, copy_i, stream);
+  if (phased) rc = phase_split(g, update_phases(g), I, copy_i, stream);
   else if (blocked_i) rc = chan_block(c, stream, I, copy_i, g.C, g.D, g.H, g.W, g.N);
   if (rc == NG_OK && blocked_e) rc = chan_block(c, stream, E, copy_e, g.K, g.M, g.P, g.Q, g.N);
   if (rc != NG_OK) return rc;
@@ -804,7 +808,7 @@ int update_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, ChunkMode mod
   tc_fill_mma(p, lay);
   fill_taps(p, g, mode);
   p.R = tb.nr; p.S = tb.ns; p.RS = tb.nr * tb.ns; p.tap_w = tb.bw; p.tap_h = tb.bh;
-  if (phased) fill_phases(p, g);
+  if (phased) fill_phases(p, update_phases(g));
   fill_decode(p, g.N, g.Q, g.P, g.M, mode);
   p.oob_y = g.H;
   p.C = Dt; p.Cold = nullptr; p.ldc = ld; p.c_zstride = 0;
@@ -815,7 +819,7 @@ int update_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, ChunkMode mod
   rc = act_map(&mapA, E, g.K, g.M, g.P, g.Q, g.N, mode, lay.a_box_rows, blocked_e);
   if (rc != NG_OK) return rc;
   rc = blocks ? act_map_tapblock(&mapB, I, g, tb)
-              : (phased ? phase_map(&mapB, I, g, tb.rows) : act_map(&mapB, I, g.C, g.D, g.H, g.W, g.N, mode, tb.rows, blocked_i));
+              : (phased ? phase_map(&mapB, I, g, update_phases(g), tb.rows) : act_map(&mapB, I, g.C, g.D, g.H, g.W, g.N, mode, tb.rows, blocked_i));
   if (rc != NG_OK) return rc;
   rc = tc_launch(c, mapA, mapB, p, stream);
   if (rc != NG_OK) return rc;
@@ -1157,7 +1161,7 @@ int ng_conv_fprop(const ng_conv_desc* d, const void* I, const void* F, void* O, 
   }
   tc_fill_mma(p, lay);
   fill_taps(p, g, mode);
-  if (phased) fill_phases(p, g);
+  if (phased) fill_phases(p, g.str_w);
   if (stack) { ++p.R; p.RS += g.S; p.str_h = 2; }
   fill_decode(p, g.N, g.Q, stack ? p.cmap.y_count : g.P, g.M, mode);
   p.oob_y = g.H;
@@ -1170,11 +1174,11 @@ int ng_conv_fprop(const ng_conv_desc* d, const void* I, const void* F, void* O, 
   // few tiles (a small minibatch, e.g. the shard of one GPU): the reduction is split over the SMs too
   if (!stack) p.splits = choose_splits(c, 1ll * p.tiles_m * p.tiles_n, p.num_kb, 1ll * g.K * cols, true);
   if (phased) {
-    const size_t bytes = phase_split_bytes(g);
+    const size_t bytes = phase_split_bytes(g, g.str_w);
     void* copy = nullptr;
     rc = chan_block_room(c, stream, p, &bytes, &copy, 1);
-    if (rc == NG_OK) rc = phase_split(g, I, copy, stream);
-    if (rc == NG_OK) rc = phase_map(&mapB, copy, g, lay.kb_rows);
+    if (rc == NG_OK) rc = phase_split(g, g.str_w, I, copy, stream);
+    if (rc == NG_OK) rc = phase_map(&mapB, copy, g, g.str_w, lay.kb_rows);
     if (rc != NG_OK) return rc;
     return tc_launch(c, mapA, mapB, p, stream);
   }
@@ -1303,7 +1307,7 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
     }
     tc_fill_mma(p, lay);
     fill_taps(p, g, mode);
-    if (phased) fill_phases(p, g);
+    if (phased) fill_phases(p, update_phases(g));
     fill_decode(p, g.N, g.Q, g.P, g.M, mode);
     p.oob_y = g.H;
     p.C = gradF; p.Cold = nullptr; p.ldc = 1ll * RST * g.K; p.c_zstride = g.K;
@@ -1316,18 +1320,18 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
     const bool blocked_i = !phased && wants_chan_block(g.D, g.H, g.W, g.N, RST);
     const bool blocked_e = wants_chan_block(g.M, g.P, g.Q, g.N, RST);
     if (phased || blocked_i || blocked_e) {
-      const size_t bytes[2] = {phased ? phase_split_bytes(g) : blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0,
+      const size_t bytes[2] = {phased ? phase_split_bytes(g, update_phases(g)) : blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0,
                                blocked_e ? chan_block_bytes(g.K, g.M, g.P, g.Q, g.N) : 0};
       void* copies[2] = {nullptr, nullptr};
       rc = chan_block_room(c, stream, p, bytes, copies, 2);
-      if (rc == NG_OK && phased) rc = phase_split(g, I, copies[0], stream);
+      if (rc == NG_OK && phased) rc = phase_split(g, update_phases(g), I, copies[0], stream);
       if (rc == NG_OK && blocked_i) rc = chan_block(c, stream, I, copies[0], g.C, g.D, g.H, g.W, g.N);
       if (rc == NG_OK && blocked_e) rc = chan_block(c, stream, E, copies[1], g.K, g.M, g.P, g.Q, g.N);
       if (rc != NG_OK) return rc;
       if (phased || blocked_i) I = copies[0];
       if (blocked_e) E = copies[1];
     }
-    rc = phased ? phase_map(&mapA, I, g, a_rows) : act_map(&mapA, I, g.C, g.D, g.H, g.W, g.N, mode, a_rows, blocked_i);
+    rc = phased ? phase_map(&mapA, I, g, update_phases(g), a_rows) : act_map(&mapA, I, g.C, g.D, g.H, g.W, g.N, mode, a_rows, blocked_i);
     if (rc != NG_OK) return rc;
     rc = act_map(&mapB, E, g.K, g.M, g.P, g.Q, g.N, mode, p.block_n, blocked_e);
     if (rc != NG_OK) return rc;

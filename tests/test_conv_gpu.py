@@ -468,3 +468,17 @@ def test_two_image_rows_per_tile(ng, lib, name):
     for one, two in zip(*finite):
         assert np.array_equal(one, two), name
         assert not one.all()
+
+
+@pytest.mark.parametrize("name", ["n24_5x5_s3", "n40_2x3_s3_h1", "n8_3x3_s2", "n24_odd_rows_s2"])
+def test_strided_update_keeps_nan_to_the_taps_it_meets(ng, name):
+    """Rows of no whole number of chunks: a NaN in the input reaches the taps that the oracle's reach."""
+    cfg = STRIDED.get(name, (24, 17, 24, 1, 9, 8, 1, 3, 3, 0, 1, 1, 1, 2, 2))
+    cd = rm.ConvDims(*cfg)
+    I, F, E = _inputs(cd, 1017)
+    for y, x in ((0, 0), (2, I.shape[3] - 1), (3, I.shape[3] - 2), (4, 3)):
+        I2 = I.copy()
+        I2[3, 0, y, x, 5] = np.nan
+        dU = ng.empty(cd.dimF, dtype=np.float32)
+        ng.update_conv(_layer(ng, cfg, "auto"), ng.array(I2), ng.array(E), dU)
+        assert np.array_equal(np.isnan(dU.get()), np.isnan(rm.conv_update_fast(cd, I2, E))), (name, y, x)
