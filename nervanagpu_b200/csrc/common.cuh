@@ -289,18 +289,19 @@ __device__ __forceinline__ void tc_mma_f16_run(uint32_t d_tmem, uint32_t a_lo, u
 #undef NG_MMA_STEP
 #undef NG_MMA_OP
 }
-// One k-block accumulated into some of the 128 lanes: `off_lo` / `off_hi` are the disable masks of lanes
-// 0-63 and 64-127 (all ones = leave that half of D as it is).
+// One k-block into some of the 128 lanes: `off_lo` / `off_hi` are the disable masks of lanes 0-63 and
+// 64-127 (all ones = leave that half of D as it is); the first MMA takes `accumulate`, the others add.
 template <int kCount>
 __device__ __forceinline__ void tc_mma_f16_run_half(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
                                                     uint32_t b_hi, uint32_t idesc, uint32_t off_lo, uint32_t off_hi,
-                                                    uint32_t a_kstep, uint32_t b_kstep) {
+                                                    uint32_t accumulate, uint32_t a_kstep, uint32_t b_kstep) {
 #pragma unroll
   for (int i = 0; i < kCount; ++i) {
     asm volatile(
-        "{\n .reg .pred q;\n .reg .b64 da, db;\n setp.eq.b32 q, %5, %5;\n mov.b64 da, {%1, %2};\n mov.b64 db, {%3, %4};\n"
+        "{\n .reg .pred q;\n .reg .b64 da, db;\n setp.ne.b32 q, %8, 0;\n mov.b64 da, {%1, %2};\n mov.b64 db, {%3, %4};\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, {%6, %6, %7, %7}, q;\n}\n" ::"r"(d_tmem),
-        "r"(a_lo + i * a_kstep), "r"(a_hi), "r"(b_lo + i * b_kstep), "r"(b_hi), "r"(idesc), "r"(off_lo), "r"(off_hi)
+        "r"(a_lo + i * a_kstep), "r"(a_hi), "r"(b_lo + i * b_kstep), "r"(b_hi), "r"(idesc), "r"(off_lo), "r"(off_hi),
+        "r"(i == 0 ? accumulate : 1u)
         : "memory");
   }
 }

@@ -150,8 +150,9 @@ __device__ __forceinline__ WorkItem decode_work(const TcParams& p, int w) {
 // once: row i meets filter row i for the first and i - 1 for the second, the two stacked as the A operand
 // (backward pass: i - 1 and i, the error rows run the other way), so that two image rows cost R + 1 steps
 // instead of 2 R. The first and the last of them belong to one half only: the MMA leaves the lanes of the
-// other alone (a product with zeros would spread infinities beyond the filter's reach). They come last,
-// so that the first k-block may overwrite both halves.
+// other alone (a product with zeros would spread infinities beyond the filter's reach). Each half so sums
+// its products in the order of the plain form and gives the same bits; the k-block in which the second half
+// starts is issued half by half, one that adds and one that overwrites.
 // kPair instances run as clusters of two CTAs on the two SMs of a pair (tcgen05 cta_group::2):
 // a work item is a tile of 256 rows, 128 in the tensor memory of each CTA; each CTA loads its own
 // 128 rows of A and its own half of the columns of B (plain TMA loads, no multicast) and the MMA,
@@ -429,9 +430,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         // (All lanes poll: one polling lane plus a broadcast measured the same or slower.)
         int c0 = 0, c1 = 0, c2 = 0, c3 = 0, c4 = 0;
         if (linear) {
-          // (two image rows: input rows 1 to R first, then row 0)
-          const int tr = !kStack ? wk.tap.r : (wk.tap.r + 1 == p.R ? 0 : wk.tap.r + 1);
-          const int ts = phased ? wk.tap.sq : wk.tap.s, tt = wk.tap.t, rc = wk.rc;
+          const int ts = phased ? wk.tap.sq : wk.tap.s, tr = wk.tap.r, tt = wk.tap.t, rc = wk.rc;
           c0 = lb0 + ts * ls[0] + tr * lr[0] + tt * lt[0] + rc * lc[0];
           c1 = lb1 + ts * ls[1] + tr * lr[1] + tt * lt[1] + rc * lc[1];
           c2 = lb2 + ts * ls[2] + tr * lr[2] + tt * lt[2] + rc * lc[2];
@@ -559,8 +558,10 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
           return true;
         };
         int kb = it.kb0;
-        ok = general_kb(0u);
-        ++kb;
+        if (!kStack) {
+          ok = general_kb(0u);
+          ++kb;
+        }
         // The steady state of the common tilings (one or two accumulators) runs in loops that hold
         // nothing but the wait, the MMAs of a fixed count and the commit: with the accumulator
         // loop, the count switch and the first-k-block test inside, the same work took the issuing
@@ -577,9 +578,35 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     release_and_step();                                                                                             \
   }
         if (kStack) {
-          // two image rows: per filter plane the input rows that both halves need, then the last and the first
+          // two image rows: per filter plane the input row that the first of them to start meets alone, those
+          // that both meet, then the one that is left to the other
           const int row_kb = p.S * p.red_chunks;
-          for (int stop = it.kb0; ok && stop < it.kb1;) {
+          const uint32_t first_off = kMode == TC_FPROP ? 0u : 0xffffffffu;    // lanes 0-63 off in row 0 (backward)
+#define NG_STACK_MMA(count, off_lo, accumulate) \
+  tc_mma_f16_run_half<count>(d_base, a_lo0 | sa, a_hi, b_lo0 | (sa + b_off), b_hi, idesc, off_lo, ~(off_lo), accumulate, a_kstep, b_kstep)
+#define NG_STACK_MMA_ANY(off_lo, accumulate)                     \
+  switch (mma_per_kb) {                                          \
+    case 4: NG_STACK_MMA(4, off_lo, accumulate); break;          \
+    case 3: NG_STACK_MMA(3, off_lo, accumulate); break;          \
+    case 2: NG_STACK_MMA(2, off_lo, accumulate); break;          \
+    default: NG_STACK_MMA(1, off_lo, accumulate); break;         \
+  }
+          for (int stop = it.kb0; ok && kb < it.kb1;) {
+            stop += row_kb;
+            for (; ok && kb < stop; ++kb) {
+              if (!wait_operands()) { ok = false; break; }
+              if (issuer) { NG_STACK_MMA_ANY(first_off, kb != it.kb0) }
+              release_and_step();
+            }
+            if (stop == it.kb0 + row_kb && ok) {    // the second half starts here
+              if (!wait_operands()) { ok = false; break; }
+              if (issuer) {
+                NG_STACK_MMA_ANY(first_off, 1u)
+                NG_STACK_MMA_ANY(~first_off, 0u)
+              }
+              release_and_step();
+              ++kb;
+            }
             stop += (p.R - 2) * row_kb;
             switch (mma_per_kb) {
               case 4: NG_STEADY_LOOP(4, false) break;
@@ -587,27 +614,15 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
               case 2: NG_STEADY_LOOP(2, false) break;
               default: NG_STEADY_LOOP(1, false) break;
             }
-            for (int edge = 0; edge < 2; ++edge) {
-              stop += row_kb;
-              // (forward: filter row R does not exist for the first image row, row -1 not for the second)
-              const uint32_t off_lo = (edge == 0) == (kMode == TC_FPROP) ? 0xffffffffu : 0u, off_hi = ~off_lo;
-#define NG_STACK_MMA(count) \
-  tc_mma_f16_run_half<count>(d_base, a_lo0 | sa, a_hi, b_lo0 | (sa + b_off), b_hi, idesc, off_lo, off_hi, a_kstep, b_kstep)
-              for (; ok && kb < stop; ++kb) {
-                if (!wait_operands()) { ok = false; break; }
-                if (issuer) {
-                  switch (mma_per_kb) {
-                    case 4: NG_STACK_MMA(4); break;
-                    case 3: NG_STACK_MMA(3); break;
-                    case 2: NG_STACK_MMA(2); break;
-                    default: NG_STACK_MMA(1); break;
-                  }
-                }
-                release_and_step();
-              }
-#undef NG_STACK_MMA
+            stop += row_kb;
+            for (; ok && kb < stop; ++kb) {
+              if (!wait_operands()) { ok = false; break; }
+              if (issuer) { NG_STACK_MMA_ANY(~first_off, 1u) }
+              release_and_step();
             }
           }
+#undef NG_STACK_MMA_ANY
+#undef NG_STACK_MMA
         }
         const int stop = it.kb1;
         if (kStack) {

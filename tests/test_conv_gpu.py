@@ -470,6 +470,27 @@ def test_two_image_rows_per_tile(ng, lib, name):
         assert not one.all()
 
 
+@pytest.mark.parametrize("name", sorted(ROW_PAIRS))
+def test_two_image_rows_per_tile_give_the_bits_of_one(ng, lib, name):
+    """Every output sums its products in the order of the plain form (unsplit reductions in both)."""
+    cfg = ROW_PAIRS[name]
+    cd = rm.ConvDims(*cfg)
+    rng = np.random.default_rng(1019)
+    I, F, E = (rng.normal(0, 1, dim).astype(np.float16) for dim in (cd.dimI, cd.dimF, cd.dimO))
+    layer = _layer(ng, cfg, "auto")
+    got = []
+    try:
+        assert lib.ng_tune(b"conv_splits", 1) == 0
+        for form in (0, 2):
+            assert lib.ng_tune(b"row_stack", form) == 0
+            got.append(_run_all(ng, layer, I, F, E, relu=True, ops="fb"))
+    finally:
+        assert lib.ng_tune(b"row_stack", -1) == 0
+        assert lib.ng_tune(b"conv_splits", -1) == 0
+    for key in ("O", "gradI"):
+        assert np.array_equal(got[0][key].view(np.uint16), got[1][key].view(np.uint16)), (name, key)
+
+
 @pytest.mark.parametrize("name", ["n24_5x5_s3", "n40_2x3_s3_h1", "n8_3x3_s2", "n24_odd_rows_s2"])
 def test_strided_update_keeps_nan_to_the_taps_it_meets(ng, name):
     """Rows of no whole number of chunks: a NaN in the input reaches the taps that the oracle's reach."""
