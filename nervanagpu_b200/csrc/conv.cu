@@ -772,25 +772,8 @@ int update_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, ChunkMode mod
   const int per = 256 / tb.rows;
   const int tiles = (ntb + per - 1) / per;
   const int ld = tiles * 256;
-  // second buffer: the gradient in tap order, then copies of the operands (the partials of the split
-  // reduction are in the first)
   const bool blocked_i = !blocks && !phased && wants_chan_block(g.D, g.H, g.W, g.N, ntb);
   const bool blocked_e = !blocks && wants_chan_block(g.M, g.P, g.Q, g.N, ntb);
-  const size_t dt_bytes = (static_cast<size_t>(g.K) * ld * 4 + 255) & ~size_t(255);
-  const size_t i_bytes = phased ? phase_split_bytes(g, update_phases(g)) : (blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0);
-  const size_t e_bytes = blocked_e ? chan_block_bytes(g.K, g.M, g.P, g.Q, g.N) : 0;
-  void* aux = nullptr;
-  int rc = ensure_aux(c, stream, dt_bytes + i_bytes + e_bytes, &aux);
-  if (rc != NG_OK) return rc;
-  float* Dt = static_cast<float*>(aux);
-  void* copy_i = static_cast<uint8_t*>(aux) + dt_bytes;
-  void* copy_e = static_cast<uint8_t*>(copy_i) + i_bytes;
-  if (phased) rc = phase_split(g, update_phases(g), I, copy_i, stream);
-  else if (blocked_i) rc = chan_block(c, stream, I, copy_i, g.C, g.D, g.H, g.W, g.N);
-  if (rc == NG_OK && blocked_e) rc = chan_block(c, stream, E, copy_e, g.K, g.M, g.P, g.Q, g.N);
-  if (rc != NG_OK) return rc;
-  if (i_bytes) I = copy_i;
-  if (e_bytes) E = copy_e;
   TcParams p = {};
   p.mode = TC_UPDATE;
   p.swap_ab = 1;
@@ -811,10 +794,26 @@ int update_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, ChunkMode mod
   if (phased) fill_phases(p, update_phases(g));
   fill_decode(p, g.N, g.Q, g.P, g.M, mode);
   p.oob_y = g.H;
-  p.C = Dt; p.Cold = nullptr; p.ldc = ld; p.c_zstride = 0;
+  p.Cold = nullptr; p.ldc = ld; p.c_zstride = 0;
   p.alpha = alpha; p.beta = 0.0f; p.relu = 0; p.sr_bits = 0; p.out_f32 = 1; p.vec_ok = 1;
   p.splits = choose_splits(c, p.tiles_n, p.num_kb, 1ll * g.K * ld);
   if (!blocks) p.splits = shorter_partitions(c, tiles, p.num_kb, p.splits, 1ll * g.K * ld, 2);
+  // behind the partials: the gradient in tap order and copies of the operands. (Not in the second buffer,
+  // where I and the gradient of a layer that was rewritten by space to depth lie.)
+  const size_t bytes[3] = {(static_cast<size_t>(g.K) * ld * 4 + 255) & ~size_t(255),
+                           phased ? phase_split_bytes(g, update_phases(g)) : (blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0),
+                           blocked_e ? chan_block_bytes(g.K, g.M, g.P, g.Q, g.N) : 0};
+  void* room[3] = {nullptr, nullptr, nullptr};
+  int rc = chan_block_room(c, stream, p, bytes, room, 3);
+  if (rc != NG_OK) return rc;
+  float* Dt = static_cast<float*>(room[0]);
+  p.C = Dt;
+  if (phased) rc = phase_split(g, update_phases(g), I, room[1], stream);
+  else if (blocked_i) rc = chan_block(c, stream, I, room[1], g.C, g.D, g.H, g.W, g.N);
+  if (rc == NG_OK && blocked_e) rc = chan_block(c, stream, E, room[2], g.K, g.M, g.P, g.Q, g.N);
+  if (rc != NG_OK) return rc;
+  if (bytes[1]) I = room[1];
+  if (bytes[2]) E = room[2];
   CUtensorMap mapA, mapB;
   rc = act_map(&mapA, E, g.K, g.M, g.P, g.Q, g.N, mode, lay.a_box_rows, blocked_e);
   if (rc != NG_OK) return rc;
@@ -975,7 +974,7 @@ __global__ void s2d_filter_grad_kernel(Geo g, SpaceToDepth z, const float* __res
 // `copied`: the channel-blocked copy of E, made by the first phase that wants it.
 // ------------------------------------------------------------------------------------------
 int bprop_phase(DeviceCtx* c, const Geo& g, const int first[3], ChunkMode mode, const void* F, const void* E, void* gradI,
-                float alpha, bool blocked, const void*& copied, cudaStream_t stream) {
+                float alpha, bool blocked, AuxClaim& aux, const void*& copied, cudaStream_t stream) {
   const int str[3] = {g.str_d, g.str_h, g.str_w}, flt[3] = {g.T, g.R, g.S}, pad[3] = {g.pad_d, g.pad_h, g.pad_w},
             ext[3] = {g.D, g.H, g.W};
   int taps[3], lo[3], n[3], off[3];     // taps of the phase; first x' and number of its pixels; first pixel
@@ -1032,11 +1031,11 @@ int bprop_phase(DeviceCtx* c, const Geo& g, const int first[3], ChunkMode mode, 
   int rc = filter_map_phase(&mapA, F, g, first, taps, a_rows);
   if (rc != NG_OK) return rc;
   if (blocked && !copied) {   // large channel planes: the product reads a copy in (z, y, chan, x, n) order
-    void* aux = nullptr;
-    rc = ensure_aux(c, stream, chan_block_bytes(g.K, g.M, g.P, g.Q, g.N), &aux);
-    if (rc == NG_OK) rc = chan_block(c, stream, E, aux, g.K, g.M, g.P, g.Q, g.N);
+    void* room = nullptr;
+    rc = aux.room(c, stream, chan_block_bytes(g.K, g.M, g.P, g.Q, g.N), &room);
+    if (rc == NG_OK) rc = chan_block(c, stream, E, room, g.K, g.M, g.P, g.Q, g.N);
     if (rc != NG_OK) return rc;
-    copied = aux;
+    copied = room;
   }
   if (blocked) E = copied;
   if (!stack) p.splits = choose_splits(c, 1ll * p.tiles_m * p.tiles_n, p.num_kb, 1ll * g.C * cols, true);
@@ -1085,11 +1084,12 @@ int ng_conv_fprop(const ng_conv_desc* d, const void* I, const void* F, void* O, 
     const SpaceToDepth z = pick_space_to_depth(g);
     if (z.ok) {
       const size_t i2_bytes = round256(2ull * z.C2 * z.H2 * z.W2 * g.N), f2_bytes = round256(2ull * z.C2 * z.R2 * z.S2 * g.K);
-      void* aux = nullptr;
-      rc = ensure_aux(c, stream, i2_bytes + f2_bytes, &aux);
+      AuxClaim aux;
+      void* room = nullptr;
+      rc = aux.room(c, stream, i2_bytes + f2_bytes, &room);
       if (rc != NG_OK) return rc;
-      uint4* I2 = static_cast<uint4*>(aux);
-      uint4* F2 = reinterpret_cast<uint4*>(static_cast<uint8_t*>(aux) + i2_bytes);
+      uint4* I2 = static_cast<uint4*>(room);
+      uint4* F2 = reinterpret_cast<uint4*>(static_cast<uint8_t*>(room) + i2_bytes);
       s2d_input_kernel<<<z.C2 * z.H2, 256, 0, stream>>>(g, z, static_cast<const uint4*>(I), I2);
       NG_CHECK_LAUNCH();
       s2d_filter_kernel<<<launch_1d(1ll * z.C2 * z.R2 * z.S2 * (g.K / 8), 256, c), 256, 0, stream>>>(
@@ -1111,10 +1111,11 @@ int ng_conv_fprop(const ng_conv_desc* d, const void* I, const void* F, void* O, 
     if (path == NG_PATH_IM2COL && !im2col) return fail(NG_ERR_UNSUPPORTED, "shape not addressable by the im2col path");
     if (im2col) {
       const size_t col_bytes = static_cast<size_t>(g.C) * RST * span * 2;
-      void* aux = nullptr;       // (the product keeps its partials, if any, in the workspace)
-      rc = ensure_aux(c, stream, col_bytes, &aux);
+      AuxClaim aux;              // (the product keeps its partials, if any, in the workspace)
+      void* room = nullptr;
+      rc = aux.room(c, stream, col_bytes, &room);
       if (rc != NG_OK) return rc;
-      __half* col = static_cast<__half*>(aux);
+      __half* col = static_cast<__half*>(room);
       im2col_kernel<<<im2col_grid(g), 256, 0, stream>>>(g, static_cast<const __half*>(I), col);
       NG_CHECK_LAUNCH();
       GemmCall gc = {};
@@ -1224,12 +1225,13 @@ int ng_conv_bprop(const ng_conv_desc* d, const void* F, const void* E, void* gra
   if (str[0] > flt[0] || str[1] > flt[1] || str[2] > flt[2])
     NG_CUDA(cudaMemsetAsync(gradI, 0, static_cast<size_t>(g.sizeI()) * 2, stream));
   const bool blocked = wants_chan_block(g.M, g.P, g.Q, g.N, g.T * g.R * g.S);
+  AuxClaim aux;
   const void* copied = nullptr;
   for (int pt = 0; pt < std::min(str[0], flt[0]); ++pt)
     for (int pr = 0; pr < std::min(str[1], flt[1]); ++pr)
       for (int ps = 0; ps < std::min(str[2], flt[2]); ++ps) {
         const int first[3] = {pt, pr, ps};
-        rc = bprop_phase(c, g, first, mode, F, E, gradI, alpha, blocked, copied, stream);
+        rc = bprop_phase(c, g, first, mode, F, E, gradI, alpha, blocked, aux, copied, stream);
         if (rc != NG_OK) return rc;
       }
   return NG_OK;
@@ -1264,11 +1266,12 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
     const SpaceToDepth z = pick_space_to_depth(g);   // see there
     if (z.ok) {
       const size_t i2_bytes = round256(2ull * z.C2 * z.H2 * z.W2 * g.N), g2_bytes = round256(4ull * z.C2 * z.R2 * z.S2 * g.K);
-      void* aux = nullptr;
-      rc = ensure_aux(c, stream, i2_bytes + g2_bytes, &aux);
+      AuxClaim aux;
+      void* room = nullptr;
+      rc = aux.room(c, stream, i2_bytes + g2_bytes, &room);
       if (rc != NG_OK) return rc;
-      uint4* I2 = static_cast<uint4*>(aux);
-      float* G2 = reinterpret_cast<float*>(static_cast<uint8_t*>(aux) + i2_bytes);
+      uint4* I2 = static_cast<uint4*>(room);
+      float* G2 = reinterpret_cast<float*>(static_cast<uint8_t*>(room) + i2_bytes);
       s2d_input_kernel<<<z.C2 * z.H2, 256, 0, stream>>>(g, z, static_cast<const uint4*>(I), I2);
       NG_CHECK_LAUNCH();
       const ng_conv_desc d2 = space_to_depth_desc(g, z);

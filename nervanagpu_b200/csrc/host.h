@@ -25,7 +25,7 @@ struct DeviceCtx {
   };
   std::map<cudaStream_t, Scratch> scratch;
   // second buffer per stream, for operands that a call re-lays-out before it hands them to another
-  // entry point of the library (which uses the first buffer as it likes)
+  // entry point of the library (which uses the first buffer as it likes); see AuxClaim
   std::map<cudaStream_t, Scratch> aux;
   float* ws = nullptr;
   size_t ws_bytes = 0;
@@ -82,7 +82,20 @@ DeviceCtx* current_ctx();
 // Ensure the workspace of `stream` holds at least `bytes` and make c->ws point at it; may
 // synchronise the device when it has to grow.
 int ensure_workspace(DeviceCtx* c, cudaStream_t stream, size_t bytes);
-int ensure_aux(DeviceCtx* c, cudaStream_t stream, size_t bytes, void** ptr);
+// Hold on the second buffer of a stream, for as long as what lies in it is needed. It has one holder: a call
+// that an outer call of the same thread makes meanwhile is refused room there (growing would free the
+// outer call's operands, and what fits would be laid over them).
+class AuxClaim {
+ public:
+  AuxClaim() = default;
+  AuxClaim(const AuxClaim&) = delete;
+  AuxClaim& operator=(const AuxClaim&) = delete;
+  ~AuxClaim();
+  int room(DeviceCtx* c, cudaStream_t stream, size_t bytes, void** ptr);
+
+ private:
+  bool held_ = false;
+};
 
 // Rank-5 tiled tensor map over fp16 (elem_bytes 2) data. dims[0] is the contiguous dimension;
 // strides_bytes[i] is the byte stride of dims[i+1]. Swizzle is chosen from the inner box width.

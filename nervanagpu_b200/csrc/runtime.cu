@@ -143,12 +143,21 @@ int ensure_workspace(DeviceCtx* c, cudaStream_t stream, size_t bytes) {
   return NG_OK;
 }
 
-int ensure_aux(DeviceCtx* c, cudaStream_t stream, size_t bytes, void** ptr) {
+// (one call works on one stream, so a thread holds at most one)
+static thread_local bool t_aux_held = false;
+
+int AuxClaim::room(DeviceCtx* c, cudaStream_t stream, size_t bytes, void** ptr) {
+  if (t_aux_held) return fail(NG_ERR_UNSUPPORTED, "internal: an outer call holds the stream's second scratch buffer");
   DeviceCtx::Scratch& s = c->aux[stream];
   const int rc = grow_scratch(c, s, bytes);
   if (rc != NG_OK) return rc;
+  t_aux_held = held_ = true;
   *ptr = s.ptr;
   return NG_OK;
+}
+
+AuxClaim::~AuxClaim() {
+  if (held_) t_aux_held = false;
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

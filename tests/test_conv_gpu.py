@@ -203,6 +203,36 @@ def test_strided_first_layers_of_small_minibatches_run_as_space_to_depth(ng, lib
     assert_close(dU.get(), ref["gradF"], f32_tol(aU, M * P * Q * cd.N) + 2.0 ** -11 * np.abs(ref["gradF"]), name + " fp16 dW")
 
 
+@pytest.mark.parametrize("name", sorted(STRIDED_FIRST_LAYERS))
+@pytest.mark.parametrize("warm", [False, True])
+def test_space_to_depth_update_with_exchanged_operands_and_copies(ng, lib, name, warm):
+    """The update of the rewritten layer in its exchanged form, with channel-blocked copies of its operands: its
+    scratch and the outer call's must not share memory, on a stream without scratch buffers and on one whose
+    buffers are large already."""
+    cfg = STRIDED_FIRST_LAYERS[name]
+    cd = rm.ConvDims(*cfg)
+    I, F, E = _inputs(cd, 1021)
+    ref = {"O": rm.conv_fprop_fast(cd, I, F), "gradF": rm.conv_update_fast(cd, I, E)}
+    layer = _layer(ng, cfg)
+    dI, dF, dE, dO, dU = ng.array(I), ng.array(F), ng.array(E), ng.empty(layer.dimO), ng.empty(layer.dimF, dtype=np.float32)
+    ng.synchronize()
+    default, ng.stream = ng.stream, ng.new_stream()
+    try:
+        for key in (b"update_swap", b"chan_block"):
+            assert lib.ng_tune(key, 2) == 0
+        for _ in range(3 if warm else 1):
+            dU.fill(0.0)
+            ng.update_conv(layer, dI, dE, dU)
+            ng.fprop_conv(layer, dI, dF, dO)
+        ng.synchronize()
+        got = {"O": dO.get(), "gradF": dU.get()}
+    finally:
+        for key in (b"update_swap", b"chan_block"):
+            assert lib.ng_tune(key, -1) == 0
+        ng.stream = default
+    _check(cd, got, I, F, E, ref, name)
+
+
 @pytest.mark.parametrize("name", sorted(SHARDED))
 def test_sharded_minibatch_shapes_run_on_the_tensor_core_path(ng, name):
     cfg = SHARDED[name]
