@@ -971,10 +971,11 @@ __global__ void s2d_filter_grad_kernel(Geo g, SpaceToDepth z, const float* __res
 // a unit-stride layer over the phase's share of the taps, whose outputs are stored every st-th pixel
 // (ColumnMap). A unit-stride layer is its only phase. (Issuing every tap for every pixel and letting
 // the copy engine fill zeros where the stride does not divide took st^2 times the operands and MMAs.)
-// `copied`: the channel-blocked copy of E, made by the first phase that wants it.
+// `blocked`: E is its channel-blocked copy. `partials`, if given, is raised to the bytes of the phase's split
+// partials, and nothing is launched.
 // ------------------------------------------------------------------------------------------
 int bprop_phase(DeviceCtx* c, const Geo& g, const int first[3], ChunkMode mode, const void* F, const void* E, void* gradI,
-                float alpha, bool blocked, AuxClaim& aux, const void*& copied, cudaStream_t stream) {
+                float alpha, bool blocked, size_t* partials, cudaStream_t stream) {
   const int str[3] = {g.str_d, g.str_h, g.str_w}, flt[3] = {g.T, g.R, g.S}, pad[3] = {g.pad_d, g.pad_h, g.pad_w},
             ext[3] = {g.D, g.H, g.W};
   int taps[3], lo[3], n[3], off[3];     // taps of the phase; first x' and number of its pixels; first pixel
@@ -1027,18 +1028,14 @@ int bprop_phase(DeviceCtx* c, const Geo& g, const int first[3], ChunkMode mode, 
   p.C = static_cast<__half*>(gradI) + ((1ll * off[0] * g.H + off[1]) * g.W + off[2]) * g.N;
   p.Cold = nullptr; p.ldc = 1ll * g.D * g.H * g.W * g.N; p.c_zstride = stack ? out_row : 0;
   p.alpha = alpha; p.beta = 0.0f; p.relu = 0; p.sr_bits = 0; p.out_f32 = 0; p.vec_ok = 1;
+  if (!stack) p.splits = choose_splits(c, 1ll * p.tiles_m * p.tiles_n, p.num_kb, 1ll * g.C * cols, true);
+  if (partials) {
+    if (p.splits > 1) *partials = std::max(*partials, static_cast<size_t>(p.splits) * p.M * p.N * sizeof(float));
+    return NG_OK;
+  }
   CUtensorMap mapA, mapB, mapBm;
   int rc = filter_map_phase(&mapA, F, g, first, taps, a_rows);
   if (rc != NG_OK) return rc;
-  if (blocked && !copied) {   // large channel planes: the product reads a copy in (z, y, chan, x, n) order
-    void* room = nullptr;
-    rc = aux.room(c, stream, chan_block_bytes(g.K, g.M, g.P, g.Q, g.N), &room);
-    if (rc == NG_OK) rc = chan_block(c, stream, E, room, g.K, g.M, g.P, g.Q, g.N);
-    if (rc != NG_OK) return rc;
-    copied = room;
-  }
-  if (blocked) E = copied;
-  if (!stack) p.splits = choose_splits(c, 1ll * p.tiles_m * p.tiles_n, p.num_kb, 1ll * g.C * cols, true);
   rc = act_map(&mapB, E, g.K, g.M, g.P, g.Q, g.N, mode, kChunk, blocked);
   if (rc != NG_OK) return rc;
   // the error pixels of a column tile inside one image row as one box
@@ -1225,16 +1222,29 @@ int ng_conv_bprop(const ng_conv_desc* d, const void* F, const void* E, void* gra
   if (str[0] > flt[0] || str[1] > flt[1] || str[2] > flt[2])
     NG_CUDA(cudaMemsetAsync(gradI, 0, static_cast<size_t>(g.sizeI()) * 2, stream));
   const bool blocked = wants_chan_block(g.M, g.P, g.Q, g.N, g.T * g.R * g.S);
-  AuxClaim aux;
-  const void* copied = nullptr;
-  for (int pt = 0; pt < std::min(str[0], flt[0]); ++pt)
-    for (int pr = 0; pr < std::min(str[1], flt[1]); ++pr)
-      for (int ps = 0; ps < std::min(str[2], flt[2]); ++ps) {
-        const int first[3] = {pt, pr, ps};
-        rc = bprop_phase(c, g, first, mode, F, E, gradI, alpha, blocked, aux, copied, stream);
-        if (rc != NG_OK) return rc;
-      }
-  return NG_OK;
+  auto phases = [&](size_t* partials) -> int {
+    for (int pt = 0; pt < std::min(str[0], flt[0]); ++pt)
+      for (int pr = 0; pr < std::min(str[1], flt[1]); ++pr)
+        for (int ps = 0; ps < std::min(str[2], flt[2]); ++ps) {
+          const int first[3] = {pt, pr, ps};
+          const int rc = bprop_phase(c, g, first, mode, F, E, gradI, alpha, blocked, partials, stream);
+          if (rc != NG_OK) return rc;
+        }
+    return NG_OK;
+  };
+  if (blocked) {   // large channel planes: the products read a copy in (z, y, chan, x, n) order, behind their partials
+    size_t off = 0;
+    rc = phases(&off);
+    if (rc != NG_OK) return rc;
+    off = round256(off);
+    rc = ensure_workspace(c, stream, off + chan_block_bytes(g.K, g.M, g.P, g.Q, g.N));
+    if (rc != NG_OK) return rc;
+    void* copy = reinterpret_cast<uint8_t*>(c->ws) + off;
+    rc = chan_block(c, stream, E, copy, g.K, g.M, g.P, g.Q, g.N);
+    if (rc != NG_OK) return rc;
+    E = copy;
+  }
+  return phases(nullptr);
 }
 
 int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gradF, int out_f32, float alpha,

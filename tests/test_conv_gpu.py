@@ -533,3 +533,30 @@ def test_strided_update_keeps_nan_to_the_taps_it_meets(ng, name):
         dU = ng.empty(cd.dimF, dtype=np.float32)
         ng.update_conv(_layer(ng, cfg, "auto"), ng.array(I2), ng.array(E), dU)
         assert np.array_equal(np.isnan(dU.get()), np.isnan(rm.conv_update_fast(cd, I2, E))), (name, y, x)
+
+
+def test_operand_copies_of_all_passes_share_one_scratch_buffer(ng, lib):
+    """Channel-blocked copies: a pass finds room in the buffer that the pass before it left."""
+    import ctypes
+    layer = _layer(ng, (32, 64, 64, 8, 28, 28, 3, 3, 3, 1, 1, 1, 1, 1, 1))
+    copy_bytes = 2 * layer.sizeI                  # 26 MB; the error tensor has the same size
+    I, F, E = ng.zeros(layer.dimI), ng.zeros(layer.dimF), ng.zeros(layer.dimO)
+    O, gI, gF = ng.empty(layer.dimO), ng.empty(layer.dimI), ng.empty(layer.dimF, dtype=np.float32)
+
+    def free():
+        ng.synchronize()
+        f, t = ctypes.c_size_t(0), ctypes.c_size_t(0)
+        assert lib.ng_mem_info(ctypes.byref(f), ctypes.byref(t)) == 0
+        return f.value
+    ng.synchronize()
+    default, ng.stream = ng.stream, ng.new_stream()
+    try:
+        assert lib.ng_tune(b"chan_block", 2) == 0
+        ng.update_conv(layer, I, E, gF)           # copies of both operands
+        before = free()
+        ng.fprop_conv(layer, I, F, O)
+        ng.bprop_conv(layer, F, E, gI)
+        assert before - free() < copy_bytes // 2
+    finally:
+        assert lib.ng_tune(b"chan_block", -1) == 0
+        ng.stream = default
