@@ -193,8 +193,8 @@ __global__ void pool_gather_kernel(PoolGeo g, const int* __restrict__ arg, const
 // its windows share is read and reduced along x once: with one output per thread a 3x3 stride-1
 // window fetches every input nine times through L1, with strips of four rows 4.5 times, and takes
 // nine compares per output instead of six. Measured (fp16, forward / backward, before -> now):
-// 3x3/1 pad 1 on 192 x 28 x 28 x 128: 63.7 -> 18.7 us (4.1 TB/s) / 236 -> 85 us; 3x3/2 on
-// 64 x 55 x 55 x 128: 16.9 -> 10.2 us (6.0 TB/s); 2x2/2 on 64 x 224 x 224 x 64 backward without a
+// 3x3/1 pad 1 on 192 x 28 x 28 x 128: 63.7 -> 22.7 us (3.4 TB/s) / 236 -> 85 us; 3x3/2 on
+// 64 x 55 x 55 x 128: 16.9 -> 10.4 us (5.9 TB/s); 2x2/2 on 64 x 224 x 224 x 64 backward without a
 // record: 164 -> 136 us (6.8 TB/s, HBM bound); 2x2/2 fp32 on 50 x 107 x 107 x 112: 78 -> 47 us /
 // 363 -> 87 us (6.7 TB/s). The 3x3/1 backward pass is bound by its compares: every input is tested
 // against the records of nine windows (strips of 1, 2, 3, 4 rows: 90, 85, 92, 88 us).
@@ -291,11 +291,13 @@ struct Best<__half> {
 #pragma unroll
     for (int i = 0; i < 4; ++i) merge(i, v.w[i], static_cast<uint32_t>(tap) * 0x00010001u);
   }
-  __device__ void raise(const Vec16<__half>& v) {   // the maximum without its tap
+  // The maximum without its tap. (__hmax2 ranks -0 below +0, of which the first is wanted; with it the padded 3x3
+  // windows took 18.7 us at stride 1 and 10.5 at stride 2, on 192 x 28 x 28 x 128, instead of 22.7 and 12.5.)
+  __device__ void raise(const Vec16<__half>& v) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const __half2 h = __hmax2(*reinterpret_cast<const __half2*>(&best[i]), *reinterpret_cast<const __half2*>(&v.w[i]));
-      best[i] = *reinterpret_cast<const uint32_t*>(&h);
+      const uint32_t m = __hgt2_mask(*reinterpret_cast<const __half2*>(&v.w[i]), *reinterpret_cast<const __half2*>(&best[i]));
+      best[i] = (v.w[i] & m) | (best[i] & ~m);
     }
   }
   __device__ void take(const Best<__half>& row, int tap) {   // the row's taps start at `tap`

@@ -231,3 +231,29 @@ def test_windows_without_a_largest_value(ng, dtype, kind, shape):
         got.append((O.get(), B.get()))
     for a, b in zip(*got):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [np.float16, np.float32])
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("shape", [(3, 2, 0, 1), (2, 2, 0, 1), (3, 1, 1, 1), (3, 3, 0, 1), (3, 2, 1, 1), (2, 2, 0, 2)])
+def test_zeros_of_both_signs_keep_the_first(ng, dtype, shift, shape):
+    """-0 and +0 are equal: the first of a window's largest values is stored, sign included, by the
+    vectorised kernels and (tensors one element off a 16-byte boundary) by the general ones."""
+    R, st, pad, T = shape
+    rng = np.random.default_rng(6)
+    L = ng.pool_layer(dtype, "max", 16, 3, 4 if T == 2 else 1, 9, 9, 1, T, R, R, 0, 0, pad, pad, 1, T, st, st)
+    x = rng.choice(np.array([-0.0, 0.0, -1.0], dtype), L.dimI)
+    C, D, H, W, N = L.dimI
+    K, M, P, Q, _ = L.dimO
+    padded = np.full((C, D, H + 2 * pad + st, W + 2 * pad + st, N), -np.inf, dtype)
+    padded[:, :, pad:pad + H, pad:pad + W] = x
+    taps = np.stack([padded[:, t::T, r:r + P * st:st, s:s + Q * st:st][:, :M, :P, :Q]
+                     for t in range(T) for r in range(R) for s in range(R)])
+    ref = np.take_along_axis(taps, taps.argmax(axis=0)[None], axis=0)[0]     # (argmax: the first of equal values)
+    assert (np.signbit(ref) & (ref == 0)).any() and (~np.signbit(ref) & (ref == 0)).any()
+    n_in, n_out = int(np.prod(L.dimI)), int(np.prod(L.dimO))
+    I = ng.empty((n_in + 8,), dtype=dtype)[shift:shift + n_in].reshape(L.dimI).set(x)
+    O = ng.empty((n_out + 8,), dtype=dtype)[shift:shift + n_out].reshape(L.dimO)
+    ng.fprop_pool(L, I, O)
+    bits = np.uint16 if dtype is np.float16 else np.uint32
+    assert np.array_equal(O.get().view(bits), ref.view(bits))
