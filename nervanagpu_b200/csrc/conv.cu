@@ -164,46 +164,70 @@ int chan_block(DeviceCtx* c, cudaStream_t stream, const void* src, void* dst, in
 // product itself needs no other change than this walk over the taps. One read and one write of the
 // input; the CUDA-core kernels it replaces ran at 2.3 TFLOP/s: 96 -> 72 channels, 5x5 stride 2,
 // 102x102, 88 images, 100.8 -> 0.8 ms.
-// The update multiplies a row's last chunk, zeros in the error tensor past the row's end, with whatever the
-// copy holds there: with ragged rows its copy has a row of Q pixels for every tap instead (`phases` = S), so
-// that a NaN or infinity meets no zero of a tap that does not reach it.
-int update_phases(const Geo& g) { return (1ll * g.Q * g.N) % kChunk == 0 ? g.str_w : std::max(g.str_w, g.S); }
-int phase_row(const Geo& g, int phases) { return g.Q + (g.S - 1) / phases; }       // pixels per phase of a row
-size_t phase_split_bytes(const Geo& g, int phases) {
-  return (static_cast<size_t>(2) * g.C * g.D * g.H * phases * phase_row(g, phases) * g.N + 255) & ~size_t(255);
+// The CUDA-core kernels skip the taps that fall outside the tensor; here they meet zeros, and a product of zero
+// and an infinity or NaN is NaN. Where that can show, the CUDA-core kernel runs once more over the result:
+// forward and backward when a filter value is not finite (nonfinite_scan), and for the elements of a weight
+// gradient that are NaN (conv_update_redo; its errors meet padding pixels, its last chunk of a row the pixels
+// that follow the row's last output).
+int phase_row(const Geo& g) { return g.Q + (g.S - 1) / g.str_w; }       // pixels per phase of a row
+size_t phase_split_bytes(const Geo& g) {
+  return (static_cast<size_t>(2) * g.C * g.D * g.H * g.str_w * phase_row(g) * g.N + 255) & ~size_t(255);
 }
-// one block per (z, y, c) row
-__global__ void __launch_bounds__(128) phase_split_kernel(Geo g, int phases, int wp, const uint4* __restrict__ I, uint4* __restrict__ dst) {
+constexpr int kScanFlags = 128;      // blocks that scan a filter, each with a flag of its own (at most a block's threads)
+// Whether this block's share of `n` vectors of eight values holds an infinity or NaN, in flags[blockIdx.x]
+__device__ __forceinline__ void scan_share(const uint4* F, long long n, int blocks, int* flags) {
+  int found = 0;
+  for (long long i = blockIdx.x * 1ll * blockDim.x + threadIdx.x; i < n; i += 1ll * blocks * blockDim.x) {
+    const uint4 v = __ldg(F + i);
+    found |= __vcmpeq2(v.x & 0x7c007c00u, 0x7c007c00u) | __vcmpeq2(v.y & 0x7c007c00u, 0x7c007c00u) |
+             __vcmpeq2(v.z & 0x7c007c00u, 0x7c007c00u) | __vcmpeq2(v.w & 0x7c007c00u, 0x7c007c00u);
+  }
+  found = __syncthreads_or(found);
+  if (threadIdx.x == 0) flags[blockIdx.x] = found;
+}
+__global__ void __launch_bounds__(256) nonfinite_scan(const uint4* __restrict__ F, long long n, int* flags) {
+  grid_dependency_wait();
+  grid_launch_dependents();   // (the product sets itself up meanwhile)
+  scan_share(F, n, gridDim.x, flags);
+}
+// one block per (z, y, c) row; the first `scans` of them also scan the filter (n_filter vectors)
+__global__ void __launch_bounds__(128) phase_split_kernel(Geo g, int wp, const uint4* __restrict__ I, uint4* __restrict__ dst,
+                                                          const uint4* __restrict__ F, long long n_filter, int scans, int* flags) {
   const int nvec = g.N >> 3, c = blockIdx.x % g.C;
   const long long zy = blockIdx.x / g.C;
   const uint4* src = I + (1ll * c * g.D * g.H + zy) * g.W * nvec;
-  uint4* out = dst + 1ll * blockIdx.x * phases * wp * nvec;
-  for (int i = threadIdx.x; i < phases * wp * nvec; i += 128) {
+  uint4* out = dst + 1ll * blockIdx.x * g.str_w * wp * nvec;
+  for (int i = threadIdx.x; i < g.str_w * wp * nvec; i += 128) {
     const int pix = i / nvec, ph = pix / wp;
     const int x = (pix - ph * wp) * g.str_w + ph - g.pad_w;
     out[i] = x >= 0 && x < g.W ? __ldg(src + x * nvec + (i - pix * nvec)) : make_uint4(0, 0, 0, 0);
   }
+  if (blockIdx.x < scans) scan_share(F, n_filter, scans, flags);
 }
-int phase_split(const Geo& g, int phases, const void* I, void* dst, cudaStream_t stream) {
+// F and flags (kScanFlags ints, of which `scans` are set) may be null
+int phase_split(const Geo& g, const void* I, void* dst, const void* F, int* flags, int* scans, cudaStream_t stream) {
   const long long rows = 1ll * g.C * g.D * g.H;
   if (rows > 0x7fffffffll) return fail(NG_ERR_TOO_LARGE, "tensor too large for the phase-split copy");
-  phase_split_kernel<<<static_cast<unsigned>(rows), 128, 0, stream>>>(g, phases, phase_row(g, phases), static_cast<const uint4*>(I),
-                                                                      static_cast<uint4*>(dst));
+  const int n = F ? static_cast<int>(std::min<long long>(rows, kScanFlags)) : 0;
+  if (scans) *scans = n;
+  phase_split_kernel<<<static_cast<unsigned>(rows), 128, 0, stream>>>(g, phase_row(g), static_cast<const uint4*>(I),
+                                                                      static_cast<uint4*>(dst), static_cast<const uint4*>(F),
+                                                                      g.sizeF() / 8, n, flags);
   NG_CHECK_LAUNCH();
   return NG_OK;
 }
 // the copy seen as (x' n, phase, y, z, chan)
-int phase_map(CUtensorMap* m, const void* base, const Geo& g, int phases, uint32_t box_chan) {
-  const uint64_t row = 2ull * phase_row(g, phases) * g.N;
-  const uint64_t dims[5] = {1ull * phase_row(g, phases) * g.N, static_cast<uint64_t>(phases), static_cast<uint64_t>(g.H),
+int phase_map(CUtensorMap* m, const void* base, const Geo& g, uint32_t box_chan) {
+  const uint64_t row = 2ull * phase_row(g) * g.N;
+  const uint64_t dims[5] = {1ull * phase_row(g) * g.N, static_cast<uint64_t>(g.str_w), static_cast<uint64_t>(g.H),
                             static_cast<uint64_t>(g.D), static_cast<uint64_t>(g.C)};
-  const uint64_t chan = row * phases;
+  const uint64_t chan = row * g.str_w;
   const uint64_t str[4] = {row, chan * g.C, chan * g.C * g.H, chan};
   const uint32_t box[5] = {kChunk, 1, 1, 1, box_chan};
   return make_tensor_map(m, base, dims, str, box);
 }
-void fill_phases(TcParams& p, int phases) {
-  p.phase_w = phases;
+void fill_phases(TcParams& p, const Geo& g) {
+  p.phase_w = g.str_w;
   p.pad_w = 0;         // (part of the copy)
 }
 
@@ -371,8 +395,15 @@ int pick_kb_rows(int C) {
 // ------------------------------------------------------------------------------------------
 // SIMT fall-backs (one thread per output element, fp32 accumulation)
 // ------------------------------------------------------------------------------------------
+// With flags (see phase_split): whether the result stands, after a wait for the kernel that made it
+__device__ __forceinline__ bool skip_unflagged(const int* flags, int n) {
+  if (!flags) return false;
+  grid_dependency_wait();
+  return !__syncthreads_or(threadIdx.x < n && flags[threadIdx.x] != 0);
+}
 __global__ void conv_fprop_simt(Geo g, const __half* __restrict__ I, const __half* __restrict__ F, __half* O,
-                                float alpha, int relu) {
+                                float alpha, int relu, const int* flags, int n_flags) {
+  if (skip_unflagged(flags, n_flags)) return;
   const long long total = g.sizeO();
   for (long long i = blockIdx.x * 1ll * blockDim.x + threadIdx.x; i < total; i += 1ll * gridDim.x * blockDim.x) {
     long long r = i;
@@ -405,7 +436,8 @@ __global__ void conv_fprop_simt(Geo g, const __half* __restrict__ I, const __hal
 }
 
 __global__ void conv_bprop_simt(Geo g, const __half* __restrict__ F, const __half* __restrict__ E, __half* dI,
-                                float alpha) {
+                                float alpha, const int* flags, int n_flags) {
+  if (skip_unflagged(flags, n_flags)) return;
   const long long total = g.sizeI();
   for (long long i = blockIdx.x * 1ll * blockDim.x + threadIdx.x; i < total; i += 1ll * gridDim.x * blockDim.x) {
     long long r = i;
@@ -442,43 +474,82 @@ __global__ void conv_bprop_simt(Geo g, const __half* __restrict__ F, const __hal
   }
 }
 
-// one warp per filter element: lanes stride over (pixel, n), shuffle reduction
+// one filter element by a whole warp: lanes stride over (pixel, n), shuffle reduction
+__device__ __forceinline__ void update_element(const Geo& g, const __half* __restrict__ I, const __half* __restrict__ E,
+                                               void* dF, int out_f32, float alpha, long long i, int lane) {
+  long long r = i;
+  const int k = r % g.K; r /= g.K;
+  const int s = r % g.S; r /= g.S;
+  const int rr = r % g.R; r /= g.R;
+  const int t = r % g.T; r /= g.T;
+  const int c = static_cast<int>(r);
+  float acc = 0.0f;
+  const long long span = 1ll * g.M * g.P * g.Q * g.N;
+  for (long long j = lane; j < span; j += 32) {
+    long long rj = j;
+    const int n = rj % g.N; rj /= g.N;
+    const int q = rj % g.Q; rj /= g.Q;
+    const int p = rj % g.P; rj /= g.P;
+    const int m = static_cast<int>(rj);
+    const int z = m * g.str_d - g.pad_d + t, y = p * g.str_h - g.pad_h + rr, x = q * g.str_w - g.pad_w + s;
+    if (z < 0 || z >= g.D || y < 0 || y >= g.H || x < 0 || x >= g.W) continue;
+    const float iv = __half2float(I[(((1ll * c * g.D + z) * g.H + y) * g.W + x) * g.N + n]);
+    const float ev = __half2float(E[1ll * k * span + j]);
+    acc = fmaf(iv, ev, acc);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0) {
+    acc *= alpha;
+    if (out_f32) static_cast<float*>(dF)[i] = acc;
+    else static_cast<__half*>(dF)[i] = __float2half_rn(acc);
+  }
+}
 __global__ void conv_update_simt(Geo g, const __half* __restrict__ I, const __half* __restrict__ E, void* dF,
                                  int out_f32, float alpha) {
   const long long total = g.sizeF();
   const int lane = threadIdx.x & 31;
   const long long warp0 = (blockIdx.x * 1ll * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = (1ll * gridDim.x * blockDim.x) >> 5;
-  for (long long i = warp0; i < total; i += nwarps) {
-    long long r = i;
-    const int k = r % g.K; r /= g.K;
-    const int s = r % g.S; r /= g.S;
-    const int rr = r % g.R; r /= g.R;
-    const int t = r % g.T; r /= g.T;
-    const int c = static_cast<int>(r);
-    float acc = 0.0f;
-    const long long span = 1ll * g.M * g.P * g.Q * g.N;
-    for (long long j = lane; j < span; j += 32) {
-      long long rj = j;
-      const int n = rj % g.N; rj /= g.N;
-      const int q = rj % g.Q; rj /= g.Q;
-      const int p = rj % g.P; rj /= g.P;
-      const int m = static_cast<int>(rj);
-      const int z = m * g.str_d - g.pad_d + t, y = p * g.str_h - g.pad_h + rr, x = q * g.str_w - g.pad_w + s;
-      if (z < 0 || z >= g.D || y < 0 || y >= g.H || x < 0 || x >= g.W) continue;
-      const float iv = __half2float(I[(((1ll * c * g.D + z) * g.H + y) * g.W + x) * g.N + n]);
-      const float ev = __half2float(E[1ll * k * span + j]);
-      acc = fmaf(iv, ev, acc);
+  for (long long i = warp0; i < total; i += nwarps) update_element(g, I, E, dF, out_f32, alpha, i, lane);
+}
+// The elements of a gradient that are NaN, again, without the pixels outside the tensor. One read of the gradient
+// when there are none.
+__global__ void __launch_bounds__(256) conv_update_redo(Geo g, const __half* __restrict__ I, const __half* __restrict__ E,
+                                                        void* dF, int out_f32, float alpha) {
+  grid_dependency_wait();
+  const long long total = g.sizeF();
+  const int lane = threadIdx.x & 31;
+  const long long warp0 = (blockIdx.x * 1ll * blockDim.x + threadIdx.x) >> 5;
+  const long long nwarps = (1ll * gridDim.x * blockDim.x) >> 5;
+  for (long long i0 = warp0 * 32; i0 < total; i0 += nwarps * 32) {
+    bool nan = false;
+    if (i0 + lane < total) {
+      const float v = out_f32 ? static_cast<const float*>(dF)[i0 + lane] : __half2float(static_cast<const __half*>(dF)[i0 + lane]);
+      nan = v != v;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) {
-      acc *= alpha;
-      if (out_f32) static_cast<float*>(dF)[i] = acc;
-      else static_cast<__half*>(dF)[i] = __float2half_rn(acc);
-    }
+    for (uint32_t left = __ballot_sync(0xffffffffu, nan); left != 0u; left &= left - 1u)
+      update_element(g, I, E, dF, out_f32, alpha, i0 + __ffs(static_cast<int>(left)) - 1, lane);
   }
 }
+
+// A kernel that waits for the one before it by itself
+template <typename... P, typename... A>
+int launch_dependent(int blocks, cudaStream_t stream, void (*kernel)(P...), A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = tuning().dependent_launch != 0 ? 1 : 0;
+  NG_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+  NG_CHECK_LAUNCH();
+  return NG_OK;
+}
+int redo_blocks(const DeviceCtx* c) { return 8 * c->sm_count; }    // (that run all at once)
 
 // ------------------------------------------------------------------------------------------
 // im2col: col[crst][pixel * N + n] = I[c, z, y, x, n] (zero outside the image); 8 images per thread
@@ -791,7 +862,7 @@ int update_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, ChunkMode mod
   tc_fill_mma(p, lay);
   fill_taps(p, g, mode);
   p.R = tb.nr; p.S = tb.ns; p.RS = tb.nr * tb.ns; p.tap_w = tb.bw; p.tap_h = tb.bh;
-  if (phased) fill_phases(p, update_phases(g));
+  if (phased) fill_phases(p, g);
   fill_decode(p, g.N, g.Q, g.P, g.M, mode);
   p.oob_y = g.H;
   p.Cold = nullptr; p.ldc = ld; p.c_zstride = 0;
@@ -801,14 +872,14 @@ int update_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, ChunkMode mod
   // behind the partials: the gradient in tap order and copies of the operands. (Not in the second buffer,
   // where I and the gradient of a layer that was rewritten by space to depth lie.)
   const size_t bytes[3] = {(static_cast<size_t>(g.K) * ld * 4 + 255) & ~size_t(255),
-                           phased ? phase_split_bytes(g, update_phases(g)) : (blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0),
+                           phased ? phase_split_bytes(g) : (blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0),
                            blocked_e ? chan_block_bytes(g.K, g.M, g.P, g.Q, g.N) : 0};
   void* room[3] = {nullptr, nullptr, nullptr};
   int rc = chan_block_room(c, stream, p, bytes, room, 3);
   if (rc != NG_OK) return rc;
   float* Dt = static_cast<float*>(room[0]);
   p.C = Dt;
-  if (phased) rc = phase_split(g, update_phases(g), I, room[1], stream);
+  if (phased) rc = phase_split(g, I, room[1], nullptr, nullptr, nullptr, stream);
   else if (blocked_i) rc = chan_block(c, stream, I, room[1], g.C, g.D, g.H, g.W, g.N);
   if (rc == NG_OK && blocked_e) rc = chan_block(c, stream, E, room[2], g.K, g.M, g.P, g.Q, g.N);
   if (rc != NG_OK) return rc;
@@ -818,7 +889,7 @@ int update_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, ChunkMode mod
   rc = act_map(&mapA, E, g.K, g.M, g.P, g.Q, g.N, mode, lay.a_box_rows, blocked_e);
   if (rc != NG_OK) return rc;
   rc = blocks ? act_map_tapblock(&mapB, I, g, tb)
-              : (phased ? phase_map(&mapB, I, g, update_phases(g), tb.rows) : act_map(&mapB, I, g.C, g.D, g.H, g.W, g.N, mode, tb.rows, blocked_i));
+              : (phased ? phase_map(&mapB, I, g, tb.rows) : act_map(&mapB, I, g.C, g.D, g.H, g.W, g.N, mode, tb.rows, blocked_i));
   if (rc != NG_OK) return rc;
   rc = tc_launch(c, mapA, mapB, p, stream);
   if (rc != NG_OK) return rc;
@@ -1126,7 +1197,7 @@ int ng_conv_fprop(const ng_conv_desc* d, const void* I, const void* F, void* O, 
   if (!tc) {
     count_fallback_launch();
     conv_fprop_simt<<<launch_1d(g.sizeO(), 256, c), 256, 0, stream>>>(
-        g, static_cast<const __half*>(I), static_cast<const __half*>(F), static_cast<__half*>(O), alpha, relu);
+        g, static_cast<const __half*>(I), static_cast<const __half*>(F), static_cast<__half*>(O), alpha, relu, nullptr, 0);
     NG_CHECK_LAUNCH();
     return NG_OK;
   }
@@ -1159,7 +1230,7 @@ int ng_conv_fprop(const ng_conv_desc* d, const void* I, const void* F, void* O, 
   }
   tc_fill_mma(p, lay);
   fill_taps(p, g, mode);
-  if (phased) fill_phases(p, g.str_w);
+  if (phased) fill_phases(p, g);
   if (stack) { ++p.R; p.RS += g.S; p.str_h = 2; }
   fill_decode(p, g.N, g.Q, stack ? p.cmap.y_count : g.P, g.M, mode);
   p.oob_y = g.H;
@@ -1172,13 +1243,17 @@ int ng_conv_fprop(const ng_conv_desc* d, const void* I, const void* F, void* O, 
   // few tiles (a small minibatch, e.g. the shard of one GPU): the reduction is split over the SMs too
   if (!stack) p.splits = choose_splits(c, 1ll * p.tiles_m * p.tiles_n, p.num_kb, 1ll * g.K * cols, true);
   if (phased) {
-    const size_t bytes = phase_split_bytes(g, g.str_w);
-    void* copy = nullptr;
-    rc = chan_block_room(c, stream, p, &bytes, &copy, 1);
-    if (rc == NG_OK) rc = phase_split(g, g.str_w, I, copy, stream);
-    if (rc == NG_OK) rc = phase_map(&mapB, copy, g, g.str_w, lay.kb_rows);
+    const size_t bytes[2] = {phase_split_bytes(g), kScanFlags * sizeof(int)};
+    void* room[2] = {nullptr, nullptr};
+    int scans = 0;
+    rc = chan_block_room(c, stream, p, bytes, room, 2);
+    int* flags = static_cast<int*>(room[1]);
+    if (rc == NG_OK) rc = phase_split(g, I, room[0], F, flags, &scans, stream);
+    if (rc == NG_OK) rc = phase_map(&mapB, room[0], g, lay.kb_rows);
+    if (rc == NG_OK) rc = tc_launch(c, mapA, mapB, p, stream);
     if (rc != NG_OK) return rc;
-    return tc_launch(c, mapA, mapB, p, stream);
+    return launch_dependent(redo_blocks(c), stream, conv_fprop_simt, g, static_cast<const __half*>(I), static_cast<const __half*>(F),
+                       static_cast<__half*>(O), alpha, relu, static_cast<const int*>(flags), scans);
   }
   const bool blocked = wants_chan_block(g.D, g.H, g.W, g.N, RST);
   if (blocked) {   // large channel planes: the product reads a copy in (z, y, chan, x, n) order
@@ -1213,7 +1288,7 @@ int ng_conv_bprop(const ng_conv_desc* d, const void* F, const void* E, void* gra
   if (!tc) {
     count_fallback_launch();
     conv_bprop_simt<<<launch_1d(g.sizeI(), 256, c), 256, 0, stream>>>(
-        g, static_cast<const __half*>(F), static_cast<const __half*>(E), static_cast<__half*>(gradI), alpha);
+        g, static_cast<const __half*>(F), static_cast<const __half*>(E), static_cast<__half*>(gradI), alpha, nullptr, 0);
     NG_CHECK_LAUNCH();
     return NG_OK;
   }
@@ -1232,19 +1307,33 @@ int ng_conv_bprop(const ng_conv_desc* d, const void* F, const void* E, void* gra
         }
     return NG_OK;
   };
-  if (blocked) {   // large channel planes: the products read a copy in (z, y, chan, x, n) order, behind their partials
+  const bool scan = !in_place;      // (see phase_split)
+  const void* E0 = E;
+  int* flags = nullptr;
+  if (blocked || scan) {   // behind the products' partials: the copy of E, the flags
     size_t off = 0;
     rc = phases(&off);
     if (rc != NG_OK) return rc;
     off = round256(off);
-    rc = ensure_workspace(c, stream, off + chan_block_bytes(g.K, g.M, g.P, g.Q, g.N));
+    const size_t copy_bytes = blocked ? chan_block_bytes(g.K, g.M, g.P, g.Q, g.N) : 0;
+    rc = ensure_workspace(c, stream, off + copy_bytes + kScanFlags * sizeof(int));
     if (rc != NG_OK) return rc;
-    void* copy = reinterpret_cast<uint8_t*>(c->ws) + off;
-    rc = chan_block(c, stream, E, copy, g.K, g.M, g.P, g.Q, g.N);
-    if (rc != NG_OK) return rc;
-    E = copy;
+    uint8_t* room = reinterpret_cast<uint8_t*>(c->ws) + off;
+    if (blocked) {   // large channel planes: the products read a copy in (z, y, chan, x, n) order
+      rc = chan_block(c, stream, E, room, g.K, g.M, g.P, g.Q, g.N);
+      if (rc != NG_OK) return rc;
+      E = room;
+    }
+    if (scan) {
+      flags = reinterpret_cast<int*>(room + copy_bytes);
+      rc = launch_dependent(kScanFlags, stream, nonfinite_scan, static_cast<const uint4*>(F), g.sizeF() / 8, flags);
+      if (rc != NG_OK) return rc;
+    }
   }
-  return phases(nullptr);
+  rc = phases(nullptr);
+  if (rc != NG_OK || !scan) return rc;
+  return launch_dependent(redo_blocks(c), stream, conv_bprop_simt, g, static_cast<const __half*>(F), static_cast<const __half*>(E0),
+                     static_cast<__half*>(gradI), alpha, static_cast<const int*>(flags), kScanFlags);
 }
 
 int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gradF, int out_f32, float alpha,
@@ -1292,10 +1381,14 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
       return NG_OK;
     }
   }
+  auto redo = [&, I0 = static_cast<const __half*>(I), E0 = static_cast<const __half*>(E)] {   // (see phase_split)
+    return launch_dependent(redo_blocks(c), stream, conv_update_redo, g, I0, E0, gradF, out_f32, alpha);
+  };
   if (direct && wants_update_swap(g, 1ll * g.M * g.P * row_chunks(g.N, g.Q, mode))) {
     TapBlock taps;
     taps.bw = taps.bh = 1; taps.rows = swap_rows(g.C); taps.nr = g.R; taps.ns = g.S; taps.ok = true;
-    return update_swapped(c, g, taps, mode, phased, I, E, gradF, out_f32, alpha, stream);
+    rc = update_swapped(c, g, taps, mode, phased, I, E, gradF, out_f32, alpha, stream);
+    return rc == NG_OK && phased ? redo() : rc;
   }
   if (direct) {
     TcParams p = {};
@@ -1320,7 +1413,7 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
     }
     tc_fill_mma(p, lay);
     fill_taps(p, g, mode);
-    if (phased) fill_phases(p, update_phases(g));
+    if (phased) fill_phases(p, g);
     fill_decode(p, g.N, g.Q, g.P, g.M, mode);
     p.oob_y = g.H;
     p.C = gradF; p.Cold = nullptr; p.ldc = 1ll * RST * g.K; p.c_zstride = g.K;
@@ -1333,22 +1426,23 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
     const bool blocked_i = !phased && wants_chan_block(g.D, g.H, g.W, g.N, RST);
     const bool blocked_e = wants_chan_block(g.M, g.P, g.Q, g.N, RST);
     if (phased || blocked_i || blocked_e) {
-      const size_t bytes[2] = {phased ? phase_split_bytes(g, update_phases(g)) : blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0,
+      const size_t bytes[2] = {phased ? phase_split_bytes(g) : blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0,
                                blocked_e ? chan_block_bytes(g.K, g.M, g.P, g.Q, g.N) : 0};
       void* copies[2] = {nullptr, nullptr};
       rc = chan_block_room(c, stream, p, bytes, copies, 2);
-      if (rc == NG_OK && phased) rc = phase_split(g, update_phases(g), I, copies[0], stream);
+      if (rc == NG_OK && phased) rc = phase_split(g, I, copies[0], nullptr, nullptr, nullptr, stream);
       if (rc == NG_OK && blocked_i) rc = chan_block(c, stream, I, copies[0], g.C, g.D, g.H, g.W, g.N);
       if (rc == NG_OK && blocked_e) rc = chan_block(c, stream, E, copies[1], g.K, g.M, g.P, g.Q, g.N);
       if (rc != NG_OK) return rc;
       if (phased || blocked_i) I = copies[0];
       if (blocked_e) E = copies[1];
     }
-    rc = phased ? phase_map(&mapA, I, g, update_phases(g), a_rows) : act_map(&mapA, I, g.C, g.D, g.H, g.W, g.N, mode, a_rows, blocked_i);
+    rc = phased ? phase_map(&mapA, I, g, a_rows) : act_map(&mapA, I, g.C, g.D, g.H, g.W, g.N, mode, a_rows, blocked_i);
     if (rc != NG_OK) return rc;
     rc = act_map(&mapB, E, g.K, g.M, g.P, g.Q, g.N, mode, p.block_n, blocked_e);
     if (rc != NG_OK) return rc;
-    return tc_launch(c, mapA, mapB, p, stream);
+    rc = tc_launch(c, mapA, mapB, p, stream);
+    return rc == NG_OK && phased ? redo() : rc;
   }
   if (im2col) {
     // dF[crst][k] = col[crst][span] * E[k][span]^T  (both K-major: an "nt" GEMM with split-K)

@@ -560,3 +560,57 @@ def test_operand_copies_of_all_passes_share_one_scratch_buffer(ng, lib):
     finally:
         assert lib.ng_tune(b"chan_block", -1) == 0
         ng.stream = default
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("name", ["n24_5x5_s3", "n88_7x7_s2_c96", "n40_2x3_s3_h1", "n32_3d_s222", "n16_1x1_s2", "n8_3x3_s2"])
+def test_strided_layers_keep_infinities_from_outputs_that_do_not_meet_them(ng, name, value):
+    """Minibatches that are no multiple of 64: an infinity or NaN in any operand reaches what it reaches on the
+    CUDA-core kernels, which skip the pixels outside the tensors that the tensor cores multiply as zeros."""
+    cfg = STRIDED[name]
+    cd = rm.ConvDims(*cfg)
+    I, F, E = _inputs(cd, 1023)
+    C, T, R, S, K = F.shape
+
+    def check(I, F, E, ops):
+        got = [_run_all(ng, _layer(ng, cfg, path), I, F, E, relu=True, ops=ops) for path in ("auto", "simt")]
+        for key in got[0]:
+            a, b = got[0][key].astype(np.float64), got[1][key].astype(np.float64)
+            assert not np.isfinite(b).all() and np.isfinite(b).any()
+            for what in (np.isnan, np.isposinf, np.isneginf):
+                assert np.array_equal(what(a), what(b)), (name, key)
+
+    for t, r, s in ((0, 0, 0), (T - 1, R - 1, S - 1)):           # corner taps: most outputs at a border miss one
+        bad = F.copy()
+        bad[C // 2, t, r, s, 1] = value
+        got = [_run_all(ng, _layer(ng, cfg, path), I, bad, E, ops="fb") for path in ("auto", "simt")]
+        for key in ("O", "gradI"):
+            np.testing.assert_array_equal(got[0][key], got[1][key])
+            assert not np.isfinite(got[1][key]).all()
+        if value > 0:      # (negative ones and NaN are gone after a ReLU)
+            check(I, bad, E, "f")
+    P, Q = E.shape[2:4]
+    for p, q in ((0, 0), (P - 1, Q - 1)):
+        bad = E.copy()
+        bad[3, 0, p, q, 2] = value
+        check(I, F, bad, "bu")
+    bad = I.copy()
+    bad[1, 0, 0, I.shape[3] - 1, 5] = value
+    if R > 1:              # (a 1x1 filter steps over that pixel)
+        check(bad, F, E, "u")
+
+
+def test_strided_update_in_fp16_keeps_infinities_apart_too(ng):
+    cfg = STRIDED["n24_5x5_s3"]
+    cd = rm.ConvDims(*cfg)
+    I, F, E = _inputs(cd, 1025)
+    E[3, 0, 0, 0, 2] = np.inf
+    got = []
+    for path in ("auto", "simt"):
+        layer = _layer(ng, cfg, path)
+        dU = ng.empty(layer.dimF)
+        ng.update_conv(layer, ng.array(I), ng.array(E), dU)
+        got.append(dU.get())
+    for what in (np.isnan, np.isposinf, np.isneginf):
+        assert np.array_equal(what(got[0]), what(got[1]))
+    assert np.isfinite(got[1][:, :, 0]).all() and not np.isfinite(got[1]).all()
