@@ -80,9 +80,10 @@ int ng_launch_count(unsigned long long* count);
  * prefix, in lower case ("pair_mma", "tile_rows", ...). For tests and measurements: results do
  * not depend on them beyond fp32 summation order. No counterpart in the reference. */
 int ng_tune(const char* name, int value);
-/* Number of GEMM / convolution calls so far that ran on the plain CUDA-core fall-back kernels
- * (operands TMA cannot address, strided layers with fewer than 64 images) instead of the
- * tensor-core engine. A benchmark that claims the tensor-core path checks that this stays 0. */
+/* Number of GEMM / convolution calls so far that had to run on the plain CUDA-core fall-back kernels
+ * (unaligned tensors of a convolution, sizes beyond the engine's) instead of the tensor-core engine.
+ * Very small calls that run there because they are shorter there are not counted. A benchmark that
+ * claims the tensor-core path checks that this stays 0. */
 int ng_fallback_launch_count(unsigned long long* count);
 
 /* Record-and-replay of a sequence of calls (a CUDA graph). The reference drives every kernel

@@ -3,10 +3,11 @@
 // Mirrors NervanaGPU.dot / batched_dot (nervanagpu/nervanagpu.py:820-1105) and the C interface
 // nervana_hgemm (nervanagpu/kernels/C_interface/nervana_c_api.h:31-128).
 //
-// Everything runs on the tcgen05 engine. Operands that TMA cannot address (base not 16-byte
-// aligned, leading dimension or batch stride no multiple of 8 elements) are first copied into
-// rows that it can (pack_rows_kernel). The plain CUDA-core kernel serves ng_hgemm_simt, the
-// second opinion of the tests.
+// The tcgen05 engine runs them. Operands that TMA cannot address (base not 16-byte aligned, leading
+// dimension or batch stride no multiple of 8 elements) are first copied into rows that it can
+// (pack_rows_kernel). The plain CUDA-core kernel serves very short products of such operands
+// (shorter_unpacked), operands of more than 2^30 packed groups, calls that are both batched and summed
+// over a batch, and ng_hgemm_simt, the second opinion of the tests.
 #include <algorithm>
 
 #include "../../include/nervana_b200.h"
@@ -162,6 +163,19 @@ bool plan_pack(PackArgs& a, const void* src, long long ld, long long zstride, lo
   return true;
 }
 
+// Whether a product whose operands would have to be packed is shorter on the CUDA cores, which take about
+// 2.1 us per 16 rows of the reduction after the first 4.5 while the device holds all tiles, and need no second
+// launch. Packing and product take 5.5 to 8.1 us with up to 128 columns and 10 beyond, hardly more for longer
+// reductions. CUDA cores / packed, in a recorded sequence (us): 65 x 65 x 9 4.6 / 7.3, x 25 6.6 / 7.3 (one by
+// one 8.5 / 7.7), x 33 8.8 / 7.4; 513 x 513 x 9 4.8 / 10.0, x 25 6.7 / 10.2, x 41 9.4 / 10.2 (one by one 10.9 / 10.7);
+// 1001 x 1001 x 25 9.3 / 10.4, x 33 12.1 / 10.5.
+bool shorter_unpacked(const DeviceCtx* c, const GemmCall& g) {
+  if (tuning().pack_odd >= 0) return tuning().pack_odd == 0;
+  const long long steps = (g.k + 15ll) / 16 * g.loops;
+  const long long tiles = ((g.m + 63ll) / 64) * ((g.n + 63ll) / 64) * g.batch;
+  return tiles <= 2ll * c->sm_count && (steps <= 1 || (steps == 2 && g.n > 128));
+}
+
 bool tma_ok(const void* p, long long ld, long long zstride) {
   return (reinterpret_cast<uintptr_t>(p) & 15u) == 0 && (ld & 7) == 0 && (zstride & 7) == 0;
 }
@@ -194,7 +208,8 @@ int run_gemm(const GemmCall& call, cudaStream_t stream) {
     use_tc = plan_pack(packA, g.A, g.lda, zsa, nza, g.a_t ? g.k : g.m, g.a_t ? g.m : g.k);
   if (use_tc && !tma_ok(g.B, g.ldb, zsb))
     use_tc = plan_pack(packB, g.B, g.ldb, zsb, nzb, g.b_t ? g.n : g.k, g.b_t ? g.k : g.n);
-  if (!use_tc) {
+  const bool by_rule = use_tc && (packA.total || packB.total) && shorter_unpacked(c, g);
+  if (!use_tc || by_rule) {
     SimtGemmArgs s;
     s.A = static_cast<const __half*>(g.A); s.B = static_cast<const __half*>(g.B); s.C = g.C;
     s.a_t = g.a_t; s.b_t = g.b_t; s.m = g.m; s.n = g.n; s.k = g.k;
@@ -202,7 +217,7 @@ int run_gemm(const GemmCall& call, cudaStream_t stream) {
     s.az = g.az; s.bz = g.bz; s.cz = g.cz; s.loops = g.loops; s.alz = g.alz; s.blz = g.blz;
     s.out_f32 = g.out_f32; s.ea = ea;
     dim3 grid((g.n + 63) / 64, (g.m + 63) / 64, g.batch);
-    count_fallback_launch();
+    if (!by_rule) count_fallback_launch();
     gemm_simt_kernel<<<grid, 256, 0, stream>>>(s);
     NG_CHECK_LAUNCH();
     return NG_OK;

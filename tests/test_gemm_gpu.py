@@ -146,6 +146,35 @@ def test_operands_at_odd_addresses(ng, op, mnk):
         assert_close(C.get(), ref, tol, "%s %s +%d" % (op, mnk, shift))
 
 
+@pytest.mark.parametrize("op", ["nn", "nt", "tn"])
+@pytest.mark.parametrize("mnk", [(1, 1, 1), (7, 9, 8), (65, 63, 16), (33, 129, 17), (33, 128, 17), (65, 300, 32), (65, 300, 33)])
+def test_short_products_of_odd_operands_packed_and_unpacked(ng, lib, op, mnk):
+    """Both sides of the line between the CUDA-core kernel and the packed product, and the rule itself."""
+    m, n, k = mnk
+    rng = np.random.default_rng(19 + m)
+    A, B = _operands(rng, m, n, k, op)
+    bigA, bigB = (np.pad(x, ((0, 0), (0, 1 + x.shape[1] % 2))) for x in (A, B))      # odd leading dimensions
+    dA, dB = ng.array(bigA)[:, :A.shape[1]], ng.array(bigB)[:, :B.shape[1]]
+    C0 = rng.standard_normal((m, n)).astype(np.float16)
+    ref = rm.gemm(A, B, op[0] == "t", op[1] == "t", alpha=0.5, beta=0.25, C=C0)
+    tol = rn16_tol(ref, rm.gemm_abs(A, B, op[0] == "t", op[1] == "t"), k) + 2.0 ** -11 * np.abs(C0.astype(np.float32))
+    before, after = ctypes.c_ulonglong(0), ctypes.c_ulonglong(0)
+    launches = []
+    try:
+        for form in (0, 2, -1):
+            assert lib.ng_tune(b"pack_odd", form) == 0
+            C = ng.array(C0)
+            assert lib.ng_launch_count(ctypes.byref(before)) == 0
+            ng.dot(dA.T if op[0] == "t" else dA, dB.T if op[1] == "t" else dB, C, alpha=0.5, beta=0.25)
+            assert lib.ng_launch_count(ctypes.byref(after)) == 0
+            launches.append(after.value - before.value)
+            assert_close(C.get(), ref, tol, "%s %s form %d" % (op, mnk, form))
+    finally:
+        assert lib.ng_tune(b"pack_odd", -1) == 0
+    assert launches[0] == 1 and launches[1] >= 2
+    assert launches[2] == launches[0 if k <= 16 or (k <= 32 and n > 128) else 1]
+
+
 @pytest.mark.parametrize("dims", [(2, 8, 8, 8), (3, 129, 72, 65), (5, 33, 17, 130), (17, 128, 128, 64), (1, 40, 24, 72)])
 @pytest.mark.parametrize("shared", [None, "A", "B"])
 def test_batched_dot_forms(ng, dims, shared):
