@@ -16,11 +16,13 @@
 // a row runs past its end, where TMA zero-fills (or, between rows of the input, reads pixels
 // whose products land in columns that are never stored).
 // Strided layers: the backward pass runs phase by phase (the input pixels of one residue modulo the
-// strides see a unit-stride layer over their share of the taps); with a minibatch that is no multiple
-// of 64 the forward pass and the update read a copy of the input whose rows are split by x modulo the
-// stride (phase_split). Small-C weight updates run as im2col + tensor-core GEMM. The plain CUDA-core
-// kernels serve unaligned tensors and the tests.
+// strides see a unit-stride layer over their share of the taps), small ones in a single launch
+// (bprop_by_phases); with a minibatch that is no multiple of 64 the forward pass and the update read a copy
+// of the input whose rows are split by x modulo the stride (phase_split), or, for small updates, a patch
+// matrix. Small-C weight updates run as im2col + tensor-core GEMM. The plain CUDA-core kernels serve
+// unaligned tensors, small strided backward passes and the tests.
 #include <algorithm>
+#include <cmath>
 
 #include "../../include/nervana_b200.h"
 #include "epilogue.cuh"
@@ -1042,22 +1044,31 @@ __global__ void s2d_filter_grad_kernel(Geo g, SpaceToDepth z, const float* __res
 // a unit-stride layer over the phase's share of the taps, whose outputs are stored every st-th pixel
 // (ColumnMap). A unit-stride layer is its only phase. (Issuing every tap for every pixel and letting
 // the copy engine fill zeros where the stride does not divide took st^2 times the operands and MMAs.)
-// `blocked`: E is its channel-blocked copy. `partials`, if given, is raised to the bytes of the phase's split
-// partials, and nothing is launched.
+// `blocked`: E is its channel-blocked copy. `gather`: the whole layer, every tap for every pixel. `plan`: if
+// given, it is filled in and nothing is launched.
 // ------------------------------------------------------------------------------------------
+struct BpropPlan {
+  size_t partials = 0;     // bytes of the split partials, raised to the largest of the phases
+  long long steps = 0;     // k-blocks that an SM works on, one after the other
+  int splits = 1;
+};
 int bprop_phase(DeviceCtx* c, const Geo& g, const int first[3], ChunkMode mode, const void* F, const void* E, void* gradI,
-                float alpha, bool blocked, size_t* partials, cudaStream_t stream) {
+                float alpha, bool blocked, bool gather, BpropPlan* plan, cudaStream_t stream) {
   const int str[3] = {g.str_d, g.str_h, g.str_w}, flt[3] = {g.T, g.R, g.S}, pad[3] = {g.pad_d, g.pad_h, g.pad_w},
             ext[3] = {g.D, g.H, g.W};
   int taps[3], lo[3], n[3], off[3];     // taps of the phase; first x' and number of its pixels; first pixel
   for (int i = 0; i < 3; ++i) {
+    if (gather) {
+      taps[i] = flt[i]; lo[i] = pad[i]; off[i] = 0; n[i] = ext[i];
+      continue;
+    }
     taps[i] = (flt[i] - first[i] + str[i] - 1) / str[i];
     lo[i] = pad[i] > first[i] ? (pad[i] - first[i] + str[i] - 1) / str[i] : 0;
     off[i] = str[i] * lo[i] + first[i] - pad[i];
     if (off[i] >= ext[i]) return NG_OK;
     n[i] = (ext[i] - off[i] + str[i] - 1) / str[i];
   }
-  const bool unit = str[0] == 1 && str[1] == 1 && str[2] == 1;
+  const bool unit = gather || (str[0] == 1 && str[1] == 1 && str[2] == 1);
   TcParams p = {};
   p.mode = TC_BPROP;
   const long long cols = pixel_columns(p, 1ll * n[0] * n[1], n[2], g.N, mode);
@@ -1080,8 +1091,8 @@ int bprop_phase(DeviceCtx* c, const Geo& g, const int first[3], ChunkMode mode, 
   // fewer input channels than tile rows (one row tile): the filter box carries the real rows only
   int a_rows = p.tiles_m == 1 ? std::min(kTileM * p.m_halves, (g.C + 7) / 8 * 8) : kTileM * p.m_halves;
   const int n_taps = taps[0] * taps[1] * taps[2];
-  const int stack = pick_row_stack(c, g.C, a_rows, n_taps, taps[1], p.red_chunks, kChunk, n[1], n[0],
-                                   1ll * row_chunks(g.N, n[2], mode) * kChunk, alpha);
+  const int stack = gather ? 0 : pick_row_stack(c, g.C, a_rows, n_taps, taps[1], p.red_chunks, kChunk, n[1], n[0],
+                                                1ll * row_chunks(g.N, n[2], mode) * kChunk, alpha);
   const long long out_row = 1ll * g.str_h * g.W * g.N;
   if (stack) {
     fill_row_pairs(p, stack, g.N, n[2], n[1], n[0], mode, g.str_w * g.N, out_row, 1ll * g.str_d * g.H * g.W * g.N);
@@ -1094,25 +1105,73 @@ int bprop_phase(DeviceCtx* c, const Geo& g, const int first[3], ChunkMode mode, 
   p.pad_d = lo[0]; p.pad_h = lo[1] + (stack ? 1 : 0); p.pad_w = lo[2];
   p.inner_tap = mode == CH_FLAT ? g.N : 0;
   p.x_tap = mode == CH_FLAT ? 0 : 1;
+  p.gather = gather;
+  p.str_d = g.str_d; p.str_h = g.str_h; p.str_w = g.str_w;
   fill_decode(p, g.N, n[2], stack ? p.cmap.y_count : n[1], n[0], mode);
   p.oob_y = g.P;
   p.C = static_cast<__half*>(gradI) + ((1ll * off[0] * g.H + off[1]) * g.W + off[2]) * g.N;
   p.Cold = nullptr; p.ldc = 1ll * g.D * g.H * g.W * g.N; p.c_zstride = stack ? out_row : 0;
   p.alpha = alpha; p.beta = 0.0f; p.relu = 0; p.sr_bits = 0; p.out_f32 = 0; p.vec_ok = 1;
   if (!stack) p.splits = choose_splits(c, 1ll * p.tiles_m * p.tiles_n, p.num_kb, 1ll * g.C * cols, true);
-  if (partials) {
-    if (p.splits > 1) *partials = std::max(*partials, static_cast<size_t>(p.splits) * p.M * p.N * sizeof(float));
+  if (plan) {
+    if (p.splits > 1) plan->partials = std::max(plan->partials, static_cast<size_t>(p.splits) * p.M * p.N * sizeof(float));
+    plan->splits = p.splits;
+    plan->steps = (1ll * p.tiles_m * p.tiles_n + c->sm_count - 1) / c->sm_count * ((p.num_kb + p.splits - 1) / p.splits);
     return NG_OK;
   }
   CUtensorMap mapA, mapB, mapBm;
-  int rc = filter_map_phase(&mapA, F, g, first, taps, a_rows);
+  int rc = gather ? filter_map_rows(&mapA, F, g.K, g.S, g.R, g.T, g.C, a_rows) : filter_map_phase(&mapA, F, g, first, taps, a_rows);
   if (rc != NG_OK) return rc;
   rc = act_map(&mapB, E, g.K, g.M, g.P, g.Q, g.N, mode, kChunk, blocked);
   if (rc != NG_OK) return rc;
   // the error pixels of a column tile inside one image row as one box
-  if (mode == CH_PIXEL)
+  if (mode == CH_PIXEL && !gather)
     p.b_merge = act_map_merged(&mapBm, E, g.K, g.M, g.P, g.Q, g.N, kChunk, p.block_n / kChunk, blocked);
   return tc_launch(c, mapA, mapB, p, stream, p.b_merge ? &mapBm : nullptr);
+}
+
+// Whether the backward pass of a strided layer runs phase by phase. Every phase is a product (and, with few
+// tiles, a second stage) of its own, some 5 us before it has done any work. Small layers are shorter as one
+// product over every tap of every pixel (`in_place`: minibatches that are multiples of 64), or on the CUDA
+// cores. The estimates are fits to 120 layers of 1 to 7 taps and strides 2 to 4, each timed in both forms; by
+// phases / the other form, us:
+//   one product: 128 -> 64, 4x4 / 4, 8x8, 128 images 82 / 13; 64 -> 64, 3x3 / 2, 14x14, 128 images 22 / 12; 96 -> 32,
+//   3x3 / 2, 23x23, 64 images 25 / 15; 64 -> 64, 3x3 / 2, 56x56, 64 images 32 / 52; 96 -> 96, 3x3 / 2, 55x55, 128 images 53 / 169
+//   CUDA cores: 16 -> 16, 4x4 / 4, 8x8, 8 images 82 / 7; 32 -> 32, 3x3 / 2, 8x8, 16 images 25 / 11; 24 -> 64, 7x7 / 2, 11x11,
+//   48 images 39 / 86; 64 -> 64, 3x3 / 2, 56x56, 24 images 33 / 858
+bool bprop_by_phases(DeviceCtx* c, const Geo& g, bool in_place) {
+  const int strides = g.str_d * g.str_h * g.str_w, taps = g.T * g.R * g.S;
+  if (strides == 1) return true;
+  if (tuning().stride_phases >= 0) return tuning().stride_phases != 0;
+  const double phases = 1.0 * std::min(g.str_d, g.T) * std::min(g.str_h, g.R) * std::min(g.str_w, g.S);
+  const double pixels = 1.0 * g.D * g.H * g.W;
+  const int chunks = (g.K + kChunk - 1) / kChunk, row_tiles = (g.C + kTileM - 1) / kTileM;
+  auto tiles = [&](double px) { return row_tiles * std::ceil(px * g.N / 256); };
+  const double kb = taps / phases * chunks, waves = tiles(pixels / strides) / c->sm_count;
+  double by_phases = 3.0 + phases * (5.0 + (waves < 1.0 ? 0.3 * std::min(kb, 8.0 + kb * waves) : 0.5 * std::ceil(waves) * (kb + 1)));
+  if (in_place) {       // (the producer takes 0.86 us to find the pixels of a k-block, whatever its size)
+    const int first[3] = {0, 0, 0};
+    BpropPlan one;
+    bprop_phase(c, g, first, g.N % kChunk == 0 ? CH_PIXEL : CH_FLAT, nullptr, nullptr, nullptr, 1.0f, false, true, &one, nullptr);
+    return by_phases < 5.0 + (one.splits > 1 ? 3.0 : 0.0) + 0.86 * one.steps;
+  }
+  by_phases += 5.0;      // (the scan of the filter, the second look at the result)
+  const double chain = std::ceil(1.0 * g.T / g.str_d) * std::ceil(1.0 * g.R / g.str_h) * std::ceil(1.0 * g.S / g.str_w) * g.K;
+  return by_phases < 7.0 + 0.03 * chain + 1e-6 * g.sizeI() * (17.0 + 0.4 * taps + 1.0 * g.K * taps / strides);
+}
+// Whether the update of a strided layer whose minibatch is no multiple of 64 reads a phase-split copy, or a
+// patch matrix: small ones, and those with about as many input pixels as patch elements or fewer, of which
+// patches read only what they need. Phase-split / patches, us (patches, their ratio to the input):
+// 128 -> 128, 1x1 / 2, 28x28, 24 images (1.2 MB, 0.25) 17 / 15; 256 -> 32, 3x3 / 2, 16x16, 24 images (7.1 MB, 2.3) 18 / 17; 256 -> 32,
+// 7x7 / 3, 19x19, 8 images (9.8 MB, 6.6) 18 / 21; 512 -> 512, 3x3 / 3, 22x22, 32 images (18 MB, 1.2) 41 / 34; 64 -> 64, 3x3 / 2, 56x56,
+// 24 images (22 MB, 2.3) 27 / 29; 512 -> 512, 1x1 / 2, 34x34, 96 images (27 MB, 0.25) 76 / 45; 96 -> 512, 3x3 / 4, 85x85, 48 images
+// (38 MB, 0.6) 58 / 54; 256 -> 64, 2x2 / 2, 62x62, 32 images (64 MB, 1.1) 46 / 61; 96 -> 72, 5x5 / 2, 51x51, 88 images (1.1 GB, 6.3) 91 / 218.
+constexpr long long kPatchBytes = 8ll << 20;
+bool update_by_phases(const Geo& g) {
+  if (tuning().stride_phases >= 0) return tuning().stride_phases != 0;
+  const long long rows = 1ll * g.C * g.T * g.R * g.S, patches = rows * g.M * g.P * g.Q * g.N;
+  if (rows > 65535) return true;          // (the patch kernel has a block row for each)
+  return 2 * patches > kPatchBytes && (2 * patches > 3 * g.sizeI() || (2 * patches > 4 * kPatchBytes && 5 * patches > 4 * g.sizeI()));
 }
 
 size_t round256(size_t b) { return (b + 255) & ~size_t(255); }
@@ -1139,7 +1198,8 @@ int ng_conv_fprop(const ng_conv_desc* d, const void* I, const void* F, void* O, 
   if (!c) return NG_ERR_CUDA;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   ChunkMode mode = pick_chunk_mode(g.N, g.str_w);
-  const bool phased = mode == CH_NONE && path == NG_PATH_AUTO;    // a phase-split copy in flattened rows
+  // a phase-split copy in flattened rows (never slower than the CUDA cores: 16 -> 128, 1x1 / 2, 6x6, 96 images 13 / 15 us)
+  const bool phased = mode == CH_NONE && path == NG_PATH_AUTO;
   if (phased) mode = CH_FLAT;
   const bool al = aligned16(I) && aligned16(F) && aligned16(O);
   const bool tc = path != NG_PATH_SIMT && path != NG_PATH_IM2COL && mode != CH_NONE && al;
@@ -1283,26 +1343,28 @@ int ng_conv_bprop(const ng_conv_desc* d, const void* F, const void* E, void* gra
   // (the error tensor is read pixel by pixel whatever the strides are; see bprop_phase)
   const ChunkMode mode = g.N % kChunk == 0 ? CH_PIXEL : CH_FLAT;
   const bool in_place = pick_chunk_mode(g.N, g.str_w) != CH_NONE;
-  const bool tc = path != NG_PATH_SIMT && (in_place || path == NG_PATH_AUTO) && aligned16(F) && aligned16(E) && aligned16(gradI);
-  if (path == NG_PATH_TENSOR && !tc) return fail(NG_ERR_UNSUPPORTED, "shape not addressable by the tensor-core path");
-  if (!tc) {
-    count_fallback_launch();
+  const bool addressable = path != NG_PATH_SIMT && (in_place || path == NG_PATH_AUTO) && aligned16(F) && aligned16(E) && aligned16(gradI);
+  if (path == NG_PATH_TENSOR && !addressable) return fail(NG_ERR_UNSUPPORTED, "shape not addressable by the tensor-core path");
+  const bool by_phases = addressable && bprop_by_phases(c, g, in_place);
+  if (!addressable || !(by_phases || in_place)) {
+    if (!addressable) count_fallback_launch();
     conv_bprop_simt<<<launch_1d(g.sizeI(), 256, c), 256, 0, stream>>>(
         g, static_cast<const __half*>(F), static_cast<const __half*>(E), static_cast<__half*>(gradI), alpha, nullptr, 0);
     NG_CHECK_LAUNCH();
     return NG_OK;
   }
   const int str[3] = {g.str_d, g.str_h, g.str_w}, flt[3] = {g.T, g.R, g.S};
+  const bool gather = !by_phases;
   // a phase that no tap falls on, because the stride is larger than the filter, gets no error at all
-  if (str[0] > flt[0] || str[1] > flt[1] || str[2] > flt[2])
+  if (!gather && (str[0] > flt[0] || str[1] > flt[1] || str[2] > flt[2]))
     NG_CUDA(cudaMemsetAsync(gradI, 0, static_cast<size_t>(g.sizeI()) * 2, stream));
   const bool blocked = wants_chan_block(g.M, g.P, g.Q, g.N, g.T * g.R * g.S);
-  auto phases = [&](size_t* partials) -> int {
-    for (int pt = 0; pt < std::min(str[0], flt[0]); ++pt)
-      for (int pr = 0; pr < std::min(str[1], flt[1]); ++pr)
-        for (int ps = 0; ps < std::min(str[2], flt[2]); ++ps) {
+  auto phases = [&](BpropPlan* plan) -> int {
+    for (int pt = 0; pt < (gather ? 1 : std::min(str[0], flt[0])); ++pt)
+      for (int pr = 0; pr < (gather ? 1 : std::min(str[1], flt[1])); ++pr)
+        for (int ps = 0; ps < (gather ? 1 : std::min(str[2], flt[2])); ++ps) {
           const int first[3] = {pt, pr, ps};
-          const int rc = bprop_phase(c, g, first, mode, F, E, gradI, alpha, blocked, partials, stream);
+          const int rc = bprop_phase(c, g, first, mode, F, E, gradI, alpha, blocked, gather, plan, stream);
           if (rc != NG_OK) return rc;
         }
     return NG_OK;
@@ -1311,10 +1373,10 @@ int ng_conv_bprop(const ng_conv_desc* d, const void* F, const void* E, void* gra
   const void* E0 = E;
   int* flags = nullptr;
   if (blocked || scan) {   // behind the products' partials: the copy of E, the flags
-    size_t off = 0;
-    rc = phases(&off);
+    BpropPlan plan;
+    rc = phases(&plan);
     if (rc != NG_OK) return rc;
-    off = round256(off);
+    const size_t off = round256(plan.partials);
     const size_t copy_bytes = blocked ? chan_block_bytes(g.K, g.M, g.P, g.Q, g.N) : 0;
     rc = ensure_workspace(c, stream, off + copy_bytes + kScanFlags * sizeof(int));
     if (rc != NG_OK) return rc;
@@ -1346,11 +1408,11 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
   if (!c) return NG_ERR_CUDA;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   ChunkMode mode = pick_chunk_mode(g.N, g.str_w);
-  const bool phased = mode == CH_NONE && path == NG_PATH_AUTO;    // a phase-split copy in flattened rows
-  if (phased) mode = CH_FLAT;
   const bool al = aligned16(I) && aligned16(E) && aligned16(gradF);
   const int RST = g.T * g.R * g.S;
   const long long span = 1ll * g.M * g.P * g.Q * g.N;
+  const bool phased = mode == CH_NONE && path == NG_PATH_AUTO && update_by_phases(g);
+  if (phased) mode = CH_FLAT;    // a phase-split copy in flattened rows
   const bool direct = path != NG_PATH_SIMT && path != NG_PATH_IM2COL && mode != CH_NONE && al &&
                       (g.C >= 16 || path == NG_PATH_TENSOR);
   const bool im2col = !direct && path != NG_PATH_SIMT && path != NG_PATH_TENSOR && al &&

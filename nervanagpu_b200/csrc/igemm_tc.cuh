@@ -105,6 +105,7 @@ struct TcParams {
   int str_d, str_h, str_w;
   int inner_tap;                   // N in flattened-(W,N) mode else 0
   int x_tap;                       // 0 in flattened mode else 1
+  int gather;                      // backward pass of a strided layer: 1 = every tap for every pixel in one product
   int phase_w;                     // > 1: the input is a copy whose rows are split into this many x phases
                                    // (strided layers in flattened mode): tap s reads phase s % phase_w
   int dec_cpi, dec_q, dec_p, dec_m;  // chunk decode of the pixel space the chunks walk

@@ -77,6 +77,21 @@ struct Walk {
   int trs, rc;
 };
 
+// Exact division for the strided gather of the backward pass: returns false when `num` is not
+// a multiple of `den` (that tap does not touch this pixel).
+__device__ __forceinline__ bool div_exact(int num, int den, int& out) {
+  if (den == 1) {
+    out = num;
+    return true;
+  }
+  if (num < 0) {
+    out = -1;  // out of range either way
+    return true;
+  }
+  out = num / den;
+  return out * den == num;
+}
+
 // Memory offset (elements, inside a row of the output) of column `col`, a multiple of 8; false for
 // columns that pad an image row to whole chunks.
 // `slice`: which row of a pair.
@@ -245,7 +260,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     uint32_t phase = 0;
     bool ok = true;
     // steps of the box coordinates per tap (s, r, t) and per reduction chunk, see below
-    constexpr bool linear = kMode == TC_FPROP || kMode == TC_BPROP;
+    const bool linear = kMode == TC_FPROP || (kMode == TC_BPROP && (kStack || !p.gather));
     const bool phased = kMode == TC_FPROP && p.phase_w > 1 && !is_a;
     int ls[5] = {0, 0, 0, 0, 0}, lr[5] = {0, 0, 0, 0, 0}, lt[5] = {0, 0, 0, 0, 0}, lc[5] = {0, 0, 0, 0, 0};
     int steps_for = -1;   // form of the B box (0 per chunk, 1 merged) the steps were taken for; -1 = not yet
@@ -332,6 +347,14 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
           } else if (kMode == TC_BPROP) {
             if (is_a) {  // filter rows c0.., 64 output channels k of the tap
               c0 = rc * kChunk; c1 = tap.s; c2 = kStack ? tap.r - 1 + bi : tap.r; c3 = tap.t; c4 = m0;
+            } else if (!kStack && p.gather) {   // the same for every tap, zeros where a stride does not divide
+              bool v = cp.valid;
+              int q = 0, pp = 0, mm = 0;
+              if (p.x_tap) v &= div_exact(cp.q + p.pad_w - tap.s, p.str_w, q);
+              v &= div_exact(cp.p + p.pad_h - tap.r, p.str_h, pp);
+              v &= div_exact(cp.m + p.pad_d - tap.t, p.str_d, mm);
+              c0 = cp.inner0 + (p.x_tap ? 0 : (p.pad_w - tap.s) * p.inner_tap);
+              c1 = q; c2 = v ? pp : p.oob_y + kFarRows; c3 = mm; c4 = rc * kChunk;
             } else {     // error pixels that reach this input pixel through the tap
               c0 = cp.inner0 + (p.x_tap ? 0 : (p.pad_w - tap.s) * p.inner_tap);
               c1 = p.x_tap ? cp.q + p.pad_w - tap.s : 0;

@@ -57,6 +57,7 @@ const Tuning& tuning() {
     t.space_to_depth = num("NG_SPACE_TO_DEPTH", -1);
     t.row_stack = num("NG_ROW_STACK", -1);
     t.pack_odd = num("NG_PACK_ODD", -1);
+    t.stride_phases = num("NG_STRIDE_PHASES", -1);
     t.dependent_launch = num("NG_DEPENDENT_LAUNCH", -1);
     t.max_ctas = num("NG_MAX_CTAS", 0);
     t.conv_splits = num("NG_CONV_SPLITS", -1);
@@ -399,7 +400,7 @@ int ng_tune(const char* name, int value) {
       {"reduce_lanes", &t.reduce_lanes}, {"update_groups", &t.update_groups}, {"update_stack", &t.update_stack},
       {"update_min_stages", &t.update_min_stages}, {"max_ctas", &t.max_ctas}, {"conv_splits", &t.conv_splits},
       {"max_stages", &t.max_stages}, {"feed_bytes_per_ns", &t.feed_bytes_per_ns}, {"merge_boxes", &t.merge_boxes}, {"split_tail", &t.split_tail},
-      {"lean_kernels", &t.lean_kernels}, {"update_swap", &t.update_swap}, {"pair_mma", &t.pair_mma}, {"chan_block", &t.chan_block}, {"space_to_depth", &t.space_to_depth}, {"row_stack", &t.row_stack}, {"pack_odd", &t.pack_odd}, {"dependent_launch", &t.dependent_launch}};
+      {"lean_kernels", &t.lean_kernels}, {"update_swap", &t.update_swap}, {"pair_mma", &t.pair_mma}, {"chan_block", &t.chan_block}, {"space_to_depth", &t.space_to_depth}, {"row_stack", &t.row_stack}, {"pack_odd", &t.pack_odd}, {"stride_phases", &t.stride_phases}, {"dependent_launch", &t.dependent_launch}};
   for (const Field& f : fields)
     if (strcmp(f.name, name) == 0) {
       *f.slot = value;

@@ -562,9 +562,17 @@ def test_operand_copies_of_all_passes_share_one_scratch_buffer(ng, lib):
         ng.stream = default
 
 
+@pytest.fixture
+def by_phases(lib):
+    """Strided layers of every size in their forms by phases."""
+    assert lib.ng_tune(b"stride_phases", 2) == 0
+    yield
+    assert lib.ng_tune(b"stride_phases", -1) == 0
+
+
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
 @pytest.mark.parametrize("name", ["n24_5x5_s3", "n88_7x7_s2_c96", "n40_2x3_s3_h1", "n32_3d_s222", "n16_1x1_s2", "n8_3x3_s2"])
-def test_strided_layers_keep_infinities_from_outputs_that_do_not_meet_them(ng, name, value):
+def test_strided_layers_keep_infinities_from_outputs_that_do_not_meet_them(ng, by_phases, name, value):
     """Minibatches that are no multiple of 64: an infinity or NaN in any operand reaches what it reaches on the
     CUDA-core kernels, which skip the pixels outside the tensors that the tensor cores multiply as zeros."""
     cfg = STRIDED[name]
@@ -600,7 +608,7 @@ def test_strided_layers_keep_infinities_from_outputs_that_do_not_meet_them(ng, n
         check(bad, F, E, "u")
 
 
-def test_strided_update_in_fp16_keeps_infinities_apart_too(ng):
+def test_strided_update_in_fp16_keeps_infinities_apart_too(ng, by_phases):
     cfg = STRIDED["n24_5x5_s3"]
     cd = rm.ConvDims(*cfg)
     I, F, E = _inputs(cd, 1025)
@@ -614,3 +622,42 @@ def test_strided_update_in_fp16_keeps_infinities_apart_too(ng):
     for what in (np.isnan, np.isposinf, np.isneginf):
         assert np.array_equal(what(got[0]), what(got[1]))
     assert np.isfinite(got[1][:, :, 0]).all() and not np.isfinite(got[1]).all()
+
+
+@pytest.mark.parametrize("form", [0, 2])
+@pytest.mark.parametrize("name", sorted(STRIDED) + ["n64_3d_s222", "n24_1x3_s_h2"])
+def test_strided_layers_in_both_forms(ng, lib, name, form):
+    """Phase by phase, and in one launch: the size of the layer decides, the results do not show it."""
+    cfg = STRIDED.get(name) or {"n64_3d_s222": (64, 32, 40, 4, 6, 7, 2, 3, 3, 1, 1, 1, 2, 2, 2),
+                                "n24_1x3_s_h2": (24, 32, 40, 1, 9, 7, 1, 3, 3, 0, 1, 1, 1, 2, 1)}[name]
+    cd = rm.ConvDims(*cfg)
+    I, F, E = _inputs(cd, 1027)
+    ref = {"gradI": rm.conv_bprop_fast(cd, F, E, alpha=0.5), "gradF": rm.conv_update_fast(cd, I, E, alpha=0.5)}
+    layer = _layer(ng, cfg)
+    pad = 4096                  # guard cells
+    buf = ng.empty((layer.sizeI + 2 * pad,))
+    buf.fill(7.0)
+    dB, dU = buf[pad:pad + layer.sizeI].reshape(layer.dimI), ng.empty(layer.dimF, dtype=np.float32)
+    try:
+        assert lib.ng_tune(b"stride_phases", form) == 0
+        ng.bprop_conv(layer, ng.array(F), ng.array(E), dB, alpha=0.5)
+        ng.update_conv(layer, ng.array(I), ng.array(E), dU, alpha=0.5)
+    finally:
+        assert lib.ng_tune(b"stride_phases", -1) == 0
+    _check(cd, {"gradI": dB.get(), "gradF": dU.get()}, I, F, E, ref, "%s form %d" % (name, form))
+    guard = buf.get()
+    assert (guard[:pad] == 7.0).all() and (guard[-pad:] == 7.0).all()
+
+
+@pytest.mark.parametrize("cfg, launches", [
+    ((64, 64, 64, 1, 32, 32, 1, 4, 4, 0, 0, 0, 1, 4, 4), 1), ((128, 96, 96, 1, 55, 55, 1, 3, 3, 0, 1, 1, 1, 2, 2), 4),
+    ((8, 16, 16, 1, 8, 8, 1, 4, 4, 0, 0, 0, 1, 4, 4), 1), ((48, 64, 64, 1, 56, 56, 1, 3, 3, 0, 1, 1, 1, 2, 2), 6)])
+def test_small_strided_backward_passes_take_one_launch(ng, lib, cfg, launches):
+    import ctypes
+    layer = _layer(ng, cfg)
+    F, E, gI = ng.zeros(layer.dimF), ng.zeros(layer.dimO), ng.empty(layer.dimI)
+    before, after = ctypes.c_ulonglong(0), ctypes.c_ulonglong(0)
+    assert lib.ng_launch_count(ctypes.byref(before)) == 0
+    ng.bprop_conv(layer, F, E, gI)
+    assert lib.ng_launch_count(ctypes.byref(after)) == 0
+    assert after.value - before.value == launches
