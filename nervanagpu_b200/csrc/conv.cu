@@ -631,19 +631,6 @@ void set_update_groups(TcParams& p, int taps, int a_rows) {
   p.nz_out = taps;
 }
 
-// Partitions of a weight update that replaces a form with shorter sums. The error of an fp32 sum grows with
-// its length, so long ones run as up to `max_waves` waves of partitions instead of one. Exchanged operands:
-// 64 -> 64, 3x3x3, 16x56x56, 32 images 4.6e-5 off the sum in 64 bits (plain form 6.5e-5), 24 -> 16, 7x7,
-// 80x80, 96 images 1.5e-5 (1.8e-5; one wave 2.3e-5). Strided: 96 -> 72, 5x5, 51x51, 88 images 3.8e-6
-// (CUDA cores 4.9e-6; 85 k-blocks per partition 6.0e-6).
-int shorter_partitions(const DeviceCtx* c, long long tiles, int num_kb, int splits, long long out_elems, int max_waves) {
-  for (int w = 2; w <= max_waves && num_kb / splits > 64; ++w) {
-    const long long s = std::min<long long>(kMaxSplits, 1ll * w * c->sm_count / tiles);
-    if (s > splits && s * out_elems * 4 <= (256ll << 20)) splits = static_cast<int>(s);
-  }
-  return splits;
-}
-
 // Rows of one tap among the MMA columns of update_swapped: whole groups of 8, and no more than 16 boxes
 // per column tile (a lane of the producer warp loads each).
 int swap_rows(int C) { return std::max(16, (C + 7) / 8 * 8); }
@@ -870,7 +857,7 @@ int update_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, ChunkMode mod
   p.Cold = nullptr; p.ldc = ld; p.c_zstride = 0;
   p.alpha = alpha; p.beta = 0.0f; p.relu = 0; p.sr_bits = 0; p.out_f32 = 1; p.vec_ok = 1;
   p.splits = choose_splits(c, p.tiles_n, p.num_kb, 1ll * g.K * ld);
-  if (!blocks) p.splits = shorter_partitions(c, tiles, p.num_kb, p.splits, 1ll * g.K * ld, 2);
+  if (!blocks) p.splits = shorter_partitions(c, tiles, p.num_kb, p.splits, 1ll * g.K * ld, 2, 64);
   // behind the partials: the gradient in tap order and copies of the operands. (Not in the second buffer,
   // where I and the gradient of a layer that was rewritten by space to depth lie.)
   const size_t bytes[3] = {(static_cast<size_t>(g.K) * ld * 4 + 255) & ~size_t(255),
@@ -1166,6 +1153,13 @@ bool bprop_by_phases(DeviceCtx* c, const Geo& g, bool in_place) {
 // 7x7 / 3, 19x19, 8 images (9.8 MB, 6.6) 18 / 21; 512 -> 512, 3x3 / 3, 22x22, 32 images (18 MB, 1.2) 41 / 34; 64 -> 64, 3x3 / 2, 56x56,
 // 24 images (22 MB, 2.3) 27 / 29; 512 -> 512, 1x1 / 2, 34x34, 96 images (27 MB, 0.25) 76 / 45; 96 -> 512, 3x3 / 4, 85x85, 48 images
 // (38 MB, 0.6) 58 / 54; 256 -> 64, 2x2 / 2, 62x62, 32 images (64 MB, 1.1) 46 / 61; 96 -> 72, 5x5 / 2, 51x51, 88 images (1.1 GB, 6.3) 91 / 218.
+// Longest partitions (k-blocks) of the strided updates' sums, so that no gradient is further off the sum in 64
+// bits than on the paths these forms replace: patches in one wave / phase-split with up to 64 /
+// now, in units of 1e-7: 128 -> 128, 1x1 / 2, 57x57, 120 images 8.5 / 8.2 / 7.9; 512 -> 512, 1x1 / 2, 34x34, 96 images 18.7 / 11.0 / 9.5;
+// 128 -> 256, 3x3 / 2, 41x41, 40 images 13.0 / 13.2 / 7.3; 64 -> 64, 3x3 / 2, 14x14, 16 images 3.8 / 3.4 / 2.6; 96 -> 72, 5x5 / 2,
+// 51x51, 88 images 47 / 42 / 33. The longer second stage costs 2 % over 70 layers (32 -> 16, 1x1 / 2, 75x75, 96
+// images 23 -> 29 us).
+constexpr int kLongSum = 16, kLongPatchSum = 3;
 constexpr long long kPatchBytes = 8ll << 20;
 bool update_by_phases(const Geo& g) {
   if (tuning().stride_phases >= 0) return tuning().stride_phases != 0;
@@ -1482,7 +1476,7 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
     p.alpha = alpha; p.beta = 0.0f; p.relu = 0; p.sr_bits = 0; p.out_f32 = out_f32; p.vec_ok = 1;
     p.splits = choose_splits(c, 1ll * p.tiles_m * p.tiles_n * p.nz, p.num_kb, 1ll * g.C * g.K * RST);
     if (phased)
-      p.splits = shorter_partitions(c, 1ll * p.tiles_m * p.tiles_n * p.nz, p.num_kb, p.splits, 1ll * g.C * g.K * RST, 4);
+      p.splits = shorter_partitions(c, 1ll * p.tiles_m * p.tiles_n * p.nz, p.num_kb, p.splits, 1ll * g.C * g.K * RST, 4, kLongSum);
     CUtensorMap mapA, mapB;
     // large channel planes: the product reads copies in (z, y, chan, x, n) order
     const bool blocked_i = !phased && wants_chan_block(g.D, g.H, g.W, g.N, RST);
@@ -1524,6 +1518,7 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
     gc.k = static_cast<int>(span);
     gc.lda = span; gc.ldb = span; gc.ldc = g.K;
     gc.alpha = alpha; gc.beta = 0.0f; gc.batch = 1; gc.loops = 1; gc.out_f32 = out_f32;
+    if (mode == CH_NONE) gc.long_kb = kLongPatchSum;
     return run_gemm(gc, stream);
   }
   const long long warps = g.sizeF();

@@ -262,6 +262,8 @@ int run_gemm(const GemmCall& call, cudaStream_t stream) {
   p.seed_lo = ea.seed_lo; p.seed_hi = ea.seed_hi; p.rng_offset = g.rng_offset;
   p.splits = choose_splits(c, static_cast<long long>(p.tiles_m) * p.tiles_n * p.nz, p.num_kb,
                            static_cast<long long>(g.m) * g.n * g.batch);
+  if (g.long_kb > 0)
+    p.splits = shorter_partitions(c, 1ll * p.tiles_m * p.tiles_n * p.nz, p.num_kb, p.splits, 1ll * g.m * g.n * g.batch, 2, g.long_kb);
   if (p.splits > 1 && (g.n & 7)) {
     // partials with whole 16-byte groups per row: they leave through the staged output stage, and
     // the second stage stores the columns that exist

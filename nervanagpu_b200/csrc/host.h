@@ -135,6 +135,8 @@ void tc_pick_tile(const DeviceCtx* c, TcParams& p, long long cols, int num_kb, i
 // Picks the number of split-K partitions for `tiles` output tiles and `num_kb` k-blocks.
 constexpr int kMaxSplits = 160;
 int choose_splits(const DeviceCtx* c, long long tiles, int num_kb, long long out_elems, bool charge_reduction = false);
+// The same for a sum that replaces one with shorter partitions (see tc_host.cu).
+int shorter_partitions(const DeviceCtx* c, long long tiles, int num_kb, int splits, long long out_elems, int max_waves, int long_kb);
 
 // One GEMM request: C[m x n] = epilogue(op(A) * op(B)); see ng_hgemm for the conventions.
 struct GemmCall {
@@ -153,6 +155,7 @@ struct GemmCall {
   long long alz, blz;
   int out_f32;
   int force_simt;
+  int long_kb;               // > 0: partitions of no more k-blocks than this, in up to two waves (shorter_partitions)
 };
 int run_gemm(const GemmCall& g, cudaStream_t stream);
 

@@ -267,6 +267,18 @@ int choose_splits(const DeviceCtx* c, long long tiles, int num_kb, long long out
   return static_cast<int>(best);
 }
 
+// Partitions of a weight update that replaces a form with shorter sums. The error of an fp32 sum grows with
+// its length: partitions of more than `long_kb` k-blocks run as up to `max_waves` waves of shorter ones. Exchanged
+// operands: 64 -> 64, 3x3x3, 16x56x56, 32 images 4.6e-5 off the sum in 64 bits (plain form 6.5e-5), 24 -> 16, 7x7,
+// 80x80, 96 images 1.5e-5 (1.8e-5; one wave 2.3e-5). Strided layers: see kLongSum.
+int shorter_partitions(const DeviceCtx* c, long long tiles, int num_kb, int splits, long long out_elems, int max_waves, int long_kb) {
+  for (int w = 1; w <= max_waves && num_kb / splits > long_kb; ++w) {
+    const long long s = std::min<long long>(std::min(kMaxSplits, num_kb / 2), 1ll * w * c->sm_count / tiles);
+    if (s > splits && s * out_elems * 4 <= (256ll << 20)) splits = static_cast<int>(s);
+  }
+  return splits;
+}
+
 // Threads that share one 8-column group of the split-K reduction: more when the output is small
 // and the partitions many, so that the device is filled and no thread walks a long chain.
 static int splitk_reduce_lanes(long long groups, int splits, int sm_count) {

@@ -661,3 +661,40 @@ def test_small_strided_backward_passes_take_one_launch(ng, lib, cfg, launches):
     ng.bprop_conv(layer, F, E, gI)
     assert lib.ng_launch_count(ctypes.byref(after)) == 0
     assert after.value - before.value == launches
+
+
+STRIDED_SUMS = {
+    # name: layer, longest partition of its sums in k-blocks of 64: patches (at most 3), a phase-split copy (294 k-blocks
+    # in 32 partitions)
+    "c64_3x3_n16_patches": ((16, 64, 64, 1, 14, 14, 1, 3, 3, 0, 1, 1, 1, 2, 2), 3),
+    "c128_1x1_n24_patches": ((24, 128, 128, 1, 28, 28, 1, 1, 1, 0, 0, 0, 1, 2, 2), 3),
+    "c24_3x3_n96_patches": ((96, 24, 512, 1, 13, 13, 1, 3, 3, 0, 1, 1, 1, 2, 2), 3),
+    "c128_3x3_n40_phases": ((40, 128, 256, 1, 41, 41, 1, 3, 3, 0, 1, 1, 1, 2, 2), 10),
+}
+
+
+@pytest.mark.parametrize("name", sorted(STRIDED_SUMS))
+def test_strided_gradients_are_summed_in_short_partitions(ng, name):
+    """Against sums in 64 bits. Each of the four MMAs of a k-block cuts its sum to 24 bits: 0.36 2^-23 of it on average. A
+    partition's sum grows like a random walk, so that the sums cut are two thirds of its end on average, and the
+    partitions' errors, like their ends, add as a random walk: 4 * 0.36 * 2/3 * 2^-23 of the result per k-block."""
+    cfg, longest = STRIDED_SUMS[name]
+    cd = rm.ConvDims(*cfg)
+    rng = np.random.default_rng(1029)
+    I = rng.uniform(0, 1, cd.dimI).astype(np.float16)
+    E = rng.normal(0, 0.1, cd.dimO).astype(np.float16)
+    layer = _layer(ng, cfg)
+    dU = ng.empty(layer.dimF, dtype=np.float32)
+    ng.update_conv(layer, ng.array(I), ng.array(E), dU)
+    N, C, K, _, H, W, _, R, S = cfg[:9]
+    pad, st = cfg[10], cfg[13]
+    _, P, Q = cd.MPQ
+    padded = np.zeros((C, H + 2 * pad + st, W + 2 * pad + st, N))
+    padded[:, pad:pad + H, pad:pad + W] = I[:, 0]
+    e = E.astype(np.float64).reshape(K, -1)
+    ref = np.empty((C, 1, R, S, K))
+    for r in range(R):
+        for s in range(S):
+            ref[:, 0, r, s] = padded[:, r:r + P * st:st, s:s + Q * st:st][:, :P, :Q].reshape(C, -1) @ e.T
+    got = dU.get().astype(np.float64)
+    assert np.linalg.norm(got - ref) <= 4 * 0.36 * 2 / 3 * 2.0 ** -23 * longest * np.linalg.norm(ref)
