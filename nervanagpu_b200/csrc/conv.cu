@@ -235,12 +235,14 @@ void fill_phases(TcParams& p, const Geo& g) {
 
 // Room for the copies behind the split-K partials of the product `p` (whose tiling and number of
 // partitions are final): `n` copies of the given sizes, returned as pointers into the workspace.
-int chan_block_room(DeviceCtx* c, cudaStream_t stream, const TcParams& p, const size_t* bytes, void** ptrs, int n) {
+// NG_ERR_TOO_LARGE: none to be had, for a product that has a form without scratch (`optional`).
+int chan_block_room(DeviceCtx* c, cudaStream_t stream, const TcParams& p, const size_t* bytes, void** ptrs, int n, bool optional = false) {
   const int nz_out = p.nz_out < 1 ? p.nz : p.nz_out;
   size_t off = p.splits > 1 ? static_cast<size_t>(p.splits) * nz_out * p.M * p.N * sizeof(float) : 0;
   off = (off + 255) & ~size_t(255);
   size_t total = off;
   for (int i = 0; i < n; ++i) total += bytes[i];
+  if (optional && !scratch_or_none(c, stream, total)) return NG_ERR_TOO_LARGE;
   const int rc = ensure_workspace(c, stream, total);
   if (rc != NG_OK) return rc;
   for (int i = 0; i < n; ++i) {
@@ -864,7 +866,7 @@ int update_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, ChunkMode mod
                            phased ? phase_split_bytes(g) : (blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0),
                            blocked_e ? chan_block_bytes(g.K, g.M, g.P, g.Q, g.N) : 0};
   void* room[3] = {nullptr, nullptr, nullptr};
-  int rc = chan_block_room(c, stream, p, bytes, room, 3);
+  int rc = chan_block_room(c, stream, p, bytes, room, 3, phased);
   if (rc != NG_OK) return rc;
   float* Dt = static_cast<float*>(room[0]);
   p.C = Dt;
@@ -1248,19 +1250,20 @@ int ng_conv_fprop(const ng_conv_desc* d, const void* I, const void* F, void* O, 
       return run_gemm(gc, stream);
     }
   }
-  if (!tc) {
+  auto cuda_cores = [&]() -> int {
     count_fallback_launch();
     conv_fprop_simt<<<launch_1d(g.sizeO(), 256, c), 256, 0, stream>>>(
         g, static_cast<const __half*>(I), static_cast<const __half*>(F), static_cast<__half*>(O), alpha, relu, nullptr, 0);
     NG_CHECK_LAUNCH();
     return NG_OK;
-  }
+  };
+  if (!tc) return cuda_cores();
   const int RST = g.T * g.R * g.S;
   const long long ldo = 1ll * g.M * g.P * g.Q * g.N;
   TcParams p = {};
   p.mode = TC_FPROP;
   const long long cols = pixel_columns(p, 1ll * g.M * g.P, g.Q, g.N, mode);
-  if (cols > 0x7fffffffll) return fail(NG_ERR_TOO_LARGE, "output too large");
+  if (cols > 0x7fffffffll) return phased ? cuda_cores() : fail(NG_ERR_TOO_LARGE, "output too large");
   p.M = g.K; p.N = static_cast<int>(cols);
   p.nz = 1; p.splits = 1;
   TcOperandLayout lay = {1, 1, pick_kb_rows(g.C)};
@@ -1300,7 +1303,8 @@ int ng_conv_fprop(const ng_conv_desc* d, const void* I, const void* F, void* O, 
     const size_t bytes[2] = {phase_split_bytes(g), kScanFlags * sizeof(int)};
     void* room[2] = {nullptr, nullptr};
     int scans = 0;
-    rc = chan_block_room(c, stream, p, bytes, room, 2);
+    rc = chan_block_room(c, stream, p, bytes, room, 2, true);
+    if (rc == NG_ERR_TOO_LARGE) return cuda_cores();
     int* flags = static_cast<int*>(room[1]);
     if (rc == NG_OK) rc = phase_split(g, I, room[0], F, flags, &scans, stream);
     if (rc == NG_OK) rc = phase_map(&mapB, room[0], g, lay.kb_rows);
@@ -1340,18 +1344,16 @@ int ng_conv_bprop(const ng_conv_desc* d, const void* F, const void* E, void* gra
   const bool addressable = path != NG_PATH_SIMT && (in_place || path == NG_PATH_AUTO) && aligned16(F) && aligned16(E) && aligned16(gradI);
   if (path == NG_PATH_TENSOR && !addressable) return fail(NG_ERR_UNSUPPORTED, "shape not addressable by the tensor-core path");
   const bool by_phases = addressable && bprop_by_phases(c, g, in_place);
-  if (!addressable || !(by_phases || in_place)) {
-    if (!addressable) count_fallback_launch();
+  auto cuda_cores = [&](bool counted) -> int {
+    if (counted) count_fallback_launch();
     conv_bprop_simt<<<launch_1d(g.sizeI(), 256, c), 256, 0, stream>>>(
         g, static_cast<const __half*>(F), static_cast<const __half*>(E), static_cast<__half*>(gradI), alpha, nullptr, 0);
     NG_CHECK_LAUNCH();
     return NG_OK;
-  }
+  };
+  if (!addressable || !(by_phases || in_place)) return cuda_cores(!addressable);
   const int str[3] = {g.str_d, g.str_h, g.str_w}, flt[3] = {g.T, g.R, g.S};
   const bool gather = !by_phases;
-  // a phase that no tap falls on, because the stride is larger than the filter, gets no error at all
-  if (!gather && (str[0] > flt[0] || str[1] > flt[1] || str[2] > flt[2]))
-    NG_CUDA(cudaMemsetAsync(gradI, 0, static_cast<size_t>(g.sizeI()) * 2, stream));
   const bool blocked = wants_chan_block(g.M, g.P, g.Q, g.N, g.T * g.R * g.S);
   auto phases = [&](BpropPlan* plan) -> int {
     for (int pt = 0; pt < (gather ? 1 : std::min(str[0], flt[0])); ++pt)
@@ -1369,10 +1371,13 @@ int ng_conv_bprop(const ng_conv_desc* d, const void* F, const void* E, void* gra
   if (blocked || scan) {   // behind the products' partials: the copy of E, the flags
     BpropPlan plan;
     rc = phases(&plan);
+    if (rc == NG_ERR_TOO_LARGE && scan) return cuda_cores(true);
     if (rc != NG_OK) return rc;
     const size_t off = round256(plan.partials);
     const size_t copy_bytes = blocked ? chan_block_bytes(g.K, g.M, g.P, g.Q, g.N) : 0;
-    rc = ensure_workspace(c, stream, off + copy_bytes + kScanFlags * sizeof(int));
+    const size_t bytes = off + copy_bytes + kScanFlags * sizeof(int);
+    if (scan && !scratch_or_none(c, stream, bytes)) return cuda_cores(true);
+    rc = ensure_workspace(c, stream, bytes);
     if (rc != NG_OK) return rc;
     uint8_t* room = reinterpret_cast<uint8_t*>(c->ws) + off;
     if (blocked) {   // large channel planes: the products read a copy in (z, y, chan, x, n) order
@@ -1386,6 +1391,9 @@ int ng_conv_bprop(const ng_conv_desc* d, const void* F, const void* E, void* gra
       if (rc != NG_OK) return rc;
     }
   }
+  // a phase that no tap falls on, because the stride is larger than the filter, gets no error at all
+  if (!gather && (str[0] > flt[0] || str[1] > flt[1] || str[2] > flt[2]))
+    NG_CUDA(cudaMemsetAsync(gradI, 0, static_cast<size_t>(g.sizeI()) * 2, stream));
   rc = phases(nullptr);
   if (rc != NG_OK || !scan) return rc;
   return launch_dependent(redo_blocks(c), stream, conv_bprop_simt, g, static_cast<const __half*>(F), static_cast<const __half*>(E0),
@@ -1437,6 +1445,12 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
       return NG_OK;
     }
   }
+  auto cuda_cores = [&, I0 = static_cast<const __half*>(I), E0 = static_cast<const __half*>(E)]() -> int {
+    count_fallback_launch();
+    conv_update_simt<<<launch_1d(g.sizeF() * 32, 256, c), 256, 0, stream>>>(g, I0, E0, gradF, out_f32, alpha);
+    NG_CHECK_LAUNCH();
+    return NG_OK;
+  };
   auto redo = [&, I0 = static_cast<const __half*>(I), E0 = static_cast<const __half*>(E)] {   // (see phase_split)
     return launch_dependent(redo_blocks(c), stream, conv_update_redo, g, I0, E0, gradF, out_f32, alpha);
   };
@@ -1444,6 +1458,7 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
     TapBlock taps;
     taps.bw = taps.bh = 1; taps.rows = swap_rows(g.C); taps.nr = g.R; taps.ns = g.S; taps.ok = true;
     rc = update_swapped(c, g, taps, mode, phased, I, E, gradF, out_f32, alpha, stream);
+    if (rc == NG_ERR_TOO_LARGE && phased) return cuda_cores();
     return rc == NG_OK && phased ? redo() : rc;
   }
   if (direct) {
@@ -1485,7 +1500,8 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
       const size_t bytes[2] = {phased ? phase_split_bytes(g) : blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0,
                                blocked_e ? chan_block_bytes(g.K, g.M, g.P, g.Q, g.N) : 0};
       void* copies[2] = {nullptr, nullptr};
-      rc = chan_block_room(c, stream, p, bytes, copies, 2);
+      rc = chan_block_room(c, stream, p, bytes, copies, 2, phased);
+      if (rc == NG_ERR_TOO_LARGE && phased) return cuda_cores();
       if (rc == NG_OK && phased) rc = phase_split(g, I, copies[0], nullptr, nullptr, nullptr, stream);
       if (rc == NG_OK && blocked_i) rc = chan_block(c, stream, I, copies[0], g.C, g.D, g.H, g.W, g.N);
       if (rc == NG_OK && blocked_e) rc = chan_block(c, stream, E, copies[1], g.K, g.M, g.P, g.Q, g.N);
@@ -1521,12 +1537,7 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
     if (mode == CH_NONE) gc.long_kb = kLongPatchSum;
     return run_gemm(gc, stream);
   }
-  const long long warps = g.sizeF();
-  count_fallback_launch();
-  conv_update_simt<<<launch_1d(warps * 32, 256, c), 256, 0, stream>>>(
-      g, static_cast<const __half*>(I), static_cast<const __half*>(E), gradF, out_f32, alpha);
-  NG_CHECK_LAUNCH();
-  return NG_OK;
+  return cuda_cores();
 }
 
 }  // extern "C"

@@ -7,7 +7,8 @@
 // dimension or batch stride no multiple of 8 elements) are first copied into rows that it can
 // (pack_rows_kernel). The plain CUDA-core kernel serves very short products of such operands
 // (shorter_unpacked), operands of more than 2^30 packed groups, calls that are both batched and summed
-// over a batch, and ng_hgemm_simt, the second opinion of the tests.
+// over a batch, packed and summed products for which there is no scratch memory, and ng_hgemm_simt, the
+// second opinion of the tests.
 #include <algorithm>
 
 #include "../../include/nervana_b200.h"
@@ -209,7 +210,7 @@ int run_gemm(const GemmCall& call, cudaStream_t stream) {
   if (use_tc && !tma_ok(g.B, g.ldb, zsb))
     use_tc = plan_pack(packB, g.B, g.ldb, zsb, nzb, g.b_t ? g.n : g.k, g.b_t ? g.k : g.n);
   const bool by_rule = use_tc && (packA.total || packB.total) && shorter_unpacked(c, g);
-  if (!use_tc || by_rule) {
+  auto cuda_cores = [&](bool counted) -> int {
     SimtGemmArgs s;
     s.A = static_cast<const __half*>(g.A); s.B = static_cast<const __half*>(g.B); s.C = g.C;
     s.a_t = g.a_t; s.b_t = g.b_t; s.m = g.m; s.n = g.n; s.k = g.k;
@@ -217,11 +218,12 @@ int run_gemm(const GemmCall& call, cudaStream_t stream) {
     s.az = g.az; s.bz = g.bz; s.cz = g.cz; s.loops = g.loops; s.alz = g.alz; s.blz = g.blz;
     s.out_f32 = g.out_f32; s.ea = ea;
     dim3 grid((g.n + 63) / 64, (g.m + 63) / 64, g.batch);
-    if (!by_rule) count_fallback_launch();
+    if (counted) count_fallback_launch();
     gemm_simt_kernel<<<grid, 256, 0, stream>>>(s);
     NG_CHECK_LAUNCH();
     return NG_OK;
-  }
+  };
+  if (!use_tc || by_rule) return cuda_cores(!by_rule);
 
   TcParams p = {};
   p.mode = TC_GEMM;
@@ -270,12 +272,13 @@ int run_gemm(const GemmCall& call, cudaStream_t stream) {
     p.n_store = g.n;
     p.N = (g.n + 7) & ~7;
   }
+  size_t off = p.splits > 1 ? static_cast<size_t>(p.splits) * p.nz * p.M * p.N * sizeof(float) : 0;
+  off = (off + 255) & ~size_t(255);
+  const size_t bytesA = (static_cast<size_t>(packA.total) * 16 + 255) & ~size_t(255);
+  const size_t room_bytes = off + bytesA + static_cast<size_t>(packB.total) * 16;
+  // (without room, the kernel that needs none)
+  if ((packA.total || packB.total || sum) && room_bytes > 0 && !scratch_or_none(c, stream, room_bytes)) return cuda_cores(true);
   if (packA.total || packB.total) {
-    size_t off = p.splits > 1 ? static_cast<size_t>(p.splits) * p.nz * p.M * p.N * sizeof(float) : 0;
-    off = (off + 255) & ~size_t(255);
-    const size_t bytesA = (static_cast<size_t>(packA.total) * 16 + 255) & ~size_t(255);
-    int rc = ensure_workspace(c, stream, off + bytesA + static_cast<size_t>(packB.total) * 16);
-    if (rc != NG_OK) return rc;
     uint8_t* room = reinterpret_cast<uint8_t*>(c->ws) + off;
     if (packA.total) {
       packA.dst = reinterpret_cast<uint4*>(room);

@@ -82,6 +82,9 @@ DeviceCtx* current_ctx();
 // Ensure the workspace of `stream` holds at least `bytes` and make c->ws point at it; may
 // synchronise the device when it has to grow.
 int ensure_workspace(DeviceCtx* c, cudaStream_t stream, size_t bytes);
+// The same for a call that has a form without scratch: false when there is none to be had (an open capture on
+// a stream whose buffer would have to grow, or no device memory), with no error left behind.
+bool scratch_or_none(DeviceCtx* c, cudaStream_t stream, size_t bytes);
 // Hold on the second buffer of a stream, for as long as what lies in it is needed. It has one holder: a call
 // that an outer call of the same thread makes meanwhile is refused room there (growing would free the
 // outer call's operands, and what fits would be laid over them).

@@ -145,6 +145,12 @@ int ensure_workspace(DeviceCtx* c, cudaStream_t stream, size_t bytes) {
   return NG_OK;
 }
 
+bool scratch_or_none(DeviceCtx* c, cudaStream_t stream, size_t bytes) {
+  if (ensure_workspace(c, stream, bytes) == NG_OK) return true;
+  cudaGetLastError();
+  return false;
+}
+
 // (one call works on one stream, so a thread holds at most one)
 static thread_local bool t_aux_held = false;
 

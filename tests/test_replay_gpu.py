@@ -4,6 +4,7 @@ import pytest
 
 from nervanagpu_b200 import NervanaGPU, _lib
 from nervanagpu_b200.convnet import ConvStack
+from oracle import reference_math as rm
 
 pytestmark = pytest.mark.gpu
 
@@ -132,3 +133,42 @@ def test_network_driver_runs_a_small_network_through_the_layer_classes():
     assert set(res) == {"fprop", "bprop", "total"}
     assert all(ms > 0 and gflops > 0 for ms, gflops in res.values())
     assert sum(l.startswith("Avg(2)") for l in lines) == 3
+
+
+def test_calls_that_need_no_scratch_can_be_recorded_on_a_cold_stream(ng, lib):
+    """Operands at odd addresses, products summed over a batch and strided layers of a minibatch that is no
+    multiple of 64 have forms without scratch memory; a stream that has none yet records those."""
+    rng = np.random.default_rng(41)
+    A, B = rng.standard_normal((65, 131)).astype(np.float16), rng.standard_normal((131, 77)).astype(np.float16)
+    A3, B3 = rng.standard_normal((40, 64, 64)).astype(np.float16), rng.standard_normal((40, 64, 64)).astype(np.float16)
+    cfg = (24, 40, 72, 1, 17, 14, 1, 5, 5, 0, 2, 2, 1, 3, 3)
+    cd = rm.ConvDims(*cfg)
+    I = rng.uniform(0, 1, cd.dimI).astype(np.float16)
+    F = rng.normal(0, 0.1, cd.dimF).astype(np.float16)
+    E = (rng.uniform(-1, 1, cd.dimO) * 0.125).astype(np.float16)
+    layer = ng.conv_layer(np.float16, *cfg)
+    dA, dB, dA3, dB3, dI, dF, dE = (ng.array(x) for x in (A, B, A3, B3, I, F, E))
+    C, S = ng.empty((65, 77)), ng.empty((64, 64))
+    O, gI, gF = ng.empty(layer.dimO), ng.empty(layer.dimI), ng.empty(layer.dimF, dtype=np.float32)
+    calls = [(lambda: ng.dot(dA, dB, C), C, A.astype(np.float32) @ B.astype(np.float32)),
+             (lambda: ng.batched_dot(dA3, dB3, S), S, np.matmul(A3.astype(np.float32), B3.astype(np.float32)).sum(axis=0)),
+             (lambda: ng.fprop_conv(layer, dI, dF, O), O, rm.conv_fprop_fast(cd, I, F)),
+             (lambda: ng.bprop_conv(layer, dF, dE, gI), gI, rm.conv_bprop_fast(cd, F, E)),
+             (lambda: ng.update_conv(layer, dI, dE, gF), gF, rm.conv_update_fast(cd, I, E))]
+    default = ng.stream
+    try:
+        assert lib.ng_tune(b"stride_phases", 2) == 0
+        for call, out, ref in calls:
+            ng.stream = ng.new_stream()
+            sequence = ng.capture(call)
+            sequence.launch()
+            ng.synchronize()
+            recorded = out.get().astype(np.float32)
+            out.fill(0)
+            call()                  # and its usual form
+            ng.synchronize()
+            for got in (recorded, out.get().astype(np.float32)):
+                assert np.abs(got - ref).max() <= 4e-3 * np.abs(ref).max() + 1e-3
+    finally:
+        assert lib.ng_tune(b"stride_phases", -1) == 0
+        ng.stream = default
