@@ -561,8 +561,11 @@ __global__ void __launch_bounds__(256) pool2d_gather_kernel(Plane2d g, int BW, c
             const int s = (WQ - 1 - wq) * SW + dx;
             if (s >= S) continue;
 #pragma unroll
-            for (int i = 0; i < V; ++i)
-              if (kAvg || idx[i] == static_cast<uint32_t>(r * S + s)) acc[l][dy][dx][i] += e[i];
+            for (int i = 0; i < V; ++i) {
+              // (the mean's shares one by one, as in the general kernel: their sum may exceed fp32 where none of them does)
+              if (kAvg) acc[l][dy][dx][i] = fmaf(e[i], 1.0f / static_cast<float>(R * S), acc[l][dy][dx][i]);
+              else if (idx[i] == static_cast<uint32_t>(r * S + s)) acc[l][dy][dx][i] += e[i];
+            }
           }
         }
     }
@@ -578,10 +581,6 @@ __global__ void __launch_bounds__(256) pool2d_gather_kernel(Plane2d g, int BW, c
         const int x = b * SW + dx - PW;
         if (x < 0 || x >= g.W) continue;
         Vec16<T> v;
-        if (kAvg) {
-#pragma unroll
-          for (int i = 0; i < V; ++i) acc[l][dy][dx][i] *= 1.0f / static_cast<float>(R * S);
-        }
         v.from_float(acc[l][dy][dx]);
         v.store(dI + ((static_cast<long long>(blockIdx.y) * g.H + y) * g.W + x) * g.N + n0);
       }

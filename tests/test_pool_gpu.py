@@ -257,3 +257,27 @@ def test_zeros_of_both_signs_keep_the_first(ng, dtype, shift, shape):
     ng.fprop_pool(L, I, O)
     bits = np.uint16 if dtype is np.float16 else np.uint32
     assert np.array_equal(O.get().view(bits), ref.view(bits))
+
+
+@pytest.mark.parametrize("dtype", [np.float16, np.float32])
+@pytest.mark.parametrize("name", sorted(WINDOWS))
+def test_mean_passes_errors_on_as_the_general_kernel_does(ng, dtype, name):
+    """Bit for bit, and without an infinity from errors whose sum is out of range while their shares are not."""
+    R, st, pad = WINDOWS[name]
+    L = ng.pool_layer(dtype, "avg", 16, 3, 1, 11, 12, 1, 1, R, R, 0, 0, pad, pad, 1, 1, st, st)
+    rng = np.random.default_rng(8)
+    largest = float(np.finfo(dtype).max)
+    e = (rng.uniform(0.4, 0.9, L.dimO) * largest).astype(dtype)
+    e[1] = rng.normal(0, 1, L.dimO[1:]).astype(dtype)
+    n_in, n_out = int(np.prod(L.dimI)), int(np.prod(L.dimO))
+    got = []
+    for shift in (0, 1):       # tensors one element off a 16-byte boundary run on the general kernel
+        I = ng.empty((n_in + 8,), dtype=dtype)[shift:shift + n_in].reshape(L.dimI)
+        I.fill(0)
+        B = ng.empty((n_in + 8,), dtype=dtype)[shift:shift + n_in].reshape(L.dimI)
+        E = ng.empty((n_out + 8,), dtype=dtype)[shift:shift + n_out].reshape(L.dimO).set(e)
+        ng.bprop_pool(L, I, E, B)
+        got.append(B.get())
+    assert np.isfinite(got[1]).all()
+    bits = np.uint16 if dtype is np.float16 else np.uint32
+    assert np.array_equal(got[0].view(bits), got[1].view(bits))
