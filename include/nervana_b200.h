@@ -111,7 +111,7 @@ int ng_graph_destroy(void* graph);
 int ng_hgemm(const void* A, const void* B, void* C, int a_t, int b_t, int m, int n, int k, int lda, int ldb, int ldc,
              float alpha, float beta, int relu, int sr_bits, unsigned long long seed, unsigned int rng_offset,
              void* stream);
-/* Same contract, always on the SIMT kernel that serves operands TMA cannot address. */
+/* Same contract, always on the plain CUDA-core kernel (the second opinion of the tests). */
 int ng_hgemm_simt(const void* A, const void* B, void* C, int a_t, int b_t, int m, int n, int k, int lda, int ldb,
                   int ldc, float alpha, float beta, int relu, int sr_bits, unsigned long long seed,
                   unsigned int rng_offset, void* stream);

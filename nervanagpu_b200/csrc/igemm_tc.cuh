@@ -122,7 +122,8 @@ struct TcParams {
   int out_f32;
   int vec_ok;                      // rows are 16-byte aligned for vector access
   int store_staged;                // 1: tiles leave through swizzled shared memory, written out in
-                                   // whole 128-byte rows; 0: stored straight from registers
+                                   // whole 128-byte rows; 2 (products): the same, row by row in single
+                                   // elements, for rows at any address; 0: stored straight from registers
   int c_box_cols;                  // columns per staged box (128 bytes worth: 64 fp16 / 32 fp32)
   ColumnMap cmap;                  // convolution outputs
   uint32_t seed_lo, seed_hi, rng_offset;

@@ -107,14 +107,6 @@ struct Tensor {
     for (int i = 0; i < nd; ++i) n *= shape[i];
     return n;
   }
-  bool contiguous() const {
-    long long want = 1;
-    for (int i = nd - 1; i >= 0; --i) {
-      if (strides[i] != want) return false;
-      want *= shape[i];
-    }
-    return true;
-  }
 };
 
 bool read_dims(PyObject* seq, long long* out, int& n) {

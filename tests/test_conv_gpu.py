@@ -271,7 +271,9 @@ def test_update_im2col_path(ng, name):
 
 
 def test_shapes_outside_the_tensor_path_run_on_simt(ng):
-    cfg = (8, 24, 16, 1, 5, 5, 1, 3, 3, 0, 1, 1, 1, 2, 2)   # N = 8 with a W stride: no 64-element chunks
+    # N = 8 with a W stride: no 64-element chunks in place. The forward pass reads a copy that has them, the small
+    # update a patch matrix, and the small backward pass runs on the CUDA cores.
+    cfg = (8, 24, 16, 1, 5, 5, 1, 3, 3, 0, 1, 1, 1, 2, 2)
     cd = rm.ConvDims(*cfg)
     I, F, E = _inputs(cd, 5)
     ref = {"O": rm.conv_fprop(cd, I, F), "gradI": rm.conv_bprop(cd, F, E), "gradF": rm.conv_update(cd, I, E)}
@@ -698,3 +700,25 @@ def test_strided_gradients_are_summed_in_short_partitions(ng, name):
             ref[:, 0, r, s] = padded[:, r:r + P * st:st, s:s + Q * st:st][:, :P, :Q].reshape(C, -1) @ e.T
     got = dU.get().astype(np.float64)
     assert np.linalg.norm(got - ref) <= 4 * 0.36 * 2 / 3 * 2.0 ** -23 * longest * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("name", sorted(STRIDED))
+def test_strided_layers_by_phases(ng, lib, by_phases, name):
+    test_strided_layers_run_on_the_tensor_core_path(ng, lib, name)
+
+
+@pytest.mark.parametrize("name", ["c40_k72_5x5_s2", "c40_k64_3x5_s3_n24"])
+def test_two_image_rows_per_tile_by_phases(ng, lib, by_phases, name):
+    test_two_image_rows_per_tile(ng, lib, name)
+    test_two_image_rows_per_tile_give_the_bits_of_one(ng, lib, name)
+
+
+@pytest.mark.parametrize("half", [False, True])
+@pytest.mark.parametrize("name", ["c48_k128_5x5_s2_n24"])
+def test_update_with_exchanged_operands_by_phases(ng, lib, by_phases, name, half):
+    test_update_with_exchanged_operands(ng, lib, name, half)
+
+
+@pytest.mark.parametrize("name", ["n24_5x5_s3", "n40_2x3_s3_h1", "n8_3x3_s2", "n24_odd_rows_s2"])
+def test_strided_update_keeps_nan_to_the_taps_it_meets_by_phases(ng, by_phases, name):
+    test_strided_update_keeps_nan_to_the_taps_it_meets(ng, name)

@@ -29,7 +29,7 @@ def _dot(ng, A, B, op, C0=None, **kw):
 @pytest.mark.parametrize("op", ["nn", "nt", "tn"])
 def test_known_answers_all_ones_and_zeros(ng, size, op):
     """The reference's C smoke test (kernels/C_interface/test.cu:27-55,70): edge tiles, aligned and
-    unaligned leading dimensions (the latter run on the SIMT kernel)."""
+    unaligned leading dimensions (the latter are packed, and run on the SIMT kernel when very short)."""
     ones = np.ones((size, size), dtype=np.float16)
     assert (_dot(ng, ones, ones, op) == size).all()
     zeros = np.zeros((size, size), dtype=np.float16)
