@@ -113,9 +113,9 @@ int act_map(CUtensorMap* m, const void* base, int chan, int Z, int Y, int X, int
 // A TMA box of an activation tensor is [channels][64 elements]: one 128-byte row per channel, the
 // rows one channel plane (z * y * x * n elements) apart. When a plane is larger than a 2 MB page
 // every row of every box lies in another page, and the loads run at less than half their rate:
-// with planes of 1.8 MB the 3-D layer 64 -> 64, 3x3x3, 56x56, N = 32 runs at 620 TFLOP/s, with
-// planes of 2.0 MB at 390, of 3.2 MB at 280, whatever the tensor's total size, and with 16
-// instead of 64 filters (a quarter of the output) in the same time. The remedy is one pass over
+// with planes of 1.8 MB the 3-D layer 64 -> 64, 3x3x3, 56x56, N = 32 ran at 620 TFLOP/s (with one image
+// row per tile), with planes of 2.0 MB at 390, of 3.2 MB at 280, whatever the tensor's total size, and
+// with 16 instead of 64 filters (a quarter of the output) in the same time. The remedy is one pass over
 // the tensor before the product: a copy in (z, y, chan, x, n) order, whose channel rows are one
 // image row (x * n elements) apart, so that a box spans a few hundred KB. The product reads the
 // copy through a tensor map with the same dimensions and other strides; nothing in the kernel
