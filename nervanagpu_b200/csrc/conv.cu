@@ -166,14 +166,18 @@ int chan_block(DeviceCtx* c, cudaStream_t stream, const void* src, void* dst, in
 // product itself needs no other change than this walk over the taps. One read and one write of the
 // input; the CUDA-core kernels it replaces ran at 2.3 TFLOP/s: 96 -> 72 channels, 5x5 stride 2,
 // 102x102, 88 images, 100.8 -> 0.8 ms.
+// The update multiplies a row's last chunk, zeros in the error tensor past the row's end, with whatever the
+// copy holds there: with ragged rows its copy has a row of Q pixels for every tap instead (`phases` = S), so
+// that a NaN or infinity meets no zero of a tap that does not reach it.
 // The CUDA-core kernels skip the taps that fall outside the tensor; here they meet zeros, and a product of zero
-// and an infinity or NaN is NaN. Where that can show, the CUDA-core kernel runs once more over the result:
-// forward and backward when a filter value is not finite (nonfinite_scan), and for the elements of a weight
-// gradient that are NaN (conv_update_redo; its errors meet padding pixels, its last chunk of a row the pixels
-// that follow the row's last output).
-int phase_row(const Geo& g) { return g.Q + (g.S - 1) / g.str_w; }       // pixels per phase of a row
-size_t phase_split_bytes(const Geo& g) {
-  return (static_cast<size_t>(2) * g.C * g.D * g.H * g.str_w * phase_row(g) * g.N + 255) & ~size_t(255);
+// and an infinity or NaN is NaN. Where those kernels ran before and that can show, they run once more over the
+// result: forward and backward when a filter value is not finite (nonfinite_scan), and for the elements of a weight
+// gradient beyond_patches that are NaN (conv_update_redo). Smaller updates took their patches, zeros included,
+// to the tensor cores already.
+int update_phases(const Geo& g) { return (1ll * g.Q * g.N) % kChunk == 0 ? g.str_w : std::max(g.str_w, g.S); }
+int phase_row(const Geo& g, int phases) { return g.Q + (g.S - 1) / phases; }       // pixels per phase of a row
+size_t phase_split_bytes(const Geo& g, int phases) {
+  return (static_cast<size_t>(2) * g.C * g.D * g.H * phases * phase_row(g, phases) * g.N + 255) & ~size_t(255);
 }
 constexpr int kScanFlags = 128;      // blocks that scan a filter, each with a flag of its own (at most a block's threads)
 // Whether this block's share of `n` vectors of eight values holds an infinity or NaN, in flags[blockIdx.x]
@@ -193,13 +197,13 @@ __global__ void __launch_bounds__(256) nonfinite_scan(const uint4* __restrict__ 
   scan_share(F, n, gridDim.x, flags);
 }
 // one block per (z, y, c) row; the first `scans` of them also scan the filter (n_filter vectors)
-__global__ void __launch_bounds__(128) phase_split_kernel(Geo g, int wp, const uint4* __restrict__ I, uint4* __restrict__ dst,
+__global__ void __launch_bounds__(128) phase_split_kernel(Geo g, int phases, int wp, const uint4* __restrict__ I, uint4* __restrict__ dst,
                                                           const uint4* __restrict__ F, long long n_filter, int scans, int* flags) {
   const int nvec = g.N >> 3, c = blockIdx.x % g.C;
   const long long zy = blockIdx.x / g.C;
   const uint4* src = I + (1ll * c * g.D * g.H + zy) * g.W * nvec;
-  uint4* out = dst + 1ll * blockIdx.x * g.str_w * wp * nvec;
-  for (int i = threadIdx.x; i < g.str_w * wp * nvec; i += 128) {
+  uint4* out = dst + 1ll * blockIdx.x * phases * wp * nvec;
+  for (int i = threadIdx.x; i < phases * wp * nvec; i += 128) {
     const int pix = i / nvec, ph = pix / wp;
     const int x = (pix - ph * wp) * g.str_w + ph - g.pad_w;
     out[i] = x >= 0 && x < g.W ? __ldg(src + x * nvec + (i - pix * nvec)) : make_uint4(0, 0, 0, 0);
@@ -207,32 +211,33 @@ __global__ void __launch_bounds__(128) phase_split_kernel(Geo g, int wp, const u
   if (blockIdx.x < scans) scan_share(F, n_filter, scans, flags);
 }
 // F and flags (kScanFlags ints, of which `scans` are set) may be null
-int phase_split(const Geo& g, const void* I, void* dst, const void* F, int* flags, int* scans, cudaStream_t stream) {
+int phase_split(const Geo& g, int phases, const void* I, void* dst, const void* F, int* flags, int* scans, cudaStream_t stream) {
   const long long rows = 1ll * g.C * g.D * g.H;
   if (rows > 0x7fffffffll) return fail(NG_ERR_TOO_LARGE, "tensor too large for the phase-split copy");
   const int n = F ? static_cast<int>(std::min<long long>(rows, kScanFlags)) : 0;
   if (scans) *scans = n;
-  phase_split_kernel<<<static_cast<unsigned>(rows), 128, 0, stream>>>(g, phase_row(g), static_cast<const uint4*>(I),
+  phase_split_kernel<<<static_cast<unsigned>(rows), 128, 0, stream>>>(g, phases, phase_row(g, phases), static_cast<const uint4*>(I),
                                                                       static_cast<uint4*>(dst), static_cast<const uint4*>(F),
                                                                       g.sizeF() / 8, n, flags);
   NG_CHECK_LAUNCH();
   return NG_OK;
 }
 // the copy seen as (x' n, phase, y, z, chan)
-int phase_map(CUtensorMap* m, const void* base, const Geo& g, uint32_t box_chan) {
-  const uint64_t row = 2ull * phase_row(g) * g.N;
-  const uint64_t dims[5] = {1ull * phase_row(g) * g.N, static_cast<uint64_t>(g.str_w), static_cast<uint64_t>(g.H),
+int phase_map(CUtensorMap* m, const void* base, const Geo& g, int phases, uint32_t box_chan) {
+  const uint64_t row = 2ull * phase_row(g, phases) * g.N;
+  const uint64_t dims[5] = {1ull * phase_row(g, phases) * g.N, static_cast<uint64_t>(phases), static_cast<uint64_t>(g.H),
                             static_cast<uint64_t>(g.D), static_cast<uint64_t>(g.C)};
-  const uint64_t chan = row * g.str_w;
+  const uint64_t chan = row * phases;
   const uint64_t str[4] = {row, chan * g.C, chan * g.C * g.H, chan};
   const uint32_t box[5] = {kChunk, 1, 1, 1, box_chan};
   return make_tensor_map(m, base, dims, str, box);
 }
-void fill_phases(TcParams& p, const Geo& g) {
-  p.phase_w = g.str_w;
+void fill_phases(TcParams& p, int phases) {
+  p.phase_w = phases;
   p.pad_w = 0;         // (part of the copy)
 }
 
+size_t round256(size_t b) { return (b + 255) & ~size_t(255); }
 // Room for the copies behind the split-K partials of the product `p` (whose tiling and number of
 // partitions are final): `n` copies of the given sizes, returned as pointers into the workspace.
 // NG_ERR_TOO_LARGE: none to be had, for a product that has a form without scratch (`optional`).
@@ -489,17 +494,20 @@ __device__ __forceinline__ void update_element(const Geo& g, const __half* __res
   const int c = static_cast<int>(r);
   float acc = 0.0f;
   const long long span = 1ll * g.M * g.P * g.Q * g.N;
-  for (long long j = lane; j < span; j += 32) {
+  for (long long j0 = 0; j0 < span; j0 += 32) {
+    const long long j = j0 + lane;
     long long rj = j;
     const int n = rj % g.N; rj /= g.N;
     const int q = rj % g.Q; rj /= g.Q;
     const int p = rj % g.P; rj /= g.P;
     const int m = static_cast<int>(rj);
     const int z = m * g.str_d - g.pad_d + t, y = p * g.str_h - g.pad_h + rr, x = q * g.str_w - g.pad_w + s;
-    if (z < 0 || z >= g.D || y < 0 || y >= g.H || x < 0 || x >= g.W) continue;
-    const float iv = __half2float(I[(((1ll * c * g.D + z) * g.H + y) * g.W + x) * g.N + n]);
-    const float ev = __half2float(E[1ll * k * span + j]);
-    acc = fmaf(iv, ev, acc);
+    if (j < span && z >= 0 && z < g.D && y >= 0 && y < g.H && x >= 0 && x < g.W) {
+      const float iv = __half2float(I[(((1ll * c * g.D + z) * g.H + y) * g.W + x) * g.N + n]);
+      const float ev = __half2float(E[1ll * k * span + j]);
+      acc = fmaf(iv, ev, acc);
+    }
+    if (__any_sync(0xffffffffu, acc != acc)) break;   // (NaN whatever follows: a gradient full of them is done at once)
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -822,6 +830,43 @@ __global__ void filter_unpack_t_kernel(Geo g, TapBlock tb, int per, int ld, cons
   }
 }
 
+// Strided updates that ran on the CUDA cores because their patch matrix would exceed 6 GB (or 65535 rows): their
+// sums were serial sums in fp32, rounded, some ten times closer than the tensor cores' truncated ones of the same
+// length. Partitions of at most kShortSum k-blocks get there, more of them than fit in the partials' share
+// of the workspace: the sum runs in several launches, each adding to the gradient in its second stage. Off the
+// sum in 64 bits / time, CUDA cores -> partitions of one wave -> now: 96 -> 72, 5x5 / 2, 224x224, 120 images (7.2 GB) 4.0e-6,
+// 1452 ms -> 5.9e-5, 2.0 ms -> 3.2e-7, 4.4 ms; 1400 -> 64, 7x7 / 2, 40x40, 24 images (68600 rows) 3.0e-7, 204 ms -> 5.7e-6,
+// 0.29 ms -> 2.6e-7, 0.72 ms.
+constexpr int kShortSum = 3;
+bool beyond_patches(const Geo& g) {
+  const long long rows = 1ll * g.C * g.T * g.R * g.S;
+  return rows > 65535 || 2 * rows * g.M * g.P * g.Q * g.N > (6ll << 30) || tuning().stride_phases == 3;   // (3: tests)
+}
+// Sets p.splits and returns the number of launches.
+int short_sums(TcParams& p, long long out_elems) {
+  const long long parts = (p.num_kb + kShortSum - 1) / kShortSum;
+  if (parts < 2) return 1;
+  const long long room = tuning().conv_splits > 1 ? tuning().conv_splits      // (tests: several launches for small sums)
+                                                  : std::max<long long>(2, std::min<long long>(kMaxSplits, (256ll << 20) / (out_elems * 4)));
+  const long long launches = (parts + room - 1) / room;
+  p.splits = static_cast<int>(std::max<long long>(2, (parts + launches - 1) / launches));
+  return static_cast<int>(launches);
+}
+int launch_sums(DeviceCtx* c, const CUtensorMap& mapA, const CUtensorMap& mapB, const TcParams& p, int launches, cudaStream_t stream) {
+  for (int i = 0; i < launches; ++i) {
+    TcParams q = p;
+    q.kb_base = static_cast<int>(1ll * p.num_kb * i / launches);
+    q.num_kb = static_cast<int>(1ll * p.num_kb * (i + 1) / launches) - q.kb_base;
+    if (i > 0) { q.beta = 1.0f; q.Cold = q.C; }
+    const int rc = tc_launch(c, mapA, mapB, q, stream);
+    if (rc != NG_OK) return rc;
+  }
+  return NG_OK;
+}
+__global__ void round_kernel(const float* __restrict__ src, __half* dst, long long n) {
+  for (long long i = blockIdx.x * 1ll * blockDim.x + threadIdx.x; i < n; i += 1ll * gridDim.x * blockDim.x) dst[i] = __float2half_rn(src[i]);
+}
+
 // Few filters (K <= 128) as well as few channels: the roles of the operands are exchanged, so that
 // the 128 MMA rows carry the filters and the 256 MMA columns carry the rows of several taps or tap
 // blocks (an MMA with 64 columns costs nearly as much as one with 256). Column tile j owns tap blocks
@@ -853,24 +898,25 @@ int update_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, ChunkMode mod
   tc_fill_mma(p, lay);
   fill_taps(p, g, mode);
   p.R = tb.nr; p.S = tb.ns; p.RS = tb.nr * tb.ns; p.tap_w = tb.bw; p.tap_h = tb.bh;
-  if (phased) fill_phases(p, g);
+  if (phased) fill_phases(p, update_phases(g));
   fill_decode(p, g.N, g.Q, g.P, g.M, mode);
   p.oob_y = g.H;
   p.Cold = nullptr; p.ldc = ld; p.c_zstride = 0;
   p.alpha = alpha; p.beta = 0.0f; p.relu = 0; p.sr_bits = 0; p.out_f32 = 1; p.vec_ok = 1;
   p.splits = choose_splits(c, p.tiles_n, p.num_kb, 1ll * g.K * ld);
   if (!blocks) p.splits = shorter_partitions(c, tiles, p.num_kb, p.splits, 1ll * g.K * ld, 2, 64);
+  const int launches = phased && beyond_patches(g) ? short_sums(p, 1ll * g.K * ld) : 1;
   // behind the partials: the gradient in tap order and copies of the operands. (Not in the second buffer,
   // where I and the gradient of a layer that was rewritten by space to depth lie.)
   const size_t bytes[3] = {(static_cast<size_t>(g.K) * ld * 4 + 255) & ~size_t(255),
-                           phased ? phase_split_bytes(g) : (blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0),
+                           phased ? phase_split_bytes(g, update_phases(g)) : (blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0),
                            blocked_e ? chan_block_bytes(g.K, g.M, g.P, g.Q, g.N) : 0};
   void* room[3] = {nullptr, nullptr, nullptr};
   int rc = chan_block_room(c, stream, p, bytes, room, 3, phased);
   if (rc != NG_OK) return rc;
   float* Dt = static_cast<float*>(room[0]);
   p.C = Dt;
-  if (phased) rc = phase_split(g, I, room[1], nullptr, nullptr, nullptr, stream);
+  if (phased) rc = phase_split(g, update_phases(g), I, room[1], nullptr, nullptr, nullptr, stream);
   else if (blocked_i) rc = chan_block(c, stream, I, room[1], g.C, g.D, g.H, g.W, g.N);
   if (rc == NG_OK && blocked_e) rc = chan_block(c, stream, E, room[2], g.K, g.M, g.P, g.Q, g.N);
   if (rc != NG_OK) return rc;
@@ -880,9 +926,9 @@ int update_swapped(DeviceCtx* c, const Geo& g, const TapBlock& tb, ChunkMode mod
   rc = act_map(&mapA, E, g.K, g.M, g.P, g.Q, g.N, mode, lay.a_box_rows, blocked_e);
   if (rc != NG_OK) return rc;
   rc = blocks ? act_map_tapblock(&mapB, I, g, tb)
-              : (phased ? phase_map(&mapB, I, g, tb.rows) : act_map(&mapB, I, g.C, g.D, g.H, g.W, g.N, mode, tb.rows, blocked_i));
+              : (phased ? phase_map(&mapB, I, g, update_phases(g), tb.rows) : act_map(&mapB, I, g.C, g.D, g.H, g.W, g.N, mode, tb.rows, blocked_i));
   if (rc != NG_OK) return rc;
-  rc = tc_launch(c, mapA, mapB, p, stream);
+  rc = launch_sums(c, mapA, mapB, p, launches, stream);
   if (rc != NG_OK) return rc;
   filter_unpack_t_kernel<<<launch_1d(g.sizeF(), 256, c), 256, 0, stream>>>(g, tb, per, ld, Dt, gradF, out_f32);
   NG_CHECK_LAUNCH();
@@ -1154,7 +1200,7 @@ bool bprop_by_phases(DeviceCtx* c, const Geo& g, bool in_place) {
 // 128 -> 128, 1x1 / 2, 28x28, 24 images (1.2 MB, 0.25) 17 / 15; 256 -> 32, 3x3 / 2, 16x16, 24 images (7.1 MB, 2.3) 18 / 17; 256 -> 32,
 // 7x7 / 3, 19x19, 8 images (9.8 MB, 6.6) 18 / 21; 512 -> 512, 3x3 / 3, 22x22, 32 images (18 MB, 1.2) 41 / 34; 64 -> 64, 3x3 / 2, 56x56,
 // 24 images (22 MB, 2.3) 27 / 29; 512 -> 512, 1x1 / 2, 34x34, 96 images (27 MB, 0.25) 76 / 45; 96 -> 512, 3x3 / 4, 85x85, 48 images
-// (38 MB, 0.6) 58 / 54; 256 -> 64, 2x2 / 2, 62x62, 32 images (64 MB, 1.1) 46 / 61; 96 -> 72, 5x5 / 2, 51x51, 88 images (1.1 GB, 6.3) 91 / 218.
+// (38 MB, 0.6) 58 / 54; 256 -> 64, 2x2 / 2, 62x62, 32 images (64 MB, 1.1) 46 / 61; 96 -> 72, 5x5 / 2, 51x51, 88 images (284 MB, 6.4) 100 / 218.
 // Longest partitions (k-blocks) of the strided updates' sums, so that no gradient is further off the sum in 64
 // bits than on the paths these forms replace: patches in one wave / phase-split with up to 64 /
 // now, in units of 1e-7: 128 -> 128, 1x1 / 2, 57x57, 120 images 8.5 / 8.2 / 7.9; 512 -> 512, 1x1 / 2, 34x34, 96 images 18.7 / 11.0 / 9.5;
@@ -1170,7 +1216,6 @@ bool update_by_phases(const Geo& g) {
   return 2 * patches > kPatchBytes && (2 * patches > 3 * g.sizeI() || (2 * patches > 4 * kPatchBytes && 5 * patches > 4 * g.sizeI()));
 }
 
-size_t round256(size_t b) { return (b + 255) & ~size_t(255); }
 
 extern "C" {
 
@@ -1287,7 +1332,7 @@ int ng_conv_fprop(const ng_conv_desc* d, const void* I, const void* F, void* O, 
   }
   tc_fill_mma(p, lay);
   fill_taps(p, g, mode);
-  if (phased) fill_phases(p, g);
+  if (phased) fill_phases(p, g.str_w);
   if (stack) { ++p.R; p.RS += g.S; p.str_h = 2; }
   fill_decode(p, g.N, g.Q, stack ? p.cmap.y_count : g.P, g.M, mode);
   p.oob_y = g.H;
@@ -1300,14 +1345,14 @@ int ng_conv_fprop(const ng_conv_desc* d, const void* I, const void* F, void* O, 
   // few tiles (a small minibatch, e.g. the shard of one GPU): the reduction is split over the SMs too
   if (!stack) p.splits = choose_splits(c, 1ll * p.tiles_m * p.tiles_n, p.num_kb, 1ll * g.K * cols, true);
   if (phased) {
-    const size_t bytes[2] = {phase_split_bytes(g), kScanFlags * sizeof(int)};
+    const size_t bytes[2] = {phase_split_bytes(g, g.str_w), kScanFlags * sizeof(int)};
     void* room[2] = {nullptr, nullptr};
     int scans = 0;
     rc = chan_block_room(c, stream, p, bytes, room, 2, true);
     if (rc == NG_ERR_TOO_LARGE) return cuda_cores();
     int* flags = static_cast<int*>(room[1]);
-    if (rc == NG_OK) rc = phase_split(g, I, room[0], F, flags, &scans, stream);
-    if (rc == NG_OK) rc = phase_map(&mapB, room[0], g, lay.kb_rows);
+    if (rc == NG_OK) rc = phase_split(g, g.str_w, I, room[0], F, flags, &scans, stream);
+    if (rc == NG_OK) rc = phase_map(&mapB, room[0], g, g.str_w, lay.kb_rows);
     if (rc == NG_OK) rc = tc_launch(c, mapA, mapB, p, stream);
     if (rc != NG_OK) return rc;
     return launch_dependent(redo_blocks(c), stream, conv_fprop_simt, g, static_cast<const __half*>(I), static_cast<const __half*>(F),
@@ -1459,7 +1504,7 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
     taps.bw = taps.bh = 1; taps.rows = swap_rows(g.C); taps.nr = g.R; taps.ns = g.S; taps.ok = true;
     rc = update_swapped(c, g, taps, mode, phased, I, E, gradF, out_f32, alpha, stream);
     if (rc == NG_ERR_TOO_LARGE && phased) return cuda_cores();
-    return rc == NG_OK && phased ? redo() : rc;
+    return rc == NG_OK && phased && beyond_patches(g) ? redo() : rc;
   }
   if (direct) {
     TcParams p = {};
@@ -1484,7 +1529,7 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
     }
     tc_fill_mma(p, lay);
     fill_taps(p, g, mode);
-    if (phased) fill_phases(p, g);
+    if (phased) fill_phases(p, update_phases(g));
     fill_decode(p, g.N, g.Q, g.P, g.M, mode);
     p.oob_y = g.H;
     p.C = gradF; p.Cold = nullptr; p.ldc = 1ll * RST * g.K; p.c_zstride = g.K;
@@ -1492,29 +1537,37 @@ int ng_conv_update(const ng_conv_desc* d, const void* I, const void* E, void* gr
     p.splits = choose_splits(c, 1ll * p.tiles_m * p.tiles_n * p.nz, p.num_kb, 1ll * g.C * g.K * RST);
     if (phased)
       p.splits = shorter_partitions(c, 1ll * p.tiles_m * p.tiles_n * p.nz, p.num_kb, p.splits, 1ll * g.C * g.K * RST, 4, kLongSum);
+    const int launches = phased && beyond_patches(g) ? short_sums(p, 1ll * g.C * g.K * RST) : 1;
+    const bool rounded = launches > 1 && !out_f32;      // (summed in fp32, then rounded)
     CUtensorMap mapA, mapB;
     // large channel planes: the product reads copies in (z, y, chan, x, n) order
     const bool blocked_i = !phased && wants_chan_block(g.D, g.H, g.W, g.N, RST);
     const bool blocked_e = wants_chan_block(g.M, g.P, g.Q, g.N, RST);
     if (phased || blocked_i || blocked_e) {
-      const size_t bytes[2] = {phased ? phase_split_bytes(g) : blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0,
-                               blocked_e ? chan_block_bytes(g.K, g.M, g.P, g.Q, g.N) : 0};
-      void* copies[2] = {nullptr, nullptr};
-      rc = chan_block_room(c, stream, p, bytes, copies, 2, phased);
+      const size_t bytes[3] = {phased ? phase_split_bytes(g, update_phases(g)) : blocked_i ? chan_block_bytes(g.C, g.D, g.H, g.W, g.N) : 0,
+                               blocked_e ? chan_block_bytes(g.K, g.M, g.P, g.Q, g.N) : 0,
+                               rounded ? round256(4ull * g.sizeF()) : 0};
+      void* copies[3] = {nullptr, nullptr, nullptr};
+      rc = chan_block_room(c, stream, p, bytes, copies, 3, phased);
       if (rc == NG_ERR_TOO_LARGE && phased) return cuda_cores();
-      if (rc == NG_OK && phased) rc = phase_split(g, I, copies[0], nullptr, nullptr, nullptr, stream);
+      if (rc == NG_OK && phased) rc = phase_split(g, update_phases(g), I, copies[0], nullptr, nullptr, nullptr, stream);
       if (rc == NG_OK && blocked_i) rc = chan_block(c, stream, I, copies[0], g.C, g.D, g.H, g.W, g.N);
       if (rc == NG_OK && blocked_e) rc = chan_block(c, stream, E, copies[1], g.K, g.M, g.P, g.Q, g.N);
       if (rc != NG_OK) return rc;
       if (phased || blocked_i) I = copies[0];
       if (blocked_e) E = copies[1];
+      if (rounded) { p.C = copies[2]; p.out_f32 = 1; }
     }
-    rc = phased ? phase_map(&mapA, I, g, a_rows) : act_map(&mapA, I, g.C, g.D, g.H, g.W, g.N, mode, a_rows, blocked_i);
+    rc = phased ? phase_map(&mapA, I, g, update_phases(g), a_rows) : act_map(&mapA, I, g.C, g.D, g.H, g.W, g.N, mode, a_rows, blocked_i);
     if (rc != NG_OK) return rc;
     rc = act_map(&mapB, E, g.K, g.M, g.P, g.Q, g.N, mode, p.block_n, blocked_e);
     if (rc != NG_OK) return rc;
-    rc = tc_launch(c, mapA, mapB, p, stream);
-    return rc == NG_OK && phased ? redo() : rc;
+    rc = launch_sums(c, mapA, mapB, p, launches, stream);
+    if (rc == NG_OK && rounded) {
+      round_kernel<<<launch_1d(g.sizeF(), 256, c), 256, 0, stream>>>(static_cast<const float*>(p.C), static_cast<__half*>(gradF), g.sizeF());
+      NG_CHECK_LAUNCH();
+    }
+    return rc == NG_OK && phased && beyond_patches(g) ? redo() : rc;
   }
   if (im2col) {
     // dF[crst][k] = col[crst][span] * E[k][span]^T  (both K-major: an "nt" GEMM with split-K)

@@ -42,6 +42,7 @@ struct TcParams {
   int tiles_m, tiles_n, nz, splits;
   int num_kb;          // k-blocks in the whole reduction
   int kb_per_split;    // ceil(num_kb / splits)
+  int kb_base;         // weight update: first k-block of this launch (0 but for sums taken in several launches)
   int full_items;      // items [0, full_items) are whole tiles; from there on, item pairs are the two
   int total_items;     // 128-row halves of one 256-row tile (the cut last wave); all items
   int block_n;         // UMMA N: 64, 128 or 256

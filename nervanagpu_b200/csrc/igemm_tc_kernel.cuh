@@ -311,7 +311,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         const int zt = p.swap_ab ? it.tile_n * p.b_boxes + (is_a ? 0 : bi) : it.z * p.taps_per_z + (is_a ? bi : 0);
         wk.tap = decode_tap(p, zt);
         tap_live = p.swap_ab ? zt < p.taps_per_z : (zt < p.nz_out && (!is_a || bi < p.taps_per_z));
-        wk.cp = decode_chunk(p, it.kb0);
+        wk.cp = decode_chunk(p, p.kb_base + it.kb0);
       }
       // box coordinates of this lane's box at walker position `s`
       auto coords = [&](const Walk& s, int& c0, int& c1, int& c2, int& c3, int& c4) {

@@ -574,9 +574,9 @@ def by_phases(lib):
 
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
 @pytest.mark.parametrize("name", ["n24_5x5_s3", "n88_7x7_s2_c96", "n40_2x3_s3_h1", "n32_3d_s222", "n16_1x1_s2", "n8_3x3_s2"])
-def test_strided_layers_keep_infinities_from_outputs_that_do_not_meet_them(ng, by_phases, name, value):
-    """Minibatches that are no multiple of 64: an infinity or NaN in any operand reaches what it reaches on the
-    CUDA-core kernels, which skip the pixels outside the tensors that the tensor cores multiply as zeros."""
+def test_strided_layers_keep_infinities_from_outputs_that_do_not_meet_them(ng, lib, by_phases, name, value):
+    """Minibatches that are no multiple of 64: an infinity or NaN reaches what it reaches on the CUDA-core
+    kernels, which skip the pixels outside the tensors that the tensor cores multiply as zeros."""
     cfg = STRIDED[name]
     cd = rm.ConvDims(*cfg)
     I, F, E = _inputs(cd, 1023)
@@ -603,14 +603,20 @@ def test_strided_layers_keep_infinities_from_outputs_that_do_not_meet_them(ng, b
     for p, q in ((0, 0), (P - 1, Q - 1)):
         bad = E.copy()
         bad[3, 0, p, q, 2] = value
-        check(I, F, bad, "bu")
+        check(I, F, bad, "b")
+        try:                    # (updates whose patch matrix is too large; smaller ones multiply patches, zeros included)
+            assert lib.ng_tune(b"stride_phases", 3) == 0
+            check(I, F, bad, "u")
+        finally:
+            assert lib.ng_tune(b"stride_phases", 2) == 0
     bad = I.copy()
     bad[1, 0, 0, I.shape[3] - 1, 5] = value
     if R > 1:              # (a 1x1 filter steps over that pixel)
         check(bad, F, E, "u")
 
 
-def test_strided_update_in_fp16_keeps_infinities_apart_too(ng, by_phases):
+def test_strided_update_in_fp16_keeps_infinities_apart_too(ng, lib, by_phases):
+    assert lib.ng_tune(b"stride_phases", 3) == 0
     cfg = STRIDED["n24_5x5_s3"]
     cd = rm.ConvDims(*cfg)
     I, F, E = _inputs(cd, 1025)
@@ -722,3 +728,31 @@ def test_update_with_exchanged_operands_by_phases(ng, lib, by_phases, name, half
 @pytest.mark.parametrize("name", ["n24_5x5_s3", "n40_2x3_s3_h1", "n8_3x3_s2", "n24_odd_rows_s2"])
 def test_strided_update_keeps_nan_to_the_taps_it_meets_by_phases(ng, by_phases, name):
     test_strided_update_keeps_nan_to_the_taps_it_meets(ng, name)
+
+
+@pytest.mark.parametrize("swap", [0, 2])
+@pytest.mark.parametrize("half", [False, True])
+@pytest.mark.parametrize("name", ["n88_7x7_s2_c96", "n24_5x5_s3", "n32_3d_s222", "n40_2x3_s3_h1", "n24_c48_5x5_s2"])
+def test_strided_sums_in_several_launches(ng, lib, name, half, swap):
+    """The form of updates beyond the patch matrix, forced on small layers: partitions of six k-blocks, two to a launch."""
+    cfg = STRIDED.get(name, (24, 48, 128, 1, 17, 15, 1, 5, 5, 0, 2, 2, 1, 2, 2))
+    cd = rm.ConvDims(*cfg)
+    I, F, E = _inputs(cd, 1031)
+    ref = rm.conv_update_fast(cd, I, E, alpha=0.5)
+    layer = _layer(ng, cfg)
+    pad = 4096                  # guard cells
+    buf = ng.empty((layer.sizeF + 2 * pad,), dtype=np.float16 if half else np.float32)
+    buf.fill(7.0)
+    try:
+        for key, value in ((b"stride_phases", 3), (b"conv_splits", 2), (b"update_swap", swap)):
+            assert lib.ng_tune(key, value) == 0
+        ng.update_conv(layer, ng.array(I), ng.array(E), buf[pad:pad + layer.sizeF].reshape(layer.dimF), alpha=0.5)
+    finally:
+        for key in (b"stride_phases", b"conv_splits", b"update_swap"):
+            assert lib.ng_tune(key, -1) == 0
+    got = buf.get()
+    assert (got[:pad] == 7.0).all() and (got[-pad:] == 7.0).all()
+    tol = f32_tol(_abs_terms(cd, I, F, E)[2], int(np.prod(cd.MPQ)) * cd.N)
+    if half:
+        tol = tol + 2.0 ** -11 * np.abs(ref) + 2.0 ** -25
+    assert_close(got[pad:-pad].reshape(layer.dimF), ref, tol, name)
